@@ -12,9 +12,6 @@
 // Work items are ordered heaviest first.  The sorts are stable radix sorts
 // keyed by (frame, tile), so entries of a tile are in sample order and the
 // spread's summation order, hence its result, is the same in every run.
-// (The host planner additionally reorders the entries of heavy 3-D tiles by
-// a hash of the sample index for balance; the device lists keep sample
-// order, which gives the same result up to float rounding.)
 //
 // The reference has no such step: its CPU kernels loop over samples and its
 // CuPy kernels scatter with global atomics
@@ -86,14 +83,19 @@ __global__ void __launch_bounds__(256) bin_count_kernel(const BinParams<R> p) {
     if (!sample_taps(p, m, kf)) atomicOr(p.err, 1);
     const int f = frame_of(p.foff, p.F, m);
     int lin = 0, mul = 1;
-    int n = 1;
+    int n = 1, nv = 1;
     for (int d = 0; d < p.ndim; ++d) {
         lin += (wrapk(kf[d], p.K[d]) / p.Tg[d]) * mul;
         mul *= p.ntg[d];
         AxisHits h;
         axis_hits(kf[d], p.J[d], p.K[d], p.Ts[d], h);
         n *= h.n;
+        axis_hits(kf[d], p.J[d], p.K[d], p.B[d], h);
+        nv *= h.n;
     }
+    const unsigned peers = __activemask();
+    const unsigned wsum = __reduce_add_sync(peers, (unsigned)nv);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(p.nvisits, (unsigned long long)wsum);
     p.gkey[m] = (unsigned)(f * p.ntiles_g + lin);
     p.gval[m] = (unsigned)m;
     p.ecount[m] = n;
@@ -148,6 +150,12 @@ __global__ void __launch_bounds__(256) bin_parts_kernel(const ItemParams p) {
         p.sparts[b] = parts;
         p.rslots[b] = parts > 1 ? parts : 0;
         p.rflag[b] = parts > 1 ? 1 : 0;
+        const int per = (c + parts - 1) / parts, last = c - per * (parts - 1);
+        for (int q = 0; q < SPREAD_HEAVY_LEVELS; ++q) {
+            const int t = SPREAD_SHARE_ENTRIES << q;
+            const int n = (per > t ? parts - 1 : 0) + (last > t ? 1 : 0);
+            if (n) atomicAdd(&p.nheavy[q], n);
+        }
     }
 }
 

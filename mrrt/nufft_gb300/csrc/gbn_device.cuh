@@ -50,6 +50,19 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ void sincos_r(float x, float* s, float* c) { sincosf(x, s, c); }
 __device__ __forceinline__ void sincos_r(double x, double* s, double* c) { sincos(x, s, c); }
 
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+// Complex product with its roundings fixed (which of a product's two terms
+// is contracted is otherwise the compiler's choice at each call site): the
+// spread kernels of the entry and the visit lists agree bit for bit.
+template <typename C>
+__device__ __forceinline__ C cmul_fixed(C a, C b) {
+    C r;
+    r.x = fma_rn(a.x, b.x, -mul_rn(a.y, b.y));
+    r.y = fma_rn(a.x, b.y, mul_rn(a.y, b.x));
+    return r;
+}
+
 // k mod K for k in a few periods around [0, K).
 __device__ __forceinline__ int wrapk(int k, int K) {
     int r = k % K;

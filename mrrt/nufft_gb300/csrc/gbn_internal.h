@@ -1,5 +1,5 @@
 // Internal declarations shared by the host planner (gbn_plan.cu) and the
-// device kernels (gbn_gather.cu, gbn_spread.cu, gbn_padcrop.cu, gbn_grad.cu,
+// device kernels (gbn_gather.cu, gbn_visit.cuh, gbn_spread.cu, gbn_padcrop.cu, gbn_grad.cu,
 // gbn_colfft.cu, ...).
 #pragma once
 
@@ -11,15 +11,16 @@ namespace gbn {
 // Kernel width limit of the register-resident coefficient arrays.
 constexpr int JMAX = 8;
 
-// Spread register blocks: each warp of a spread CTA (at most 8 warps) owns
-// SB0 x SB1 x SB2 cells of its tile (16 accumulators per lane).
+// Spread register blocks: a warp sums SB0 x SB1 x SB2 cells of its tile at a
+// time (16 accumulators per lane); a tile has at most 8 of them.
 template <int NDIM> struct SpreadBlock;
 template <> struct SpreadBlock<1> { static constexpr int B0 = 16, B1 = 1, B2 = 1; };
 template <> struct SpreadBlock<2> { static constexpr int B0 = 4, B1 = 4, B2 = 1; };
 template <> struct SpreadBlock<3> { static constexpr int B0 = 4, B1 = 4, B2 = 1; };
-// Entries staged per spread chunk (two chunks in flight: one accumulated
-// while the next is copied in).
-constexpr int SPREAD_CHUNK_ENTRIES = 64;
+// Spread items are counted by size: level q holds those of more entries than
+// SPREAD_SHARE_ENTRIES << q.  A launch shares the items of one level among the
+// warps of a CTA each.
+constexpr int SPREAD_SHARE_ENTRIES = 32, SPREAD_HEAVY_LEVELS = 6;
 
 template <typename R> struct Cx;
 template <> struct Cx<float> { typedef float2 T; };
@@ -116,26 +117,61 @@ struct GatherParams {
     int chunks;                     // coil chunks of LS lanes
 };
 
+// Visit lists (gbn_visit.cuh): per (work item, register block) the samples
+// whose window touches the block, and their coefficients clipped to it.
 template <typename R>
-struct SpreadParams {
+struct VisitBuildParams {
     Geom<R> g;
-    Lanes ln;
     SampleList<R> s;
     const int4* items;              // {frame, tile, start, count}
-    const int2* parts;              // {scratch slot or -1, nparts}
-    int nitems;
-    int coils;
+    int nitems, nblk;               // register blocks per tile
     const int64_t* foff;
+    const R* wr[3];                 // sparse-matrix weights, or nullptr: the tables
+    const R* wi[3];
+    int cx;
+    int* count;                     // [nitems * nblk], multiples of four
+    const long long* start;         // exclusive scan of the counts, [nitems * nblk + 1]
+    int* vidx;                      // [nvisits] sample index within its frame (without vco: list
+                                    // position), -1 for padding
+    R* vco;                         // [nvisits][coefficients], or nullptr: computed in the spread
+};
+
+// Sample values of a call, coil-minor and times conj(sample phase).
+template <typename R>
+struct ValuesParams {
+    const typename Cx<R>::T* y;     // samples [frame][coil][m]
+    const typename Cx<R>::T* ph;    // sample phase, sample order, or nullptr
+    typename Cx<R>::T* out;         // [frame][m][coil]
+    const int64_t* foff;
+    int F, coils, row;              // row: values per sample of out (coils rounded up to 16 bytes)
+    int64_t M;                      // samples of all frames
+    unsigned* check;
+    int64_t out_elems;
+};
+
+template <typename R>
+struct VisitParams {
+    Geom<R> g;
+    SampleList<R> s;                // the entries, where the coefficients are computed on the way
+    const long long* start;
+    const int* vidx;
+    const R* vco;                   // or nullptr: from the tables
+    int64_t nvisits;
+    const int4* items;
+    const int2* parts;              // {scratch slot or -1, nparts}
+    int nitems, nblk;
+    int nheavy[SPREAD_HEAVY_LEVELS];   // leading items of more entries than 32 << level
+    short4 borg[8];                 // set by the launcher: block origins within the tile
+    int nshared;                    // set by the launcher: leading items shared by a CTA's warps
+    int coils, LS, chunks, row;
+    const int64_t* foff;
+    const typename Cx<R>::T* vals;  // [frame][m][row] (launch_values), or nullptr: read y in place
     const typename Cx<R>::T* y;
+    const typename Cx<R>::T* ph;    // with y: sample phase, sample order, or nullptr
     typename Cx<R>::T* grid;
     typename Cx<R>::T* scratch;     // [slot][chunk][LS][tile cells] partial sums
-    int64_t tile_cells;             // T0*T1*T2
-    int64_t scratch_elems;          // scratch extent (complex elements)
+    int64_t tile_cells, scratch_elems;
     int apply_pb;
-    int apply_ph;
-    int chunks;                     // coil chunks of LS lanes (gridDim.y)
-    int cpf;                        // set by the launcher: precomputed coefficients prefetched
-                                    // into shared memory a chunk ahead
 };
 
 template <typename R>
@@ -222,6 +258,8 @@ struct BinParams {
     unsigned* gval;                // [M] sample index (sort payload)
     int* ecount;                   // [M] spread entries of each sample
     const int* eoff;               // [M] exclusive scan of ecount (emit pass)
+    int B[3];                      // register block edges
+    unsigned long long* nvisits;   // sum over samples of the register blocks their windows touch
     unsigned* skey;                // [entries] spread bin
     unsigned* sval;                // [entries] entry index (sort payload)
     int* em;                       // [entries] sample index
@@ -252,6 +290,7 @@ struct ItemParams {
     unsigned* ssize;
     unsigned* sorder;
     int4* rtiles;
+    int* nheavy;                   // parts pass: spread items of more than 32 << level entries
 };
 
 // List packing: position i of a sorted list takes sample em[order[i]] (or
@@ -321,17 +360,19 @@ bool rowfft_supported(int L);
 cudaError_t launch_rowfft(const RowFftParams& p, int sign, cudaStream_t s);
 
 template <typename R> cudaError_t launch_gather(const GatherParams<R>& p, cudaStream_t s);
-template <typename R> cudaError_t launch_spread(const SpreadParams<R>& p, cudaStream_t s);
+template <typename R> cudaError_t launch_visit_count(const VisitBuildParams<R>& p, cudaStream_t s);
+template <typename R> cudaError_t launch_visit_fill(const VisitBuildParams<R>& p, cudaStream_t s);
+template <typename R> cudaError_t launch_values(const ValuesParams<R>& p, cudaStream_t s);
+template <typename R> cudaError_t launch_spread_visits(const VisitParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_reduce(const ReduceParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_pad(const PadParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_crop(const CropParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_grad(const GradParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_coef(const CoefParams<R>& p, cudaStream_t s);
 
-// Shared-memory bytes needed by the gather / spread kernels for a lane layout.
+// Shared-memory bytes needed by the gather kernel for a lane layout.
 template <typename R> size_t gather_smem(const Geom<R>& g, const Lanes& ln);
-template <typename R> size_t spread_smem(const Geom<R>& g, const Lanes& ln);
-// Threads of a spread CTA for a tiling (one warp per register block).
+// 32 x the register blocks of a spread tile.
 int spread_threads(int ndim, const int* T);
 
 // Raise a kernel's dynamic shared-memory limit to at least `bytes` on the

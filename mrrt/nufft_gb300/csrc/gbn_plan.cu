@@ -110,6 +110,13 @@ int next_pow2(int v) {
     return p;
 }
 
+// Edges of the spread's register blocks.
+void spread_block(int ndim, int* B) {
+    B[0] = ndim == 1 ? SpreadBlock<1>::B0 : ndim == 2 ? SpreadBlock<2>::B0 : SpreadBlock<3>::B0;
+    B[1] = ndim == 1 ? 1 : ndim == 2 ? SpreadBlock<2>::B1 : SpreadBlock<3>::B1;
+    B[2] = ndim == 3 ? SpreadBlock<3>::B2 : 1;
+}
+
 int ilog2(int v) {
     int l = 0;
     while ((1 << l) < v) ++l;
@@ -213,8 +220,14 @@ struct gbn_plan {
     DevBuf check;         // status word of the checked build's bounds tests
     DevBuf tickets;       // work counters of the persistent gather launch
     DevBuf weights;       // sparse-matrix mode: per-axis [M_total][J] weights (re, then im)
-    DevBuf gcoef, scoef;  // precomputed coefficients in gather / spread list order
-    bool coefs = false;   // gcoef / scoef hold the current lists' coefficients
+    DevBuf gcoef;         // precomputed coefficients in gather list order
+    // visit lists of the spread (gbn_visit.cuh): offsets per (item, block), sample
+    // indices, clipped coefficients; the sample phase in sample order; the values of a
+    // call, coil-minor (grown on demand)
+    DevBuf vstart, vidx, vco, vwork, phnat, vals;
+    int64_t nvisits = 0;  // extent of vidx and vco in visits
+    int n_heavy[SPREAD_HEAVY_LEVELS] = {0};   // leading spread items of more entries than 32 << level
+    bool coefs = false;   // gcoef and vco hold the current points' coefficients
     DevBuf glist, gitems;
     DevBuf bin_ws, bin_ws2;   // device binning workspaces (grown on demand)
     DevBuf slist, sitems, sparts, rtiles;
@@ -379,8 +392,8 @@ SampleList<R> make_list(const gbn_plan* P, const DevBuf& buf, int64_t len, bool 
     for (int d = 0; d < P->geom.ndim; ++d) s.t[d] = reinterpret_cast<const R*>(b + L.t[d]);
     s.idx = reinterpret_cast<const int*>(b + L.idx);
     s.len = len;
-    if (P->coefs) {
-        const DevBuf& cb = with_ls ? P->scoef : P->gcoef;
+    if (P->coefs && !with_ls) {
+        const DevBuf& cb = P->gcoef;
         int jsum = 0;
         for (int d = 0; d < P->geom.ndim; ++d) jsum += P->geom.Jd[d];
         s.jsum = jsum;
@@ -434,11 +447,11 @@ void choose_tiles(gbn_plan* P) {
     }
     P->ntiles_g = P->ntg[0] * P->ntg[1] * P->ntg[2];
     // spread: 8 register blocks (warps) per tile by default
-    int B[3] = {1, 1, 1}, S[3] = {1, 1, 1};
-    if (ndim == 1) { B[0] = SpreadBlock<1>::B0; S[0] = 8 * B[0]; }
-    else if (ndim == 2) { B[0] = SpreadBlock<2>::B0; B[1] = SpreadBlock<2>::B1; S[0] = 4 * B[0]; S[1] = 2 * B[1]; }
+    int B[3], S[3] = {1, 1, 1};
+    spread_block(ndim, B);
+    if (ndim == 1) S[0] = 8 * B[0];
+    else if (ndim == 2) { S[0] = 4 * B[0]; S[1] = 2 * B[1]; }
     else {
-        B[0] = SpreadBlock<3>::B0; B[1] = SpreadBlock<3>::B1; B[2] = SpreadBlock<3>::B2;
         // 8 x 4 x 4: measured best of the 8-block shapes on a 3-D kooshball
         S[0] = 2 * B[0]; S[1] = B[1]; S[2] = 4 * B[2];
     }
@@ -561,38 +574,6 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
                     sls[(size_t)at] = ls;
                 });
     }
-    // 3-D: within a tile, entries in sample order come in a few trajectory
-    // segments at a time, so a staged chunk loads some warps' register
-    // blocks much more than others, and every warp waits for the busiest one
-    // at the chunk's barrier.  Runs of four consecutive samples (one 32-byte
-    // sector of each coil's values) are put in a fixed pseudo-random order
-    // instead, so every chunk spreads over the whole tile (kooshball spread
-    // 6.08 -> 5.73 ms).  2-D keeps sample order: with 32 coils a chunk's
-    // values are 16 KB, and scattering their reads cost more than the
-    // balance gained (0.159 -> 0.180 ms).
-    if (ndim == 3) {
-        std::vector<std::pair<uint32_t, int64_t>> key;
-        std::vector<int64_t> o2;
-        std::vector<short4> l2;
-        for (int64_t b = 0; b < nbins_s; ++b) {
-            const int64_t lo = scount[(size_t)b], hi = scount[(size_t)b + 1];
-            if (hi - lo <= SPREAD_CHUNK_ENTRIES) continue;   // one chunk: order irrelevant
-            key.resize((size_t)(hi - lo));
-            for (int64_t i = lo; i < hi; ++i) {
-                const uint32_t run = (uint32_t)(sorder[(size_t)i] >> 2);
-                key[(size_t)(i - lo)] = {run * 2654435761u, i};
-            }
-            std::sort(key.begin(), key.end());
-            o2.resize(key.size());
-            l2.resize(key.size());
-            for (size_t q = 0; q < key.size(); ++q) {
-                o2[q] = sorder[(size_t)key[q].second];
-                l2[q] = sls[(size_t)key[q].second];
-            }
-            std::copy(o2.begin(), o2.end(), sorder.begin() + lo);
-            std::copy(l2.begin(), l2.end(), sls.begin() + lo);
-        }
-    }
     // ---- pack lists (SoA) -------------------------------------------------
     auto pack = [&](const std::vector<int64_t>& order, const short4* ls, DevBuf& dst, int64_t len) -> int {
         const ListLayout<R> L(P, len, ls != nullptr);
@@ -628,6 +609,12 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
     if (rc) return rc;
     P->glen = Mt;
     P->slen = slen;
+    if (P->has_phase) {
+        cudaError_t e = P->phnat.alloc(std::max<size_t>((size_t)Mt * sizeof(C), 16));
+        if (e == cudaSuccess && Mt)
+            e = cudaMemcpy(P->phnat.p, phase, (size_t)Mt * sizeof(C), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(e, "phase upload");
+    }
 
     // ---- work items ---------------------------------------------------------
     struct Item { int4 a; int2 b; };
@@ -662,6 +649,10 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
     auto heavy_first = [](const Item& x, const Item& y) { return x.a.w > y.a.w; };
     std::stable_sort(gi.begin(), gi.end(), heavy_first);
     std::stable_sort(si.begin(), si.end(), heavy_first);
+    for (int q = 0; q < SPREAD_HEAVY_LEVELS; ++q) {
+        const int t = SPREAD_SHARE_ENTRIES << q;
+        P->n_heavy[q] = (int)std::count_if(si.begin(), si.end(), [t](const Item& x) { return x.a.w > t; });
+    }
     std::vector<int4> ga(gi.size()), sa(si.size());
     std::vector<int2> sb(si.size());
     for (size_t i = 0; i < gi.size(); ++i) ga[i] = gi[i].a;
@@ -689,6 +680,16 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
     return GBN_OK;
 }
 
+// Coil-minor values are worth their pass above this many coils: up to four,
+// a visit's coils fill no more sectors read in place.
+constexpr int VALUES_MIN_COILS = 5;
+
+// Values per sample of the coil-minor buffer: the coils, rounded up to 16 bytes.
+int value_row(int coils, size_t csz) {
+    const int unit = (int)(16 / csz);
+    return (coils + unit - 1) / unit * unit;
+}
+
 // Scratch for the partial tiles of split spread work items.
 int ensure_scratch(gbn_plan* P, int coils) {
     const size_t csz = (size_t)2 * P->rsize;
@@ -702,6 +703,12 @@ int ensure_scratch(gbn_plan* P, int coils) {
         cudaError_t e = P->scratch.alloc((size_t)need * csz);
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "scratch allocation failed");
         P->scratch_cap = need;
+    }
+    // the coil-minor values of the visit-list spread
+    const size_t vbytes = (size_t)P->M_total * value_row(coils, csz) * csz;
+    if (coils >= VALUES_MIN_COILS && vbytes > P->vals.bytes) {
+        cudaError_t e = P->vals.alloc(vbytes);
+        if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "sample value allocation failed");
     }
     return GBN_OK;
 }
@@ -1012,14 +1019,14 @@ int fft_inverse(gbn_plan* P, int planes, cudaStream_t s) {
 }
 
 // Coil lanes for a call: as many as the coil count asks for, halved until
-// the gather and spread shared memory fit the per-CTA limit with the plan's
+// the gather's shared memory fits the per-CTA limit with the plan's
 // tiles (a plan tiled for few coils still runs wide batches, in more chunks).
 // Both directions use the same lane count so the scratch bound holds.
 template <typename R>
 Lanes call_lanes(const gbn_plan* P, int coils) {
-    const Geom<R> gg = make_geom<R>(P, false), gs = make_geom<R>(P, true);
+    const Geom<R> gg = make_geom<R>(P, false);
     Lanes ln = make_lanes(P->geom.ndim, coils);
-    while (ln.LS > 1 && (gather_smem<R>(gg, ln) > SMEM_LIMIT || spread_smem<R>(gs, ln) > SMEM_LIMIT))
+    while (ln.LS > 1 && gather_smem<R>(gg, ln) > SMEM_LIMIT)
         ln = make_lanes(P->geom.ndim, ln.LS / 2);
     return ln;
 }
@@ -1051,49 +1058,86 @@ int run_gather(gbn_plan* P, const void* grid, void* y, int coils, bool phases, c
     return GBN_OK;
 }
 
+// The spread over visit lists into `grid`, then the reduction of split tiles.
+// vals: room for the coil-minor values (or nullptr: the samples are read in
+// place), scratch: the partial sums.
 template <typename R>
-int run_spread(gbn_plan* P, const void* y, void* grid, int coils, bool phases, cudaStream_t s) {
+int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, bool phases, void* vals, int64_t vals_elems,
+                  void* scratch, int64_t scratch_elems, cudaStream_t s) {
     typedef typename Cx<R>::T C;
-    int rc = ensure_scratch(P, coils);
-    if (rc) return rc;
-    SpreadParams<R> p;
+    const Lanes ln = call_lanes<R>(P, coils);
+    if (ln.LS < 8) vals = nullptr;   // narrow lanes read the samples in place
+    const C* ph = phases && P->has_phase ? reinterpret_cast<const C*>(P->phnat.p) : nullptr;
+    const int64_t* foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
+    VisitParams<R> p;
     std::memset(&p, 0, sizeof(p));
     p.g = make_geom<R>(P, true);
-    p.ln = call_lanes<R>(P, coils);
+    if (phases) internal_layout(P, P->F * coils, p.g);   // the transform's own grid
+    p.g.grid_elems = (int64_t)P->F * coils * P->Kprod;
+    p.g.sample_elems = (int64_t)coils * P->M_total;
     p.s = make_list<R>(P, P->slist, P->slen, true);
+    p.start = static_cast<const long long*>(P->vstart.p);
+    p.vidx = static_cast<const int*>(P->vidx.p);
+    p.vco = P->coefs ? static_cast<const R*>(P->vco.p) : nullptr;
+    for (int q = 0; q < SPREAD_HEAVY_LEVELS; ++q) p.nheavy[q] = P->n_heavy[q];
+    p.nvisits = P->nvisits;
     p.items = reinterpret_cast<const int4*>(P->sitems.p);
     p.parts = reinterpret_cast<const int2*>(P->sparts.p);
     p.nitems = P->n_sitems;
+    p.nblk = spread_threads(P->geom.ndim, P->Ts) / 32;
     p.coils = coils;
-    p.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
-    if (phases) internal_layout(P, P->F * coils, p.g);   // the transform's own grid
-    p.y = reinterpret_cast<const C*>(y);
-    p.grid = reinterpret_cast<C*>(grid);
-    p.scratch = reinterpret_cast<C*>(P->scratch.p);
+    p.LS = ln.LS;
+    p.chunks = (coils + ln.LS - 1) / ln.LS;
+    p.row = value_row(coils, sizeof(C));
+    p.foff = foff;
+    p.vals = static_cast<const C*>(vals);
+    p.y = static_cast<const C*>(y);
+    p.ph = ph;
+    p.grid = static_cast<C*>(grid);
+    p.scratch = static_cast<C*>(scratch);
     p.tile_cells = (int64_t)P->Ts[0] * P->Ts[1] * P->Ts[2];
-    p.scratch_elems = P->scratch_cap;
-    p.chunks = (coils + p.ln.LS - 1) / p.ln.LS;
-    p.g.grid_elems = (int64_t)P->F * coils * P->Kprod;
-    p.g.sample_elems = (int64_t)coils * P->M_total;
+    p.scratch_elems = scratch_elems;
     p.apply_pb = phases && P->geom.phasing == GBN_PHASING_REAL;
-    p.apply_ph = phases && P->has_phase;
-    GBN_CUDA(launch_spread<R>(p, s), "spread launch");
+    if (vals) {
+        ValuesParams<R> v;
+        std::memset(&v, 0, sizeof(v));
+        v.y = p.y;
+        v.ph = ph;
+        v.out = static_cast<C*>(vals);
+        v.foff = foff;
+        v.F = P->F;
+        v.coils = coils;
+        v.row = p.row;
+        v.M = P->M_total;
+        v.check = p.g.check;
+        v.out_elems = vals_elems;
+        GBN_CUDA(launch_values<R>(v, s), "sample values launch");
+    }
+    GBN_CUDA(launch_spread_visits<R>(p, s), "spread launch");
     if (P->n_rtiles) {
         ReduceParams<R> q;
         std::memset(&q, 0, sizeof(q));
         q.g = p.g;
-        q.ln = p.ln;
+        q.ln = ln;
         q.tiles = reinterpret_cast<const int4*>(P->rtiles.p);
         q.ntiles = P->n_rtiles;
         q.coils = coils;
         q.scratch = p.scratch;
         q.grid = p.grid;
         q.tile_cells = p.tile_cells;
-        q.scratch_elems = p.scratch_elems;
+        q.scratch_elems = scratch_elems;
         q.apply_pb = p.apply_pb;
         GBN_CUDA(launch_reduce<R>(q, s), "reduce launch");
     }
     return GBN_OK;
+}
+
+template <typename R>
+int run_spread(gbn_plan* P, const void* y, void* grid, int coils, bool phases, cudaStream_t s) {
+    int rc = ensure_scratch(P, coils);
+    if (rc) return rc;
+    return launch_visits<R>(P, y, grid, coils, phases, coils >= VALUES_MIN_COILS ? P->vals.p : nullptr,
+                            (int64_t)(P->vals.bytes / sizeof(typename Cx<R>::T)), P->scratch.p, P->scratch_cap, s);
 }
 
 // The spread of run_spread with the split-tile partial sums kept in the
@@ -1119,43 +1163,13 @@ int run_spread_noalloc(gbn_plan* P, const void* y, void* grid, int coils, cudaSt
                       (long long)need, coils, cap);
         return fail(GBN_ERR_TOOLARGE, msg);
     }
-    SpreadParams<R> p;
-    std::memset(&p, 0, sizeof(p));
-    p.g = make_geom<R>(P, true);
-    p.ln = ln;
-    p.s = make_list<R>(P, P->slist, P->slen, true);
-    p.items = reinterpret_cast<const int4*>(P->sitems.p);
-    p.parts = reinterpret_cast<const int2*>(P->sparts.p);
-    p.nitems = P->n_sitems;
-    p.coils = coils;
-    p.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
-    p.y = reinterpret_cast<const C*>(y);
-    p.grid = reinterpret_cast<C*>(grid);
-    p.scratch = reinterpret_cast<C*>(scratch);
-    p.tile_cells = tile_cells;
-    p.scratch_elems = (int64_t)(cap / sizeof(C));
-    p.chunks = (coils + ln.LS - 1) / ln.LS;
-    p.g.grid_elems = (int64_t)P->F * coils * P->Kprod;
-    p.g.sample_elems = (int64_t)coils * P->M_total;
-    p.apply_pb = 0;
-    p.apply_ph = 0;
-    GBN_CUDA(launch_spread<R>(p, s), "no-alloc spread launch");
-    if (P->n_rtiles) {
-        ReduceParams<R> q;
-        std::memset(&q, 0, sizeof(q));
-        q.g = p.g;
-        q.ln = p.ln;
-        q.tiles = reinterpret_cast<const int4*>(P->rtiles.p);
-        q.ntiles = P->n_rtiles;
-        q.coils = coils;
-        q.scratch = p.scratch;
-        q.grid = p.grid;
-        q.tile_cells = p.tile_cells;
-        q.scratch_elems = p.scratch_elems;
-        q.apply_pb = 0;
-        GBN_CUDA(launch_reduce<R>(q, s), "no-alloc reduce launch");
-    }
-    return GBN_OK;
+    // the values take what the partial sums leave of the array, if they fit;
+    // else the samples are read in place
+    const int64_t used = (need + 255) & ~(int64_t)255;
+    const int64_t velems = P->M_total * value_row(coils, sizeof(C));
+    void* vals = coils >= VALUES_MIN_COILS && used + velems * (int64_t)sizeof(C) <= (int64_t)cap
+                     ? static_cast<char*>(scratch) + used : nullptr;
+    return launch_visits<R>(P, y, grid, coils, false, vals, velems, scratch, need / (int64_t)sizeof(C), s);
 }
 
 template <typename R>
@@ -1450,55 +1464,102 @@ int validate(const gbn_geometry* g) {
     return GBN_OK;
 }
 
-// Precompute both lists' interpolation coefficients (list order): from the
-// sparse-mode weights when set, else from the tables unless the geometry
-// asks for table interpolation inside the kernels (GBN_FLAG_TABLE_ONLY).
+// Per-axis sparse-mode weights on the device (re, then im), or nullptr.
 template <typename R>
-int fill_coefs(gbn_plan* P, cudaStream_t stream = 0, bool sync = true) {
+void weight_pointers(const gbn_plan* P, const R* (&wr)[3], const R* (&wi)[3]) {
+    const R* w = reinterpret_cast<const R*>(P->weights.p);
+    if (!w) return;
+    for (int part = 0; part < (P->cx ? 2 : 1); ++part)
+        for (int d = 0; d < P->geom.ndim; ++d) {
+            (part ? wi : wr)[d] = w;
+            w += (size_t)P->M_total * P->geom.Jd[d];
+        }
+}
+
+// Visit lists of the spread (gbn_visit.cuh), with their coefficients unless
+// the geometry asks for table interpolation inside the kernels.  `total`: the
+// visits before padding where the caller knows them (device binning), else -1
+// and the padded sum is read back.
+template <typename R>
+int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
+    VisitBuildParams<R> b;
+    std::memset(&b, 0, sizeof(b));
+    b.g = make_geom<R>(P, true);
+    b.s = make_list<R>(P, P->slist, P->slen, true);
+    b.items = reinterpret_cast<const int4*>(P->sitems.p);
+    b.nitems = P->n_sitems;
+    b.nblk = spread_threads(P->geom.ndim, P->Ts) / 32;
+    b.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
+    weight_pointers<R>(P, b.wr, b.wi);
+    b.cx = P->cx ? 1 : 0;
+    const int64_t units = (int64_t)b.nitems * b.nblk;
+    auto ensure = [](DevBuf& d, size_t bytes) {
+        return d.bytes >= bytes && d.p ? cudaSuccess : d.alloc(std::max<size_t>(bytes, 256));
+    };
+    const size_t cbytes = ((size_t)units * sizeof(int) + 255) & ~(size_t)255;
+    GBN_CUDA(ensure(P->vwork, cbytes + scan_temp_bytes(units)), "visit workspace");
+    GBN_CUDA(ensure(P->vstart, (size_t)(units + 1) * sizeof(long long)), "visit offsets");
+    b.count = static_cast<int*>(P->vwork.p);
+    long long* start = static_cast<long long*>(P->vstart.p);
+    GBN_CUDA(launch_visit_count<R>(b, stream), "visit count launch");
+    GBN_CUDA(exclusive_scan64(b.count, start, units, start + units, static_cast<char*>(P->vwork.p) + cbytes, stream),
+             "visit scan");
+    if (total < 0) {
+        long long h = 0;
+        GBN_CUDA(cudaMemcpyAsync(&h, start + units, sizeof(h), cudaMemcpyDeviceToHost, stream), "visit count readback");
+        GBN_CUDA(cudaStreamSynchronize(stream), "visit count readback");
+        total = h;
+    } else {
+        total += 3 * units;   // padding, at most
+    }
+    const int NC = P->geom.ndim == 1 ? 16 : 8;
+    GBN_CUDA(ensure(P->vidx, (size_t)total * sizeof(int)), "visit allocation");
+    if (coefs)
+        GBN_CUDA(ensure(P->vco, (size_t)total * NC * (P->cx ? 2 : 1) * sizeof(R)), "visit allocation");
+    else
+        GBN_CUDA(P->vco.alloc(0), "coefficient release");
+    b.start = start;
+    b.vidx = static_cast<int*>(P->vidx.p);
+    b.vco = static_cast<R*>(P->vco.p);
+    GBN_CUDA(launch_visit_fill<R>(b, stream), "visit launch");
+    P->nvisits = total;
+    return GBN_OK;
+}
+
+// Precompute the interpolation coefficients, of the gather in list order and
+// of the spread per visit: from the sparse-mode weights when set, else from
+// the tables unless the geometry asks for table interpolation inside the
+// kernels (GBN_FLAG_TABLE_ONLY).  `total`: as for build_visits.
+template <typename R>
+int fill_coefs(gbn_plan* P, cudaStream_t stream = 0, bool sync = true, int64_t total = -1) {
     P->coefs = false;
     const gbn_geometry& G = P->geom;
-    if (!P->weights.p && (G.flags & GBN_FLAG_TABLE_ONLY)) {
-        GBN_CUDA(P->gcoef.alloc(0), "coefficient release");
-        GBN_CUDA(P->scoef.alloc(0), "coefficient release");
-        return GBN_OK;
-    }
-    int jsum = 0;
-    for (int d = 0; d < G.ndim; ++d) jsum += G.Jd[d];
-    const size_t parts = P->cx ? 2 : 1;
-    const size_t gb = (size_t)P->glen * jsum * parts * sizeof(R);
-    const size_t sb = (size_t)P->slen * jsum * parts * sizeof(R);
-    GBN_CUDA(P->gcoef.alloc(std::max<size_t>(gb, 16)), "gather coefficient allocation");
-    GBN_CUDA(P->scoef.alloc(std::max<size_t>(sb, 16)), "spread coefficient allocation");
-    for (int which = 0; which < 2; ++which) {
-        const bool spread = which == 1;
+    const bool keep = P->weights.p || !(G.flags & GBN_FLAG_TABLE_ONLY);
+    if (keep) {
+        int jsum = 0;
+        for (int d = 0; d < G.ndim; ++d) jsum += G.Jd[d];
+        const size_t bytes = std::max<size_t>((size_t)P->glen * jsum * (P->cx ? 2 : 1) * sizeof(R), 16);
+        if (P->gcoef.bytes < bytes) GBN_CUDA(P->gcoef.alloc(bytes), "gather coefficient allocation");
         CoefParams<R> c;
         std::memset(&c, 0, sizeof(c));
-        c.g = make_geom<R>(P, spread);
-        c.s = make_list<R>(P, spread ? P->slist : P->glist, spread ? P->slen : P->glen, spread);
-        c.items = reinterpret_cast<const int4*>(spread ? P->sitems.p : P->gitems.p);
-        c.nitems = spread ? P->n_sitems : P->n_gitems;
+        c.g = make_geom<R>(P, false);
+        c.s = make_list<R>(P, P->glist, P->glen, false);
+        c.items = reinterpret_cast<const int4*>(P->gitems.p);
+        c.nitems = P->n_gitems;
         c.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
-        if (P->weights.p) {
-            const R* w = reinterpret_cast<const R*>(P->weights.p);
-            size_t woff = 0;
-            for (int d = 0; d < G.ndim; ++d) {
-                c.wr[d] = w + woff;
-                woff += (size_t)P->M_total * G.Jd[d];
-            }
-            for (int d = 0; d < G.ndim && P->cx; ++d) {
-                c.wi[d] = w + woff;
-                woff += (size_t)P->M_total * G.Jd[d];
-            }
-        }
-        const int64_t len = spread ? P->slen : P->glen;
-        c.out_r = reinterpret_cast<R*>(spread ? P->scoef.p : P->gcoef.p);
-        c.out_i = P->cx ? c.out_r + (size_t)len * jsum : nullptr;
+        weight_pointers<R>(P, c.wr, c.wi);
+        c.out_r = reinterpret_cast<R*>(P->gcoef.p);
+        c.out_i = P->cx ? c.out_r + (size_t)P->glen * jsum : nullptr;
         c.jsum = jsum;
         c.cx = P->cx ? 1 : 0;
         GBN_CUDA(launch_coef<R>(c, stream), "coefficient launch");
+    } else {
+        GBN_CUDA(P->gcoef.alloc(0), "coefficient release");
     }
+    int rc = build_visits<R>(P, keep, stream, total);
+    if (rc) return rc;
     if (sync) GBN_CUDA(cudaDeviceSynchronize(), "coefficient precompute");
-    P->coefs = true;
+    P->coefs = keep;
     return GBN_OK;
 }
 
@@ -1560,8 +1621,7 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     unsigned *gkey, *gval;
     void* scan_tmp;
     auto layout_a = [&](Bump& b) {
-        err = b.take<int>(16);
-        tot = b.take<int>(16);
+        err = b.take<int>(32);
         gkey = b.take<unsigned>(M);
         gval = b.take<unsigned>(M);
         ecount = b.take<int>(M);
@@ -1578,6 +1638,7 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
         Bump b(P->bin_ws.p);
         layout_a(b);
     }
+    tot = err + 16;   // entry count, item counts (1-4), heavy items (5-10), visit count (12-13)
     BinParams<R> bp;
     std::memset(&bp, 0, sizeof(bp));
     bp.ndim = ndim;
@@ -1590,6 +1651,8 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
         bp.Ts[d] = P->Ts[d];
         bp.nts[d] = P->nts[d];
     }
+    spread_block(ndim, bp.B);
+    bp.nvisits = reinterpret_cast<unsigned long long*>(tot + 12);
     bp.ntiles_g = ntg;
     bp.ntiles_s = nts;
     bp.tm_limit = TM_LIMIT;
@@ -1604,12 +1667,13 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     GBN_CUDA(cudaMemsetAsync(err, 0, 32 * sizeof(int), s), "binning reset");
     GBN_CUDA(launch_bin_count<R>(bp, s), "bin count launch");
     GBN_CUDA(exclusive_scan(ecount, eoff, M, tot, scan_tmp, s), "entry scan");
-    int hA[2] = {0, 0};
-    GBN_CUDA(cudaMemcpyAsync(&hA[0], err, sizeof(int), cudaMemcpyDeviceToHost, s), "binning readback");
-    GBN_CUDA(cudaMemcpyAsync(&hA[1], tot, sizeof(int), cudaMemcpyDeviceToHost, s), "binning readback");
+    int hA[32] = {0};
+    GBN_CUDA(cudaMemcpyAsync(hA, err, sizeof(hA), cudaMemcpyDeviceToHost, s), "binning readback");
     GBN_CUDA(cudaStreamSynchronize(s), "binning readback");
     if (hA[0]) return fail(GBN_ERR_INVALID, "sample coordinate is not finite or |tm| > 2^22");
-    const int64_t slen = hA[1];
+    const int64_t slen = hA[16];
+    unsigned long long nvisits = 0;
+    std::memcpy(&nvisits, hA + 28, sizeof(nvisits));
 
     // ---- phase B: spread entries, sorts, bins, items ---------------------
     const int64_t nsort = std::max<int64_t>(std::max<int64_t>(M, slen), nbs);
@@ -1685,13 +1749,14 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     ip.sparts = sp;
     ip.rslots = rs;
     ip.rflag = rf;
+    ip.nheavy = tot + 5;
     GBN_CUDA(launch_bin_parts(ip, s), "bin parts launch");
     GBN_CUDA(exclusive_scan(gp, go, nbg, tot + 1, scan_tmp, s), "gather item scan");
     GBN_CUDA(exclusive_scan(sp, so, nbs, tot + 2, scan_tmp, s), "spread item scan");
     GBN_CUDA(exclusive_scan(rs, slo, nbs, tot + 3, scan_tmp, s), "slot scan");
     GBN_CUDA(exclusive_scan(rf, ro, nbs, tot + 4, scan_tmp, s), "split tile scan");
-    int hB[4] = {0, 0, 0, 0};
-    GBN_CUDA(cudaMemcpyAsync(hB, tot + 1, 4 * sizeof(int), cudaMemcpyDeviceToHost, s), "binning readback");
+    int hB[4 + SPREAD_HEAVY_LEVELS] = {0};
+    GBN_CUDA(cudaMemcpyAsync(hB, tot + 1, sizeof(hB), cudaMemcpyDeviceToHost, s), "binning readback");
     GBN_CUDA(cudaStreamSynchronize(s), "binning readback");
     const int n_gi = hB[0], n_si = hB[1], n_slots = hB[2], n_rt = hB[3];
     auto ensure = [&](DevBuf& b, size_t bytes, const char* what) -> int {
@@ -1760,7 +1825,12 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     P->n_sitems = n_si;
     P->n_rtiles = n_rt;
     P->n_slots = n_slots;
-    return fill_coefs<R>(P, s, false);
+    for (int q = 0; q < SPREAD_HEAVY_LEVELS; ++q) P->n_heavy[q] = hB[4 + q];
+    if (ph) {
+        if ((rc = ensure(P->phnat, (size_t)M * sizeof(C), "phase allocation"))) return rc;
+        GBN_CUDA(cudaMemcpyAsync(P->phnat.p, ph, (size_t)M * sizeof(C), cudaMemcpyDeviceToDevice, s), "phase copy");
+    }
+    return fill_coefs<R>(P, s, false, (int64_t)nvisits);
 }
 
 }  // namespace
@@ -2107,7 +2177,9 @@ int gbn_plan_stats(const gbn_plan* P, int64_t* o) {
     o[3] = P->glen;
     o[4] = P->slen;
     o[5] = (int64_t)P->ntiles_s * P->F;
-    o[6] = (int64_t)(P->tables.bytes + P->weights.bytes + P->gcoef.bytes + P->scoef.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
+    o[6] = (int64_t)(P->tables.bytes + P->weights.bytes + P->gcoef.bytes +
+                     P->vstart.bytes + P->vidx.bytes + P->vco.bytes + P->vwork.bytes + P->phnat.bytes +
+                     P->vals.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
                      P->grid.bytes + P->scratch.bytes);
     o[7] = P->M_total;
     return GBN_OK;

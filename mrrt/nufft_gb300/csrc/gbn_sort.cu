@@ -28,44 +28,46 @@ inline size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Exclusive scan of a CTA's values held one per thread; *out_total gets the
 // CTA total.
-__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int* out_total) {
+template <typename T>
+__device__ __forceinline__ T block_exclusive_scan(T v, T* warp_sums, T* out_total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
+    T x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        const T y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
     if (lane == 31) warp_sums[warp] = x;
     __syncthreads();
     if (warp == 0) {
         const int nw = blockDim.x >> 5;
-        int w = lane < nw ? warp_sums[lane] : 0;
+        T w = lane < nw ? warp_sums[lane] : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            const T y = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += y;
         }
         if (lane < nw) warp_sums[lane] = w;   // inclusive
     }
     __syncthreads();
-    const int before = warp > 0 ? warp_sums[warp - 1] : 0;
+    const T before = warp > 0 ? warp_sums[warp - 1] : 0;
     *out_total = warp_sums[(blockDim.x >> 5) - 1];
     return before + x - v;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) scan_tile_kernel(const int* in, int* out, int64_t n, int* bsum) {
-    __shared__ int ws[32];
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(SCAN_THREADS) scan_tile_kernel(const TI* in, TO* out, int64_t n, TO* bsum) {
+    __shared__ TO ws[32];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_PER_THREAD;
-    int v[SCAN_PER_THREAD];
-    int s = 0;
+    TO v[SCAN_PER_THREAD];
+    TO s = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_PER_THREAD; ++k) {
         v[k] = base + k < n ? in[base + k] : 0;
         s += v[k];
     }
-    int total;
-    int run = block_exclusive_scan(s, ws, &total);
+    TO total;
+    TO run = block_exclusive_scan(s, ws, &total);
 #pragma unroll
     for (int k = 0; k < SCAN_PER_THREAD; ++k) {
         if (base + k < n) out[base + k] = run;
@@ -74,15 +76,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_tile_kernel(const int* in, 
     if (threadIdx.x == 0 && bsum) bsum[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) scan_add_kernel(int* out, int64_t n, const int* boff) {
+template <typename TO>
+__global__ void __launch_bounds__(SCAN_THREADS) scan_add_kernel(TO* out, int64_t n, const TO* boff) {
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_PER_THREAD;
-    const int add = boff[blockIdx.x];
+    const TO add = boff[blockIdx.x];
 #pragma unroll
     for (int k = 0; k < SCAN_PER_THREAD; ++k)
         if (base + k < n) out[base + k] += add;
 }
 
-__global__ void scan_total_kernel(const int* in, const int* out, int64_t n, int* total) {
+template <typename TI, typename TO>
+__global__ void scan_total_kernel(const TI* in, const TO* out, int64_t n, TO* total) {
     *total = n > 0 ? out[n - 1] + in[n - 1] : 0;
 }
 
@@ -164,38 +168,47 @@ __global__ void __launch_bounds__(RADIX_THREADS) radix_scatter_kernel(const unsi
     }
 }
 
+template <typename TI, typename TO>
+cudaError_t scan_any(const TI* in, TO* out, int64_t n, TO* total, void* temp, cudaStream_t s) {
+    if (n <= 0) {
+        if (total) return cudaMemsetAsync(total, 0, sizeof(TO), s);
+        return cudaSuccess;
+    }
+    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+    if (nb == 1) {
+        scan_tile_kernel<TI, TO><<<1, SCAN_THREADS, 0, s>>>(in, out, n, nullptr);
+    } else {
+        char* t = reinterpret_cast<char*>(temp);
+        const size_t part = round256((size_t)nb * sizeof(long long));
+        TO* bsum = reinterpret_cast<TO*>(t);
+        TO* boff = reinterpret_cast<TO*>(t + part);
+        scan_tile_kernel<TI, TO><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, bsum);
+        cudaError_t e = scan_any<TO, TO>(bsum, boff, nb, nullptr, t + 2 * part, s);
+        if (e != cudaSuccess) return e;
+        scan_add_kernel<TO><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(out, n, boff);
+    }
+    if (total) scan_total_kernel<TI, TO><<<1, 1, 0, s>>>(in, out, n, total);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 size_t scan_temp_bytes(int64_t n) {
     size_t bytes = 0;
     while (n > SCAN_TILE) {
         const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-        bytes += 2 * round256((size_t)nb * sizeof(int));
+        bytes += 2 * round256((size_t)nb * sizeof(long long));
         n = nb;
     }
     return bytes + 256;
 }
 
 cudaError_t exclusive_scan(const int* in, int* out, int64_t n, int* total, void* temp, cudaStream_t s) {
-    if (n <= 0) {
-        if (total) return cudaMemsetAsync(total, 0, sizeof(int), s);
-        return cudaSuccess;
-    }
-    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-    if (nb == 1) {
-        scan_tile_kernel<<<1, SCAN_THREADS, 0, s>>>(in, out, n, nullptr);
-    } else {
-        char* t = reinterpret_cast<char*>(temp);
-        int* bsum = reinterpret_cast<int*>(t);
-        int* boff = reinterpret_cast<int*>(t + round256((size_t)nb * sizeof(int)));
-        void* rest = t + 2 * round256((size_t)nb * sizeof(int));
-        scan_tile_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, bsum);
-        cudaError_t e = exclusive_scan(bsum, boff, nb, nullptr, rest, s);
-        if (e != cudaSuccess) return e;
-        scan_add_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(out, n, boff);
-    }
-    if (total) scan_total_kernel<<<1, 1, 0, s>>>(in, out, n, total);
-    return cudaGetLastError();
+    return scan_any<int, int>(in, out, n, total, temp, s);
+}
+
+cudaError_t exclusive_scan64(const int* in, long long* out, int64_t n, long long* total, void* temp, cudaStream_t s) {
+    return scan_any<int, long long>(in, out, n, total, temp, s);
 }
 
 // temp layout: keys and values of the other ping-pong side, the digit

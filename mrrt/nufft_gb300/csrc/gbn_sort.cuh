@@ -11,6 +11,8 @@ size_t scan_temp_bytes(int64_t n);
 // out[i] = in[0] + ... + in[i-1] (int32; in and out may not alias); total
 // (device, optional) receives the sum of all n.  Asynchronous on s.
 cudaError_t exclusive_scan(const int* in, int* out, int64_t n, int* total, void* temp, cudaStream_t s);
+// The same with 64-bit sums.
+cudaError_t exclusive_scan64(const int* in, long long* out, int64_t n, long long* total, void* temp, cudaStream_t s);
 
 // Bytes of device temporaries radix_sort_pairs needs for n pairs.
 size_t radix_temp_bytes(int64_t n);

@@ -1,0 +1,851 @@
+// Adjoint table interpolation (samples -> grid) over plan-time visit lists.
+// Replaces the reference's scatters (serial per coil on the CPU,
+// mrrt/nufft/_extensions/c/nufft_table.template.c:144-531, 924-1206; global
+// atomicAdd per tap on the GPU, mrrt/nufft/cuda/jinja/table_*_adjoint.jinja)
+// with an "owner computes" decomposition and register accumulation.
+//
+// The grid is cut into register blocks of 16 cells (4 x 4, one z-plane; 16 in
+// 1-D); a warp holds a block's 16 complex sums in every lane, lane = (visit
+// slot, coil), LS coils per chunk.  Which samples touch a block, and with
+// which coefficients, is fixed by the coordinates, so the plan stores it:
+//
+//   * visits: for each work item (a tile's entries, or a part of them) and
+//     each block of the tile, in entry order, the samples whose window
+//     touches the block, padded to a multiple of four;
+//   * each visit's coefficients clipped to the block and zero-padded: B0
+//     values of axis 0, then (2-D, 3-D) B1 values w of the other axes, w = c1
+//     or c1 c2.  Rows the window misses hold -0, so that a row is skipped by
+//     a test of its bits and not by its value.
+//
+// At run time nothing is searched or sorted: a warp streams visits.  (The
+// kernel this replaces staged a tile's entries chunk by chunk with two
+// barriers each, and every warp balloted which of them touched its block:
+// 515 warp instructions a sample at the 2-D 32-coil workload, 101 of them
+// the multiply-adds.)  Measured, spread alone, before -> now, plus the pass
+// that lays the values out: 128^3 kooshball, 8 coils 4892 -> 2014 + 115 us;
+// 64-frame series, 8 coils 949 -> 452 + 64; 2-D 256^2, 32 coils 143 -> 109 +
+// 24; 128^2, one coil 29 -> 18; 192^2 double, 4 coils 345 -> 227.  Bound by
+// instruction issue (3-D: 80% of the issue slots, 45% of them multiply-adds).
+//
+// The sample values come coil-minor, [sample][coil], with conj(sample phase)
+// applied (values_kernel: one transposition per call), so that one visit's
+// coils are one segment: read straight from [coil][sample], a 32-coil visit
+// touches 32 sectors.  Up to four coils, where the segment is no longer than
+// a sector, the values are read in place and the phase applied on reading.
+//
+// Order of summation: entry order per slot, slots combined in a fixed
+// pattern, warps sharing a block in warp order, parts of split tiles by
+// reduce_kernel: the same in every run.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "gbn_device.cuh"
+#include "gbn_internal.h"
+
+namespace gbn {
+
+template <int NDIM>
+struct VisitBlock {
+    static constexpr int B0 = SpreadBlock<NDIM>::B0, B1 = SpreadBlock<NDIM>::B1, B2 = SpreadBlock<NDIM>::B2;
+    static constexpr int NB = B0 * B1;               // cells (B2 = 1: w carries axis 2)
+    static constexpr int NC = B0 + (NDIM > 1 ? B1 : 0);   // coefficients per visit
+    static_assert(B2 == 1 && NB == 16, "register blocks of 16 cells, one z-plane");
+};
+
+// Origin of register block `blk` within its tile (blocks of axis 0 fastest).
+template <int NDIM, typename R>
+__host__ __device__ __forceinline__ void block_origin(const Geom<R>& g, int blk, int& b0, int& b1, int& b2) {
+    typedef VisitBlock<NDIM> VB;
+    const int n0 = g.T[0] / VB::B0, n1 = NDIM > 1 ? g.T[1] / VB::B1 : 1;
+    b0 = (blk % n0) * VB::B0;
+    b1 = NDIM > 1 ? ((blk / n0) % n1) * VB::B1 : 0;
+    b2 = NDIM > 2 ? blk / (n0 * n1) : 0;
+}
+// The same from the table the launcher put in the parameters (no division).
+template <typename R>
+__device__ __forceinline__ void block_origin_of(const VisitParams<R>& p, int blk, int& b0, int& b1, int& b2) {
+    const short4 o = p.borg[blk];
+    b0 = o.x;
+    b1 = o.y;
+    b2 = o.z;
+}
+
+__device__ __forceinline__ bool is_neg_zero(float v) { return __float_as_uint(v) == 0x80000000u; }
+__device__ __forceinline__ bool is_neg_zero(double v) {
+    return (unsigned long long)__double_as_longlong(v) == 0x8000000000000000ull;
+}
+
+// N values, 16 bytes at a time (16-byte aligned records, global or shared).
+template <int N>
+__device__ __forceinline__ void load_run(const float* src, float (&o)[N]) {
+    static_assert(N % 4 == 0, "whole vectors");
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(src + i);
+        o[i] = v.x;
+        o[i + 1] = v.y;
+        o[i + 2] = v.z;
+        o[i + 3] = v.w;
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_run(const double* src, double (&o)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(src + i);
+        o[i] = v.x;
+        o[i + 1] = v.y;
+    }
+}
+
+// 16-byte asynchronous copy of `bytes` (16 or 0) source bytes, zero-filled.
+__device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, bool valid) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    const int n = valid ? 16 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(n) : "memory");
+}
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait_pending() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// Coefficient k of the visit of list entry e (sample idx of the frame at
+// offset fo) to the block at (b0, b1, b2): from the per-sample weights when
+// set, else from the tables; conjugated for a complex kernel.
+template <typename R, int NDIM, bool CX>
+__device__ __forceinline__ typename Cx<R>::T visit_coef(const Geom<R>& g, const SampleList<R>& s, int64_t e, short4 ls,
+                                                        int64_t m, const R* const* wr, const R* const* wi, int b0,
+                                                        int b1, int b2, int k) {
+    typedef VisitBlock<NDIM> VB;
+    typedef typename Cx<R>::T C;
+    auto coef = [&](int d, int j) -> C {
+        R cr, ci = (R)0;
+        if (wr && wr[0]) {
+            cr = wr[d][m * g.J[d] + j];
+            if (CX) ci = wi[d][m * g.J[d] + j];
+        } else {
+            const R t = s.t[d][e];
+            table_coef<R, CX>(g, d, t, first_tap(t, g.J[d]) + j, cr, ci);
+        }
+        return cmake<R>(cr, CX ? -ci : (R)0);
+    };
+    if (k < VB::B0) {
+        const int j = b0 + k - ls.x;
+        return j >= 0 && j < g.J[0] ? coef(0, j) : cmake<R>((R)0, (R)0);
+    }
+    const int j = b1 + (k - VB::B0) - ls.y;
+    if (NDIM < 2 || j < 0 || j >= g.J[1]) return cmake<R>((R)-0.0, (R)0);
+    C w = coef(1, j);
+    if (NDIM > 2) {
+        const C c2 = coef(2, b2 - ls.z);
+        w = CX ? cmul_fixed(w, c2) : cmake<R>(mul_rn(w.x, c2.x), (R)0);
+    }
+    return w;
+}
+
+// ---- plan time ---------------------------------------------------------------
+
+// The tile's block at (b0, b1, b2) holds cells of the grid (tile edges may
+// reach past it); the others are never written and have no visits.
+template <int NDIM, typename R>
+__device__ __forceinline__ bool block_in_grid(const Geom<R>& g, int tile, int b0, int b1, int b2) {
+    int org[3] = {0, 0, 0};
+    tile_origin<NDIM>(tile, g.nt, g.T, org);
+    return org[0] + b0 < g.K[0] && (NDIM < 2 || org[1] + b1 < g.K[1]) && (NDIM < 3 || org[2] + b2 < g.K[2]);
+}
+
+// A window starting at s (tile coordinates) touches the block at (b0, b1, b2).
+template <int NDIM, typename R>
+__device__ __forceinline__ bool visits_block(const Geom<R>& g, short4 s, int b0, int b1, int b2) {
+    typedef VisitBlock<NDIM> VB;
+    bool hit = s.x < b0 + VB::B0 && s.x + g.J[0] > b0;
+    if (NDIM > 1) hit = hit && s.y < b1 + VB::B1 && s.y + g.J[1] > b1;
+    if (NDIM > 2) hit = hit && s.z < b2 + VB::B2 && s.z + g.J[2] > b2;
+    return hit;
+}
+
+// Visits per (item, block), rounded up to whole groups of four: one CTA per
+// item, one warp per block.
+template <typename R, int NDIM>
+__global__ void __launch_bounds__(256) visit_count_kernel(const VisitBuildParams<R> p) {
+    const int item = blockIdx.x, blk = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int4 it = p.items[item];
+    int b0, b1, b2;
+    block_origin<NDIM>(p.g, blk, b0, b1, b2);
+    int n = 0;
+    const int count = block_in_grid<NDIM>(p.g, it.y, b0, b1, b2) ? it.w : 0;
+    for (int base = 0; base < count; base += 32) {
+        bool hit = false;
+        if (base + lane < count) hit = visits_block<NDIM>(p.g, p.s.ls[it.z + base + lane], b0, b1, b2);
+        n += __popc(__ballot_sync(0xffffffffu, hit));
+    }
+    if (lane == 0) p.count[(int64_t)item * p.nblk + blk] = (n + 3) & ~3;
+}
+
+// The visits: sample indices (list positions where the coefficients are
+// computed during the call) and coefficients; padding is index -1.
+template <typename R, int NDIM, bool CX>
+__global__ void __launch_bounds__(256) visit_fill_kernel(const VisitBuildParams<R> p) {
+    typedef VisitBlock<NDIM> VB;
+    typedef typename Cx<R>::T C;
+    constexpr int NR = VB::NC * (CX ? 2 : 1);   // reals per visit
+    const Geom<R>& g = p.g;
+    const int item = blockIdx.x, blk = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int4 it = p.items[item];
+    const int64_t fo = p.foff[it.x];
+    int b0, b1, b2;
+    block_origin<NDIM>(g, blk, b0, b1, b2);
+    int64_t at = p.start[(int64_t)item * p.nblk + blk];
+    const int64_t end = p.start[(int64_t)item * p.nblk + blk + 1];
+    const int count = block_in_grid<NDIM>(g, it.y, b0, b1, b2) ? it.w : 0;
+    for (int base = 0; base < count; base += 32) {
+        const int64_t e = (int64_t)it.z + base + lane;
+        short4 s = make_short4(0, 0, 0, 0);
+        bool hit = false;
+        if (base + lane < count) {
+            s = p.s.ls[e];
+            hit = visits_block<NDIM>(g, s, b0, b1, b2);
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, hit);
+        const int64_t pos = at + __popc(mask & ((1u << lane) - 1u));
+        if (hit && pos < end) {
+            const int idx = p.s.idx[e];
+            p.vidx[pos] = p.vco ? idx : (int)e;
+            if (p.vco) {
+                R* o = p.vco + pos * NR;
+#pragma unroll
+                for (int k = 0; k < VB::NC; ++k) {
+                    const C c = visit_coef<R, NDIM, CX>(g, p.s, e, s, fo + idx, p.wr, p.wi, b0, b1, b2, k);
+                    if (CX) {
+                        o[2 * k] = c.x;
+                        o[2 * k + 1] = c.y;
+                    } else {
+                        o[k] = c.x;
+                    }
+                }
+            }
+        }
+        at += __popc(mask);
+    }
+    if (at + lane < end) {
+        p.vidx[at + lane] = -1;
+        if (p.vco)
+            for (int k = 0; k < NR; ++k) p.vco[(at + lane) * NR + k] = !CX && k >= VB::B0 ? (R)-0.0 : (R)0;
+    }
+}
+
+// ---- per call ----------------------------------------------------------------
+
+// Samples [frame][coil][m] -> values [frame][m][coil] times conj(phase).  A
+// CTA transposes 64 consecutive samples of 32 coils at a time through shared
+// memory: 512-byte reads along m, contiguous writes along (m, coil).
+constexpr int VAL_SAMPLES = 64, VAL_COILS = 32;
+
+template <typename R>
+__global__ void __launch_bounds__(256) values_kernel(const ValuesParams<R> p) {
+    typedef typename Cx<R>::T C;
+    __shared__ C sm[VAL_SAMPLES * (VAL_COILS + 1)];
+    const int64_t m0 = (int64_t)blockIdx.x * VAL_SAMPLES;
+    const int ns = (int)min((int64_t)VAL_SAMPLES, p.M - m0);
+    const int c0 = blockIdx.y * VAL_COILS;
+    const int nc = min(VAL_COILS, p.coils - c0);
+    const int sl = threadIdx.x % VAL_SAMPLES, cg = threadIdx.x / VAL_SAMPLES;
+    constexpr int NG = 256 / VAL_SAMPLES;
+    if (sl < ns) {
+        const int64_t m = m0 + sl;
+        int f = 0, hi = p.F;   // foff[f] <= m < foff[hi]
+        while (hi - f > 1) {
+            const int mid = (f + hi) >> 1;
+            if (p.foff[mid] <= m) f = mid;
+            else hi = mid;
+        }
+        const int64_t fo = p.foff[f], Mf = p.foff[f + 1] - fo;
+        const C* src = p.y + fo * p.coils + (m - fo) + (int64_t)c0 * Mf;
+        const C ph = p.ph ? p.ph[m] : cmake<R>((R)1, (R)0);
+        for (int c = cg; c < nc; c += 4 * NG) {
+            C v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                v[u] = cmake<R>((R)0, (R)0);
+                if (c + u * NG < nc &&
+                    GBN_INB(p.check, fo * p.coils + (m - fo) + (int64_t)(c0 + c + u * NG) * Mf < p.M * p.coils,
+                            CHK_SAMPLE_READ))
+                    v[u] = src[(int64_t)(c + u * NG) * Mf];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c + u * NG < nc) sm[sl * (VAL_COILS + 1) + c + u * NG] = p.ph ? cmulc(v[u], ph) : v[u];
+        }
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < ns * nc; q += 256) {
+        const int s = q / nc, c = q - s * nc;
+        const int64_t o = (m0 + s) * p.row + c0 + c;
+        if (GBN_INB(p.check, o < p.out_elems, CHK_SCRATCH)) p.out[o] = sm[s * (VAL_COILS + 1) + c];
+    }
+}
+
+// ---- accumulation ------------------------------------------------------------
+
+// Add row k1 of one visit: value v, coefficients co.
+template <typename R, int NDIM, bool CX>
+__device__ __forceinline__ void add_row(typename Cx<R>::T (&acc)[VisitBlock<NDIM>::NB], typename Cx<R>::T v,
+                                        const R (&co)[VisitBlock<NDIM>::NC * (CX ? 2 : 1)], int k1) {
+    typedef typename Cx<R>::T C;
+    constexpr int B0 = VisitBlock<NDIM>::B0;
+    C tv = v;
+    if constexpr (CX) {
+        if (NDIM > 1) tv = cmul_fixed(cmake<R>(co[2 * (B0 + k1)], co[2 * (B0 + k1) + 1]), v);
+#pragma unroll
+        for (int k0 = 0; k0 < B0; ++k0) {
+            const C t = cmul_fixed(cmake<R>(co[2 * k0], co[2 * k0 + 1]), tv);
+            acc[k1 * B0 + k0].x = add_rn(acc[k1 * B0 + k0].x, t.x);
+            acc[k1 * B0 + k0].y = add_rn(acc[k1 * B0 + k0].y, t.y);
+        }
+    } else {
+        if (NDIM > 1) {
+            tv.x = mul_rn(co[B0 + k1], v.x);
+            tv.y = mul_rn(co[B0 + k1], v.y);
+        }
+        // scalar multiply-adds: as many per cycle as packed ones, and no
+        // register moves to form the (c, c) pairs
+#pragma unroll
+        for (int k0 = 0; k0 < B0; ++k0) {
+            acc[k1 * B0 + k0].x = fma_rn(co[k0], tv.x, acc[k1 * B0 + k0].x);
+            acc[k1 * B0 + k0].y = fma_rn(co[k0], tv.y, acc[k1 * B0 + k0].y);
+        }
+    }
+}
+
+// Sum a block over the warp's slots by a halving exchange: each slot ends up
+// with KEEP consecutive cells, from cell q0 on, in acc[0..KEEP).
+template <typename R, int LS, int NB>
+__device__ __forceinline__ int combine_slots(typename Cx<R>::T (&acc)[NB], int slot) {
+    typedef typename Cx<R>::T C;
+    constexpr int SW = 32 / LS;
+    int q0 = 0;
+#pragma unroll
+    for (int s = 0; (1 << s) < SW; ++s) {
+        const int half = NB >> (s + 1);
+        if (half >= 1) {
+            const bool up = (slot >> s) & 1;
+#pragma unroll
+            for (int i = 0; i < (half >= 1 ? half : 1); ++i) {
+                const C lo = acc[i], hi = acc[i + half];
+                const C send = up ? lo : hi, keep = up ? hi : lo;
+                acc[i].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, LS << s);
+                acc[i].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, LS << s);
+            }
+            if (up) q0 += half;
+        } else {   // 32 slots, 16 cells: the last stage adds the pair
+            acc[0].x += __shfl_xor_sync(0xffffffffu, acc[0].x, LS << s);
+            acc[0].y += __shfl_xor_sync(0xffffffffu, acc[0].y, LS << s);
+        }
+    }
+    return q0;
+}
+
+// Write a combined block: to the grid with conj(phase_before), or to the
+// scratch slot of a split tile.  `zero`: no visits (zeros need no phase).
+template <typename R, int NDIM, int LS>
+__device__ __forceinline__ void flush_block(const VisitParams<R>& p, typename Cx<R>::T (&acc)[16], int q0, int lane,
+                                            int f, const int* org, int blk, int scratch_slot, int chunk, bool zero) {
+    typedef typename Cx<R>::T C;
+    typedef VisitBlock<NDIM> VB;
+    constexpr int B0 = VB::B0, NB = VB::NB, SW = 32 / LS;
+    constexpr int KEEP = SW >= NB ? 1 : NB / SW;
+    const Geom<R>& g = p.g;
+    const int slot = lane / LS, coil = lane % LS;
+    const int c0 = chunk * LS, nc = min(LS, p.coils - c0);
+    int b0, b1, b2;
+    block_origin_of(p, blk, b0, b1, b2);
+    const bool direct = scratch_slot < 0;
+    if (direct && p.apply_pb && !zero) {
+        C ph = cmake<R>((R)1, (R)0);
+        if (lane < NB) {
+            int k[3] = {org[0] + b0 + lane % B0, org[1] + b1 + lane / B0, org[2] + b2};
+            if (k[0] < g.K[0] && (NDIM < 2 || k[1] < g.K[1]) && (NDIM < 3 || k[2] < g.K[2])) ph = phase_before(g, k);
+        }
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            C w;
+            w.x = __shfl_sync(0xffffffffu, ph.x, q0 + i);
+            w.y = __shfl_sync(0xffffffffu, ph.y, q0 + i);
+            acc[i] = cmulc(acc[i], w);
+        }
+    }
+    if (coil >= nc || (SW > NB && (slot >> 4))) return;
+    const bool vec_ok = sizeof(R) == 4 && (g.K[0] % 2) == 0 && (g.gsp % 2) == 0 && (g.gs1 % 2) == 0 &&
+                        (g.gs2 % 2) == 0;
+    constexpr int STEP = KEEP >= 2 ? 2 : 1;
+#pragma unroll
+    for (int i = 0; i < KEEP; i += STEP) {
+        const int q = q0 + i;
+        const int l0 = b0 + q % B0, l1 = b1 + q / B0, l2 = b2;
+        const bool row_in = (NDIM < 2 || org[1] + l1 < g.K[1]) && (NDIM < 3 || org[2] + l2 < g.K[2]);
+        const bool in0 = row_in && org[0] + l0 < g.K[0];
+        const bool in1 = STEP == 2 && row_in && org[0] + l0 + 1 < g.K[0];
+        C* dst;
+        if (direct) {
+            const int64_t gi = ((int64_t)f * p.coils + c0 + coil) * g.gsp + (org[0] + l0) +
+                               (int64_t)(org[1] + l1) * g.gs1 + (int64_t)(org[2] + l2) * g.gs2;
+            if ((in0 || in1) && !GBN_INB(g.check, gi >= 0 && gi + (in1 ? 1 : 0) < g.grid_elems, CHK_GRID_WRITE))
+                continue;
+            dst = p.grid + gi;
+        } else {
+            const int64_t cell = l0 + (int64_t)g.T[0] * (l1 + (int64_t)g.T[1] * l2);
+            const int64_t si = (((int64_t)scratch_slot * p.chunks + chunk) * LS + coil) * p.tile_cells + cell;
+            if ((in0 || in1) && !GBN_INB(g.check, si >= 0 && si + (in1 ? 1 : 0) < p.scratch_elems, CHK_SCRATCH))
+                continue;
+            dst = p.scratch + si;
+        }
+        if (in0 && in1 && vec_ok && direct) {
+            store_pair(dst, acc[i], acc[i + STEP - 1]);
+        } else {
+            if (in0) dst[0] = acc[i];
+            if (in1) dst[1] = acc[i + STEP - 1];
+        }
+    }
+}
+
+// ---- values read in place: one (item, block) per warp ---------------------------
+//
+// Up to four coil lanes, and wider batches of calls that may not allocate
+// the coil-minor values.  U visits per slot are in flight at a time.
+constexpr int VISIT_THREADS = 128;   // four (item, block) units per CTA
+
+template <typename R, int NDIM, bool CX, int LS, bool TAB>
+__global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const VisitParams<R> p) {
+    typedef typename Cx<R>::T C;
+    typedef VisitBlock<NDIM> VB;
+    constexpr int NB = VB::NB, NC = VB::NC * (CX ? 2 : 1), B1 = NDIM > 1 ? VB::B1 : 1;
+    constexpr int SW = 32 / LS;
+    // visits in flight per slot, fewer the more registers one takes
+    constexpr int WORDS = (int)sizeof(R) / 4 * (CX ? 2 : 1) * (NDIM == 1 ? 2 : 1);
+    constexpr int U = WORDS > 2 || SW > 8 || TAB ? 1 : (WORDS > 1 || SW > 4 ? 2 : 4);
+    const Geom<R>& g = p.g;
+    const int lane = threadIdx.x & 31;
+    const unsigned unit = blockIdx.x * (VISIT_THREADS / 32) + (threadIdx.x >> 5);
+    if (unit >= (unsigned)(p.nitems * p.nblk)) return;   // whole warps only; no barrier below
+    const int item = (int)(unit / (unsigned)p.nblk), blk = (int)(unit - (unsigned)item * p.nblk);
+    const int chunk = blockIdx.y;
+    const int4 it = p.items[item];
+    const int2 part = p.parts[item];
+    const int f = it.x;
+    const int64_t st = p.start[unit];
+    const int n = (int)(min(p.start[unit + 1], (long long)p.nvisits) - st);
+    if (!GBN_INB(g.check, st >= 0 && n >= 0, CHK_LIST)) return;
+    const int c0 = chunk * LS;
+    const int nc = min(LS, p.coils - c0);
+    const int slot = lane / LS, coil = lane % LS;
+
+    const int64_t fo = p.foff[f];
+    const int Mf = (int)(p.foff[f + 1] - fo);
+    // samples of this lane's coil (lanes past the last coil repeat it)
+    const C* yb = p.y + fo * p.coils + (int64_t)(c0 + min(coil, nc - 1)) * Mf;
+    const C* ph = p.ph ? p.ph + fo : nullptr;
+    int b0, b1, b2;
+    block_origin_of(p, blk, b0, b1, b2);
+
+    C acc[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) acc[q] = cmake<R>((R)0, (R)0);
+    const int* vidx = p.vidx + st;
+    for (int i0 = 0; i0 < n; i0 += U * SW) {
+        // past the last visit, and for padding, the value is zero by selection:
+        // an infinity or NaN must not meet a zero coefficient
+        int id[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * SW + slot;
+            id[u] = i < n ? vidx[i] : -1;
+        }
+        C v[U], w[U];
+        R co[U][NC];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (TAB) {
+                const int64_t e = max(id[u], 0);
+                id[u] = id[u] < 0 ? -1 : p.s.idx[e];
+                const short4 ls = p.s.ls[e];
+#pragma unroll
+                for (int k = 0; k < VB::NC; ++k) {
+                    const C c = visit_coef<R, NDIM, CX>(g, p.s, e, ls, 0, nullptr, nullptr, b0, b1, b2, k);
+                    if (CX) {
+                        co[u][2 * k] = c.x;
+                        co[u][2 * k + (CX ? 1 : 0)] = c.y;
+                    } else {
+                        co[u][k] = c.x;
+                    }
+                }
+            } else {
+                load_run(p.vco + (st + min(i0 + u * SW + slot, n - 1)) * NC, co[u]);
+            }
+            const int m = max(id[u], 0);
+            v[u] = cmake<R>((R)0, (R)0);
+            if (GBN_INB(g.check, m < Mf, CHK_SAMPLE_READ)) v[u] = yb[m];
+            if (ph) w[u] = ph[m];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (ph) v[u] = cmulc(v[u], w[u]);
+            if (id[u] < 0) v[u] = cmake<R>((R)0, (R)0);
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < B1; ++k1)
+#pragma unroll
+            for (int u = 0; u < U; ++u) add_row<R, NDIM, CX>(acc, v[u], co[u], k1);
+    }
+    const int q0 = combine_slots<R, LS, NB>(acc, slot);
+    int org[3] = {0, 0, 0};
+    tile_origin<NDIM>(it.y, g.nt, g.T, org);
+    flush_block<R, NDIM, LS>(p, acc, q0, lane, f, org, blk, part.x, chunk, n == 0);
+}
+
+// ---- coil-minor values: a warp streams visits through a shared-memory ring ------
+//
+// The visits of an item's blocks lie one after another, so a warp runs over
+// a whole range of them, blocks in turn, with the copies (values and
+// coefficients, cp.async into the warp's own ring, no barrier) running
+// STAGES - 1 stages ahead across block boundaries: with loads into registers
+// the same sums waited 58% of the time on the four visits a lane could hold.
+//
+// An item of many entries is shared by the eight warps of a CTA, each taking
+// an equal run of the visits wherever the block boundaries fall (a block cut
+// by a run's end is completed by the warp that began it, from shared
+// memory, in warp order); lighter items go one to a warp, eight to a CTA.
+// Sharing costs a barrier and, where blocks are cut, an exchange; not sharing
+// leaves the last warps alone with the heavy tiles of the k-space centre.
+constexpr int STREAM_WARPS = 8;
+
+template <typename R, int NDIM, bool CX, int LS>
+struct StreamLayout {
+    typedef typename Cx<R>::T C;
+    static constexpr int NC = VisitBlock<NDIM>::NC * (CX ? 2 : 1);
+    static constexpr int VROW = LS * (int)sizeof(C);            // bytes of one visit's values
+    static constexpr int VBYTES = 2048;                         // values of a stage
+    static constexpr int RV = VBYTES / VROW;                    // visits per stage
+    static constexpr int CBYTES = RV * NC * (int)sizeof(R);     // coefficients of a stage
+    static constexpr int STAGE = VBYTES + CBYTES;
+    static constexpr int HEAD = 16 * LS * (int)sizeof(C);       // one combined block
+    static constexpr int WARP = 2 * STAGE + HEAD;
+    static constexpr int SMEM = STREAM_WARPS * WARP;
+    static_assert(RV % 4 == 0 && RV <= 32 && VROW <= 512 && STAGE % 16 == 0, "stage layout");
+};
+
+template <typename R, int NDIM, bool CX, int LS, bool TAB>
+__global__ void __launch_bounds__(32 * STREAM_WARPS, sizeof(R) == 4 && !CX ? (LS == 32 ? 2 : 3) : 1)
+spread_stream_kernel(const VisitParams<R> p) {
+    typedef typename Cx<R>::T C;
+    typedef VisitBlock<NDIM> VB;
+    typedef StreamLayout<R, NDIM, CX, LS> SL;
+    constexpr int NB = VB::NB, NC = SL::NC, B1 = NDIM > 1 ? VB::B1 : 1, SW = 32 / LS, RV = SL::RV;
+    constexpr int KEEP = NB / SW;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Geom<R>& g = p.g;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool shared_item = (int)blockIdx.x < p.nshared;
+    const int item = shared_item ? (int)blockIdx.x
+                                 : p.nshared + ((int)blockIdx.x - p.nshared) * STREAM_WARPS + warp;
+    if (item >= p.nitems) return;   // only in a CTA of unshared items: no barrier there
+    const int chunk = blockIdx.y;
+    const int4 it = p.items[item];
+    const int part = p.parts[item].x;
+    const int f = it.x;
+    const int c0 = chunk * LS;
+    const int slot = lane / LS, coil = lane % LS;
+    unsigned char* ring = smem_raw + warp * SL::WARP;
+    C* head = reinterpret_cast<C*>(ring + 2 * SL::STAGE);
+
+    // visit offsets of the item's blocks: lane b holds block b's, from base on
+    const int nblk = p.nblk;
+    const long long* st = p.start + (int64_t)item * nblk;
+    const long long base = st[0];
+    const int rel = (int)(min(st[min(lane, nblk)], (long long)p.nvisits) - base);
+    const int N = __shfl_sync(0xffffffffu, rel, nblk);
+    // this warp's run [lo, hi): the whole item, or its share; whole blocks
+    // where the largest is close enough to an equal share
+    int lo = 0, hi = N, per = N;
+    bool whole = false;
+    if (shared_item) {
+        per = ((N + STREAM_WARPS - 1) / STREAM_WARPS + 3) & ~3;
+        const int nxt = __shfl_down_sync(0xffffffffu, rel, 1);
+        const int most = __reduce_max_sync(0xffffffffu, (unsigned)(lane < nblk ? nxt - rel : 0));
+        whole = most <= per + 8 * SW;
+        lo = whole ? __shfl_sync(0xffffffffu, rel, min(warp, nblk)) : min(N, warp * per);
+        hi = whole ? __shfl_sync(0xffffffffu, rel, min(warp + 1, nblk)) : min(N, (warp + 1) * per);
+    }
+    const int64_t fo = p.foff[f];
+    const int Mf = (int)(p.foff[f + 1] - fo);
+    int org[3] = {0, 0, 0};
+    tile_origin<NDIM>(it.y, g.nt, g.T, org);
+
+    // ---- copies: stage k holds visits lo + k RV ... of the run -----------------
+    // A lane copies 16 bytes at a fixed place of every (512 / VROW)-th visit.
+    const int row_bytes = p.row * (int)sizeof(C);
+    const int off = lane * 16 % SL::VROW;
+    const bool lane_ok = c0 * (int)sizeof(C) + off < row_bytes;
+    const char* vsrc = reinterpret_cast<const char*>(p.vals + fo * p.row + c0) + (lane_ok ? off : 0);
+    const int* isrc = p.vidx + base + lo + lane;
+    const char* csrc = reinterpret_cast<const char*>(p.vco + (base + lo) * NC) + lane * 16;
+    int to_load = hi - lo - lane;                        // this lane's visits not yet read
+    int to_copy = (hi - lo) * NC * (int)sizeof(R) - lane * 16;   // coefficient bytes not yet copied
+    int issued = 0;                                      // visits whose copies were issued
+    // index of the visit this lane reads for the stage to come (-1: none)
+    auto load_id = [&]() {
+        const int id = lane < RV && to_load > 0 ? *isrc : -1;
+        isrc += RV;
+        to_load -= RV;
+        return id;
+    };
+    auto issue = [&](unsigned char* sb, int id) {
+        if (issued < hi - lo) {
+            const int e_mine = id;
+            if (TAB) id = id < 0 ? -1 : p.s.idx[id];
+            // no copy of a sample out of range, nor past the last coil: zeros
+            if (!GBN_INB(g.check, id < Mf, CHK_SAMPLE_READ)) id = -1;
+#pragma unroll
+            for (int j = 0; j < SL::VBYTES / 512; ++j) {
+                const int m = __shfl_sync(0xffffffffu, id, lane * 16 / SL::VROW + j * (512 / SL::VROW));
+                const bool ok = m >= 0 && lane_ok;
+                cp_async16_zfill(sb + lane * 16 + j * 512, vsrc + (ok ? (int64_t)m * row_bytes : 0), ok);
+            }
+            if (TAB) {
+                R* cb = reinterpret_cast<R*>(sb + SL::VBYTES);
+                for (int q = lane; q - lane < RV * VB::NC; q += 32) {
+                    const int vi = q / VB::NC, k1 = q - vi * VB::NC;
+                    const int e = __shfl_sync(0xffffffffu, e_mine, min(vi, RV - 1));
+                    if (vi < RV && e >= 0) {
+                        int blk = 0;   // the block this visit belongs to
+                        for (int b = 1; b < nblk; ++b) blk += (int)(st[b] - base) <= lo + issued + vi;
+                        int b0, b1, b2;
+                        block_origin_of(p, blk, b0, b1, b2);
+                        const C c = visit_coef<R, NDIM, CX>(g, p.s, e, p.s.ls[e], 0, nullptr, nullptr, b0, b1, b2, k1);
+                        if (CX) {
+                            cb[2 * q] = c.x;
+                            cb[2 * q + 1] = c.y;
+                        } else {
+                            cb[q] = c.x;
+                        }
+                    } else if (vi < RV) {
+                        cb[(CX ? 2 : 1) * q] = (R)0;
+                        if (CX) cb[2 * q + 1] = (R)0;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < SL::CBYTES; q += 512) {
+                    if (SL::CBYTES - q < 512 && lane * 16 >= SL::CBYTES - q) break;
+                    const bool ok = q < to_copy;
+                    cp_async16_zfill(sb + SL::VBYTES + lane * 16 + q,
+                                     ok ? csrc + q : reinterpret_cast<const char*>(p.vco), ok);
+                }
+                csrc += SL::CBYTES;
+                to_copy -= SL::CBYTES;
+            }
+            issued += RV;
+        }
+        cp_async_commit();
+    };
+    int id = load_id();
+    {
+        const int nx = load_id();
+        issue(ring, id);
+        id = nx;
+    }
+
+    C acc[NB];
+    const unsigned char* sb = ring + SL::STAGE;   // the stage being read (none yet)
+    const C* vp = nullptr;
+    const R* cp = nullptr;
+    int left = 0, pos = lo;                       // visits left in it; next visit of the run
+    int pending = -1, pending_end = 0, q_pending = 0;
+    for (int b = 0; b < nblk; ++b) {
+        const int rb = __shfl_sync(0xffffffffu, rel, b), re = __shfl_sync(0xffffffffu, rel, b + 1);
+        const bool owned = shared_item ? (whole ? b == warp
+                                                : lo <= rb && (rb < hi || warp == STREAM_WARPS - 1))
+                                       : true;
+        const int end = min(re, hi);
+        if (!owned && max(rb, lo) >= end) continue;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) acc[q] = cmake<R>((R)0, (R)0);
+        while (pos < end) {
+            if (left == 0) {
+                // the next stage has landed, for every lane; the buffer just
+                // read takes the one after it
+                cp_async_wait_all();
+                __syncwarp();
+                const int nx = load_id();
+                unsigned char* done = const_cast<unsigned char*>(sb);
+                sb = sb == ring ? ring + SL::STAGE : ring;
+                issue(done, id);
+                id = nx;
+                left = RV;
+                vp = reinterpret_cast<const C*>(sb) + slot * LS + coil;
+                cp = reinterpret_cast<const R*>(sb + SL::VBYTES) + slot * NC;
+            }
+            const int n = min(end - pos, left);
+            pos += n;
+            left -= n;
+            // groups of four visits (blocks begin and end on whole groups)
+#pragma unroll 1
+            for (int q = n; q > 0; q -= 4) {
+                unsigned rows = 0xffffu;
+                if (NDIM > 1 && !CX && SW == 1) {
+                    // one visit at a time: bit 4 u + k1 is set where visit u's
+                    // window covers row k1; the warp skips the others
+                    rows = __ballot_sync(0xffffffffu,
+                                         lane < 16 && !is_neg_zero(cp[(lane >> 2) * NC + NC - B1 + (lane & 3)]));
+                }
+#pragma unroll
+                for (int u = 0; u < 4 / SW; ++u) {
+                    const C v = vp[u * 32];
+                    R co[NC];
+                    load_run(cp + u * SW * NC, co);
+#pragma unroll
+                    for (int k1 = 0; k1 < B1; ++k1)
+                        if (!(NDIM > 1 && !CX && SW == 1) || (rows >> (4 * u + k1) & 1))
+                            add_row<R, NDIM, CX>(acc, v, co, k1);
+                }
+                vp += 4 * LS;
+                cp += 4 * NC;
+            }
+        }
+        const int q0 = combine_slots<R, LS, NB>(acc, slot);
+        if (!owned) {   // begun by an earlier warp: hand it over
+#pragma unroll
+            for (int i = 0; i < KEEP; ++i) head[(q0 + i) * LS + coil] = acc[i];
+        } else if (re > hi) {   // continued by later warps (the last block of the run)
+            pending = b;
+            pending_end = re;
+            q_pending = q0;
+        } else {
+            flush_block<R, NDIM, LS>(p, acc, q0, lane, f, org, b, part, chunk, re == rb);
+        }
+    }
+    if (!shared_item || whole) return;   // the same for the whole CTA
+    __syncthreads();
+    if (pending >= 0) {
+        for (int w = warp + 1; w < STREAM_WARPS && w * per < pending_end; ++w) {
+            const C* h = reinterpret_cast<const C*>(smem_raw + w * SL::WARP + 2 * SL::STAGE);
+#pragma unroll
+            for (int i = 0; i < KEEP; ++i) acc[i] = cadd(acc[i], h[(q_pending + i) * LS + coil]);
+        }
+        flush_block<R, NDIM, LS>(p, acc, q_pending, lane, f, org, pending, part, chunk, false);
+    }
+}
+
+// ---- launchers -----------------------------------------------------------------
+
+template <typename R>
+cudaError_t launch_visit_count(const VisitBuildParams<R>& p, cudaStream_t s) {
+    if (p.nitems == 0) return cudaSuccess;
+    const int threads = 32 * p.nblk;
+    switch (p.g.ndim) {
+        case 1: visit_count_kernel<R, 1><<<p.nitems, threads, 0, s>>>(p); break;
+        case 2: visit_count_kernel<R, 2><<<p.nitems, threads, 0, s>>>(p); break;
+        case 3: visit_count_kernel<R, 3><<<p.nitems, threads, 0, s>>>(p); break;
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t launch_visit_fill(const VisitBuildParams<R>& p, cudaStream_t s) {
+    if (p.nitems == 0) return cudaSuccess;
+    const int threads = 32 * p.nblk;
+    switch (p.g.ndim * 2 + (p.cx ? 1 : 0)) {
+        case 2: visit_fill_kernel<R, 1, false><<<p.nitems, threads, 0, s>>>(p); break;
+        case 3: visit_fill_kernel<R, 1, true><<<p.nitems, threads, 0, s>>>(p); break;
+        case 4: visit_fill_kernel<R, 2, false><<<p.nitems, threads, 0, s>>>(p); break;
+        case 5: visit_fill_kernel<R, 2, true><<<p.nitems, threads, 0, s>>>(p); break;
+        case 6: visit_fill_kernel<R, 3, false><<<p.nitems, threads, 0, s>>>(p); break;
+        case 7: visit_fill_kernel<R, 3, true><<<p.nitems, threads, 0, s>>>(p); break;
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t launch_values(const ValuesParams<R>& p, cudaStream_t s) {
+    if (p.M == 0 || p.coils == 0) return cudaSuccess;
+    const int64_t bx = (p.M + VAL_SAMPLES - 1) / VAL_SAMPLES;
+    const int64_t by = (p.coils + VAL_COILS - 1) / VAL_COILS;
+    if (bx > INT32_MAX || by > 65535) return cudaErrorInvalidValue;
+    values_kernel<R><<<dim3((unsigned)bx, (unsigned)by), 256, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+template <typename R, int NDIM, bool CX, int LS, bool TAB>
+cudaError_t stream_launch(const VisitParams<R>& p0, cudaStream_t s) {
+    VisitParams<R> p = p0;
+    // An item goes to one warp up to 32 entries per slot (a longer one would
+    // outlast the rest of a small launch), more where each of the device's
+    // warps has many times that to do anyway.
+    const int64_t load = p.s.len * p.chunks / (3 * STREAM_WARPS * 152) / 8;
+    int q = LS >= 32 ? 0 : LS >= 16 ? 1 : 2;
+    while (q < SPREAD_HEAVY_LEVELS - 1 && (SPREAD_SHARE_ENTRIES << q) < load) ++q;
+    p.nshared = p.nheavy[q];
+    const int64_t ctas = p.nshared + ((int64_t)p.nitems - p.nshared + STREAM_WARPS - 1) / STREAM_WARPS;
+    if (ctas > INT32_MAX || p.chunks > 65535) return cudaErrorInvalidValue;
+    constexpr size_t smem = StreamLayout<R, NDIM, CX, LS>::SMEM;
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(spread_stream_kernel<R, NDIM, CX, LS, TAB>), smem);
+    if (e != cudaSuccess) return e;
+    spread_stream_kernel<R, NDIM, CX, LS, TAB>
+        <<<dim3((unsigned)ctas, (unsigned)p.chunks), 32 * STREAM_WARPS, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
+template <typename R, int NDIM, bool CX, int LS, bool TAB>
+cudaError_t unit_launch(const VisitParams<R>& p, cudaStream_t s) {
+    const int64_t units = (int64_t)p.nitems * p.nblk;
+    const int64_t ctas = (units + VISIT_THREADS / 32 - 1) / (VISIT_THREADS / 32);
+    if (units > INT32_MAX || p.chunks > 65535) return cudaErrorInvalidValue;
+    spread_unit_kernel<R, NDIM, CX, LS, TAB><<<dim3((unsigned)ctas, (unsigned)p.chunks), VISIT_THREADS, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+template <typename R, int NDIM, bool CX, bool TAB>
+cudaError_t visit_lanes(const VisitParams<R>& p, cudaStream_t s) {
+    switch (p.LS) {
+        case 1: return unit_launch<R, NDIM, CX, 1, TAB>(p, s);
+        case 2: return unit_launch<R, NDIM, CX, 2, TAB>(p, s);
+        case 4: return unit_launch<R, NDIM, CX, 4, TAB>(p, s);
+        case 8: return p.vals ? stream_launch<R, NDIM, CX, 8, TAB>(p, s) : unit_launch<R, NDIM, CX, 8, TAB>(p, s);
+        case 16: return p.vals ? stream_launch<R, NDIM, CX, 16, TAB>(p, s) : unit_launch<R, NDIM, CX, 16, TAB>(p, s);
+        case 32: return p.vals ? stream_launch<R, NDIM, CX, 32, TAB>(p, s) : unit_launch<R, NDIM, CX, 32, TAB>(p, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <typename R, int NDIM, bool CX>
+cudaError_t visit_any(const VisitParams<R>& p, cudaStream_t s) {
+    return p.vco ? visit_lanes<R, NDIM, CX, false>(p, s) : visit_lanes<R, NDIM, CX, true>(p, s);
+}
+
+template <typename R>
+cudaError_t launch_spread_visits(const VisitParams<R>& p0, cudaStream_t s) {
+    if (p0.nitems == 0 || p0.coils == 0) return cudaSuccess;
+    VisitParams<R> p = p0;
+    if (p.nblk < 1 || p.nblk > 8) return cudaErrorInvalidValue;
+    for (int b = 0; b < p.nblk; ++b) {
+        int b0, b1, b2;
+        if (p.g.ndim == 1) block_origin<1>(p.g, b, b0, b1, b2);
+        else if (p.g.ndim == 2) block_origin<2>(p.g, b, b0, b1, b2);
+        else block_origin<3>(p.g, b, b0, b1, b2);
+        p.borg[b] = make_short4((short)b0, (short)b1, (short)b2, 0);
+    }
+    const bool cx = p.g.hi[0] != nullptr;
+    switch (p.g.ndim * 2 + (cx ? 1 : 0)) {
+        case 2: return visit_any<R, 1, false>(p, s);
+        case 3: return visit_any<R, 1, true>(p, s);
+        case 4: return visit_any<R, 2, false>(p, s);
+        case 5: return visit_any<R, 2, true>(p, s);
+        case 6: return visit_any<R, 3, false>(p, s);
+        case 7: return visit_any<R, 3, true>(p, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace gbn
