@@ -241,8 +241,13 @@ gather_kernel(const GatherParams<R> p) {
     int pidx = -1;                          // held output, waiting for its pair
     C pacc = cmake<R>((R)0, (R)0);
 
-    for (int base = warp * 32; base < count; base += nwarps * 32) {
-        const int nb = min(32, count - base);
+    // an equal share of the samples per warp (whole rounds of SW): items hold
+    // some 70 to 100 samples at the workloads here, which in turns of 32 per
+    // warp occupied three of the eight warps
+    const int share = ((count + nwarps - 1) / nwarps + SW - 1) / SW * SW;
+    const int last = min(count, (warp + 1) * share);
+    for (int base = warp * share; base < last; base += 32) {
+        const int nb = min(32, last - base);
         R mcr[NDIM][JL], mci[NDIM][JL];
         int mbase = 0;  // shared-memory index of the window's first cell
         int mx0 = 0;    // region x-position of the window's first cell
