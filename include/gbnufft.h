@@ -241,10 +241,13 @@ int gbn_grad_tm(gbn_plan* plan, const void* grid, const void* gy,
                 const double* phase_shift, void* gtm, int coils, void* stream);
 
 /* Device pointer of the plan's forward grid buffer (valid until the next
- * call on the plan).  Its layout is the transform's own: [K1][coils][K0] for
- * 2-D plans (row k1 of every coil plane together, so the FFT's row pass skips
- * the zero-padded rows), [coils][K...] for 1-D and 3-D plans.  The
- * interpolation-only entry points keep the [planes][K...] layout.           */
+ * call on the plan).  Its layout is the transform's own: coil-minor,
+ * [K_{ndim-1}]...[K_0][coils] per frame, for single-precision 2-D and 3-D
+ * plans whose every axis length the library's FFT passes implement (see
+ * GBN_FLAG_CUFFT_ONLY), else [K1][coils][K0] for 2-D plans and [coils][K...]
+ * for 1-D and 3-D ones.  A plan with derivative tables keeps it as
+ * gbn_grad_tm takes it, from before phase_before.  The interpolation-only
+ * entry points keep the [planes][K...] layout.                              */
 int gbn_forward_grid(gbn_plan* plan, void** grid);
 
 /* Exact direct NUDFT in double precision on the GPU (the reference's

@@ -29,6 +29,7 @@
 // other lengths and double precision run the pass through cuFFT.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "gbn_device.cuh"
@@ -43,8 +44,11 @@ namespace {
 // separate instantiation: with the second term in every kernel the 2-D
 // 512-point pass compiled to 86 instead of 80 registers, two 256-thread CTAs
 // per SM instead of three, and ran 40% slower.
-template <int L1, int L2, int CF_TC, int SIGN, bool Z>
-__global__ void __launch_bounds__(CF_TC * L1) colfft_kernel(const ColFftParams p) {
+// PH (forward): phase_before applied to the outputs, so that the gather copies
+// grid cells as they are.  (The inverse takes it in the spread's writes: here,
+// on 32 loaded values, it cost the 512-point pass 140 instead of 80 registers.)
+template <int L1, int L2, int CF_TC, int SIGN, bool Z, bool PH>
+__global__ void __launch_bounds__(CF_TC * L1, 2) colfft_kernel(const ColFftParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sm = reinterpret_cast<float2*>(smem_raw);
     const int64_t c0 = (int64_t)blockIdx.x * CF_TC;
@@ -81,6 +85,16 @@ __global__ void __launch_bounds__(CF_TC * L1) colfft_kernel(const ColFftParams p
 #pragma unroll
         for (int n1 = 0; n1 < L1; ++n1) u[n1] = sm[(k2 * L1 + n1) * CF_TC + col];
         stockham<L1, 1, SIGN>(u);
+        if (PH && c < p.S) {
+            const unsigned cells = (unsigned)p.S / (unsigned)p.coils;
+            const float2* ph = p.phase + (unsigned)c / (unsigned)p.coils;
+#pragma unroll
+            for (int k1 = 0; k1 < L1; ++k1) u[k1] = cmul(u[k1], __ldg(ph + (int64_t)(k2 + L2 * k1) * cells));
+            if (p.div != 1.f) {
+#pragma unroll
+                for (int k1 = 0; k1 < L1; ++k1) u[k1] = make_float2(u[k1].x / p.div, u[k1].y / p.div);
+            }
+        }
 #pragma unroll
         for (int k1 = 0; k1 < L1; ++k1) {
             const int k = k2 + L2 * k1;
@@ -92,29 +106,41 @@ __global__ void __launch_bounds__(CF_TC * L1) colfft_kernel(const ColFftParams p
 
 // CF_TC columns per CTA: 16 (128-byte row segments), 8 for 32-point second
 // stages (a 256-thread CTA, so that the 32-point transforms need no spills).
-template <int L1, int L2, int CF_TC>
-cudaError_t colfft_launch(const ColFftParams& p, int sign, cudaStream_t s) {
-    constexpr int L = L1 * L2;
-    const size_t smem = (size_t)CF_TC * L * sizeof(float2);
-    const bool z = p.planes2 > 1;
-    const void* k = sign < 0 ? (z ? reinterpret_cast<const void*>(colfft_kernel<L1, L2, CF_TC, -1, true>)
-                                  : reinterpret_cast<const void*>(colfft_kernel<L1, L2, CF_TC, -1, false>))
-                             : (z ? reinterpret_cast<const void*>(colfft_kernel<L1, L2, CF_TC, 1, true>)
-                                  : reinterpret_cast<const void*>(colfft_kernel<L1, L2, CF_TC, 1, false>));
-    cudaError_t e = ensure_dynamic_smem(k, smem);
+template <int L1, int L2, int CF_TC, int SIGN, bool Z, bool PH>
+cudaError_t colfft_run(const ColFftParams& p, cudaStream_t s) {
+    const size_t smem = (size_t)CF_TC * L1 * L2 * sizeof(float2);
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(colfft_kernel<L1, L2, CF_TC, SIGN, Z, PH>), smem);
     if (e != cudaSuccess) return e;
     const int64_t ctas = (p.S + CF_TC - 1) / CF_TC;
-    if (ctas > INT32_MAX || p.planes > 65535 || p.planes2 > 65535) return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)ctas, (unsigned)p.planes, (unsigned)p.planes2);
-    if (sign < 0 && z)
-        colfft_kernel<L1, L2, CF_TC, -1, true><<<grid, CF_TC * L1, smem, s>>>(p);
-    else if (sign < 0)
-        colfft_kernel<L1, L2, CF_TC, -1, false><<<grid, CF_TC * L1, smem, s>>>(p);
-    else if (z)
-        colfft_kernel<L1, L2, CF_TC, 1, true><<<grid, CF_TC * L1, smem, s>>>(p);
-    else
-        colfft_kernel<L1, L2, CF_TC, 1, false><<<grid, CF_TC * L1, smem, s>>>(p);
+    if (ctas > INT32_MAX) return cudaErrorInvalidValue;
+    // grid.y and grid.z hold 65535 arrays each
+    for (int z = 0; z < p.planes2; z += 65535)
+        for (int y = 0; y < p.planes; y += 65535) {
+            ColFftParams q = p;
+            const int64_t off = y * p.ps + z * p.ps2;
+            q.in += off;
+            q.out += off;
+            q.in_elems -= off;
+            q.out_elems -= off;
+            const dim3 grid((unsigned)ctas, (unsigned)std::min(p.planes - y, 65535),
+                            (unsigned)std::min(p.planes2 - z, 65535));
+            colfft_kernel<L1, L2, CF_TC, SIGN, Z, PH><<<grid, CF_TC * L1, smem, s>>>(q);
+        }
     return cudaGetLastError();
+}
+
+// The phase goes with the last axis, which has one array stride.
+template <int L1, int L2, int CF_TC>
+cudaError_t colfft_launch(const ColFftParams& p, int sign, cudaStream_t s) {
+    if (p.phase) {
+        if (sign > 0 || p.planes2 > 1 || p.coils < 1 || p.S > INT32_MAX) return cudaErrorInvalidValue;
+        return colfft_run<L1, L2, CF_TC, -1, false, true>(p, s);
+    }
+    if (p.planes2 > 1)
+        return sign < 0 ? colfft_run<L1, L2, CF_TC, -1, true, false>(p, s)
+                        : colfft_run<L1, L2, CF_TC, 1, true, false>(p, s);
+    return sign < 0 ? colfft_run<L1, L2, CF_TC, -1, false, false>(p, s)
+                    : colfft_run<L1, L2, CF_TC, 1, false, false>(p, s);
 }
 
 }  // namespace

@@ -81,6 +81,7 @@ __device__ __forceinline__ int first_tap(R t, int J) {
 // (mrrt/nufft/_nufft.py:703-715).
 template <typename R>
 __device__ __forceinline__ typename Cx<R>::T phase_before(const Geom<R>& g, const int* k) {
+    if (g.ptab) return g.ptab[k[0] + (int64_t)g.K[0] * (k[1] + (int64_t)g.K[1] * k[2])];
     R ph[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d)

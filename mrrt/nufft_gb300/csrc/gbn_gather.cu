@@ -122,7 +122,7 @@ gather_kernel(const GatherParams<R> p) {
     const int Rtot = region_dims(g, NDIM, Rd);
 
     // ---- stage tile + halo for nc coils --------------------------------------
-    const C* gb = p.grid + ((int64_t)f * p.coils + c0) * g.gsp;
+    const C* gb = p.grid + f * g.gsf + c0 * g.gsp;
     if constexpr (ES) {
         // (1) thread per cell: grid offset and phase_before into shared
         // memory; (2) thread per (coil, cell), consecutive threads on
@@ -141,7 +141,7 @@ gather_kernel(const GatherParams<R> p) {
             int k[3] = {0, 0, 0};
 #pragma unroll
             for (int d = 0; d < NDIM; ++d) k[d] = wrapk(org[d] + r[d], g.K[d]);
-            soff[cell] = k[0] + (int64_t)k[1] * g.gs1 + (int64_t)k[2] * g.gs2;
+            soff[cell] = k[0] * g.gs0 + (int64_t)k[1] * g.gs1 + (int64_t)k[2] * g.gs2;
             if (p.apply_pb) sph[cell] = phase_before(g, k);
         }
         __syncthreads();
@@ -157,7 +157,7 @@ gather_kernel(const GatherParams<R> p) {
                 cc[u] = c;
                 cl[u] = cell;
                 if (e + u * step < E) {
-                    const int64_t gi = ((int64_t)f * p.coils + c0 + c) * g.gsp + soff[cell];
+                    const int64_t gi = f * g.gsf + (c0 + c) * g.gsp + soff[cell];
                     if (GBN_INB(g.check, gi >= 0 && gi < g.grid_elems, CHK_GRID_READ))
                         v[u] = gb[(int64_t)c * g.gsp + soff[cell]];
                 }
@@ -189,7 +189,7 @@ gather_kernel(const GatherParams<R> p) {
         int k[3] = {0, 0, 0};
 #pragma unroll
         for (int d = 0; d < NDIM; ++d) k[d] = wrapk(org[d] + r[d], g.K[d]);
-        const int64_t off = k[0] + (int64_t)k[1] * g.gs1 + (int64_t)k[2] * g.gs2;
+        const int64_t off = k[0] * g.gs0 + (int64_t)k[1] * g.gs1 + (int64_t)k[2] * g.gs2;
         C ph = cmake<R>((R)1, (R)0);
         if (p.apply_pb) ph = phase_before(g, k);
         const int dst = cell * LSP;
@@ -199,7 +199,7 @@ gather_kernel(const GatherParams<R> p) {
 #pragma unroll
             for (int u = 0; u < 4; ++u)
                 if (c + u < nc) {
-                    const int64_t gi = ((int64_t)f * p.coils + c0 + c + u) * g.gsp + off;
+                    const int64_t gi = f * g.gsf + (c0 + c + u) * g.gsp + off;
                     if (GBN_INB(g.check, gi >= 0 && gi < g.grid_elems, CHK_GRID_READ))
                         v[u] = src[(int64_t)(c + u) * g.gsp];
                 }
@@ -270,9 +270,9 @@ gather_kernel(const GatherParams<R> p) {
                 loc[d] = wrapk(kf[d], g.K[d]) - org[d];
             }
             if (p.s.cr) {
-                // precomputed coefficients: jsum contiguous values per entry
-                load_coefs<R, NDIM, JJ, JL>(p.s.cr + (int64_t)e * p.s.jsum, g, mcr);
-                if (CX) load_coefs<R, NDIM, JJ, JL>(p.s.ci + (int64_t)e * p.s.jsum, g, mci);
+                // precomputed coefficients: contiguous values per entry
+                load_coefs<R, NDIM, JJ, JL>(p.s.cr + (int64_t)e * p.s.cstride, g, mcr);
+                if (CX) load_coefs<R, NDIM, JJ, JL>(p.s.ci + (int64_t)e * p.s.cstride, g, mci);
             } else {
 #pragma unroll
                 for (int d = 0; d < NDIM; ++d)
@@ -496,6 +496,7 @@ static cudaError_t launch_generic(const GatherParams<R>& p, cudaStream_t s) {
 }
 
 static cudaError_t gather_any(const GatherParams<float>& p, cudaStream_t s) {
+    if (gather_cm_supported(p)) return launch_gather_cm(p, s);
     const bool cx = p.g.hi[0] != nullptr;
     if (!cx && (p.g.ndim == 2 || p.g.ndim == 3)) {
         bool done = false;

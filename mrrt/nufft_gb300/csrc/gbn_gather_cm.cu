@@ -1,0 +1,302 @@
+// Forward table interpolation (grid -> samples) on a coil-minor grid, for
+// real single-precision kernels of width 4, 5 or 6 and five or more coils.
+//
+// The same decomposition as gbn_gather.cu (a CTA stages a tile with its halo
+// for LS coils in shared memory and interpolates the tile's samples there).
+// What bounded it was not the interpolation: of 666 warp instructions a sample
+// at a 3-D kooshball some 560 staged cells (divisions for the cell's place, a
+// sincos for its phase, an 8-byte load, multiply and store per coil), and a
+// further 22 shuffles a sample handed its prepared coefficients round.  Here
+//   * the grid comes coil-minor and with phase_before applied (the last FFT
+//     pass does both), so staging is 16-byte asynchronous copies of whole
+//     row segments (8-byte ones for an odd coil count);
+//   * a sample's window place, output index, phase and coefficients are one
+//     plan-time record; each warp streams the records of its share of the
+//     samples through a small ring in shared memory and reads them as
+//     broadcasts;
+//   * a lane takes two adjacent coils, so the tap loop reads 16 bytes a lane.
+//     With 8 coils two groups of four lanes share a sample and take its even
+//     and odd taps along axis 0: the eight lanes of a wavefront then read two
+//     adjacent cells, all 32 banks once.
+// Bound: shared-memory bandwidth, J^d cells of LS coils per sample (72
+// wavefronts of 128 bytes at J 6, 2-D, 32 coils; 108 in 3-D with 8).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "gbn_device.cuh"
+#include "gbn_internal.h"
+
+namespace gbn {
+
+namespace {
+
+constexpr int CM_THREADS = 256, CM_WARPS = CM_THREADS / 32;
+
+template <int NDIM, int J, int LS>
+struct CmLayout {
+    static constexpr int LL = LS / 2;                       // lanes over the coils
+    static constexpr int TSP = LS == 8 ? 2 : 1;             // lane groups over a sample's taps
+    static constexpr int GL = LL * TSP;                     // lanes per sample
+    static constexpr int SW = 32 / GL;                      // samples a warp serves at a time
+    static constexpr int NC = (NDIM * J + 3) / 4 * 4;       // coefficients of a record
+    static constexpr int REC = 16 + 4 * NC;                 // bytes of a record
+    static constexpr int B = 2 * SW;                        // records per ring stage
+    static constexpr int RING = 2 * B * REC;                // bytes per warp
+};
+
+template <int CB>
+__device__ __forceinline__ void cp_async_fill(void* smem, const void* gmem, bool valid) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    const int n = valid ? CB : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(CB), "r"(n) : "memory");
+}
+
+template <int NDIM, int J, int LS, int CB>
+__global__ void __launch_bounds__(CM_THREADS) gather_cm_kernel(const GatherParams<float> p) {
+    typedef CmLayout<NDIM, J, LS> L;
+    constexpr int LL = L::LL, TSP = L::TSP, GL = L::GL, SW = L::SW, B = L::B, REC = L::REC;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Geom<float>& g = p.g;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int4 it = p.items[blockIdx.x];
+    const int f = it.x, start = it.z, count = it.w;
+    if (!GBN_INB(g.check, start >= 0 && count >= 0 && start + (int64_t)count <= p.s.len, CHK_LIST)) return;
+    const int c0 = blockIdx.y * LS;
+    const int nc = min(LS, p.coils - c0);
+    int org[3] = {0, 0, 0};
+    tile_origin<NDIM>(it.y, g.nt, g.T, org);
+    int Rd[3];
+    const int cells = region_dims(g, NDIM, Rd);
+    float4* S = reinterpret_cast<float4*>(smem_raw);                       // [cell][LS / 2] coil pairs
+    unsigned char* ring = smem_raw + (size_t)cells * LS * sizeof(float2) + warp * L::RING;
+
+    // ---- this warp's samples: an equal share, whole rounds of SW ----------------
+    const int share = ((count + CM_WARPS - 1) / CM_WARPS + SW - 1) / SW * SW;
+    const int s0 = min(count, warp * share), ns = min(count, (warp + 1) * share) - s0;
+    const char* rsrc = reinterpret_cast<const char*>(p.s.rec) + (int64_t)(start + s0) * REC;
+    auto issue_records = [&](int k) {   // stage k: records k B ... of the share
+        const int left = (ns - k * B) * REC;
+        for (int q = lane * 16; q < B * REC; q += 512)
+            if (q < left) cp_async<16>(ring + (k & 1) * (B * REC) + q, rsrc + (int64_t)k * (B * REC) + q);
+    };
+    issue_records(0);
+
+    // ---- stage the tile and its halo: a warp per row segment ----------------------
+    {
+        constexpr int PC = LS * 8 / CB;   // copies per cell
+        const char* gb = reinterpret_cast<const char*>(p.grid + f * g.gsf + c0);
+        const int nrows = Rd[1] * (NDIM > 2 ? Rd[2] : 1);
+        const int part = lane % PC * CB;
+        const bool part_ok = part < nc * 8;
+        for (int r = warp; r < nrows; r += CM_WARPS) {
+            const int y = NDIM > 2 ? r % Rd[1] : r, z = NDIM > 2 ? r / Rd[1] : 0;
+            int64_t row = (int64_t)wrapk(org[1] + y, g.K[1]) * g.gs1;
+            if (NDIM > 2) row += (int64_t)wrapk(org[2] + z, g.K[2]) * g.gs2;
+            unsigned char* dst = smem_raw + (size_t)r * Rd[0] * (LS * 8);
+            for (int q = lane; q < Rd[0] * PC; q += 32) {
+                int kx = org[0] + q / PC;
+                if (kx >= g.K[0]) kx = wrapk(kx, g.K[0]);
+                const int64_t i = row + (int64_t)kx * g.gs0;   // complex values from gb
+                const bool ok = part_ok && GBN_INB(g.check, f * g.gsf + c0 + i + (part + CB) / 8 <= g.grid_elems,
+                                                   CHK_GRID_READ);
+                cp_async_fill<CB>(dst + q * CB, ok ? gb + i * 8 + part : gb, ok);
+            }
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+
+    // ---- interpolate --------------------------------------------------------------
+    const int grp = lane / GL, th = TSP > 1 ? (lane / LL) % TSP : 0, cl = lane % LL;   // coils 2 cl, 2 cl + 1
+    const int64_t fo = p.foff[f];
+    const int Mf = (int)(p.foff[f + 1] - fo);
+    if (!GBN_INB(g.check, (fo + Mf) * p.coils <= g.sample_elems, CHK_SAMPLE_WRITE)) return;
+    // the coil this lane writes: of two lane groups, one each; else both
+    const int wc = TSP > 1 ? 2 * cl + th : 2 * cl;
+    float2* yb = p.y + fo * p.coils + (int64_t)(c0 + wc) * Mf;
+    const int rs = Rd[0] * LL, ps = Rd[0] * Rd[1] * LL;
+    constexpr int JH = (J + TSP - 1) / TSP;   // taps of a lane along axis 0
+    int pidx = -1;                            // held output (per coil), waiting for its neighbour
+    float2 pa = make_float2(0.f, 0.f), pb = make_float2(0.f, 0.f);
+    auto put = [&](float2* y, int idx, float2 held, float2 v, bool pair) {
+        if (pair)
+            store_pair(y + idx - 1, held, v);
+        else
+            y[idx] = v;
+    };
+    for (int k = 0; k * B < ns; ++k) {
+        if (k > 0) {
+            cp_async_wait_all();
+            __syncwarp();
+        }
+        if ((k + 1) * B < ns) issue_records(k + 1);
+        const unsigned char* buf = ring + (k & 1) * (B * REC);
+#pragma unroll 1
+        for (int u = 0; u < B / SW; ++u) {
+            // a lane group takes adjacent list entries in turn
+            const int e = grp * (B / SW) + u;
+            const bool on = k * B + e < ns;
+            const unsigned char* rec = buf + (on ? e : 0) * REC;
+            const int4 meta = *reinterpret_cast<const int4*>(rec);   // region cell, index, phase
+            float q[L::NC];
+#pragma unroll
+            for (int i = 0; i < L::NC; i += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(rec + 16 + 4 * i);
+                q[i] = v.x;
+                q[i + 1] = v.y;
+                q[i + 2] = v.z;
+                q[i + 3] = v.w;
+            }
+            float qx[JH];
+#pragma unroll
+            for (int j = 0; j < JH; ++j) {
+                const int j1 = j * TSP + 1;
+                qx[j] = TSP > 1 && th ? (j1 < J ? q[j1 < J ? j1 : 0] : 0.f) : q[j * TSP];
+            }
+            const float4* w = S + (meta.x + th) * LL + cl;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto add = [](float4& a, float c, const float4& v) {
+                a.x = fmaf(c, v.x, a.x);
+                a.y = fmaf(c, v.y, a.y);
+                a.z = fmaf(c, v.z, a.z);
+                a.w = fmaf(c, v.w, a.w);
+            };
+#pragma unroll
+            for (int j2 = 0; j2 < (NDIM > 2 ? J : 1); ++j2) {
+                float4 plane = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int j1 = 0; j1 < J; ++j1) {
+                    const float4* r = w + j2 * ps + j1 * rs;
+                    float4 row = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int j = 0; j < JH; ++j) {
+                        // an odd width: the odd taps are one fewer, and the cell past the
+                        // window must not enter, not even times zero
+                        if (TSP > 1 && (J & 1) && j == JH - 1) {
+                            if (th == 0) add(row, qx[j], r[j * TSP * LL]);
+                        } else {
+                            add(row, qx[j], r[j * TSP * LL]);
+                        }
+                    }
+                    add(plane, q[J + j1], row);
+                }
+                if (NDIM > 2)
+                    add(acc, q[2 * J + j2 < L::NC ? 2 * J + j2 : 0], plane);
+                else
+                    acc = plane;
+            }
+            float2 va = make_float2(acc.x, acc.y), vb = make_float2(acc.z, acc.w);
+            if (TSP > 1) {
+                // the other half's sums; each half keeps one coil
+                const float2 send = th ? va : vb, keep = th ? vb : va;
+                va.x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, LL);
+                va.y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, LL);
+            }
+            if (!on || wc >= nc) continue;
+            const int idx = meta.y;
+            if (!GBN_INB(g.check, idx >= 0 && idx < Mf, CHK_SAMPLE_WRITE)) continue;
+            if (p.apply_ph) {
+                const float2 ph = make_float2(__int_as_float(meta.z), __int_as_float(meta.w));
+                va = cmul(va, ph);
+                if (TSP == 1) vb = cmul(vb, ph);
+            }
+            // samples idx, idx + 1 (idx even) in consecutive entries leave as
+            // one 16-byte store per coil
+            const bool two = TSP == 1 && wc + 1 < nc;
+            if (pidx >= 0 && idx == pidx + 1) {
+                put(yb, idx, pa, va, (reinterpret_cast<uintptr_t>(yb + pidx) & 15) == 0);
+                if ((reinterpret_cast<uintptr_t>(yb + pidx) & 15) != 0) yb[pidx] = pa;
+                if (two) {
+                    float2* y2 = yb + Mf;
+                    const bool al = (reinterpret_cast<uintptr_t>(y2 + pidx) & 15) == 0;
+                    put(y2, idx, pb, vb, al);
+                    if (!al) y2[pidx] = pb;
+                }
+                pidx = -1;
+            } else {
+                if (pidx >= 0) {
+                    yb[pidx] = pa;
+                    if (two) yb[Mf + pidx] = pb;
+                    pidx = -1;
+                }
+                if ((idx & 1) == 0) {
+                    pidx = idx;
+                    pa = va;
+                    pb = vb;
+                } else {
+                    yb[idx] = va;
+                    if (two) yb[Mf + idx] = vb;
+                }
+            }
+        }
+    }
+    if (pidx >= 0 && wc < nc) {
+        yb[pidx] = pa;
+        if (TSP == 1 && wc + 1 < nc) yb[Mf + pidx] = pb;
+    }
+}
+
+template <int NDIM, int J, int LS, int CB>
+cudaError_t cm_launch(const GatherParams<float>& p, cudaStream_t s) {
+    int Rd[3];
+    size_t cells = 1;
+    for (int d = 0; d < NDIM; ++d) {
+        Rd[d] = p.g.T[d] + p.g.J[d] - 1;
+        cells *= (size_t)Rd[d];
+    }
+    const size_t smem = cells * LS * sizeof(float2) + CM_WARPS * (size_t)CmLayout<NDIM, J, LS>::RING;
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(gather_cm_kernel<NDIM, J, LS, CB>), smem);
+    if (e != cudaSuccess) return e;
+    gather_cm_kernel<NDIM, J, LS, CB><<<dim3(p.nitems, p.chunks), CM_THREADS, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
+template <int NDIM, int J, int LS>
+cudaError_t cm_bytes(const GatherParams<float>& p, cudaStream_t s) {
+    // 16-byte copies where every cell's coils start on a 16-byte boundary
+    const bool even = p.coils % 2 == 0 && (reinterpret_cast<uintptr_t>(p.grid) & 15) == 0;
+    return even ? cm_launch<NDIM, J, LS, 16>(p, s) : cm_launch<NDIM, J, LS, 8>(p, s);
+}
+
+template <int NDIM, int LS>
+cudaError_t cm_width(const GatherParams<float>& p, cudaStream_t s) {
+    switch (p.g.J[0]) {
+        case 4: return cm_bytes<NDIM, 4, LS>(p, s);
+        case 5: return cm_bytes<NDIM, 5, LS>(p, s);
+        case 6: return cm_bytes<NDIM, 6, LS>(p, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+// Records exist, the grid is coil-minor with its phases and scale applied,
+// one kernel width on every axis, and the staged tile fits.
+bool gather_cm_supported(const GatherParams<float>& p) {
+    const Geom<float>& g = p.g;
+    if (!p.s.rec || g.hi[0] || g.ndim < 2 || g.gsp != 1 || g.gs0 != p.coils) return false;
+    if (p.apply_pb || p.grid_scale != 1.f || p.chunks > 65535) return false;
+    const int LS = p.ln.LS;
+    if (!(LS == 8 || (g.ndim == 2 && (LS == 16 || LS == 32)))) return false;
+    size_t cells = 1;
+    for (int d = 0; d < g.ndim; ++d) {
+        if (g.J[d] != g.J[0]) return false;
+        cells *= (size_t)(g.T[d] + g.J[d] - 1);
+    }
+    if (g.J[0] < 4 || g.J[0] > 6) return false;
+    return cells * LS * sizeof(float2) + 16 * 1024 <= 227 * 1024;
+}
+
+cudaError_t launch_gather_cm(const GatherParams<float>& p, cudaStream_t s) {
+    if (p.nitems == 0 || p.coils == 0) return cudaSuccess;
+    if (p.g.ndim == 3) return cm_width<3, 8>(p, s);
+    switch (p.ln.LS) {
+        case 8: return cm_width<2, 8>(p, s);
+        case 16: return cm_width<2, 16>(p, s);
+        case 32: return cm_width<2, 32>(p, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace gbn

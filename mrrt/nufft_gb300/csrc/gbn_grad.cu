@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) grad_kernel(const GradParams<R> p) {
 #pragma unroll
                 for (int j0 = 0; j0 < JMAX; ++j0) {
                     if (j0 >= g.J[0]) continue;
-                    const C v = gb[wrapk(kf[0] + j0, g.K[0]) + o1 + o2];
+                    const C v = gb[wrapk(kf[0] + j0, g.K[0]) * g.gs0 + o1 + o2];
                     r = cadd(r, cmul(cc[0][j0], v));
                     rd = cadd(rd, cmul(dd[0][j0], v));
                 }
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) grad2d_group_kernel(const GradParams<R> p
             d0.x = __shfl_sync(0xffffffffu, dd[0].x, base + j0);
             d0.y = __shfl_sync(0xffffffffu, dd[0].y, base + j0);
             if (row) {
-                const C v = gb[wrapk(kf[0] + j0, g.K[0]) + o1];
+                const C v = gb[wrapk(kf[0] + j0, g.K[0]) * g.gs0 + o1];
                 r = cadd(r, cmul(c0, v));
                 rd = cadd(rd, cmul(d0, v));
             }

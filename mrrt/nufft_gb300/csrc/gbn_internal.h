@@ -37,14 +37,15 @@ struct Geom {
     const R* hr[3];          // device tables (shifted past their zero padding)
     const R* hi[3];          // imaginary tables, nullptr for a real kernel
     int64_t Kprod, Nprod;
-    // Grid layout: cell (k0, k1, k2) of plane pl (= frame * coils + coil) at
-    // pl * gsp + k0 + k1 * gs1 + k2 * gs2.  Plane-major ([planes][K...]:
-    // gsp = Kprod, gs1 = K0, gs2 = K0 K1) or, for the 2-D transform's own
-    // grid, row-interleaved ([K1][planes][K0]: gsp = K0, gs1 = planes K0),
-    // the layout its pruned FFT passes need.
-    int64_t gsp, gs1, gs2;
+    // Grid layout: cell (k0, k1, k2) of coil c of frame f at f * gsf + c * gsp +
+    // k0 * gs0 + k1 * gs1 + k2 * gs2.  Plane-major ([frame][coil][K...]), for
+    // transforms on the library's own FFT passes coil-minor
+    // ([frame][K...][coil]), around cuFFT's passes in 2-D row-interleaved
+    // ([K1][frame][coil][K0]), the layout their pruning needs.
+    int64_t gsf, gsp, gs0, gs1, gs2;
     R pbc[3];                // phase_before coefficient per memory axis
     int pbo[3];              // summation order of the per-axis phases
+    const typename Cx<R>::T* ptab;   // phase_before per cell [K...], or nullptr: computed
     // Checked builds (GBN_CHECKED): the plan's status word and the extents
     // (complex elements) of the grid and sample buffers of the call
     unsigned* check;
@@ -69,31 +70,33 @@ struct SampleList {
     const int* idx;                 // sample index within its frame
     const typename Cx<R>::T* ph;    // per-sample phase (list order) or nullptr
     const short4* ls;               // spread list: window start in tile coordinates
-    // Interpolation coefficients precomputed in list order, or nullptr (the
-    // kernels then interpolate the tables): entry e holds jsum values, the
-    // J_0 taps of axis 0, then the J_1 taps of axis 1, ...; ci the imaginary
-    // parts for a complex kernel.
+    // Gather list: coefficients precomputed in list order, or nullptr (the
+    // kernels then interpolate the tables): entry e holds, from cr + e * cstride
+    // on, the J_0 taps of axis 0, then the J_1 taps of axis 1, ...; ci the
+    // imaginary parts for a complex kernel.
     const R* cr;
     const R* ci;
-    int jsum;
+    int cstride;
+    const R* rec;                   // real single precision: records of cstride values, {cell of the
+                                    // window's start in the staged tile, sample index, phase} and
+                                    // the coefficients padded with zeros to 16 bytes
     int64_t len;                    // entries in the list
 };
 
-// Fill a list's precomputed coefficients, for every entry of every work
-// item: from the tables (bitwise the values the kernels would interpolate)
-// or, in sparse-matrix mode, from per-sample weights wr[d] / wi[d]
-// ([M_total][J_d], sample order = frame offset + index).
+// Fill the gather list's precomputed coefficients: from the tables (bitwise
+// the values the kernels would interpolate) or, in sparse-matrix mode, from
+// per-sample weights wr[d] / wi[d] ([M_total][J_d], sample order = frame
+// offset + index).
 template <typename R>
 struct CoefParams {
     Geom<R> g;
     SampleList<R> s;
-    const int4* items;              // {frame, tile, start, count}
-    int nitems;
     const int64_t* foff;
+    int F;
     const R* wr[3];
     const R* wi[3];
-    R* out_r;
-    R* out_i;
+    R* out;
+    int off, stride;                // an entry's coefficients lie from out + e * stride + off on
     int jsum;
     int cx;
 };
@@ -169,7 +172,7 @@ struct VisitParams {
     const typename Cx<R>::T* y;
     const typename Cx<R>::T* ph;    // with y: sample phase, sample order, or nullptr
     typename Cx<R>::T* grid;
-    typename Cx<R>::T* scratch;     // [slot][chunk][LS][tile cells] partial sums
+    typename Cx<R>::T* scratch;     // [slot][chunk][tile cells][LS] partial sums
     int64_t tile_cells, scratch_elems;
     int apply_pb;
 };
@@ -193,7 +196,7 @@ struct PadParams {
     int ndim;
     int N[3], K[3];
     int64_t Nprod, Kprod;
-    int64_t gsp, gs1, gs2;          // layout of the padded grid (see Geom)
+    int64_t gsp, gs1, gs2;          // layout of the padded grid: plane (frame * coils + coil), rows, z-planes
     int planes;
     const typename Cx<R>::T* x;
     const R* sn;
@@ -211,7 +214,7 @@ struct CropParams {
     int ndim;
     int N[3], K[3];
     int64_t Nprod, Kprod;
-    int64_t gsp, gs1, gs2;          // layout of the grid read (see Geom)
+    int64_t gsp, gs1, gs2;          // layout of the grid read: plane (frame * coils + coil), rows, z-planes
     int planes;
     const typename Cx<R>::T* grid;
     const R* sn;
@@ -332,6 +335,12 @@ struct ColFftParams {
     int planes, planes2;
     int L, nin, nout;
     const float2* tw;               // exp(-2 pi i m / L), m < L
+    // phase_before of the grid cells, or nullptr: the forward pass multiplies
+    // its outputs by it (and divides them by `div`, the orthonormal scale).
+    // Value (row, column) lies in cell row * (S / coils) + column / coils.
+    const float2* phase;
+    int coils;
+    float div;
     unsigned* check;                // checked builds: status word and extents
     int64_t in_elems, out_elems;
 };
@@ -340,18 +349,19 @@ bool colfft_supported(int L);
 cudaError_t launch_colfft(const ColFftParams& p, int sign, cudaStream_t s);
 
 // Row passes of the 2-D and 3-D transforms with pad / crop folded in
-// (gbn_rowfft.cu).  Rows r < planes * N2 * N1 (N2 = 1 in 2-D): plane
-// r / (N1 N2), image row (n2, n1) of [planes][N2][N1][N0] and grid row at
-// plane * gsp + n2 * gs2 + n1 * gs1 (L = K0 values).  sign -1: sn * image ->
-// forward FFT -> grid row; +1: grid row -> inverse FFT -> first N0 values *
-// scale * sn -> image.
+// (gbn_rowfft.cu).  Row r < rows = frames N2 N1 coils, coil fastest: image row
+// (n2, n1) of [frames][coils][N2][N1][N0] and the coil-minor grid row at
+// f * gsf + n2 * gs2 + n1 * gs1 + c (L = K0 values, `coils` apart).  sign -1:
+// sn * image -> forward FFT -> grid row; +1: grid row -> inverse FFT -> first
+// N0 values * scale * sn -> image.
 struct RowFftParams {
     const float2* in;               // forward: image; inverse: grid
     float2* out;                    // forward: grid; inverse: image
     const float* sn;                // [N2][N1][N0]
     float scale;                    // inverse only
-    int planes, N0, N1, N2, L;
-    int64_t gsp, gs1, gs2;
+    int coils, N0, N1, N2, L;
+    int64_t rows;
+    int64_t gsf, gs1, gs2;
     const float2* tw;               // exp(-2 pi i m / L), m < L
     unsigned* check;                // checked builds: status word and extents
     int64_t in_elems, out_elems;
@@ -369,6 +379,11 @@ template <typename R> cudaError_t launch_pad(const PadParams<R>& p, cudaStream_t
 template <typename R> cudaError_t launch_crop(const CropParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_grad(const GradParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_coef(const CoefParams<R>& p, cudaStream_t s);
+// phase_before of every grid cell, [K_{ndim-1}]...[K_0].
+template <typename R> cudaError_t launch_phase_table(const Geom<R>& g, typename Cx<R>::T* out, cudaStream_t s);
+// The gather on a coil-minor grid (gbn_gather_cm.cu), and whether it takes a launch.
+bool gather_cm_supported(const GatherParams<float>& p);
+cudaError_t launch_gather_cm(const GatherParams<float>& p, cudaStream_t s);
 
 // Shared-memory bytes needed by the gather kernel for a lane layout.
 template <typename R> size_t gather_smem(const Geom<R>& g, const Lanes& ln);

@@ -234,6 +234,7 @@ struct gbn_plan {
     int n_gitems = 0, n_sitems = 0, n_rtiles = 0, n_slots = 0;
     int64_t glen = 0, slen = 0;
     DevBuf pad, grid, scratch;
+    DevBuf ptab;               // phase_before of every grid cell (real phasing)
     DevBuf mid;           // output of the forward's slab pass (2-D rows, 3-D z-planes); the
                           // slabs >= N_last the last-axis pass reads stay zero
     int64_t mid_clean = 0;     // 2-D: slabs from which mid is known to be zero
@@ -242,7 +243,8 @@ struct gbn_plan {
                                // and crop folded in (gbn_rowfft.cu, gbn_colfft.cu)
     DevBuf fft_tw[3];          // per axis d: exp(-2 pi i m / K_d), m < K_d (axes those use)
     int mid_planes = 0;        // planes the mid buffer holds
-    int cap_planes = 0;        // planes the pad/grid buffers hold
+    int cap_planes = 0;        // planes the grid buffer holds
+    int pad_planes = 0;        // planes the pad buffer holds (transforms around cuFFT)
     int64_t scratch_cap = 0;   // complex elements
     std::vector<FftEntry> ffts;
     HostIo hio;
@@ -312,11 +314,8 @@ Geom<R> make_geom(const gbn_plan* P, bool spread) {
     g.L = G.L;
     g.Kprod = P->Kprod;
     g.Nprod = P->Nprod;
-    // plane-major layout (the C ABI's grids); transform-internal grids of
-    // 2-D and 3-D plans are re-strided by internal_layout
-    g.gsp = P->Kprod;
-    g.gs1 = g.K[0];
-    g.gs2 = (int64_t)g.K[0] * g.K[1];
+    g.ptab = reinterpret_cast<const typename Cx<R>::T*>(P->ptab.p);
+    // the grid's strides are the caller's to set: abi_layout, internal_layout
     g.check = reinterpret_cast<unsigned*>(P->check.p);
     return g;
 }
@@ -353,6 +352,31 @@ void internal_layout(const gbn_plan* P, int planes, T& g) {
     }
 }
 
+// Grid strides of an interpolation kernel: the C ABI's plane-major grids, the
+// coil-minor grid of a transform on the plan's own FFT passes, or the grid
+// around cuFFT's.
+enum class Grid { abi, own, cufft };
+template <typename R>
+void grid_layout(const gbn_plan* P, int coils, Grid kind, Geom<R>& g) {
+    if (kind == Grid::own) {
+        g.gsf = P->Kprod * coils;
+        g.gsp = 1;
+        g.gs0 = coils;
+        g.gs1 = (int64_t)g.K[0] * coils;
+        g.gs2 = (int64_t)g.K[0] * g.K[1] * coils;
+        return;
+    }
+    g.gs0 = 1;
+    if (kind == Grid::cufft) {
+        internal_layout(P, P->F * coils, g);
+    } else {
+        g.gsp = P->Kprod;
+        g.gs1 = g.K[0];
+        g.gs2 = (int64_t)g.K[0] * g.K[1];
+    }
+    g.gsf = g.gsp * coils;
+}
+
 // Sample-list buffer layout: window starts (spread list only), sample
 // phase (if any), one coordinate array per axis, sample index.  Every
 // section starts on a 16-byte boundary (double2 phases need it).
@@ -380,6 +404,19 @@ struct ListLayout {
     }
 };
 
+// Layout of an entry of the gather list's coefficients: real single precision
+// keeps whole records (place, index and phase ahead of the coefficients, 16-byte
+// units), the others the coefficients alone.
+struct GatherRecord {
+    int jsum = 0, off = 0, stride = 0;
+    explicit GatherRecord(const gbn_plan* P) {
+        for (int d = 0; d < P->geom.ndim; ++d) jsum += P->geom.Jd[d];
+        const bool whole = !P->dbl && !P->cx;
+        off = whole ? 4 : 0;
+        stride = whole ? 4 + (jsum + 3) / 4 * 4 : jsum * (P->cx ? 2 : 1);
+    }
+};
+
 template <typename R>
 SampleList<R> make_list(const gbn_plan* P, const DevBuf& buf, int64_t len, bool with_ls) {
     typedef typename Cx<R>::T C;
@@ -393,12 +430,12 @@ SampleList<R> make_list(const gbn_plan* P, const DevBuf& buf, int64_t len, bool 
     s.idx = reinterpret_cast<const int*>(b + L.idx);
     s.len = len;
     if (P->coefs && !with_ls) {
-        const DevBuf& cb = P->gcoef;
-        int jsum = 0;
-        for (int d = 0; d < P->geom.ndim; ++d) jsum += P->geom.Jd[d];
-        s.jsum = jsum;
-        s.cr = reinterpret_cast<const R*>(cb.p);
-        if (P->cx) s.ci = s.cr + (size_t)len * jsum;
+        const GatherRecord r(P);
+        const R* base = reinterpret_cast<const R*>(P->gcoef.p);
+        s.cstride = r.stride;
+        s.cr = base + r.off;
+        if (P->cx) s.ci = s.cr + r.jsum;
+        if (r.off) s.rec = base;
     }
     return s;
 }
@@ -713,27 +750,32 @@ int ensure_scratch(gbn_plan* P, int coils) {
     return GBN_OK;
 }
 
-// Zero-padded FFT input, FFT output grid and scratch for F * coils planes.
-// `fused`: the call runs the 3-D transform on the plan's own passes (in
-// place on the grid), which need no slab-pass buffer.
-int ensure_buffers(gbn_plan* P, int coils, bool fused = false) {
+// FFT grid and scratch for F * coils planes; around cuFFT's passes also the
+// zero-padded input and the pruned passes' intermediate buffer.  `own`: the
+// call runs on the plan's own passes, in place on the grid.
+int ensure_buffers(gbn_plan* P, int coils, bool own) {
     const int planes = P->F * coils;
     const size_t csz = (size_t)2 * P->rsize;
+    const size_t bytes = (size_t)planes * P->Kprod * csz;
     if (planes > P->cap_planes) {
-        const size_t bytes = (size_t)planes * P->Kprod * csz;
+        P->cap_planes = 0;
+        cudaError_t e = P->grid.alloc(bytes);
+        if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "grid buffer allocation failed");
+        P->cap_planes = planes;
+    }
+    if (!own && planes > P->pad_planes) {
+        P->pad_planes = 0;
         cudaError_t e = P->pad.alloc(bytes);
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "pad buffer allocation failed");
         e = cudaMemset(P->pad.p, 0, bytes);
         if (e != cudaSuccess) return cuda_fail(e, "pad buffer clear");
-        e = P->grid.alloc(bytes);
-        if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "grid buffer allocation failed");
-        P->cap_planes = planes;
+        P->pad_planes = planes;
     }
-    // the pruned FFT's intermediate buffer: every plane in 2-D, the planes of
-    // a pruned call in 3-D (none beyond PRUNE3_MAX_PLANES)
-    const int mid_need = P->geom.ndim == 2 || (pruned_3d(P, planes) && !fused) ? planes : 0;
+    // every plane in 2-D, the planes of a pruned call in 3-D (none beyond
+    // PRUNE3_MAX_PLANES)
+    const int mid_need = !own && (P->geom.ndim == 2 || pruned_3d(P, planes)) ? planes : 0;
     if (mid_need > P->mid_planes) {
-        const size_t bytes = (size_t)mid_need * P->Kprod * csz;
+        P->mid_planes = 0;
         cudaError_t e = P->mid.alloc(bytes);
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "slab-pass buffer allocation failed");
         e = cudaMemset(P->mid.p, 0, bytes);
@@ -779,10 +821,8 @@ int setup_colfft(gbn_plan* P) {
 }
 
 // Row pass with the pad (sign -1: image -> grid rows) or the crop (sign +1:
-// grid rows -> image) folded in; 2-D: image rows to the row-interleaved
-// layout (into mid), 3-D: to the plane-major layout (the grid in place).
-int run_rowfft(gbn_plan* P, const void* in, int64_t in_elems, void* out, int64_t out_elems, int planes, int sign,
-               cudaStream_t s) {
+// grid rows -> image) folded in, on the coil-minor grid.
+int run_rowfft(gbn_plan* P, const void* in, void* out, int coils, int sign, cudaStream_t s) {
     const gbn_geometry& G = P->geom;
     RowFftParams p;
     std::memset(&p, 0, sizeof(p));
@@ -790,16 +830,20 @@ int run_rowfft(gbn_plan* P, const void* in, int64_t in_elems, void* out, int64_t
     p.out = static_cast<float2*>(out);
     p.sn = static_cast<const float*>(P->sn.p);
     p.scale = G.ortho ? (float)(G.adjoint_scale / std::sqrt((double)P->Kprod)) : (float)G.adjoint_scale;
-    p.planes = planes;
+    p.coils = coils;
     p.N0 = G.Nd[0];
     p.N1 = G.Nd[1];
     p.N2 = G.ndim > 2 ? G.Nd[2] : 1;
+    p.rows = (int64_t)P->F * coils * p.N1 * p.N2;
     p.L = G.Kd[0];
-    internal_layout(P, planes, p);
+    p.gsf = P->Kprod * coils;
+    p.gs1 = (int64_t)G.Kd[0] * coils;
+    p.gs2 = (int64_t)G.Kd[0] * G.Kd[1] * coils;
     p.tw = static_cast<const float2*>(P->fft_tw[0].p);
     p.check = static_cast<unsigned*>(P->check.p);
-    p.in_elems = in_elems;
-    p.out_elems = out_elems;
+    const int64_t img = (int64_t)P->F * coils * P->Nprod, grid = (int64_t)P->cap_planes * P->Kprod;
+    p.in_elems = sign < 0 ? img : grid;
+    p.out_elems = sign < 0 ? grid : img;
     GBN_CUDA(launch_rowfft(p, sign, s), sign < 0 ? "pad + row FFT pass" : "row FFT pass + crop");
     return GBN_OK;
 }
@@ -816,6 +860,7 @@ struct AxisPass {
     int64_t S, ps, ps2;
     int planes, planes2;
     int nin, nout;
+    int phase_coils = 0;   // coils of a coil-minor grid to which phase_before is applied (0: none)
 };
 int run_colfft(gbn_plan* P, const AxisPass& a, int sign, cudaStream_t s) {
     ColFftParams p;
@@ -831,6 +876,9 @@ int run_colfft(gbn_plan* P, const AxisPass& a, int sign, cudaStream_t s) {
     p.nin = a.nin;
     p.nout = a.nout;
     p.tw = static_cast<const float2*>(P->fft_tw[a.axis].p);
+    p.phase = a.phase_coils ? static_cast<const float2*>(P->ptab.p) : nullptr;
+    p.coils = a.phase_coils;
+    p.div = P->geom.ortho ? (float)std::sqrt((double)P->Kprod) : 1.f;
     p.check = static_cast<unsigned*>(P->check.p);
     p.in_elems = a.in_elems;
     p.out_elems = a.out_elems;
@@ -902,31 +950,33 @@ int colfft_2d(gbn_plan* P, int planes, int sign, cudaStream_t s) {
     return run_colfft(P, a, sign, s);
 }
 
-// 3-D passes along axes 1 and 2 of the grid, in place: forward axis 1 over
-// the N_2 z-slabs with data (N_1 rows read), then axis 2 (N_2 z-slabs read);
+// Whether a forward call leaves phase_before (and the orthonormal scale)
+// applied to its grid: plans with derivative tables keep the grid that
+// gbn_grad_tm takes, from before it.
+bool grid_phased(const gbn_plan* P) { return P->geom.phasing == GBN_PHASING_REAL && !P->dtables.p; }
+
+// The strided passes of a transform on the plan's own passes, in place on the
+// coil-minor grid: forward axis 1 over the N_2 z-slabs with data (N_1 rows
+// read), then in 3-D axis 2 (N_2 z-slabs read), phase_before with the last;
 // inverse axis 2 (N_2 z-slabs written), then axis 1 over those slabs (N_1
 // rows written).
-int colfft_3d(gbn_plan* P, int planes, int sign, cudaStream_t s) {
+int own_passes(gbn_plan* P, int coils, int sign, cudaStream_t s) {
     const gbn_geometry& G = P->geom;
     const int64_t ge = (int64_t)P->cap_planes * P->Kprod;
-    const int64_t slab = (int64_t)G.Kd[0] * G.Kd[1];
-    AxisPass a1{P->grid.p, ge, P->grid.p, ge, 1, G.Kd[0], slab, P->Kprod, G.Nd[2], planes, 0, 0};
-    AxisPass a2{P->grid.p, ge, P->grid.p, ge, 2, slab, P->Kprod, 0, planes, 1, 0, 0};
-    int rc;
-    if (sign < 0) {
-        a1.nin = G.Nd[1];
-        a1.nout = G.Kd[1];
-        a2.nin = G.Nd[2];
-        a2.nout = G.Kd[2];
-        if ((rc = run_colfft(P, a1, -1, s))) return rc;
-        return run_colfft(P, a2, -1, s);
+    const int64_t row = (int64_t)G.Kd[0] * coils, slab = row * G.Kd[1], vol = P->Kprod * coils;
+    const bool d3 = G.ndim == 3;
+    AxisPass a1{P->grid.p, ge, P->grid.p, ge, 1, row, d3 ? slab : vol, vol, d3 ? G.Nd[2] : P->F, d3 ? P->F : 1,
+                sign < 0 ? G.Nd[1] : G.Kd[1], sign < 0 ? G.Kd[1] : G.Nd[1]};
+    const int pc = sign < 0 && grid_phased(P) ? coils : 0;
+    if (!d3) {
+        a1.phase_coils = pc;
+        return run_colfft(P, a1, sign, s);
     }
-    a2.nin = G.Kd[2];
-    a2.nout = G.Nd[2];
-    a1.nin = G.Kd[1];
-    a1.nout = G.Nd[1];
-    if ((rc = run_colfft(P, a2, 1, s))) return rc;
-    return run_colfft(P, a1, 1, s);
+    AxisPass a2{P->grid.p, ge, P->grid.p, ge, 2, slab, vol, 0, P->F, 1,
+                sign < 0 ? G.Nd[2] : G.Kd[2], sign < 0 ? G.Kd[2] : G.Nd[2]};
+    a2.phase_coils = pc;
+    int rc = run_colfft(P, sign < 0 ? a1 : a2, sign, s);
+    return rc ? rc : run_colfft(P, sign < 0 ? a2 : a1, sign, s);
 }
 
 // Forward Kd-point FFT of the padded planes into the grid.  2-D and 3-D:
@@ -1032,7 +1082,7 @@ Lanes call_lanes(const gbn_plan* P, int coils) {
 }
 
 template <typename R>
-int run_gather(gbn_plan* P, const void* grid, void* y, int coils, bool phases, cudaStream_t s) {
+int run_gather(gbn_plan* P, const void* grid, void* y, int coils, Grid kind, cudaStream_t s) {
     typedef typename Cx<R>::T C;
     GatherParams<R> p;
     std::memset(&p, 0, sizeof(p));
@@ -1043,11 +1093,12 @@ int run_gather(gbn_plan* P, const void* grid, void* y, int coils, bool phases, c
     p.nitems = P->n_gitems;
     p.coils = coils;
     p.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
-    if (phases) internal_layout(P, P->F * coils, p.g);   // the transform's own grid
+    grid_layout<R>(P, coils, kind, p.g);
+    const bool phases = kind != Grid::abi, done = kind == Grid::own && grid_phased(P);
     p.grid = reinterpret_cast<const C*>(grid);
     p.y = reinterpret_cast<C*>(y);
-    p.apply_pb = phases && P->geom.phasing == GBN_PHASING_REAL;
-    p.grid_scale = (phases && P->geom.ortho) ? (R)std::sqrt((double)P->Kprod) : (R)1;
+    p.apply_pb = phases && !done && P->geom.phasing == GBN_PHASING_REAL;
+    p.grid_scale = phases && !done && P->geom.ortho ? (R)std::sqrt((double)P->Kprod) : (R)1;
     p.apply_ph = phases && P->has_phase;
     p.g.grid_elems = (int64_t)P->F * coils * P->Kprod;
     p.g.sample_elems = (int64_t)coils * P->M_total;
@@ -1062,17 +1113,18 @@ int run_gather(gbn_plan* P, const void* grid, void* y, int coils, bool phases, c
 // vals: room for the coil-minor values (or nullptr: the samples are read in
 // place), scratch: the partial sums.
 template <typename R>
-int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, bool phases, void* vals, int64_t vals_elems,
+int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, void* vals, int64_t vals_elems,
                   void* scratch, int64_t scratch_elems, cudaStream_t s) {
     typedef typename Cx<R>::T C;
     const Lanes ln = call_lanes<R>(P, coils);
+    const bool phases = kind != Grid::abi;
     if (ln.LS < 8) vals = nullptr;   // narrow lanes read the samples in place
     const C* ph = phases && P->has_phase ? reinterpret_cast<const C*>(P->phnat.p) : nullptr;
     const int64_t* foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
     VisitParams<R> p;
     std::memset(&p, 0, sizeof(p));
     p.g = make_geom<R>(P, true);
-    if (phases) internal_layout(P, P->F * coils, p.g);   // the transform's own grid
+    grid_layout<R>(P, coils, kind, p.g);
     p.g.grid_elems = (int64_t)P->F * coils * P->Kprod;
     p.g.sample_elems = (int64_t)coils * P->M_total;
     p.s = make_list<R>(P, P->slist, P->slen, true);
@@ -1133,10 +1185,10 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, bool phases
 }
 
 template <typename R>
-int run_spread(gbn_plan* P, const void* y, void* grid, int coils, bool phases, cudaStream_t s) {
+int run_spread(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, cudaStream_t s) {
     int rc = ensure_scratch(P, coils);
     if (rc) return rc;
-    return launch_visits<R>(P, y, grid, coils, phases, coils >= VALUES_MIN_COILS ? P->vals.p : nullptr,
+    return launch_visits<R>(P, y, grid, coils, kind, coils >= VALUES_MIN_COILS ? P->vals.p : nullptr,
                             (int64_t)(P->vals.bytes / sizeof(typename Cx<R>::T)), P->scratch.p, P->scratch_cap, s);
 }
 
@@ -1169,14 +1221,24 @@ int run_spread_noalloc(gbn_plan* P, const void* y, void* grid, int coils, cudaSt
     const int64_t velems = P->M_total * value_row(coils, sizeof(C));
     void* vals = coils >= VALUES_MIN_COILS && used + velems * (int64_t)sizeof(C) <= (int64_t)cap
                      ? static_cast<char*>(scratch) + used : nullptr;
-    return launch_visits<R>(P, y, grid, coils, false, vals, velems, scratch, need / (int64_t)sizeof(C), s);
+    return launch_visits<R>(P, y, grid, coils, Grid::abi, vals, velems, scratch, need / (int64_t)sizeof(C), s);
 }
 
 template <typename R>
 int run_forward(gbn_plan* P, const void* x, void* y, int coils, cudaStream_t s, const void* maps = nullptr) {
-    int rc = ensure_buffers(P, coils, P->rowfft && !maps);
+    // single precision only (rowfft is off for double plans)
+    const bool own = P->rowfft && !maps;
+    int rc = ensure_buffers(P, coils, own);
     if (rc) return rc;
-    if (!P->pad.p || !P->grid.p) return fail(GBN_ERR_NOMEM, "transform buffers missing");
+    if (own) {
+        {
+            NvtxRange r("gbn forward: pad + fft");
+            if ((rc = run_rowfft(P, x, P->grid.p, coils, -1, s))) return rc;
+            if ((rc = own_passes(P, coils, -1, s))) return rc;
+        }
+        NvtxRange r("gbn forward: gather");
+        return run_gather<R>(P, P->grid.p, y, coils, Grid::own, s);
+    }
     const gbn_geometry& G = P->geom;
     PadParams<R> pp;
     std::memset(&pp, 0, sizeof(pp));
@@ -1195,23 +1257,8 @@ int run_forward(gbn_plan* P, const void* x, void* y, int coils, cudaStream_t s, 
     pp.coils = coils;
     pp.check = reinterpret_cast<unsigned*>(P->check.p);
     pp.x_elems = (int64_t)(maps ? P->F : P->F * coils) * P->Nprod;
-    pp.out_elems = (int64_t)P->cap_planes * P->Kprod;
+    pp.out_elems = (int64_t)P->pad_planes * P->Kprod;
     internal_layout(P, P->F * coils, pp);
-    if (P->rowfft && !maps) {
-        // single precision only (rowfft is off for double plans); 2-D rows
-        // into mid, 3-D rows into the grid, whose passes run in place
-        {
-            NvtxRange r("gbn forward: pad + fft");
-            const int planes = P->F * coils;
-            const bool d2 = G.ndim == 2;
-            if ((rc = run_rowfft(P, x, pp.x_elems, d2 ? P->mid.p : P->grid.p,
-                                 (int64_t)(d2 ? P->mid_planes : P->cap_planes) * P->Kprod, planes, -1, s)))
-                return rc;
-            if ((rc = d2 ? colfft_2d(P, planes, -1, s) : colfft_3d(P, planes, -1, s))) return rc;
-        }
-        NvtxRange r("gbn forward: gather");
-        return run_gather<R>(P, P->grid.p, y, coils, true, s);
-    }
     {
         NvtxRange r("gbn forward: pad");
         GBN_CUDA(launch_pad<R>(pp, s), "pad launch");
@@ -1221,27 +1268,25 @@ int run_forward(gbn_plan* P, const void* x, void* y, int coils, cudaStream_t s, 
         if ((rc = fft_forward(P, P->F * coils, s))) return rc;
     }
     NvtxRange r("gbn forward: gather");
-    return run_gather<R>(P, P->grid.p, y, coils, true, s);
+    return run_gather<R>(P, P->grid.p, y, coils, Grid::cufft, s);
 }
 
 template <typename R>
 int run_adjoint(gbn_plan* P, const void* y, void* x, int coils, cudaStream_t s, const void* maps = nullptr) {
     // allocate first: the grid pointer handed to the spread must be the
     // buffer this call will use (it is null before the first call)
-    int rc = ensure_buffers(P, coils, P->rowfft && !maps);
+    const bool own = P->rowfft && !maps;
+    int rc = ensure_buffers(P, coils, own);
     if (rc) return rc;
-    if (!P->grid.p) return fail(GBN_ERR_NOMEM, "grid buffer missing");
     {
         NvtxRange r("gbn adjoint: spread");
-        rc = run_spread<R>(P, y, P->grid.p, coils, true, s);
+        rc = run_spread<R>(P, y, P->grid.p, coils, own ? Grid::own : Grid::cufft, s);
         if (rc) return rc;
     }
-    if (P->rowfft && !maps) {
+    if (own) {
         NvtxRange r("gbn adjoint: fft + crop");
-        if ((rc = P->geom.ndim == 2 ? colfft_2d(P, P->F * coils, 1, s) : colfft_3d(P, P->F * coils, 1, s)))
-            return rc;
-        return run_rowfft(P, P->grid.p, (int64_t)P->cap_planes * P->Kprod, x, (int64_t)P->F * coils * P->Nprod,
-                          P->F * coils, 1, s);
+        if ((rc = own_passes(P, coils, 1, s))) return rc;
+        return run_rowfft(P, P->grid.p, x, coils, 1, s);
     }
     {
         NvtxRange r("gbn adjoint: fft");
@@ -1437,6 +1482,17 @@ int upload_static(gbn_plan* P, const void* const* h_re, const void* const* h_im,
     return GBN_OK;
 }
 
+// phase_before of every grid cell.
+template <typename R>
+int phase_table(gbn_plan* P) {
+    if (P->geom.phasing != GBN_PHASING_REAL) return GBN_OK;
+    const Geom<R> g = make_geom<R>(P, false);   // no table yet: computed
+    GBN_CUDA(P->ptab.alloc((size_t)P->Kprod * 2 * sizeof(R)), "phase table allocation");
+    GBN_CUDA(launch_phase_table<R>(g, reinterpret_cast<typename Cx<R>::T*>(P->ptab.p), 0), "phase table launch");
+    GBN_CUDA(cudaDeviceSynchronize(), "phase table");
+    return GBN_OK;
+}
+
 int validate(const gbn_geometry* g) {
     if (!g) return fail(GBN_ERR_INVALID, "null geometry");
     if (g->ndim < 1 || g->ndim > 3) return fail(GBN_ERR_UNSUPPORTED, "ndim must be 1, 2 or 3");
@@ -1536,21 +1592,20 @@ int fill_coefs(gbn_plan* P, cudaStream_t stream = 0, bool sync = true, int64_t t
     const gbn_geometry& G = P->geom;
     const bool keep = P->weights.p || !(G.flags & GBN_FLAG_TABLE_ONLY);
     if (keep) {
-        int jsum = 0;
-        for (int d = 0; d < G.ndim; ++d) jsum += G.Jd[d];
-        const size_t bytes = std::max<size_t>((size_t)P->glen * jsum * (P->cx ? 2 : 1) * sizeof(R), 16);
+        const GatherRecord rec(P);
+        const size_t bytes = std::max<size_t>((size_t)P->glen * rec.stride * sizeof(R), 16);
         if (P->gcoef.bytes < bytes) GBN_CUDA(P->gcoef.alloc(bytes), "gather coefficient allocation");
         CoefParams<R> c;
         std::memset(&c, 0, sizeof(c));
         c.g = make_geom<R>(P, false);
         c.s = make_list<R>(P, P->glist, P->glen, false);
-        c.items = reinterpret_cast<const int4*>(P->gitems.p);
-        c.nitems = P->n_gitems;
         c.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
+        c.F = P->F;
         weight_pointers<R>(P, c.wr, c.wi);
-        c.out_r = reinterpret_cast<R*>(P->gcoef.p);
-        c.out_i = P->cx ? c.out_r + (size_t)P->glen * jsum : nullptr;
-        c.jsum = jsum;
+        c.out = reinterpret_cast<R*>(P->gcoef.p);
+        c.off = rec.off;
+        c.stride = rec.stride;
+        c.jsum = rec.jsum;
         c.cx = P->cx ? 1 : 0;
         GBN_CUDA(launch_coef<R>(c, stream), "coefficient launch");
     } else {
@@ -1843,7 +1898,7 @@ int run_grad(gbn_plan* P, const void* grid, const void* gy, const double* shift,
     GradParams<R> p;
     std::memset(&p, 0, sizeof(p));
     p.g = make_geom<R>(P, false);
-    internal_layout(P, P->F * coils, p.g);   // the grid a forward call with these coils left
+    grid_layout<R>(P, coils, P->rowfft ? Grid::own : Grid::cufft, p.g);   // as a forward call with these coils left it
     const SampleList<R> L = make_list<R>(P, P->glist, P->glen, false);
     const R* db = reinterpret_cast<const R*>(P->dtables.p);
     size_t off = 0;
@@ -1921,6 +1976,7 @@ int gbn_plan_create(gbn_plan** out, const gbn_geometry* geom, const void* const*
         }
     }
     rc = P->dbl ? upload_static<double>(P, h_re, h_im, sn) : upload_static<float>(P, h_re, h_im, sn);
+    if (!rc) rc = P->dbl ? phase_table<double>(P) : phase_table<float>(P);
     if (!rc) rc = P->dbl ? plan_points<double>(P, tm, sample_phase) : plan_points<float>(P, tm, sample_phase);
     if (rc) {
         delete P;
@@ -2046,8 +2102,8 @@ int gbn_interp_forward(gbn_plan* P, const void* grid, void* y, int coils, void* 
     std::lock_guard<std::mutex> lk(P->mu);
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    return P->dbl ? run_gather<double>(P, grid, y, coils, false, s)
-                  : run_gather<float>(P, grid, y, coils, false, s);
+    return P->dbl ? run_gather<double>(P, grid, y, coils, Grid::abi, s)
+                  : run_gather<float>(P, grid, y, coils, Grid::abi, s);
 }
 
 int gbn_interp_adjoint(gbn_plan* P, const void* y, void* grid, int coils, void* stream) {
@@ -2057,8 +2113,8 @@ int gbn_interp_adjoint(gbn_plan* P, const void* y, void* grid, int coils, void* 
     std::lock_guard<std::mutex> lk(P->mu);
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    return P->dbl ? run_spread<double>(P, y, grid, coils, false, s)
-                  : run_spread<float>(P, y, grid, coils, false, s);
+    return P->dbl ? run_spread<double>(P, y, grid, coils, Grid::abi, s)
+                  : run_spread<float>(P, y, grid, coils, Grid::abi, s);
 }
 
 int gbn_interp_adjoint_noalloc(gbn_plan* P, const void* y, void* grid, int coils, void* stream) {
@@ -2179,7 +2235,7 @@ int gbn_plan_stats(const gbn_plan* P, int64_t* o) {
     o[5] = (int64_t)P->ntiles_s * P->F;
     o[6] = (int64_t)(P->tables.bytes + P->weights.bytes + P->gcoef.bytes +
                      P->vstart.bytes + P->vidx.bytes + P->vco.bytes + P->vwork.bytes + P->phnat.bytes +
-                     P->vals.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
+                     P->vals.bytes + P->ptab.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
                      P->grid.bytes + P->scratch.bytes);
     o[7] = P->M_total;
     return GBN_OK;

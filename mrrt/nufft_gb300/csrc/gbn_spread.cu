@@ -44,9 +44,9 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceParams<R> p, co
     }
     const int TT = Td[0] * Td[1] * Td[2];
     const int q = sub * blockDim.x + threadIdx.x;
-    if (q >= TT * nc) return;
-    const int c = q / TT;
-    const int cell = q - c * TT;
+    if (q >= TT * LS) return;
+    const int cell = q >> lsh, c = q & (LS - 1);   // coils fastest, as the partial sums lie
+    if (c >= nc) return;
     int r[3];
     r[0] = cell % Td[0];
     r[1] = (cell / Td[0]) % Td[1];
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceParams<R> p, co
     for (int d = 0; d < NDIM; ++d) inside = inside && (r[d] < ext[d]);
     if (!inside) return;
     const int64_t pstride = (int64_t)gridDim.y * LS * p.tile_cells;
-    const int64_t s0 = (((int64_t)slot0 * gridDim.y + blockIdx.y) * LS + c) * p.tile_cells + cell;
+    const int64_t s0 = (((int64_t)slot0 * gridDim.y + blockIdx.y) * p.tile_cells + cell) * LS + c;
     if (!GBN_INB(g.check, slot0 >= 0 && nparts >= 1 && s0 + (int64_t)(nparts - 1) * pstride < p.scratch_elems,
                  CHK_SCRATCH))
         return;
@@ -81,9 +81,9 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceParams<R> p, co
     int k[3] = {0, 0, 0};
 #pragma unroll
     for (int d = 0; d < NDIM; ++d) k[d] = org[d] + r[d];
-    const int64_t off = k[0] + (int64_t)k[1] * g.gs1 + (int64_t)k[2] * g.gs2;
+    const int64_t off = k[0] * g.gs0 + (int64_t)k[1] * g.gs1 + (int64_t)k[2] * g.gs2;
     if (p.apply_pb) acc = cmulc(acc, phase_before(g, k));
-    const int64_t gi = ((int64_t)f * p.coils + c0 + c) * g.gsp + off;
+    const int64_t gi = f * g.gsf + (c0 + c) * g.gsp + off;
     if (GBN_INB(g.check, gi >= 0 && gi < g.grid_elems, CHK_GRID_WRITE)) p.grid[gi] = acc;
 }
 

@@ -376,7 +376,7 @@ __device__ __forceinline__ void flush_block(const VisitParams<R>& p, typename Cx
         }
     }
     if (coil >= nc || (SW > NB && (slot >> 4))) return;
-    const bool vec_ok = sizeof(R) == 4 && (g.K[0] % 2) == 0 && (g.gsp % 2) == 0 && (g.gs1 % 2) == 0 &&
+    const bool vec_ok = sizeof(R) == 4 && g.gs0 == 1 && (g.K[0] % 2) == 0 && (g.gsf % 2) == 0 && (g.gsp % 2) == 0 && (g.gs1 % 2) == 0 &&
                         (g.gs2 % 2) == 0;
     constexpr int STEP = KEEP >= 2 ? 2 : 1;
 #pragma unroll
@@ -387,16 +387,19 @@ __device__ __forceinline__ void flush_block(const VisitParams<R>& p, typename Cx
         const bool in0 = row_in && org[0] + l0 < g.K[0];
         const bool in1 = STEP == 2 && row_in && org[0] + l0 + 1 < g.K[0];
         C* dst;
+        int64_t next;   // the cell after this one along axis 0
         if (direct) {
-            const int64_t gi = ((int64_t)f * p.coils + c0 + coil) * g.gsp + (org[0] + l0) +
-                               (int64_t)(org[1] + l1) * g.gs1 + (int64_t)(org[2] + l2) * g.gs2;
-            if ((in0 || in1) && !GBN_INB(g.check, gi >= 0 && gi + (in1 ? 1 : 0) < g.grid_elems, CHK_GRID_WRITE))
+            const int64_t gi = f * g.gsf + (c0 + coil) * g.gsp + (org[0] + l0) * g.gs0 + (org[1] + l1) * g.gs1 +
+                               (org[2] + l2) * g.gs2;
+            next = g.gs0;
+            if ((in0 || in1) && !GBN_INB(g.check, gi >= 0 && gi + (in1 ? next : 0) < g.grid_elems, CHK_GRID_WRITE))
                 continue;
             dst = p.grid + gi;
         } else {
             const int64_t cell = l0 + (int64_t)g.T[0] * (l1 + (int64_t)g.T[1] * l2);
-            const int64_t si = (((int64_t)scratch_slot * p.chunks + chunk) * LS + coil) * p.tile_cells + cell;
-            if ((in0 || in1) && !GBN_INB(g.check, si >= 0 && si + (in1 ? 1 : 0) < p.scratch_elems, CHK_SCRATCH))
+            const int64_t si = (((int64_t)scratch_slot * p.chunks + chunk) * p.tile_cells + cell) * LS + coil;
+            next = LS;
+            if ((in0 || in1) && !GBN_INB(g.check, si >= 0 && si + (in1 ? next : 0) < p.scratch_elems, CHK_SCRATCH))
                 continue;
             dst = p.scratch + si;
         }
@@ -404,7 +407,7 @@ __device__ __forceinline__ void flush_block(const VisitParams<R>& p, typename Cx
             store_pair(dst, acc[i], acc[i + STEP - 1]);
         } else {
             if (in0) dst[0] = acc[i];
-            if (in1) dst[1] = acc[i + STEP - 1];
+            if (in1) dst[next] = acc[i + STEP - 1];
         }
     }
 }
