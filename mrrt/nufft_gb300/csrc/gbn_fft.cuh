@@ -1,5 +1,5 @@
-// In-register FFTs shared by the FFT pass kernels (gbn_colfft.cu,
-// gbn_rowfft.cu): Stockham autosort transforms (Govindaraju et al., "High
+// In-register FFTs shared by the FFT pass kernels (gbn_fftpass.cu):
+// Stockham autosort transforms (Govindaraju et al., "High
 // performance discrete Fourier transforms on graphics processors", SC 2008)
 // of length N dividing 96, radix 4, 2 and 3 stages fully unrolled, and the
 // four-step twiddle multiply.  Included by one translation unit each (the

@@ -82,25 +82,36 @@ __global__ void __launch_bounds__(CM_THREADS) gather_cm_kernel(const GatherParam
     };
     issue_records(0);
 
-    // ---- stage the tile and its halo: a warp per row segment ----------------------
+    // ---- stage the tile and its halo --------------------------------------------
+    // Grid offsets of the region's rows first, one per thread; then a thread
+    // keeps its place along axis 0 (and so its wrapped offset) and copies it
+    // from every row: a load of the row's offset, an add and a copy each.
+    const int nrows = Rd[1] * (NDIM > 2 ? Rd[2] : 1);
+    int64_t* rowoff = reinterpret_cast<int64_t*>(smem_raw + (size_t)cells * LS * sizeof(float2) + CM_WARPS * L::RING);
+    for (int r = threadIdx.x; r < nrows; r += CM_THREADS) {
+        const int y = NDIM > 2 ? r % Rd[1] : r, z = NDIM > 2 ? r / Rd[1] : 0;
+        int64_t o = f * g.gsf + c0 + (int64_t)wrapk(org[1] + y, g.K[1]) * g.gs1;
+        if (NDIM > 2) o += (int64_t)wrapk(org[2] + z, g.K[2]) * g.gs2;
+        rowoff[r] = o;
+    }
+    __syncthreads();
     {
         constexpr int PC = LS * 8 / CB;   // copies per cell
-        const char* gb = reinterpret_cast<const char*>(p.grid + f * g.gsf + c0);
-        const int nrows = Rd[1] * (NDIM > 2 ? Rd[2] : 1);
-        const int part = lane % PC * CB;
+        const int Q = Rd[0] * PC;
+        int tpr = 32;                     // threads per row
+        while (tpr < Q && tpr < CM_THREADS) tpr *= 2;
+        const int part = threadIdx.x % PC * CB;
         const bool part_ok = part < nc * 8;
-        for (int r = warp; r < nrows; r += CM_WARPS) {
-            const int y = NDIM > 2 ? r % Rd[1] : r, z = NDIM > 2 ? r / Rd[1] : 0;
-            int64_t row = (int64_t)wrapk(org[1] + y, g.K[1]) * g.gs1;
-            if (NDIM > 2) row += (int64_t)wrapk(org[2] + z, g.K[2]) * g.gs2;
-            unsigned char* dst = smem_raw + (size_t)r * Rd[0] * (LS * 8);
-            for (int q = lane; q < Rd[0] * PC; q += 32) {
-                int kx = org[0] + q / PC;
-                if (kx >= g.K[0]) kx = wrapk(kx, g.K[0]);
-                const int64_t i = row + (int64_t)kx * g.gs0;   // complex values from gb
-                const bool ok = part_ok && GBN_INB(g.check, f * g.gsf + c0 + i + (part + CB) / 8 <= g.grid_elems,
+        for (int q = threadIdx.x % tpr; q < Q; q += tpr) {
+            const int64_t x = (int64_t)wrapk(org[0] + q / PC, g.K[0]) * g.gs0;
+            const char* src = reinterpret_cast<const char*>(p.grid + x) + part;
+            unsigned char* dst = smem_raw + q * CB;
+#pragma unroll 4
+            for (int r = threadIdx.x / tpr; r < nrows; r += CM_THREADS / tpr) {
+                const bool ok = part_ok && GBN_INB(g.check, rowoff[r] + x + (part + CB) / 8 <= g.grid_elems,
                                                    CHK_GRID_READ);
-                cp_async_fill<CB>(dst + q * CB, ok ? gb + i * 8 + part : gb, ok);
+                cp_async_fill<CB>(dst + (size_t)r * Rd[0] * (LS * 8),
+                                  ok ? src + rowoff[r] * 8 : reinterpret_cast<const char*>(p.grid), ok);
             }
         }
     }
@@ -132,11 +143,13 @@ __global__ void __launch_bounds__(CM_THREADS) gather_cm_kernel(const GatherParam
         }
         if ((k + 1) * B < ns) issue_records(k + 1);
         const unsigned char* buf = ring + (k & 1) * (B * REC);
+        // a lane group takes adjacent list entries in turn, as few turns as the
+        // stage's entries need
+        const int have = min(B, ns - k * B), turns = (have + SW - 1) / SW;
 #pragma unroll 1
-        for (int u = 0; u < B / SW; ++u) {
-            // a lane group takes adjacent list entries in turn
-            const int e = grp * (B / SW) + u;
-            const bool on = k * B + e < ns;
+        for (int u = 0; u < turns; ++u) {
+            const int e = grp * turns + u;
+            const bool on = e < have;
             const unsigned char* rec = buf + (on ? e : 0) * REC;
             const int4 meta = *reinterpret_cast<const int4*>(rec);   // region cell, index, phase
             float q[L::NC];
@@ -239,13 +252,15 @@ __global__ void __launch_bounds__(CM_THREADS) gather_cm_kernel(const GatherParam
 
 template <int NDIM, int J, int LS, int CB>
 cudaError_t cm_launch(const GatherParams<float>& p, cudaStream_t s) {
-    int Rd[3];
+    int Rd[3] = {1, 1, 1};
     size_t cells = 1;
     for (int d = 0; d < NDIM; ++d) {
         Rd[d] = p.g.T[d] + p.g.J[d] - 1;
         cells *= (size_t)Rd[d];
     }
-    const size_t smem = cells * LS * sizeof(float2) + CM_WARPS * (size_t)CmLayout<NDIM, J, LS>::RING;
+    const size_t nrows = (size_t)Rd[1] * (NDIM > 2 ? Rd[2] : 1);
+    const size_t smem = cells * LS * sizeof(float2) + CM_WARPS * (size_t)CmLayout<NDIM, J, LS>::RING +
+                        nrows * sizeof(int64_t);
     cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(gather_cm_kernel<NDIM, J, LS, CB>), smem);
     if (e != cudaSuccess) return e;
     gather_cm_kernel<NDIM, J, LS, CB><<<dim3(p.nitems, p.chunks), CM_THREADS, smem, s>>>(p);
@@ -285,7 +300,8 @@ bool gather_cm_supported(const GatherParams<float>& p) {
         cells *= (size_t)(g.T[d] + g.J[d] - 1);
     }
     if (g.J[0] < 4 || g.J[0] > 6) return false;
-    return cells * LS * sizeof(float2) + 16 * 1024 <= 227 * 1024;
+    const size_t nrows = cells / (size_t)(g.T[0] + g.J[0] - 1);
+    return cells * LS * sizeof(float2) + nrows * sizeof(int64_t) + 16 * 1024 <= 227 * 1024;
 }
 
 cudaError_t launch_gather_cm(const GatherParams<float>& p, cudaStream_t s) {

@@ -1,6 +1,6 @@
 // Internal declarations shared by the host planner (gbn_plan.cu) and the
 // device kernels (gbn_gather.cu, gbn_visit.cuh, gbn_spread.cu, gbn_padcrop.cu, gbn_grad.cu,
-// gbn_colfft.cu, ...).
+// gbn_fftpass.cu, ...).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -323,51 +323,37 @@ cudaError_t launch_permute_int4(const int4* in, const unsigned* order, int64_t n
 cudaError_t launch_permute_int2(const int2* in, const unsigned* order, int64_t n, int2* out, cudaStream_t s);
 template <typename R> cudaError_t launch_bin_pack(const PackParams<R>& p, cudaStream_t s);
 
-// Pruned FFT pass along a strided axis (gbn_colfft.cu): planes x planes2
-// arrays at offsets y * ps + z * ps2, each [L][S] (S columns, row stride S);
-// rows >= nin are read as zero, rows >= nout are not written.  in == out is
-// allowed.
-struct ColFftParams {
+// Pruned FFT pass along one axis (gbn_fftpass.cu), of length L.
+//   Plain (sn null): ncols columns; column j = array j / S, place j % S, its
+//   element n at in[(j / S) psi + j % S + n S], at out[(j / S) pso + j % S + n S];
+//   elements >= nin are read as zero, elements >= nout are not written.
+//   Image (sn set): forward, image [frames][coils][nin][Sxy] times sn
+//   [nin][Sxy] (with maps: one image [frames][nin][Sxy] times maps
+//   [coils][nin][Sxy]) to arrays [frames (pso)][L][Sxy][coils], S = Sxy coils;
+//   inverse, arrays [frames (psi)][L][Sxy][coils] to the image's nout elements
+//   times scale sn.
+struct FftPassParams {
     const float2* in;
     float2* out;
-    int64_t S;                      // columns per array, and the row stride (elements)
-    int64_t ps, ps2;                // array strides (elements)
-    int planes, planes2;
-    int L, nin, nout;
     const float2* tw;               // exp(-2 pi i m / L), m < L
-    // phase_before of the grid cells, or nullptr: the forward pass multiplies
-    // its outputs by it (and divides them by `div`, the orthonormal scale).
-    // Value (row, column) lies in cell row * (S / coils) + column / coils.
+    int L, nin, nout;
+    int64_t ncols, S, psi, pso;
+    const float* sn;
+    const float2* maps;
+    float scale;                    // image, inverse
+    int frames, coils, Sxy;
+    int cwsh, nct, nxt;             // set by the launcher: coils per CTA (log2), CTAs over coils and places
+    // Forward, plain: outputs times phase[(array % prows) L + k] (or nullptr),
+    // divided by div, the orthonormal scale.
     const float2* phase;
-    int coils;
+    int prows;
     float div;
     unsigned* check;                // checked builds: status word and extents
     int64_t in_elems, out_elems;
 };
-bool colfft_supported(int L);
+bool fftpass_supported(int L);
 // sign -1: forward (exp(-2 pi i nk / L)), +1: inverse (unnormalised)
-cudaError_t launch_colfft(const ColFftParams& p, int sign, cudaStream_t s);
-
-// Row passes of the 2-D and 3-D transforms with pad / crop folded in
-// (gbn_rowfft.cu).  Row r < rows = frames N2 N1 coils, coil fastest: image row
-// (n2, n1) of [frames][coils][N2][N1][N0] and the coil-minor grid row at
-// f * gsf + n2 * gs2 + n1 * gs1 + c (L = K0 values, `coils` apart).  sign -1:
-// sn * image -> forward FFT -> grid row; +1: grid row -> inverse FFT -> first
-// N0 values * scale * sn -> image.
-struct RowFftParams {
-    const float2* in;               // forward: image; inverse: grid
-    float2* out;                    // forward: grid; inverse: image
-    const float* sn;                // [N2][N1][N0]
-    float scale;                    // inverse only
-    int coils, N0, N1, N2, L;
-    int64_t rows;
-    int64_t gsf, gs1, gs2;
-    const float2* tw;               // exp(-2 pi i m / L), m < L
-    unsigned* check;                // checked builds: status word and extents
-    int64_t in_elems, out_elems;
-};
-bool rowfft_supported(int L);
-cudaError_t launch_rowfft(const RowFftParams& p, int sign, cudaStream_t s);
+cudaError_t launch_fftpass(const FftPassParams& p, int sign, cudaStream_t s);
 
 template <typename R> cudaError_t launch_gather(const GatherParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_visit_count(const VisitBuildParams<R>& p, cudaStream_t s);
@@ -377,6 +363,9 @@ template <typename R> cudaError_t launch_spread_visits(const VisitParams<R>& p, 
 template <typename R> cudaError_t launch_reduce(const ReduceParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_pad(const PadParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_crop(const CropParams<R>& p, cudaStream_t s);
+// x[f] = sum_c conj(maps[c]) * images[f][c], in coil order; n values per image.
+cudaError_t launch_combine(const float2* images, const float2* maps, float2* x, int frames, int coils, int64_t n,
+                           cudaStream_t s);
 template <typename R> cudaError_t launch_grad(const GradParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_coef(const CoefParams<R>& p, cudaStream_t s);
 // phase_before of every grid cell, [K_{ndim-1}]...[K_0].

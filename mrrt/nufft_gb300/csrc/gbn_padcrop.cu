@@ -254,4 +254,31 @@ template cudaError_t launch_pad<double>(const PadParams<double>&, cudaStream_t);
 template cudaError_t launch_crop<float>(const CropParams<float>&, cudaStream_t);
 template cudaError_t launch_crop<double>(const CropParams<double>&, cudaStream_t);
 
+// Coil combination of a transform on the library's own passes, whose last
+// pass leaves one image per coil: a thread per image value, eight coils'
+// loads in flight, summed in coil order.
+__global__ void __launch_bounds__(256) combine_kernel(const float2* images, const float2* maps, float2* x, int coils,
+                                                      int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float2* im = images + (int64_t)blockIdx.y * coils * n + i;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int c = 0; c < coils; ++c) {
+        const float2 v = cmulc(im[c * n], __ldg(maps + c * n + i));
+        acc.x += v.x;
+        acc.y += v.y;
+    }
+    x[blockIdx.y * n + i] = acc;
+}
+
+cudaError_t launch_combine(const float2* images, const float2* maps, float2* x, int frames, int coils, int64_t n,
+                           cudaStream_t s) {
+    for (int f = 0; f < frames; f += 65535) {   // grid.y
+        const dim3 grid((unsigned)((n + 255) / 256), (unsigned)(frames - f < 65535 ? frames - f : 65535));
+        combine_kernel<<<grid, 256, 0, s>>>(images + (int64_t)f * coils * n, maps, x + f * n, coils, n);
+    }
+    return cudaGetLastError();
+}
+
 }  // namespace gbn

@@ -235,12 +235,13 @@ struct gbn_plan {
     int64_t glen = 0, slen = 0;
     DevBuf pad, grid, scratch;
     DevBuf ptab;               // phase_before of every grid cell (real phasing)
-    DevBuf mid;           // output of the forward's slab pass (2-D rows, 3-D z-planes); the
-                          // slabs >= N_last the last-axis pass reads stay zero
+    DevBuf coil_images;   // own passes, combining adjoint: one image per coil
+    DevBuf half;          // own passes: the array between them, N_0 of K_0 along axis 0
+    DevBuf mid;           // around cuFFT: output of the forward's slab pass (2-D rows, 3-D z-planes);
+                          // the slabs >= N_last the last-axis pass reads stay zero
     int64_t mid_clean = 0;     // 2-D: slabs from which mid is known to be zero
-    bool colfft = false;       // last-axis pass by gbn_colfft.cu (else cuFFT)
-    bool rowfft = false;       // every pass on the plan's kernels, the row passes with the pad
-                               // and crop folded in (gbn_rowfft.cu, gbn_colfft.cu)
+    bool colfft = false;       // around cuFFT: last-axis pass by gbn_fftpass.cu (else cuFFT)
+    bool own = false;          // every pass on the plan's kernels, pad and crop folded in (gbn_fftpass.cu)
     DevBuf fft_tw[3];          // per axis d: exp(-2 pi i m / K_d), m < K_d (axes those use)
     int mid_planes = 0;        // planes the mid buffer holds
     int cap_planes = 0;        // planes the grid buffer holds
@@ -751,9 +752,10 @@ int ensure_scratch(gbn_plan* P, int coils) {
 }
 
 // FFT grid and scratch for F * coils planes; around cuFFT's passes also the
-// zero-padded input and the pruned passes' intermediate buffer.  `own`: the
-// call runs on the plan's own passes, in place on the grid.
-int ensure_buffers(gbn_plan* P, int coils, bool own) {
+// zero-padded input and the pruned passes' intermediate buffer; on the plan's
+// own passes (`own`) the array between them and, for a combining adjoint
+// (`images`), the coil images.
+int ensure_buffers(gbn_plan* P, int coils, bool own, bool images = false) {
     const int planes = P->F * coils;
     const size_t csz = (size_t)2 * P->rsize;
     const size_t bytes = (size_t)planes * P->Kprod * csz;
@@ -763,6 +765,11 @@ int ensure_buffers(gbn_plan* P, int coils, bool own) {
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "grid buffer allocation failed");
         P->cap_planes = planes;
     }
+    auto grow_to = [](DevBuf& b, size_t n) { return b.bytes >= n ? cudaSuccess : b.alloc(n); };
+    if (own && grow_to(P->half, bytes / P->geom.Kd[0] * P->geom.Nd[0]) != cudaSuccess)
+        return fail(GBN_ERR_NOMEM, "FFT pass buffer allocation failed");
+    if (images && grow_to(P->coil_images, (size_t)planes * P->Nprod * csz) != cudaSuccess)
+        return fail(GBN_ERR_NOMEM, "coil image allocation failed");
     if (!own && planes > P->pad_planes) {
         P->pad_planes = 0;
         cudaError_t e = P->pad.alloc(bytes);
@@ -786,7 +793,7 @@ int ensure_buffers(gbn_plan* P, int coils, bool own) {
     return ensure_scratch(P, coils);
 }
 
-// The last-axis pass runs on the plan's own pruned kernel (gbn_colfft.cu) in
+// The last-axis pass runs on the plan's own pruned kernel (gbn_fftpass.cu) in
 // single precision, 2-D and 3-D, for the lengths it implements, unless the
 // geometry asks for cuFFT throughout.  Its twiddles are computed here in
 // double precision and rounded once.
@@ -804,85 +811,86 @@ int upload_twiddles(DevBuf& dst, int L) {
 }
 
 // When every axis has a supported length, the whole transform runs on the
-// plan's kernels, the row passes with the pad and the crop folded in
-// (gbn_rowfft.cu).
+// plan's kernels, with the pad and the crop folded in.
 int setup_colfft(gbn_plan* P) {
     const gbn_geometry& G = P->geom;
     const int L = G.Kd[G.ndim - 1];
-    P->colfft = !P->dbl && G.ndim >= 2 && !(G.flags & GBN_FLAG_CUFFT_ONLY) && colfft_supported(L);
+    P->colfft = !P->dbl && G.ndim >= 2 && !(G.flags & GBN_FLAG_CUFFT_ONLY) && fftpass_supported(L);
     if (!P->colfft) return GBN_OK;
-    P->rowfft = rowfft_supported(G.Kd[0]) && (G.ndim == 2 || colfft_supported(G.Kd[1]));
+    P->own = fftpass_supported(G.Kd[0]) && (G.ndim == 2 || fftpass_supported(G.Kd[1]));
     for (int d = 0; d < G.ndim; ++d) {
-        if (d < G.ndim - 1 && !P->rowfft) continue;
+        if (d < G.ndim - 1 && !P->own) continue;
         int rc = upload_twiddles(P->fft_tw[d], G.Kd[d]);
         if (rc) return rc;
     }
     return GBN_OK;
 }
 
-// Row pass with the pad (sign -1: image -> grid rows) or the crop (sign +1:
-// grid rows -> image) folded in, on the coil-minor grid.
-int run_rowfft(gbn_plan* P, const void* in, void* out, int coils, int sign, cudaStream_t s) {
-    const gbn_geometry& G = P->geom;
-    RowFftParams p;
-    std::memset(&p, 0, sizeof(p));
-    p.in = static_cast<const float2*>(in);
-    p.out = static_cast<float2*>(out);
-    p.sn = static_cast<const float*>(P->sn.p);
-    p.scale = G.ortho ? (float)(G.adjoint_scale / std::sqrt((double)P->Kprod)) : (float)G.adjoint_scale;
-    p.coils = coils;
-    p.N0 = G.Nd[0];
-    p.N1 = G.Nd[1];
-    p.N2 = G.ndim > 2 ? G.Nd[2] : 1;
-    p.rows = (int64_t)P->F * coils * p.N1 * p.N2;
-    p.L = G.Kd[0];
-    p.gsf = P->Kprod * coils;
-    p.gs1 = (int64_t)G.Kd[0] * coils;
-    p.gs2 = (int64_t)G.Kd[0] * G.Kd[1] * coils;
-    p.tw = static_cast<const float2*>(P->fft_tw[0].p);
-    p.check = static_cast<unsigned*>(P->check.p);
-    const int64_t img = (int64_t)P->F * coils * P->Nprod, grid = (int64_t)P->cap_planes * P->Kprod;
-    p.in_elems = sign < 0 ? img : grid;
-    p.out_elems = sign < 0 ? grid : img;
-    GBN_CUDA(launch_rowfft(p, sign, s), sign < 0 ? "pad + row FFT pass" : "row FFT pass + crop");
-    return GBN_OK;
-}
-
-// Pass along memory axis `axis` (1 or 2) over planes x planes2 arrays of
-// [K_axis][S] at strides ps, ps2: rows >= nin read as zero, rows >= nout not
-// written.
+// Plain pass along memory axis `axis` over `arrays` arrays of [K_axis][S] at
+// strides psi, pso: elements >= nin read as zero, elements >= nout not written.
 struct AxisPass {
     const void* in;
     int64_t in_elems;
     void* out;
     int64_t out_elems;
     int axis;
-    int64_t S, ps, ps2;
-    int planes, planes2;
+    int64_t S, arrays, psi, pso;
     int nin, nout;
-    int phase_coils = 0;   // coils of a coil-minor grid to which phase_before is applied (0: none)
+    bool phase = false;   // coil-minor grid rows: times phase_before
 };
-int run_colfft(gbn_plan* P, const AxisPass& a, int sign, cudaStream_t s) {
-    ColFftParams p;
+int run_pass(gbn_plan* P, const AxisPass& a, int sign, cudaStream_t s) {
+    const gbn_geometry& G = P->geom;
+    FftPassParams p;
     std::memset(&p, 0, sizeof(p));
     p.in = static_cast<const float2*>(a.in);
     p.out = static_cast<float2*>(a.out);
-    p.S = a.S;
-    p.ps = a.ps;
-    p.ps2 = a.ps2;
-    p.planes = a.planes;
-    p.planes2 = a.planes2;
-    p.L = P->geom.Kd[a.axis];
+    p.tw = static_cast<const float2*>(P->fft_tw[a.axis].p);
+    p.L = G.Kd[a.axis];
     p.nin = a.nin;
     p.nout = a.nout;
-    p.tw = static_cast<const float2*>(P->fft_tw[a.axis].p);
-    p.phase = a.phase_coils ? static_cast<const float2*>(P->ptab.p) : nullptr;
-    p.coils = a.phase_coils;
-    p.div = P->geom.ortho ? (float)std::sqrt((double)P->Kprod) : 1.f;
+    p.S = a.S;
+    p.ncols = a.S * a.arrays;
+    p.psi = a.psi;
+    p.pso = a.pso;
+    if (a.phase) {
+        p.phase = static_cast<const float2*>(P->ptab.p);
+        p.prows = (int)(P->Kprod / G.Kd[0]);
+    }
+    p.div = G.ortho ? (float)std::sqrt((double)P->Kprod) : 1.f;
     p.check = static_cast<unsigned*>(P->check.p);
     p.in_elems = a.in_elems;
     p.out_elems = a.out_elems;
-    GBN_CUDA(launch_colfft(p, sign, s), "strided-axis FFT pass");
+    GBN_CUDA(launch_fftpass(p, sign, s), "FFT pass");
+    return GBN_OK;
+}
+
+// Pass between the image and the first array of a transform on the plan's own
+// passes, along the slowest axis: forward (with maps: one image per frame
+// times the coil maps) or inverse.
+int image_pass(gbn_plan* P, const void* in, void* out, const void* maps, int coils, int sign, cudaStream_t s) {
+    const gbn_geometry& G = P->geom;
+    const int a = G.ndim - 1;
+    FftPassParams p;
+    std::memset(&p, 0, sizeof(p));
+    p.in = static_cast<const float2*>(in);
+    p.out = static_cast<float2*>(out);
+    p.tw = static_cast<const float2*>(P->fft_tw[a].p);
+    p.L = G.Kd[a];
+    p.nin = sign < 0 ? G.Nd[a] : G.Kd[a];
+    p.nout = sign < 0 ? G.Kd[a] : G.Nd[a];
+    p.sn = static_cast<const float*>(P->sn.p);
+    p.maps = static_cast<const float2*>(maps);
+    p.scale = G.ortho ? (float)(G.adjoint_scale / std::sqrt((double)P->Kprod)) : (float)G.adjoint_scale;
+    p.frames = P->F;
+    p.coils = coils;
+    p.Sxy = (int)(P->Nprod / G.Nd[a]);
+    p.S = (int64_t)p.Sxy * coils;
+    p.psi = p.pso = p.S * p.L;
+    p.check = static_cast<unsigned*>(P->check.p);
+    const int64_t img = (int64_t)P->F * (maps ? 1 : coils) * P->Nprod, arr = (int64_t)P->F * p.psi;
+    p.in_elems = sign < 0 ? img : arr;
+    p.out_elems = sign < 0 ? arr : img;
+    GBN_CUDA(launch_fftpass(p, sign, s), sign < 0 ? "pad + FFT pass" : "FFT pass + crop");
     return GBN_OK;
 }
 
@@ -935,19 +943,19 @@ int exec_fft(gbn_plan* P, cufftHandle h, void* in, void* out, int dir, cudaStrea
     return GBN_OK;
 }
 
-// 2-D last-axis pass: forward mid -> grid (the N_1 slabs with data read),
-// inverse grid -> grid in place (the N_1 slabs the crop reads written).
+// 2-D last-axis pass around cuFFT: forward mid -> grid (the N_1 slabs with
+// data read), inverse grid -> grid in place (the N_1 slabs the crop reads
+// written).
 int colfft_2d(gbn_plan* P, int planes, int sign, cudaStream_t s) {
     const int64_t ge = (int64_t)P->cap_planes * P->Kprod;
-    AxisPass a{P->grid.p, ge, P->grid.p, ge, 1, (int64_t)planes * P->geom.Kd[0], 0, 0, 1, 1,
-               P->geom.Kd[1], last_n(P)};
+    AxisPass a{P->grid.p, ge, P->grid.p, ge, 1, (int64_t)planes * P->geom.Kd[0], 1, 0, 0, P->geom.Kd[1], last_n(P)};
     if (sign < 0) {
         a.in = P->mid.p;
         a.in_elems = (int64_t)P->mid_planes * P->Kprod;
         a.nin = last_n(P);
         a.nout = P->geom.Kd[1];
     }
-    return run_colfft(P, a, sign, s);
+    return run_pass(P, a, sign, s);
 }
 
 // Whether a forward call leaves phase_before (and the orthonormal scale)
@@ -955,28 +963,30 @@ int colfft_2d(gbn_plan* P, int planes, int sign, cudaStream_t s) {
 // gbn_grad_tm takes, from before it.
 bool grid_phased(const gbn_plan* P) { return P->geom.phasing == GBN_PHASING_REAL && !P->dtables.p; }
 
-// The strided passes of a transform on the plan's own passes, in place on the
-// coil-minor grid: forward axis 1 over the N_2 z-slabs with data (N_1 rows
-// read), then in 3-D axis 2 (N_2 z-slabs read), phase_before with the last;
-// inverse axis 2 (N_2 z-slabs written), then axis 1 over those slabs (N_1
-// rows written).
-int own_passes(gbn_plan* P, int coils, int sign, cudaStream_t s) {
+// Transform on the plan's own passes, on coil-minor arrays, widening the axes
+// from the slowest to the contiguous one (sign -1) or narrowing them back:
+//   2-D: image <-> half [K1][N0] <-> grid [K1][K0];
+//   3-D: image <-> grid, as [K2][N1][N0] <-> half [K2][K1][N0] <-> grid [K2][K1][K0].
+int own_transform(gbn_plan* P, const void* x, void* xa, const void* maps, int coils, int sign, cudaStream_t s) {
     const gbn_geometry& G = P->geom;
-    const int64_t ge = (int64_t)P->cap_planes * P->Kprod;
-    const int64_t row = (int64_t)G.Kd[0] * coils, slab = row * G.Kd[1], vol = P->Kprod * coils;
     const bool d3 = G.ndim == 3;
-    AxisPass a1{P->grid.p, ge, P->grid.p, ge, 1, row, d3 ? slab : vol, vol, d3 ? G.Nd[2] : P->F, d3 ? P->F : 1,
-                sign < 0 ? G.Nd[1] : G.Kd[1], sign < 0 ? G.Kd[1] : G.Nd[1]};
-    const int pc = sign < 0 && grid_phased(P) ? coils : 0;
-    if (!d3) {
-        a1.phase_coils = pc;
-        return run_colfft(P, a1, sign, s);
+    const int64_t ge = (int64_t)P->cap_planes * P->Kprod, he = (int64_t)(P->half.bytes / sizeof(float2));
+    const int64_t rows = (int64_t)P->F * (P->Kprod / G.Kd[0]);   // grid rows of all frames
+    const int64_t rn = (int64_t)G.Nd[0] * coils, rk = (int64_t)G.Kd[0] * coils;
+    void *half = P->half.p, *grid = P->grid.p, *small = d3 ? grid : half;
+    int rc = GBN_OK;
+    if (sign < 0) {
+        if ((rc = image_pass(P, x, small, maps, coils, -1, s))) return rc;
+        if (d3 && (rc = run_pass(P, AxisPass{grid, ge, half, he, 1, rn, (int64_t)P->F * G.Kd[2], rn * G.Nd[1],
+                                             rn * G.Kd[1], G.Nd[1], G.Kd[1]}, -1, s)))
+            return rc;
+        return run_pass(P, AxisPass{half, he, grid, ge, 0, coils, rows, rn, rk, G.Nd[0], G.Kd[0], grid_phased(P)}, -1, s);
     }
-    AxisPass a2{P->grid.p, ge, P->grid.p, ge, 2, slab, vol, 0, P->F, 1,
-                sign < 0 ? G.Nd[2] : G.Kd[2], sign < 0 ? G.Kd[2] : G.Nd[2]};
-    a2.phase_coils = pc;
-    int rc = run_colfft(P, sign < 0 ? a1 : a2, sign, s);
-    return rc ? rc : run_colfft(P, sign < 0 ? a2 : a1, sign, s);
+    if ((rc = run_pass(P, AxisPass{grid, ge, half, he, 0, coils, rows, rk, rn, G.Kd[0], G.Nd[0]}, 1, s))) return rc;
+    if (d3 && (rc = run_pass(P, AxisPass{half, he, grid, ge, 1, rn, (int64_t)P->F * G.Kd[2], rn * G.Kd[1],
+                                         rn * G.Nd[1], G.Kd[1], G.Nd[1]}, 1, s)))
+        return rc;
+    return image_pass(P, small, xa, nullptr, coils, 1, s);
 }
 
 // Forward Kd-point FFT of the padded planes into the grid.  2-D and 3-D:
@@ -996,11 +1006,10 @@ int fft_forward(gbn_plan* P, int planes, cudaStream_t s) {
         for (int pl = 0; pl < planes; ++pl)
             if ((rc = exec_fft(P, f->hx, pad + pl * pb, mid + pl * pb, CUFFT_FORWARD, s))) return rc;
         if (P->colfft)
-            return run_colfft(P,
-                              AxisPass{mid, (int64_t)P->mid_planes * P->Kprod, grid,
-                                       (int64_t)P->cap_planes * P->Kprod, 2, slab_cells(P), P->Kprod, 0, planes,
-                                       1, last_n(P), P->geom.Kd[2]},
-                              -1, s);
+            return run_pass(P,
+                            AxisPass{mid, (int64_t)P->mid_planes * P->Kprod, grid, (int64_t)P->cap_planes * P->Kprod,
+                                     2, slab_cells(P), planes, P->Kprod, P->Kprod, last_n(P), P->geom.Kd[2]},
+                            -1, s);
         for (int pl = 0; pl < planes; ++pl)
             if ((rc = exec_fft(P, f->hy, mid + pl * pb, grid + pl * pb, CUFFT_FORWARD, s))) return rc;
         return GBN_OK;
@@ -1045,9 +1054,9 @@ int fft_inverse(gbn_plan* P, int planes, cudaStream_t s) {
         char* grid = static_cast<char*>(P->grid.p);
         if (P->colfft) {
             const int64_t ge = (int64_t)P->cap_planes * P->Kprod;
-            if ((rc = run_colfft(P, AxisPass{grid, ge, grid, ge, 2, slab_cells(P), P->Kprod, 0, planes, 1,
-                                             P->geom.Kd[2], last_n(P)},
-                                 1, s)))
+            if ((rc = run_pass(P, AxisPass{grid, ge, grid, ge, 2, slab_cells(P), planes, P->Kprod, P->Kprod,
+                                           P->geom.Kd[2], last_n(P)},
+                               1, s)))
                 return rc;
         } else {
             for (int pl = 0; pl < planes; ++pl)
@@ -1226,15 +1235,14 @@ int run_spread_noalloc(gbn_plan* P, const void* y, void* grid, int coils, cudaSt
 
 template <typename R>
 int run_forward(gbn_plan* P, const void* x, void* y, int coils, cudaStream_t s, const void* maps = nullptr) {
-    // single precision only (rowfft is off for double plans)
-    const bool own = P->rowfft && !maps;
+    // single precision only (`own` is off for double plans)
+    const bool own = P->own;
     int rc = ensure_buffers(P, coils, own);
     if (rc) return rc;
     if (own) {
         {
             NvtxRange r("gbn forward: pad + fft");
-            if ((rc = run_rowfft(P, x, P->grid.p, coils, -1, s))) return rc;
-            if ((rc = own_passes(P, coils, -1, s))) return rc;
+            if ((rc = own_transform(P, x, nullptr, maps, coils, -1, s))) return rc;
         }
         NvtxRange r("gbn forward: gather");
         return run_gather<R>(P, P->grid.p, y, coils, Grid::own, s);
@@ -1275,8 +1283,8 @@ template <typename R>
 int run_adjoint(gbn_plan* P, const void* y, void* x, int coils, cudaStream_t s, const void* maps = nullptr) {
     // allocate first: the grid pointer handed to the spread must be the
     // buffer this call will use (it is null before the first call)
-    const bool own = P->rowfft && !maps;
-    int rc = ensure_buffers(P, coils, own);
+    const bool own = P->own;
+    int rc = ensure_buffers(P, coils, own, own && maps);
     if (rc) return rc;
     {
         NvtxRange r("gbn adjoint: spread");
@@ -1285,8 +1293,12 @@ int run_adjoint(gbn_plan* P, const void* y, void* x, int coils, cudaStream_t s, 
     }
     if (own) {
         NvtxRange r("gbn adjoint: fft + crop");
-        if ((rc = own_passes(P, coils, 1, s))) return rc;
-        return run_rowfft(P, P->grid.p, x, coils, 1, s);
+        if (!maps) return own_transform(P, nullptr, x, nullptr, coils, 1, s);
+        if ((rc = own_transform(P, nullptr, P->coil_images.p, nullptr, coils, 1, s))) return rc;
+        GBN_CUDA(launch_combine(static_cast<const float2*>(P->coil_images.p), static_cast<const float2*>(maps),
+                                static_cast<float2*>(x), P->F, coils, P->Nprod, s),
+                 "coil combination launch");
+        return GBN_OK;
     }
     {
         NvtxRange r("gbn adjoint: fft");
@@ -1898,7 +1910,7 @@ int run_grad(gbn_plan* P, const void* grid, const void* gy, const double* shift,
     GradParams<R> p;
     std::memset(&p, 0, sizeof(p));
     p.g = make_geom<R>(P, false);
-    grid_layout<R>(P, coils, P->rowfft ? Grid::own : Grid::cufft, p.g);   // as a forward call with these coils left it
+    grid_layout<R>(P, coils, P->own ? Grid::own : Grid::cufft, p.g);   // as a forward call with these coils left it
     const SampleList<R> L = make_list<R>(P, P->glist, P->glen, false);
     const R* db = reinterpret_cast<const R*>(P->dtables.p);
     size_t off = 0;
@@ -2235,7 +2247,7 @@ int gbn_plan_stats(const gbn_plan* P, int64_t* o) {
     o[5] = (int64_t)P->ntiles_s * P->F;
     o[6] = (int64_t)(P->tables.bytes + P->weights.bytes + P->gcoef.bytes +
                      P->vstart.bytes + P->vidx.bytes + P->vco.bytes + P->vwork.bytes + P->phnat.bytes +
-                     P->vals.bytes + P->ptab.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
+                     P->vals.bytes + P->ptab.bytes + P->half.bytes + P->coil_images.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
                      P->grid.bytes + P->scratch.bytes);
     o[7] = P->M_total;
     return GBN_OK;
