@@ -351,17 +351,19 @@ def config_dict(extra=None):
     return cfg
 
 
-# FFT lengths the library transforms with its own passes (gbn_colfft.cu,
-# gbn_rowfft.cu); the other lengths use cuFFT (whose launches are not ours)
-OWN_FFT_LENGTHS = (64, 96, 128, 192, 256, 384, 512, 768)
+# FFT lengths the library transforms with its own passes (gbn_fftpass.cuh); the
+# other lengths use cuFFT (whose launches are not ours)
+OWN_FFT_LENGTHS = (60, 64, 72, 90, 96, 100, 120, 128, 144, 150, 160, 180, 192, 200, 240, 256, 288, 300, 320,
+                   360, 384, 400, 450, 480, 512, 576, 600, 640, 720, 768)
 
 
-def our_launches_per_step(Kd, split_tiles):
+def our_launches_per_step(Kd, split_tiles, coils=1):
     """Launches of this library's kernels in one forward + adjoint pair of a
-    single-precision plan: with every axis length supported, the row pass
-    (pad or crop folded in), the strided-axis passes and the interpolation
-    kernel each way; else pad / crop and the interpolation kernel, plus the
-    last-axis pass when its length is supported; the reduce of split tiles."""
+    single-precision plan: with every axis length supported, a pass per axis
+    (pad or crop folded in) and the interpolation kernel each way; else pad /
+    crop and the interpolation kernel, plus the last-axis pass when its length
+    is supported; the coil-minor sample values from five coils on; the reduce
+    of split tiles."""
     nd = len(Kd)
     if nd >= 2 and all(k in OWN_FFT_LENGTHS for k in Kd):
         per_dir = nd + 1
@@ -369,7 +371,7 @@ def our_launches_per_step(Kd, split_tiles):
         per_dir = 3
     else:
         per_dir = 2
-    return 2 * per_dir + (1 if split_tiles > 0 else 0)
+    return 2 * per_dir + (1 if split_tiles > 0 else 0) + (1 if coils >= 5 else 0)
 
 
 def _clock_path(rank):
@@ -448,7 +450,7 @@ def run_ours(args, rank, world):
         parity_gate(parity)
 
     stats = P.stats()
-    launches_per_step = our_launches_per_step(w["Kd"], stats["split_tiles"])
+    launches_per_step = our_launches_per_step(w["Kd"], stats["split_tiles"], w["coils"])
 
     # ---- batched, device resident: the step replayed from a CUDA graph -----
     for _ in range(args.warmup):
@@ -769,7 +771,7 @@ def run_series(args, rank, world):
         parity_gate(parity)
 
     stats = S.plan.stats()
-    launches_per_step = our_launches_per_step(w["Kd"], stats["split_tiles"])
+    launches_per_step = our_launches_per_step(w["Kd"], stats["split_tiles"], w["coils"])
 
     # ---- batched series from CUDA graphs, device resident -------------------
     for _ in range(args.warmup):

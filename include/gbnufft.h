@@ -55,11 +55,13 @@ extern "C" {
  * buffers and interpolates the tables inside the kernels instead (same
  * results bit for bit, less device memory).                               */
 #define GBN_FLAG_TABLE_ONLY 1
-/* By default the single-precision 2-D and 3-D plans run the FFT's pass
- * along the slowest axis on the library's own pruned kernel when that
- * axis's length is 64, 96, 128, 192, 256, 384, 512 or 768 (it reads
- * only the rows that hold data and writes only the rows the crop reads);
- * CUFFT_ONLY runs every pass through cuFFT instead.                         */
+/* By default single-precision 2-D and 3-D plans run the FFT on the library's
+ * own pruned passes (which read only the rows that hold data and write only
+ * the rows the crop reads) when every axis length is one of 60, 64, 72, 90,
+ * 96, 100, 120, 128, 144, 150, 160, 180, 192, 200, 240, 256, 288, 300, 320,
+ * 360, 384, 400, 450, 480, 512, 576, 600, 640, 720, 768; with a supported
+ * length of the slowest axis alone, that axis's pass.  CUFFT_ONLY runs every
+ * pass through cuFFT instead.                                               */
 #define GBN_FLAG_CUFFT_ONLY 2
 
 /* Geometry of one operator (or of a series of frames sharing it). */
