@@ -71,3 +71,38 @@ def test_spread_matches_oracle(gpu_lib, K, J, coils, precision, phasing):
     T, _ = _plan(K, J, tm, rdt, phasing, coils, table_only=True)
     T.interp_adjoint(yd, out[1], coils)
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("N,K,J,coils", [
+    ((30, 33), (64, 72), 6, 1), ((30, 33), (64, 72), 5, 2), ((30, 33), (64, 72), 4, 3), ((30, 33), (64, 72), 6, 4),
+    ((30, 33), (64, 72), 5, 7), ((30, 33), (64, 72), 6, 8), ((30, 33), (64, 72), 4, 13), ((30, 33), (64, 72), 6, 35),
+    ((30, 33, 32), (60, 64, 64), 6, 1), ((30, 33, 32), (60, 64, 64), 4, 2), ((30, 33, 32), (60, 64, 64), 5, 3),
+    ((30, 33, 32), (60, 64, 64), 6, 11),
+])
+def test_gather_matches_oracle(gpu_lib, N, K, J, coils):
+    """Coil-minor gather (gbn_gather_cm.cu): the forward transform for every
+    coil-lane count, odd and even coil counts (8- and 16-byte copies), ragged
+    last chunks, kernel widths whose taps fill the lane groups unevenly, heavy
+    and nearly empty tiles, against the oracle; the same bits without
+    precomputed coefficients."""
+    from mrrt.nufft_gb300 import NufftBase
+    from mrrt.nufft_gb300._kernels import kernel_table
+    from mrrt.nufft_gb300._plan import GpuPlan
+
+    rng = np.random.default_rng(coils)
+    nd, M = len(N), 2500
+    omega = rng.uniform(-np.pi, np.pi, (M, nd))
+    omega[:700] = 0.3 + 0.02 * rng.random((700, nd))
+    kw = dict(Nd=N, omega=omega, Jd=(J,) * nd, Kd=K)
+    x = (rng.standard_normal(N + (coils,)) + 1j * rng.standard_normal(N + (coils,))).astype(np.complex64)
+    y = NufftBase(max_coils=coils, **kw).fft(x)
+    assert rel_l2(y, O.OracleNufft(**kw).fft(x).reshape(y.shape)) < 1e-5
+    h = [kernel_table(N[d], J, K[d], 512, "real", np.float32) for d in range(nd)]
+    tm = (omega / (2 * np.pi / np.asarray(K))).astype(np.float32)
+    xt = torch.from_numpy(x).permute(*reversed(range(nd + 1))).contiguous().cuda()
+    out = []
+    for table_only in (False, True):
+        P = GpuPlan(N, K, (J,) * nd, 512, np.float32, h, None, np.ones(int(np.prod(N)), np.float32), tm, None,
+                    max_coils=coils, table_only=table_only)
+        out.append(P.forward(xt, torch.empty((coils, M), dtype=torch.complex64, device="cuda"), coils))
+    assert torch.equal(out[0], out[1])
