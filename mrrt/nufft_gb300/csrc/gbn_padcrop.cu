@@ -8,8 +8,8 @@
 // reference's prod(Kd) * adjoint_scalefactor with ifftn's 1/prod(Kd)
 // (or the orthonormal factors).
 //
-// One warp per image row (memory axis 0); rows are enumerated over
-// (plane, axis 1, axis 2).  The coil-sensitivity variants fuse the MRI
+// One warp per image row (memory axis 0), or per segment of a long one; rows
+// are enumerated over (plane, axis 1, axis 2).  The coil-sensitivity variants fuse the MRI
 // system operator's coil-map multiply (forward) and conjugate-map coil sum
 // (adjoint) into these passes.
 #include <cuda_runtime.h>
@@ -25,14 +25,17 @@ namespace gbn {
 // sides; a lane then moves two adjacent complex values per access (16-byte
 // loads and stores, 8-byte loads of sn), four accesses in flight.
 template <typename R, bool PAIRS>
-__global__ void __launch_bounds__(256) pad_kernel(const PadParams<R> p) {
+__global__ void __launch_bounds__(256) pad_kernel(const PadParams<R> p, const int seg) {
     typedef typename Cx<R>::T C;
     const int lane = threadIdx.x & 31;
     const int64_t rows_per_plane = (int64_t)p.N[1] * p.N[2];
     const int64_t nrows = rows_per_plane * p.planes;
+    const int64_t segs = (p.N[0] + seg - 1) / seg;   // a warp takes `seg` (even) values of a row
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t row = wid; row < nrows; row += nw) {
+    for (int64_t w = wid; w < nrows * segs; w += nw) {
+        const int64_t row = w / segs;
+        const int lo = (int)(w - row * segs) * seg, hi = min(p.N[0], lo + seg);
         const int64_t pl = row / rows_per_plane;
         const int64_t rr = row - pl * rows_per_plane;
         const int n1 = (int)(rr % p.N[1]);
@@ -49,23 +52,23 @@ __global__ void __launch_bounds__(256) pad_kernel(const PadParams<R> p) {
             const float4* s4 = reinterpret_cast<const float4*>(src);
             const float2* w2 = reinterpret_cast<const float2*>(s);
             float4* d4 = reinterpret_cast<float4*>(dst);
-            const int np = p.N[0] >> 1;
+            const int np = hi >> 1;
 #pragma unroll 4
-            for (int q = lane; q < np; q += 32) {
+            for (int q = (lo >> 1) + lane; q < np; q += 32) {
                 float4 v = s4[q];
-                const float2 w = w2[q];
-                v.x *= w.x;
-                v.y *= w.x;
-                v.z *= w.y;
-                v.w *= w.y;
+                const float2 f = w2[q];
+                v.x *= f.x;
+                v.y *= f.x;
+                v.z *= f.y;
+                v.w *= f.y;
                 d4[q] = v;
             }
         } else {
-            for (int n0 = lane; n0 < p.N[0]; n0 += 32) {
+            for (int n0 = lo + lane; n0 < hi; n0 += 32) {
                 C v = src[n0];
-                const R w = s[n0];
-                v.x *= w;
-                v.y *= w;
+                const R f = s[n0];
+                v.x *= f;
+                v.y *= f;
                 dst[n0] = v;
             }
         }
@@ -73,14 +76,17 @@ __global__ void __launch_bounds__(256) pad_kernel(const PadParams<R> p) {
 }
 
 template <typename R, bool PAIRS>
-__global__ void __launch_bounds__(256) crop_kernel(const CropParams<R> p) {
+__global__ void __launch_bounds__(256) crop_kernel(const CropParams<R> p, const int seg) {
     typedef typename Cx<R>::T C;
     const int lane = threadIdx.x & 31;
     const int64_t rows_per_plane = (int64_t)p.N[1] * p.N[2];
     const int64_t nrows = rows_per_plane * p.planes;
+    const int64_t segs = (p.N[0] + seg - 1) / seg;   // a warp takes `seg` (even) values of a row
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t row = wid; row < nrows; row += nw) {
+    for (int64_t w = wid; w < nrows * segs; w += nw) {
+        const int64_t row = w / segs;
+        const int lo = (int)(w - row * segs) * seg, hi = min(p.N[0], lo + seg);
         const int64_t pl = row / rows_per_plane;
         const int64_t rr = row - pl * rows_per_plane;
         const int n1 = (int)(rr % p.N[1]);
@@ -97,30 +103,30 @@ __global__ void __launch_bounds__(256) crop_kernel(const CropParams<R> p) {
             const float4* s4 = reinterpret_cast<const float4*>(src);
             const float2* w2 = reinterpret_cast<const float2*>(s);
             float4* d4 = reinterpret_cast<float4*>(dst);
-            const int np = p.N[0] >> 1;
+            const int np = hi >> 1;
             const float sc = (float)p.scale;
 #pragma unroll 4
-            for (int q = lane; q < np; q += 32) {
+            for (int q = (lo >> 1) + lane; q < np; q += 32) {
                 float4 v = s4[q];
-                const float2 w = w2[q];
+                const float2 f = w2[q];
                 v.x *= sc;
                 v.y *= sc;
                 v.z *= sc;
                 v.w *= sc;
-                v.x *= w.x;
-                v.y *= w.x;
-                v.z *= w.y;
-                v.w *= w.y;
+                v.x *= f.x;
+                v.y *= f.x;
+                v.z *= f.y;
+                v.w *= f.y;
                 d4[q] = v;
             }
         } else {
-            for (int n0 = lane; n0 < p.N[0]; n0 += 32) {
+            for (int n0 = lo + lane; n0 < hi; n0 += 32) {
                 C v = src[n0];
                 v.x *= p.scale;
                 v.y *= p.scale;
-                const R w = s[n0];
-                v.x *= w;
-                v.y *= w;
+                const R f = s[n0];
+                v.x *= f;
+                v.y *= f;
                 dst[n0] = v;
             }
         }
@@ -217,17 +223,24 @@ static int row_grid(int64_t nrows) {
     return (int)blocks;
 }
 
+// Values of a row a warp takes: all of them, or 128 where there are too few
+// rows to fill the device (48 rows of 1000, a 1-D batch: pad and crop 13 us
+// each with a warp per row).
+static int row_segment(int64_t nrows, int N0) { return nrows < 152 * 16 && N0 > 128 ? 128 : N0 + (N0 & 1); }
+
 template <typename R>
 cudaError_t launch_pad(const PadParams<R>& p, cudaStream_t s) {
     if (p.planes == 0 || p.Nprod == 0) return cudaSuccess;
     const int64_t nrows = (int64_t)p.N[1] * p.N[2] * p.planes;
+    const int seg = row_segment(nrows, p.N[0]);
+    const int64_t segs = (p.N[0] + seg - 1) / seg;
     if (p.maps) {
         if (p.coils < 1) return cudaErrorInvalidValue;
         pad_sense_kernel<R><<<row_grid(nrows), 256, 0, s>>>(p);
     } else if (pairs_ok<R>(p.N[0], p.Nprod, p.gsp, p.gs1, p.gs2, p.x, p.out)) {
-        pad_kernel<R, true><<<row_grid(nrows), 256, 0, s>>>(p);
+        pad_kernel<R, true><<<row_grid(nrows * segs), 256, 0, s>>>(p, seg);
     } else {
-        pad_kernel<R, false><<<row_grid(nrows), 256, 0, s>>>(p);
+        pad_kernel<R, false><<<row_grid(nrows * segs), 256, 0, s>>>(p, seg);
     }
     return cudaGetLastError();
 }
@@ -241,10 +254,12 @@ cudaError_t launch_crop(const CropParams<R>& p, cudaStream_t s) {
         crop_sense_kernel<R><<<row_grid(nrows), 256, 0, s>>>(p);
     } else {
         const int64_t nrows = (int64_t)p.N[1] * p.N[2] * p.planes;
+        const int seg = row_segment(nrows, p.N[0]);
+        const int64_t segs = (p.N[0] + seg - 1) / seg;
         if (pairs_ok<R>(p.N[0], p.Nprod, p.gsp, p.gs1, p.gs2, p.grid, p.x))
-            crop_kernel<R, true><<<row_grid(nrows), 256, 0, s>>>(p);
+            crop_kernel<R, true><<<row_grid(nrows * segs), 256, 0, s>>>(p, seg);
         else
-            crop_kernel<R, false><<<row_grid(nrows), 256, 0, s>>>(p);
+            crop_kernel<R, false><<<row_grid(nrows * segs), 256, 0, s>>>(p, seg);
     }
     return cudaGetLastError();
 }

@@ -466,6 +466,19 @@ void choose_tiles(gbn_plan* P) {
         if (ln.LS >= 4) { T[0] = 8; T[1] = 8; T[2] = 4; }
         else { T[0] = 8; T[1] = 8; T[2] = 8; }
     }
+    // two tiles per SM at least, down to edges of 8 (32 in 1-D): a 256 x 256
+    // grid of one coil in 32 x 32 tiles kept 64 SMs busy, 2000 cells in tiles
+    // of 256 sixteen CTAs (48 coils: gather 42 us)
+    for (;;) {
+        int64_t tiles = (int64_t)P->F * ((G.max_coils + ln.LS - 1) / ln.LS);
+        int dm = 0;
+        for (int d = 0; d < ndim; ++d) {
+            tiles *= (G.Kd[d] + T[d] - 1) / T[d];
+            if (T[d] > T[dm]) dm = d;
+        }
+        if (tiles >= 2 * 152 || T[dm] <= (ndim == 1 ? 32 : 8)) break;
+        T[dm] /= 2;
+    }
     for (int d = 0; d < ndim; ++d)
         if (G.tile[d] > 0) T[d] = G.tile[d];
     const size_t csz = (size_t)2 * P->rsize;
