@@ -25,6 +25,13 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def raw_stream(index):
+    """The current stream of CUDA device ``index`` as an integer handle
+    (``torch.cuda.current_stream`` builds a Stream object first: 3 of the 17 us
+    a small transform's call takes on a Grace core)."""
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
 def require_cuda():
     if not torch.cuda.is_available():
         raise RuntimeError("mrrt.nufft_gb300 needs a CUDA GPU: torch.cuda.is_available() is False")
@@ -104,6 +111,9 @@ class GpuPlan:
 
     # -- transforms on device tensors in the plan's memory layout -------------
     def _check(self, t, numel, name):
+        if type(t) is torch.Tensor and t.is_cuda and t.dtype is self.ctype and t.numel() == numel \
+                and t.is_contiguous():
+            return
         if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
             raise ValueError("%s must be a CUDA tensor" % name)
         if t.dtype != self.ctype:
@@ -117,18 +127,20 @@ class GpuPlan:
         F = len(self.frame_offsets) - 1
         self._check(x, F * coils * self.Nprod, "x")
         self._check(y, coils * self.M_total, "y")
-        with torch.cuda.device(self.device):
-            _lib.check_with(self.lib, self.lib.gbn_forward(self.handle, ctypes.c_void_p(x.data_ptr()),
-                                            ctypes.c_void_p(y.data_ptr()), int(coils), _stream()))
+        # the library switches to the plan's device itself
+        rc = self.lib.gbn_forward(self.handle, x.data_ptr(), y.data_ptr(), int(coils), raw_stream(self.device.index))
+        if rc:
+            _lib.check_with(self.lib, rc)
         return y
 
     def adjoint(self, y, x, coils):
         F = len(self.frame_offsets) - 1
         self._check(y, coils * self.M_total, "y")
         self._check(x, F * coils * self.Nprod, "x")
-        with torch.cuda.device(self.device):
-            _lib.check_with(self.lib, self.lib.gbn_adjoint(self.handle, ctypes.c_void_p(y.data_ptr()),
-                                            ctypes.c_void_p(x.data_ptr()), int(coils), _stream()))
+        # the library switches to the plan's device itself
+        rc = self.lib.gbn_adjoint(self.handle, y.data_ptr(), x.data_ptr(), int(coils), raw_stream(self.device.index))
+        if rc:
+            _lib.check_with(self.lib, rc)
         return x
 
     def _check_host(self, t, numel, name):

@@ -68,6 +68,7 @@ class NufftOperator(object):
         self._omega_t = torch.as_tensor(om, device=self.device)   # the plan's current trajectory
         self._gamma_t = torch.tensor(self.gamma, dtype=torch.float64, device=self.device)
         self._shift_t = torch.as_tensor(self.shift_vec, device=self.device)
+        self._inv_gamma_t = torch.tensor(1.0 / self.gamma, dtype=self.rtdtype, device=self.device)
 
     # ----------------------------------------------------------- trajectory
     def set_omega(self, omega):
@@ -133,8 +134,7 @@ class NufftOperator(object):
         gtm = torch.empty((self.M, self.ndim), dtype=self.rtdtype, device=self.device)
         gyc = gy.to(device=self.device, dtype=self.tdtype).contiguous()
         self.plan.grad_tm(self.plan.forward_grid(C), gyc, self.phase_shift, gtm, C)
-        inv_gamma = torch.tensor(1.0 / self.gamma, dtype=self.rtdtype, device=self.device)
-        return gtm * inv_gamma
+        return gtm * self._inv_gamma_t
 
     # ------------------------------------------------------------ public API
     def forward(self, x, omega=None):
