@@ -164,7 +164,11 @@ struct VisitParams {
     const int2* parts;              // {scratch slot or -1, nparts}
     int nitems, nblk;
     int nheavy[SPREAD_HEAVY_LEVELS];   // leading items of more entries than 32 << level
-    short4 borg[8];                 // set by the launcher: block origins within the tile
+    // set by the launcher, per block of a tile: origin, and its offset in the
+    // grid, in a scratch tile and in the phase table
+    short4 borg[8];
+    int64_t boff[8], bcell[8];
+    int bscr[8];
     int nshared;                    // set by the launcher: leading items shared by a CTA's warps
     int coils, LS, chunks, row;
     const int64_t* foff;

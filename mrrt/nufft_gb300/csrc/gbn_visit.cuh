@@ -346,71 +346,123 @@ __device__ __forceinline__ int combine_slots(typename Cx<R>::T (&acc)[NB], int s
     return q0;
 }
 
-// Write a combined block: to the grid with conj(phase_before), or to the
-// scratch slot of a split tile.  `zero`: no visits (zeros need no phase).
+// Where the blocks of an item go, for one lane: the grid (with
+// conj(phase_before)), or the scratch slot of a split tile.  Formed once per
+// item, so that a block costs an offset from the launcher's tables and a few
+// adds, and its phases come in one load ahead of use; with origins, bounds
+// and 64-bit strides worked out for each block, and the phases loaded where
+// they were used, the adjoint took 182 us instead of 168 at 256 x 256 with
+// 32 coils, 5000 instead of 4860 (with the forward) at 128^3 with 8, and 511
+// instead of 449 (with the forward) at 60 x 72 x 45 with 3.
 template <typename R, int NDIM, int LS>
-__device__ __forceinline__ void flush_block(const VisitParams<R>& p, typename Cx<R>::T (&acc)[16], int q0, int lane,
-                                            int f, const int* org, int blk, int scratch_slot, int chunk, bool zero) {
+struct BlockSink {
     typedef typename Cx<R>::T C;
     typedef VisitBlock<NDIM> VB;
-    constexpr int B0 = VB::B0, NB = VB::NB, SW = 32 / LS;
-    constexpr int KEEP = SW >= NB ? 1 : NB / SW;
-    const Geom<R>& g = p.g;
-    const int slot = lane / LS, coil = lane % LS;
-    const int c0 = chunk * LS, nc = min(LS, p.coils - c0);
-    int b0, b1, b2;
-    block_origin_of(p, blk, b0, b1, b2);
-    const bool direct = scratch_slot < 0;
-    if (direct && p.apply_pb && !zero) {
-        C ph = cmake<R>((R)1, (R)0);
-        if (lane < NB) {
-            int k[3] = {org[0] + b0 + lane % B0, org[1] + b1 + lane / B0, org[2] + b2};
-            if (k[0] < g.K[0] && (NDIM < 2 || k[1] < g.K[1]) && (NDIM < 3 || k[2] < g.K[2])) ph = phase_before(g, k);
-        }
-#pragma unroll
-        for (int i = 0; i < KEEP; ++i) {
-            C w;
-            w.x = __shfl_sync(0xffffffffu, ph.x, q0 + i);
-            w.y = __shfl_sync(0xffffffffu, ph.y, q0 + i);
-            acc[i] = cmulc(acc[i], w);
-        }
-    }
-    if (coil >= nc || (SW > NB && (slot >> 4))) return;
-    const bool vec_ok = sizeof(R) == 4 && g.gs0 == 1 && (g.K[0] % 2) == 0 && (g.gsf % 2) == 0 && (g.gsp % 2) == 0 && (g.gs1 % 2) == 0 &&
-                        (g.gs2 % 2) == 0;
-    constexpr int STEP = KEEP >= 2 ? 2 : 1;
-#pragma unroll
-    for (int i = 0; i < KEEP; i += STEP) {
-        const int q = q0 + i;
-        const int l0 = b0 + q % B0, l1 = b1 + q / B0, l2 = b2;
-        const bool row_in = (NDIM < 2 || org[1] + l1 < g.K[1]) && (NDIM < 3 || org[2] + l2 < g.K[2]);
-        const bool in0 = row_in && org[0] + l0 < g.K[0];
-        const bool in1 = STEP == 2 && row_in && org[0] + l0 + 1 < g.K[0];
-        C* dst;
-        int64_t next;   // the cell after this one along axis 0
+    static constexpr int B0 = VB::B0, NB = VB::NB, SW = 32 / LS;
+    static constexpr int KEEP = SW >= NB ? 1 : NB / SW;   // cells of a block this lane writes
+    C* dst;               // cell 0 of the tile, this lane's coil
+    int64_t pcell;        // cell 0 of the tile in the phase table
+    int tile;
+    bool direct, phased, whole, on;
+
+    __device__ __forceinline__ BlockSink(const VisitParams<R>& p, int4 it, int slot_id, int chunk, int lane) {
+        const Geom<R>& g = p.g;
+        const int coil = lane % LS, c = chunk * LS + coil;
+        int org[3] = {0, 0, 0};
+        tile = it.y;
+        tile_origin<NDIM>(tile, g.nt, g.T, org);
+        direct = slot_id < 0;
+        phased = direct && p.apply_pb;
+        whole = org[0] + g.T[0] <= g.K[0] && (NDIM < 2 || org[1] + g.T[1] <= g.K[1]) &&
+                (NDIM < 3 || org[2] + g.T[2] <= g.K[2]);
+        on = c < p.coils && !(SW > NB && ((lane / LS) >> 4));
         if (direct) {
-            const int64_t gi = f * g.gsf + (c0 + coil) * g.gsp + (org[0] + l0) * g.gs0 + (org[1] + l1) * g.gs1 +
-                               (org[2] + l2) * g.gs2;
-            next = g.gs0;
-            if ((in0 || in1) && !GBN_INB(g.check, gi >= 0 && gi + (in1 ? next : 0) < g.grid_elems, CHK_GRID_WRITE))
-                continue;
-            dst = p.grid + gi;
+            dst = p.grid + it.x * g.gsf + c * g.gsp + org[0] * g.gs0 + (NDIM > 1 ? org[1] * g.gs1 : 0) +
+                  (NDIM > 2 ? org[2] * g.gs2 : 0);
         } else {
-            const int64_t cell = l0 + (int64_t)g.T[0] * (l1 + (int64_t)g.T[1] * l2);
-            const int64_t si = (((int64_t)scratch_slot * p.chunks + chunk) * p.tile_cells + cell) * LS + coil;
-            next = LS;
-            if ((in0 || in1) && !GBN_INB(g.check, si >= 0 && si + (in1 ? next : 0) < p.scratch_elems, CHK_SCRATCH))
-                continue;
-            dst = p.scratch + si;
+            dst = p.scratch + ((int64_t)slot_id * p.chunks + chunk) * p.tile_cells * LS + coil;
         }
-        if (in0 && in1 && vec_ok && direct) {
-            store_pair(dst, acc[i], acc[i + STEP - 1]);
-        } else {
-            if (in0) dst[0] = acc[i];
-            if (in1) dst[next] = acc[i + STEP - 1];
+        pcell = org[0] + (int64_t)g.K[0] * ((NDIM > 1 ? org[1] : 0) + (int64_t)g.K[1] * (NDIM > 2 ? org[2] : 0));
+    }
+
+    // Extents of block blk that lie in the grid.
+    __device__ __forceinline__ void extent(const VisitParams<R>& p, int blk, int& n0, int& n1) const {
+        n0 = B0;
+        n1 = NB / B0;
+        if (!whole) {
+            int b0, b1, b2, org[3] = {0, 0, 0};
+            tile_origin<NDIM>(tile, p.g.nt, p.g.T, org);
+            block_origin_of(p, blk, b0, b1, b2);
+            n0 = min(B0, p.g.K[0] - org[0] - b0);
+            if (NDIM > 1) n1 = min(n1, p.g.K[1] - org[1] - b1);
+            if (NDIM > 2 && org[2] + b2 >= p.g.K[2]) n0 = 0;
         }
     }
-}
+
+    // phase_before of the block's cell `lane` (lanes below NB), to be loaded
+    // ahead of the block's sums
+    __device__ __forceinline__ C phase(const VisitParams<R>& p, int blk, int lane) const {
+        C ph = cmake<R>((R)1, (R)0);
+        if (phased && lane < NB) {
+            int n0, n1;
+            extent(p, blk, n0, n1);
+            if (lane % B0 < n0 && lane / B0 < n1) {
+                if (p.g.ptab) {
+                    ph = p.g.ptab[pcell + p.bcell[blk] + lane % B0 + (NDIM > 1 ? p.g.K[0] * (lane / B0) : 0)];
+                } else {
+                    int b0, b1, b2, org[3] = {0, 0, 0};
+                    tile_origin<NDIM>(tile, p.g.nt, p.g.T, org);
+                    block_origin_of(p, blk, b0, b1, b2);
+                    const int k[3] = {org[0] + b0 + lane % B0, org[1] + b1 + lane / B0, org[2] + b2};
+                    ph = phase_before(p.g, k);
+                }
+            }
+        }
+        return ph;
+    }
+
+    // Write a combined block; `zero`: no visits (zeros need no phase).
+    __device__ __forceinline__ void flush(const VisitParams<R>& p, C (&acc)[NB], int q0, int blk, C ph,
+                                          bool zero) const {
+        if (phased && !zero) {
+#pragma unroll
+            for (int i = 0; i < KEEP; ++i) {
+                C w;
+                w.x = __shfl_sync(0xffffffffu, ph.x, q0 + i);
+                w.y = __shfl_sync(0xffffffffu, ph.y, q0 + i);
+                acc[i] = cmulc(acc[i], w);
+            }
+        }
+        if (!on) return;
+        int n0, n1;
+        extent(p, blk, n0, n1);
+        const Geom<R>& g = p.g;
+        // within a block offsets fit 32 bits
+        const int s0 = direct ? (int)g.gs0 : LS, s1 = direct ? (int)g.gs1 : g.T[0] * LS;
+        const bool vec = sizeof(R) == 4 && direct && g.gs0 == 1 && ((g.K[0] | g.gsf | g.gsp | g.gs1 | g.gs2) & 1) == 0;
+        C* d = dst + (direct ? p.boff[blk] : p.bscr[blk] * LS);
+        constexpr int STEP = KEEP >= 2 ? 2 : 1;
+#pragma unroll
+        for (int i = 0; i < KEEP; i += STEP) {
+            const int q = q0 + i, k0 = q % B0, k1 = q / B0;
+            const bool in0 = k0 < n0 && k1 < n1, in1 = STEP == 2 && k0 + 1 < n0 && k1 < n1;
+            C* o = d + k0 * s0 + k1 * s1;
+#ifdef GBN_CHECKED
+            C* last = o + (in1 ? s0 : 0);
+            if ((in0 || in1) && !(direct ? GBN_INB(p.g.check, o >= p.grid && last < p.grid + p.g.grid_elems, CHK_GRID_WRITE)
+                                         : GBN_INB(p.g.check, o >= p.scratch && last < p.scratch + p.scratch_elems,
+                                                   CHK_SCRATCH)))
+                continue;
+#endif
+            if (in0 && in1 && vec) {
+                store_pair(o, acc[i], acc[i + STEP - 1]);
+            } else {
+                if (in0) o[0] = acc[i];
+                if (in1) o[s0] = acc[i + STEP - 1];
+            }
+        }
+    }
+};
 
 // ---- values read in place: one (item, block) per warp ---------------------------
 //
@@ -500,10 +552,11 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
 #pragma unroll
             for (int u = 0; u < U; ++u) add_row<R, NDIM, CX>(acc, v[u], co[u], k1);
     }
+    const BlockSink<R, NDIM, LS> sink(p, it, part.x, chunk, lane);
+    C phase = cmake<R>((R)1, (R)0);
+    if (n > 0) phase = sink.phase(p, blk, lane);
     const int q0 = combine_slots<R, LS, NB>(acc, slot);
-    int org[3] = {0, 0, 0};
-    tile_origin<NDIM>(it.y, g.nt, g.T, org);
-    flush_block<R, NDIM, LS>(p, acc, q0, lane, f, org, blk, part.x, chunk, n == 0);
+    sink.flush(p, acc, q0, blk, phase, n == 0);
 }
 
 // ---- coil-minor values: a warp streams visits through a shared-memory ring ------
@@ -527,13 +580,17 @@ struct StreamLayout {
     typedef typename Cx<R>::T C;
     static constexpr int NC = VisitBlock<NDIM>::NC * (CX ? 2 : 1);
     static constexpr int VROW = LS * (int)sizeof(C);            // bytes of one visit's values
-    static constexpr int VBYTES = 2048;                         // values of a stage
+    // values of a stage: at 32 coils two copies of eight visits each, 9 us of
+    // 168 faster than one (256 x 256, 32 coils)
+    static constexpr int VBYTES = LS == 32 && sizeof(C) == 8 ? 4096 : 2048;
     static constexpr int RV = VBYTES / VROW;                    // visits per stage
     static constexpr int CBYTES = RV * NC * (int)sizeof(R);     // coefficients of a stage
     static constexpr int STAGE = VBYTES + CBYTES;
     static constexpr int HEAD = 16 * LS * (int)sizeof(C);       // one combined block
-    static constexpr int WARP = 2 * STAGE + HEAD;
+    static constexpr int SINK = 32;                             // the item's BlockSink
+    static constexpr int WARP = 2 * STAGE + HEAD + SINK;
     static constexpr int SMEM = STREAM_WARPS * WARP;
+    static_assert(sizeof(BlockSink<R, 2, LS>) <= SINK, "sink");
     static_assert(RV % 4 == 0 && RV <= 32 && VROW <= 512 && STAGE % 16 == 0, "stage layout");
 };
 
@@ -581,8 +638,20 @@ spread_stream_kernel(const VisitParams<R> p) {
     }
     const int64_t fo = p.foff[f];
     const int Mf = (int)(p.foff[f + 1] - fo);
-    int org[3] = {0, 0, 0};
-    tile_origin<NDIM>(it.y, g.nt, g.T, org);
+    // the item's sink waits in shared memory: held in registers through the
+    // sums it spilled at 80, and formed anew for each block it cost 2-3%
+    BlockSink<R, NDIM, LS>* kept = reinterpret_cast<BlockSink<R, NDIM, LS>*>(ring + SL::WARP - SL::SINK);
+    {
+        const BlockSink<R, NDIM, LS> first(p, it, part, chunk, lane);
+        if (lane == 0) *kept = first;   // coil 0 of the chunk
+        __syncwarp();
+    }
+    auto sink = [&]() {   // for this lane's coil
+        BlockSink<R, NDIM, LS> k = *kept;
+        k.dst += coil * (k.direct ? g.gsp : (int64_t)1);
+        k.on = c0 + coil < p.coils;
+        return k;
+    };
 
     // ---- copies: stage k holds visits lo + k RV ... of the run -----------------
     // A lane copies 16 bytes at a fixed place of every (512 / VROW)-th visit.
@@ -658,7 +727,7 @@ spread_stream_kernel(const VisitParams<R> p) {
         id = nx;
     }
 
-    C acc[NB];
+    C acc[NB], phase = cmake<R>((R)1, (R)0);
     const unsigned char* sb = ring + SL::STAGE;   // the stage being read (none yet)
     const C* vp = nullptr;
     const R* cp = nullptr;
@@ -715,6 +784,8 @@ spread_stream_kernel(const VisitParams<R> p) {
                 cp += 4 * NC;
             }
         }
+        // loaded ahead of the exchange between slots, which hides part of it
+        if (owned && re > rb) phase = sink().phase(p, b, lane);
         const int q0 = combine_slots<R, LS, NB>(acc, slot);
         if (!owned) {   // begun by an earlier warp: hand it over
 #pragma unroll
@@ -724,7 +795,7 @@ spread_stream_kernel(const VisitParams<R> p) {
             pending_end = re;
             q_pending = q0;
         } else {
-            flush_block<R, NDIM, LS>(p, acc, q0, lane, f, org, b, part, chunk, re == rb);
+            sink().flush(p, acc, q0, b, phase, re == rb);
         }
     }
     if (!shared_item || whole) return;   // the same for the whole CTA
@@ -735,7 +806,7 @@ spread_stream_kernel(const VisitParams<R> p) {
 #pragma unroll
             for (int i = 0; i < KEEP; ++i) acc[i] = cadd(acc[i], h[(q_pending + i) * LS + coil]);
         }
-        flush_block<R, NDIM, LS>(p, acc, q_pending, lane, f, org, pending, part, chunk, false);
+        sink().flush(p, acc, q_pending, pending, phase, false);
     }
 }
 
@@ -838,6 +909,9 @@ cudaError_t launch_spread_visits(const VisitParams<R>& p0, cudaStream_t s) {
         else if (p.g.ndim == 2) block_origin<2>(p.g, b, b0, b1, b2);
         else block_origin<3>(p.g, b, b0, b1, b2);
         p.borg[b] = make_short4((short)b0, (short)b1, (short)b2, 0);
+        p.boff[b] = b0 * p.g.gs0 + (p.g.ndim > 1 ? b1 * p.g.gs1 : 0) + (p.g.ndim > 2 ? b2 * p.g.gs2 : 0);
+        p.bscr[b] = b0 + p.g.T[0] * (b1 + p.g.T[1] * b2);
+        p.bcell[b] = b0 + (int64_t)p.g.K[0] * (b1 + (int64_t)p.g.K[1] * b2);
     }
     const bool cx = p.g.hi[0] != nullptr;
     switch (p.g.ndim * 2 + (cx ? 1 : 0)) {
