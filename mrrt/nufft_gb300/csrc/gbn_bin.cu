@@ -19,6 +19,8 @@
 // are tm = omega / gamma (mrrt/nufft/_nufft.py:338-342).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "gbn_device.cuh"
 #include "gbn_internal.h"
 
@@ -128,24 +130,44 @@ __global__ void __launch_bounds__(256) bin_emit_kernel(const BinParams<R> p) {
             }
 }
 
-// Counts per bin of sorted keys: lanes holding the same key (a run of the
-// sort) add once, through their lowest lane.
-__global__ void __launch_bounds__(256) bin_hist_kernel(const unsigned* keys, int64_t n, int* counts) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned lane = threadIdx.x & 31;
-    const bool ok = i < n;
-    const unsigned k = ok ? keys[i] : 0xffffffffu;
-    const unsigned peers = __match_any_sync(0xffffffffu, k);
-    if (ok && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&counts[k], __popc(peers));
+// First positions of two lists of sorted keys that are not below b; the
+// searches' loads overlap.
+__device__ __forceinline__ int2 lower_bounds(const unsigned* ka, int na, const unsigned* kb, int nb, unsigned b) {
+    int la = 0, ha = na, lb = 0, hb = nb;
+    while (la < ha || lb < hb) {
+        const int ma = (int)(((unsigned)la + (unsigned)ha) >> 1), mb = (int)(((unsigned)lb + (unsigned)hb) >> 1);
+        const bool ga = la < ha && ka[ma] < b, gb = lb < hb && kb[mb] < b;
+        if (la < ha) (ga ? la : ha) = ga ? ma + 1 : ma;
+        if (lb < hb) (gb ? lb : hb) = gb ? mb + 1 : mb;
+    }
+    return make_int2(la, lb);
 }
 
-// parts per bin: gather chunks (none for an empty tile), spread parts (at
-// least one: an empty tile still writes its zeros), split-tile slots
-__global__ void __launch_bounds__(256) bin_parts_kernel(const ItemParams p) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < p.nbins_g) p.gparts[b] = (p.gcnt[b] + p.gchunk - 1) / p.gchunk;
+// Entries and parts per bin: gather chunks (none for an empty tile), spread
+// parts (at least one: an empty tile still writes its zeros), split-tile
+// slots.  The bins' first entries are found by a search of the sorted keys,
+// in the one launch (counting them took a reset, a histogram and a scan for
+// each list).
+constexpr int PARTS_THREADS = 64;
+
+__global__ void __launch_bounds__(PARTS_THREADS + 1) bin_parts_kernel(const ItemParams p) {
+    __shared__ int2 first[PARTS_THREADS + 1];
+    const int b = blockIdx.x * PARTS_THREADS + threadIdx.x;
+    // one thread more than bins, for the end of the last
+    first[threadIdx.x] = lower_bounds(p.gkeys, p.glen, p.skeys, p.slen, (unsigned)b);
+    __syncthreads();
+    if (threadIdx.x == PARTS_THREADS) return;
+    const int2 lo = first[threadIdx.x], hi = first[threadIdx.x + 1];
+    if (b < p.nbins_g) {
+        const int c = hi.x - lo.x;
+        p.gstart[b] = lo.x;
+        p.gcnt[b] = c;
+        p.gparts[b] = (c + p.gchunk - 1) / p.gchunk;
+    }
     if (b < p.nbins_s) {
-        const int c = p.scnt[b];
+        const int c = hi.y - lo.y;
+        p.sstart[b] = lo.y;
+        p.scnt[b] = c;
         const int parts = max(1, (c + p.schunk - 1) / p.schunk);
         p.sparts[b] = parts;
         p.rslots[b] = parts > 1 ? parts : 0;
@@ -198,14 +220,22 @@ __global__ void __launch_bounds__(256) bin_items_kernel(const ItemParams p) {
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) permute_kernel(const T* in, const unsigned* order, int64_t n, T* out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[order[i]];
+// The items of both lists in their order, with the spread's parts.
+__global__ void __launch_bounds__(256) item_order_kernel(const ItemParams p, int n_g, int n_s, int4* gout, int4* sout,
+                                                         int2* slot_out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_g) gout[i] = p.gitems[p.gorder[i]];
+    if (i < n_s) {
+        const unsigned o = p.sorder[i];
+        sout[i] = p.sitems[o];
+        slot_out[i] = p.sslot[o];
+    }
 }
 
+// Both lists (blockIdx.y).
 template <typename R>
-__global__ void __launch_bounds__(256) bin_pack_kernel(const PackParams<R> p) {
+__global__ void __launch_bounds__(256) bin_pack_kernel(const PackParams<R> g, const PackParams<R> sp) {
+    const PackParams<R>& p = blockIdx.y ? sp : g;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.len) return;
     const unsigned e = p.order[i];
@@ -235,16 +265,10 @@ cudaError_t launch_bin_emit(const BinParams<R>& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_bin_hist(const unsigned* keys, int64_t n, int* counts, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    bin_hist_kernel<<<grid_for(n, 256), 256, 0, s>>>(keys, n, counts);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_bin_parts(const ItemParams& p, cudaStream_t s) {
     const int nb = max(p.nbins_g, p.nbins_s);
     if (nb == 0) return cudaSuccess;
-    bin_parts_kernel<<<grid_for(nb, 256), 256, 0, s>>>(p);
+    bin_parts_kernel<<<grid_for(nb, PARTS_THREADS), PARTS_THREADS + 1, 0, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -255,22 +279,19 @@ cudaError_t launch_bin_items(const ItemParams& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_permute_int4(const int4* in, const unsigned* order, int64_t n, int4* out, cudaStream_t s) {
+cudaError_t launch_item_order(const ItemParams& p, int n_g, int n_s, int4* gout, int4* sout, int2* slot_out,
+                              cudaStream_t s) {
+    const int n = max(n_g, n_s);
     if (n == 0) return cudaSuccess;
-    permute_kernel<int4><<<grid_for(n, 256), 256, 0, s>>>(in, order, n, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_permute_int2(const int2* in, const unsigned* order, int64_t n, int2* out, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    permute_kernel<int2><<<grid_for(n, 256), 256, 0, s>>>(in, order, n, out);
+    item_order_kernel<<<grid_for(n, 256), 256, 0, s>>>(p, n_g, n_s, gout, sout, slot_out);
     return cudaGetLastError();
 }
 
 template <typename R>
-cudaError_t launch_bin_pack(const PackParams<R>& p, cudaStream_t s) {
-    if (p.len == 0) return cudaSuccess;
-    bin_pack_kernel<R><<<grid_for(p.len, 256), 256, 0, s>>>(p);
+cudaError_t launch_bin_pack(const PackParams<R>& gather, const PackParams<R>& spread, cudaStream_t s) {
+    const int64_t len = std::max(gather.len, spread.len);
+    if (len == 0) return cudaSuccess;
+    bin_pack_kernel<R><<<dim3(grid_for(len, 256), 2), 256, 0, s>>>(gather, spread);
     return cudaGetLastError();
 }
 
@@ -278,7 +299,7 @@ template cudaError_t launch_bin_count<float>(const BinParams<float>&, cudaStream
 template cudaError_t launch_bin_count<double>(const BinParams<double>&, cudaStream_t);
 template cudaError_t launch_bin_emit<float>(const BinParams<float>&, cudaStream_t);
 template cudaError_t launch_bin_emit<double>(const BinParams<double>&, cudaStream_t);
-template cudaError_t launch_bin_pack<float>(const PackParams<float>&, cudaStream_t);
-template cudaError_t launch_bin_pack<double>(const PackParams<double>&, cudaStream_t);
+template cudaError_t launch_bin_pack<float>(const PackParams<float>&, const PackParams<float>&, cudaStream_t);
+template cudaError_t launch_bin_pack<double>(const PackParams<double>&, const PackParams<double>&, cudaStream_t);
 
 }  // namespace gbn

@@ -277,10 +277,13 @@ struct BinParams {
 struct ItemParams {
     int nbins_g, nbins_s, ntiles_g, ntiles_s;
     int gchunk, schunk;
-    const int* gcnt;
-    const int* gstart;
-    const int* scnt;
-    const int* sstart;
+    const unsigned* gkeys;         // sorted bins of the lists' entries
+    const unsigned* skeys;
+    int glen, slen;
+    int* gcnt;                     // parts pass: entries per bin, and the first
+    int* gstart;
+    int* scnt;
+    int* sstart;
     int* gparts;                   // parts pass: gather items per bin
     int* sparts;                   //   spread items per bin
     int* rslots;                   //   scratch slots per bin (parts of split tiles)
@@ -320,12 +323,12 @@ struct PackParams {
 
 template <typename R> cudaError_t launch_bin_count(const BinParams<R>& p, cudaStream_t s);
 template <typename R> cudaError_t launch_bin_emit(const BinParams<R>& p, cudaStream_t s);
-cudaError_t launch_bin_hist(const unsigned* keys, int64_t n, int* counts, cudaStream_t s);
 cudaError_t launch_bin_parts(const ItemParams& p, cudaStream_t s);
 cudaError_t launch_bin_items(const ItemParams& p, cudaStream_t s);
-cudaError_t launch_permute_int4(const int4* in, const unsigned* order, int64_t n, int4* out, cudaStream_t s);
-cudaError_t launch_permute_int2(const int2* in, const unsigned* order, int64_t n, int2* out, cudaStream_t s);
-template <typename R> cudaError_t launch_bin_pack(const PackParams<R>& p, cudaStream_t s);
+cudaError_t launch_item_order(const ItemParams& p, int n_g, int n_s, int4* gout, int4* sout, int2* slot_out,
+                              cudaStream_t s);
+template <typename R>
+cudaError_t launch_bin_pack(const PackParams<R>& gather, const PackParams<R>& spread, cudaStream_t s);
 
 // Pruned FFT pass along one axis (gbn_fftpass.cu), of length L.
 //   Plain (sn null): ncols columns; column j = array j / S, place j % S, its

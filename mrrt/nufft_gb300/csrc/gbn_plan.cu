@@ -1746,7 +1746,8 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     bp.eoff = eoff;
     GBN_CUDA(cudaMemsetAsync(err, 0, 32 * sizeof(int), s), "binning reset");
     GBN_CUDA(launch_bin_count<R>(bp, s), "bin count launch");
-    GBN_CUDA(exclusive_scan(ecount, eoff, M, tot, scan_tmp, s), "entry scan");
+    const ScanJob entries = {ecount, eoff, M, tot};
+    GBN_CUDA(exclusive_scans(&entries, 1, scan_tmp, s), "entry scan");
     int hA[32] = {0};
     GBN_CUDA(cudaMemcpyAsync(hA, err, sizeof(hA), cudaMemcpyDeviceToHost, s), "binning readback");
     GBN_CUDA(cudaStreamSynchronize(s), "binning readback");
@@ -1756,14 +1757,13 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     std::memcpy(&nvisits, hA + 28, sizeof(nvisits));
 
     // ---- phase B: spread entries, sorts, bins, items ---------------------
-    const int64_t nsort = std::max<int64_t>(std::max<int64_t>(M, slen), nbs);
     const int64_t nitem_max = nbg + M / GATHER_CHUNK + 1 + nbs + slen / SCH + 1;
     unsigned *skey, *sval, *gsize, *gorder, *ssize, *sorder;
     int *em, *cg, *cs, *sg, *ss, *gp, *sp, *rs, *rf, *go, *so, *slo, *ro;
     short4* els;
     int4 *gi_tmp, *si_tmp;
     int2* sl_tmp;
-    void* rtmp;
+    void *list_tmp[2], *item_tmp[2];
     auto layout_b = [&](Bump& b) {
         skey = b.take<unsigned>(slen);
         sval = b.take<unsigned>(slen);
@@ -1788,7 +1788,10 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
         gorder = b.take<unsigned>(nitem_max);
         ssize = b.take<unsigned>(nitem_max);
         sorder = b.take<unsigned>(nitem_max);
-        rtmp = b.take<char>((int64_t)radix_temp_bytes(nsort));
+        // the sorted lists may end in their temporaries, and are read to the end
+        list_tmp[0] = b.take<char>((int64_t)radix_temp_bytes(M));
+        list_tmp[1] = b.take<char>((int64_t)radix_temp_bytes(slen));
+        for (int j = 0; j < 2; ++j) item_tmp[j] = b.take<char>((int64_t)radix_temp_bytes(nitem_max));
     };
     {
         Bump sz(nullptr);
@@ -1805,14 +1808,8 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     bp.em = em;
     bp.els = els;
     GBN_CUDA(launch_bin_emit<R>(bp, s), "bin emit launch");
-    GBN_CUDA(radix_sort_pairs(gkey, gval, M, bits_for(nbg), rtmp, s), "gather sort");
-    GBN_CUDA(radix_sort_pairs(skey, sval, slen, bits_for(nbs), rtmp, s), "spread sort");
-    GBN_CUDA(cudaMemsetAsync(cg, 0, sizeof(int) * nbg, s), "bin count reset");
-    GBN_CUDA(cudaMemsetAsync(cs, 0, sizeof(int) * nbs, s), "bin count reset");
-    GBN_CUDA(launch_bin_hist(gkey, M, cg, s), "gather bin counts");
-    GBN_CUDA(launch_bin_hist(skey, slen, cs, s), "spread bin counts");
-    GBN_CUDA(exclusive_scan(cg, sg, nbg, nullptr, scan_tmp, s), "gather bin scan");
-    GBN_CUDA(exclusive_scan(cs, ss, nbs, nullptr, scan_tmp, s), "spread bin scan");
+    SortJob lists[SORT_JOBS] = {{gkey, gval, M, bits_for(nbg)}, {skey, sval, slen, bits_for(nbs)}};
+    GBN_CUDA(radix_sort_pairs(lists, list_tmp, s), "list sort");
     ItemParams ip;
     std::memset(&ip, 0, sizeof(ip));
     ip.nbins_g = (int)nbg;
@@ -1821,6 +1818,10 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     ip.ntiles_s = nts;
     ip.gchunk = GATHER_CHUNK;
     ip.schunk = SCH;
+    ip.gkeys = lists[0].keys;
+    ip.skeys = lists[1].keys;
+    ip.glen = (int)M;
+    ip.slen = (int)slen;
     ip.gcnt = cg;
     ip.gstart = sg;
     ip.scnt = cs;
@@ -1831,10 +1832,9 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     ip.rflag = rf;
     ip.nheavy = tot + 5;
     GBN_CUDA(launch_bin_parts(ip, s), "bin parts launch");
-    GBN_CUDA(exclusive_scan(gp, go, nbg, tot + 1, scan_tmp, s), "gather item scan");
-    GBN_CUDA(exclusive_scan(sp, so, nbs, tot + 2, scan_tmp, s), "spread item scan");
-    GBN_CUDA(exclusive_scan(rs, slo, nbs, tot + 3, scan_tmp, s), "slot scan");
-    GBN_CUDA(exclusive_scan(rf, ro, nbs, tot + 4, scan_tmp, s), "split tile scan");
+    const ScanJob counts[SCAN_JOBS] = {{gp, go, nbg, tot + 1}, {sp, so, nbs, tot + 2}, {rs, slo, nbs, tot + 3},
+                                       {rf, ro, nbs, tot + 4}};
+    GBN_CUDA(exclusive_scans(counts, SCAN_JOBS, scan_tmp, s), "item scans");
     int hB[4 + SPREAD_HEAVY_LEVELS] = {0};
     GBN_CUDA(cudaMemcpyAsync(hB, tot + 1, sizeof(hB), cudaMemcpyDeviceToHost, s), "binning readback");
     GBN_CUDA(cudaStreamSynchronize(s), "binning readback");
@@ -1867,27 +1867,31 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
     GBN_CUDA(launch_bin_items(ip, s), "bin items launch");
     // heaviest first, ties in bin order (a stable sort by chunk - count), as
     // the host planner's stable_sort
-    GBN_CUDA(radix_sort_pairs(gsize, gorder, n_gi, bits_for(GATHER_CHUNK + 1), rtmp, s), "gather item sort");
-    GBN_CUDA(radix_sort_pairs(ssize, sorder, n_si, bits_for(SCH + 1), rtmp, s), "spread item sort");
-    GBN_CUDA(launch_permute_int4(gi_tmp, gorder, n_gi, reinterpret_cast<int4*>(P->gitems.p), s), "item order");
-    GBN_CUDA(launch_permute_int4(si_tmp, sorder, n_si, reinterpret_cast<int4*>(P->sitems.p), s), "item order");
-    GBN_CUDA(launch_permute_int2(sl_tmp, sorder, n_si, reinterpret_cast<int2*>(P->sparts.p), s), "item order");
+    SortJob items[SORT_JOBS] = {{gsize, gorder, n_gi, bits_for(GATHER_CHUNK + 1)},
+                                {ssize, sorder, n_si, bits_for(SCH + 1)}};
+    GBN_CUDA(radix_sort_pairs(items, item_tmp, s), "item sort");
+    ip.gorder = items[0].vals;
+    ip.sorder = items[1].vals;
+    GBN_CUDA(launch_item_order(ip, n_gi, n_si, reinterpret_cast<int4*>(P->gitems.p),
+                               reinterpret_cast<int4*>(P->sitems.p), reinterpret_cast<int2*>(P->sparts.p), s),
+             "item order");
 
     // ---- lists (SoA, the layout of build_lists) --------------------------
     P->has_phase = ph != nullptr;
     if ((rc = ensure(P->glist, list_bytes<R>(P, M, false), "list allocation"))) return rc;
     if ((rc = ensure(P->slist, list_bytes<R>(P, slen, true), "list allocation"))) return rc;
+    PackParams<R> packs[2];
     for (int which = 0; which < 2; ++which) {
         const bool spread = which == 1;
         const int64_t len = spread ? slen : M;
         const ListLayout<R> L(P, len, spread);
         char* base = reinterpret_cast<char*>(spread ? P->slist.p : P->glist.p);
-        PackParams<R> pk;
+        PackParams<R>& pk = packs[which];
         std::memset(&pk, 0, sizeof(pk));
         pk.ndim = ndim;
         pk.F = P->F;
         pk.len = len;
-        pk.order = spread ? sval : gval;
+        pk.order = lists[which].vals;
         pk.em = spread ? em : nullptr;
         pk.els = spread ? els : nullptr;
         pk.tm = tm;
@@ -1897,8 +1901,8 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
         pk.ph_out = ph ? reinterpret_cast<C*>(base + L.ph) : nullptr;
         for (int d = 0; d < ndim; ++d) pk.t_out[d] = reinterpret_cast<R*>(base + L.t[d]);
         pk.idx_out = reinterpret_cast<int*>(base + L.idx);
-        GBN_CUDA(launch_bin_pack<R>(pk, s), "list pack launch");
     }
+    GBN_CUDA(launch_bin_pack<R>(packs[0], packs[1], s), "list pack launch");
     P->glen = M;
     P->slen = slen;
     P->n_gitems = n_gi;

@@ -6,18 +6,35 @@
 
 namespace gbn {
 
-// Bytes of device temporaries exclusive_scan needs for n elements.
+// Exclusive scans, several in one launch: out[i] = in[0] + ... + in[i-1]
+// (in and out may not alias); total (device, optional) receives the sum of
+// all n.  Each is asynchronous on s.
+struct ScanJob {
+    const int* in;
+    int* out;
+    int64_t n;
+    int* total;
+};
+constexpr int SCAN_JOBS = 4;
+// Bytes of device temporaries for scans of at most n elements each.
 size_t scan_temp_bytes(int64_t n);
-// out[i] = in[0] + ... + in[i-1] (int32; in and out may not alias); total
-// (device, optional) receives the sum of all n.  Asynchronous on s.
-cudaError_t exclusive_scan(const int* in, int* out, int64_t n, int* total, void* temp, cudaStream_t s);
-// The same with 64-bit sums.
+cudaError_t exclusive_scans(const ScanJob* jobs, int count, void* temp, cudaStream_t s);
+// One scan with 64-bit sums.
 cudaError_t exclusive_scan64(const int* in, long long* out, int64_t n, long long* total, void* temp, cudaStream_t s);
 
-// Bytes of device temporaries radix_sort_pairs needs for n pairs.
+// A stable sort of (keys, vals) by the low `bits` bits of keys.
+struct SortJob {
+    unsigned* keys;
+    unsigned* vals;
+    int64_t n;
+    int bits;
+};
+constexpr int SORT_JOBS = 2;
+// Bytes of device temporaries for a sort of n pairs.
 size_t radix_temp_bytes(int64_t n);
-// Stable sort of (keys, vals) by the low `bits` bits of keys, in place.
-// Asynchronous on s; the result is the same in every run.
-cudaError_t radix_sort_pairs(unsigned* keys, unsigned* vals, int64_t n, int bits, void* temp, cudaStream_t s);
+// Sorts both jobs, pass by pass in shared launches.  Asynchronous on s; the
+// result is the same in every run, and lies where the job's keys and vals
+// point on return (its own arrays or its temporaries).
+cudaError_t radix_sort_pairs(SortJob (&jobs)[SORT_JOBS], void* const (&temp)[SORT_JOBS], cudaStream_t s);
 
 }  // namespace gbn

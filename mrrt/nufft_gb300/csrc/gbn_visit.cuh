@@ -130,14 +130,12 @@ __device__ __forceinline__ typename Cx<R>::T visit_coef(const Geom<R>& g, const 
         }
         return cmake<R>(cr, CX ? -ci : (R)0);
     };
-    if (k < VB::B0) {
-        const int j = b0 + k - ls.x;
-        return j >= 0 && j < g.J[0] ? coef(0, j) : cmake<R>((R)0, (R)0);
-    }
-    const int j = b1 + (k - VB::B0) - ls.y;
-    if (NDIM < 2 || j < 0 || j >= g.J[1]) return cmake<R>((R)-0.0, (R)0);
-    C w = coef(1, j);
-    if (NDIM > 2) {
+    // one path for both axes: lanes of a warp hold coefficients of either
+    const int d = NDIM > 1 && k >= VB::B0 ? 1 : 0;
+    const int j = d ? b1 + (k - VB::B0) - ls.y : b0 + k - ls.x;
+    if (j < 0 || j >= g.J[d]) return cmake<R>(d ? (R)-0.0 : (R)0, (R)0);
+    C w = coef(d, j);
+    if (NDIM > 2 && d) {
         const C c2 = coef(2, b2 - ls.z);
         w = CX ? cmul_fixed(w, c2) : cmake<R>(mul_rn(w.x, c2.x), (R)0);
     }
@@ -165,6 +163,23 @@ __device__ __forceinline__ bool visits_block(const Geom<R>& g, short4 s, int b0,
     return hit;
 }
 
+// Entries e with base + 32 u + lane = e of a count-long run that touch the
+// block, as one mask per u; the starts' loads are independent of each other.
+constexpr int VISIT_UNROLL = 4;
+
+template <typename R, int NDIM>
+__device__ __forceinline__ void block_hits(const VisitBuildParams<R>& p, int first, int count, int base, int lane, int b0,
+                                           int b1, int b2, unsigned (&mask)[VISIT_UNROLL]) {
+    short4 s[VISIT_UNROLL];
+#pragma unroll
+    for (int u = 0; u < VISIT_UNROLL; ++u)
+        if (base + 32 * u + lane < count) s[u] = p.s.ls[(int64_t)first + base + 32 * u + lane];
+#pragma unroll
+    for (int u = 0; u < VISIT_UNROLL; ++u)
+        mask[u] = __ballot_sync(0xffffffffu,
+                                base + 32 * u + lane < count && visits_block<NDIM>(p.g, s[u], b0, b1, b2));
+}
+
 // Visits per (item, block), rounded up to whole groups of four: one CTA per
 // item, one warp per block.
 template <typename R, int NDIM>
@@ -175,63 +190,104 @@ __global__ void __launch_bounds__(256) visit_count_kernel(const VisitBuildParams
     block_origin<NDIM>(p.g, blk, b0, b1, b2);
     int n = 0;
     const int count = block_in_grid<NDIM>(p.g, it.y, b0, b1, b2) ? it.w : 0;
-    for (int base = 0; base < count; base += 32) {
-        bool hit = false;
-        if (base + lane < count) hit = visits_block<NDIM>(p.g, p.s.ls[it.z + base + lane], b0, b1, b2);
-        n += __popc(__ballot_sync(0xffffffffu, hit));
+    for (int base = 0; base < count; base += 32 * VISIT_UNROLL) {
+        unsigned mask[VISIT_UNROLL];
+        block_hits<R, NDIM>(p, it.z, count, base, lane, b0, b1, b2, mask);
+#pragma unroll
+        for (int u = 0; u < VISIT_UNROLL; ++u) n += __popc(mask[u]);
     }
     if (lane == 0) p.count[(int64_t)item * p.nblk + blk] = (n + 3) & ~3;
 }
 
-// The visits: sample indices (list positions where the coefficients are
-// computed during the call) and coefficients; padding is index -1.
-template <typename R, int NDIM, bool CX>
+// The visits as list positions; padding is -1.
+template <typename R, int NDIM>
 __global__ void __launch_bounds__(256) visit_fill_kernel(const VisitBuildParams<R> p) {
-    typedef VisitBlock<NDIM> VB;
-    typedef typename Cx<R>::T C;
-    constexpr int NR = VB::NC * (CX ? 2 : 1);   // reals per visit
-    const Geom<R>& g = p.g;
     const int item = blockIdx.x, blk = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int4 it = p.items[item];
-    const int64_t fo = p.foff[it.x];
     int b0, b1, b2;
-    block_origin<NDIM>(g, blk, b0, b1, b2);
+    block_origin<NDIM>(p.g, blk, b0, b1, b2);
     int64_t at = p.start[(int64_t)item * p.nblk + blk];
     const int64_t end = p.start[(int64_t)item * p.nblk + blk + 1];
-    const int count = block_in_grid<NDIM>(g, it.y, b0, b1, b2) ? it.w : 0;
-    for (int base = 0; base < count; base += 32) {
-        const int64_t e = (int64_t)it.z + base + lane;
-        short4 s = make_short4(0, 0, 0, 0);
-        bool hit = false;
-        if (base + lane < count) {
-            s = p.s.ls[e];
-            hit = visits_block<NDIM>(g, s, b0, b1, b2);
-        }
-        const unsigned mask = __ballot_sync(0xffffffffu, hit);
-        const int64_t pos = at + __popc(mask & ((1u << lane) - 1u));
-        if (hit && pos < end) {
-            const int idx = p.s.idx[e];
-            p.vidx[pos] = p.vco ? idx : (int)e;
-            if (p.vco) {
-                R* o = p.vco + pos * NR;
+    const int count = block_in_grid<NDIM>(p.g, it.y, b0, b1, b2) ? it.w : 0;
+    for (int base = 0; base < count; base += 32 * VISIT_UNROLL) {
+        unsigned mask[VISIT_UNROLL];
+        block_hits<R, NDIM>(p, it.z, count, base, lane, b0, b1, b2, mask);
 #pragma unroll
-                for (int k = 0; k < VB::NC; ++k) {
-                    const C c = visit_coef<R, NDIM, CX>(g, p.s, e, s, fo + idx, p.wr, p.wi, b0, b1, b2, k);
-                    if (CX) {
-                        o[2 * k] = c.x;
-                        o[2 * k + 1] = c.y;
-                    } else {
-                        o[k] = c.x;
-                    }
-                }
+        for (int u = 0; u < VISIT_UNROLL; ++u) {
+            const int64_t pos = at + __popc(mask[u] & ((1u << lane) - 1u));
+            if ((mask[u] >> lane & 1u) && pos < end) p.vidx[pos] = it.z + base + 32 * u + lane;
+            at += __popc(mask[u]);
+        }
+    }
+    if (at + lane < end) p.vidx[at + lane] = -1;
+}
+
+// Their coefficients, a thread to each, and the sample indices in place of
+// the positions.  A visit waits for four loads in a chain (position, sample,
+// coordinate, table), so an item's visits, up to some thousands, go to the
+// threads of up to VISIT_SLICES CTAs, VISIT_UNROLL at a time; most items need
+// one.  Bound by the instructions of a coefficient: 34 us for 330,000 visits
+// (512 x 512 grid, J = 6).  With the warp of each block computing them where
+// it found the visits, a lane to a visit, one launch took 90 us; with both
+// axes in separate branches this one took 51.
+constexpr int VISIT_SLICES = 4;
+
+template <typename R, int NDIM, bool CX>
+__global__ void __launch_bounds__(256) visit_coef_kernel(const VisitBuildParams<R> p) {
+    typedef VisitBlock<NDIM> VB;
+    typedef typename Cx<R>::T C;
+    constexpr int NC = VB::NC, PER = 256 / NC;   // visits a CTA takes at a time
+    const Geom<R>& g = p.g;
+    const int item = blockIdx.x;
+    const long long* st = p.start + (int64_t)item * p.nblk;
+    const int64_t first = st[0];
+    const int n = (int)(st[p.nblk] - first);
+    if ((int)blockIdx.y * PER * VISIT_UNROLL >= n) return;   // the whole CTA
+    // origins and first visits of the item's blocks
+    __shared__ int4 block[8];
+    if ((int)threadIdx.x < p.nblk) {
+        int4 o;
+        block_origin<NDIM>(g, threadIdx.x, o.x, o.y, o.z);
+        o.w = (int)(st[threadIdx.x] - first);
+        block[threadIdx.x] = o;
+    }
+    __syncthreads();
+    const int64_t fo = p.foff[p.items[item].x];
+    const int k = threadIdx.x % NC;
+    int* vidx = p.vidx + first;
+    R* vco = p.vco + first * NC * (CX ? 2 : 1);
+    for (int v0 = blockIdx.y * PER * VISIT_UNROLL; v0 < n; v0 += PER * VISIT_UNROLL * VISIT_SLICES) {
+        int e[VISIT_UNROLL], idx[VISIT_UNROLL], blk[VISIT_UNROLL];
+        C c[VISIT_UNROLL];
+#pragma unroll
+        for (int u = 0; u < VISIT_UNROLL; ++u) {
+            const int v = v0 + u * PER + threadIdx.x / NC;
+            e[u] = v < n ? vidx[v] : -1;
+            blk[u] = 0;
+        }
+        for (int b = 1; b < p.nblk; ++b) {
+            const int at = block[b].w;
+#pragma unroll
+            for (int u = 0; u < VISIT_UNROLL; ++u) blk[u] += at <= v0 + u * PER + (int)threadIdx.x / NC;
+        }
+#pragma unroll
+        for (int u = 0; u < VISIT_UNROLL; ++u) {
+            idx[u] = e[u] < 0 ? -1 : p.s.idx[e[u]];
+            c[u] = cmake<R>(!CX && k >= VB::B0 ? (R)-0.0 : (R)0, (R)0);
+            if (e[u] >= 0) {
+                const int4 o = block[blk[u]];
+                c[u] = visit_coef<R, NDIM, CX>(g, p.s, e[u], p.s.ls[e[u]], fo + idx[u], p.wr, p.wi, o.x, o.y, o.z, k);
             }
         }
-        at += __popc(mask);
-    }
-    if (at + lane < end) {
-        p.vidx[at + lane] = -1;
-        if (p.vco)
-            for (int k = 0; k < NR; ++k) p.vco[(at + lane) * NR + k] = !CX && k >= VB::B0 ? (R)-0.0 : (R)0;
+        __syncwarp();   // a visit's lanes, one warp, have read its position
+#pragma unroll
+        for (int u = 0; u < VISIT_UNROLL; ++u) {
+            const int v = v0 + u * PER + threadIdx.x / NC;
+            if (v >= n) continue;
+            if (k == 0) vidx[v] = idx[u];
+            if (CX) reinterpret_cast<C*>(vco)[(int64_t)v * NC + k] = c[u];
+            else vco[(int64_t)v * NC + k] = c[u].x;
+        }
     }
 }
 
@@ -825,20 +881,27 @@ cudaError_t launch_visit_count(const VisitBuildParams<R>& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <typename R, int NDIM>
+cudaError_t visit_fill_any(const VisitBuildParams<R>& p, cudaStream_t s) {
+    visit_fill_kernel<R, NDIM><<<p.nitems, 32 * p.nblk, 0, s>>>(p);
+    if (p.vco) {
+        const dim3 grid((unsigned)p.nitems, VISIT_SLICES);
+        if (p.cx) visit_coef_kernel<R, NDIM, true><<<grid, 256, 0, s>>>(p);
+        else visit_coef_kernel<R, NDIM, false><<<grid, 256, 0, s>>>(p);
+    }
+    return cudaGetLastError();
+}
+
 template <typename R>
 cudaError_t launch_visit_fill(const VisitBuildParams<R>& p, cudaStream_t s) {
     if (p.nitems == 0) return cudaSuccess;
-    const int threads = 32 * p.nblk;
-    switch (p.g.ndim * 2 + (p.cx ? 1 : 0)) {
-        case 2: visit_fill_kernel<R, 1, false><<<p.nitems, threads, 0, s>>>(p); break;
-        case 3: visit_fill_kernel<R, 1, true><<<p.nitems, threads, 0, s>>>(p); break;
-        case 4: visit_fill_kernel<R, 2, false><<<p.nitems, threads, 0, s>>>(p); break;
-        case 5: visit_fill_kernel<R, 2, true><<<p.nitems, threads, 0, s>>>(p); break;
-        case 6: visit_fill_kernel<R, 3, false><<<p.nitems, threads, 0, s>>>(p); break;
-        case 7: visit_fill_kernel<R, 3, true><<<p.nitems, threads, 0, s>>>(p); break;
-        default: return cudaErrorInvalidValue;
+    if (p.nblk < 1 || p.nblk > 8) return cudaErrorInvalidValue;
+    switch (p.g.ndim) {
+        case 1: return visit_fill_any<R, 1>(p, s);
+        case 2: return visit_fill_any<R, 2>(p, s);
+        case 3: return visit_fill_any<R, 3>(p, s);
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 template <typename R>
