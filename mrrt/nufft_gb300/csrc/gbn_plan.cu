@@ -731,9 +731,14 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
     return GBN_OK;
 }
 
-// Coil-minor values are worth their pass above this many coils: up to four,
-// a visit's coils fill no more sectors read in place.
-constexpr int VALUES_MIN_COILS = 5;
+// Coil-minor values are worth their pass from five coils on, and from three
+// in single-precision volumes, whose samples have three times the visits
+// (64^3 image, 4 coils: 265 us, against 361 with the samples read in place).
+// In the plane a pass more, and a warp per tile instead of one per block,
+// cost more than they save (256 x 256, 3 coils: 61 against 55 us; 64 x 64,
+// 4 coils: 29 against 23), and in double precision a visit's coils fill whole
+// sectors either way (192 x 192, 4 coils: 521 against 506).
+bool use_values(const gbn_plan* P, int coils) { return coils >= (!P->dbl && P->geom.ndim == 3 ? 3 : 5); }
 
 // Values per sample of the coil-minor buffer: the coils, rounded up to 16 bytes.
 int value_row(int coils, size_t csz) {
@@ -757,7 +762,7 @@ int ensure_scratch(gbn_plan* P, int coils) {
     }
     // the coil-minor values of the visit-list spread
     const size_t vbytes = (size_t)P->M_total * value_row(coils, csz) * csz;
-    if (coils >= VALUES_MIN_COILS && vbytes > P->vals.bytes) {
+    if (use_values(P, coils) && vbytes > P->vals.bytes) {
         cudaError_t e = P->vals.alloc(vbytes);
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "sample value allocation failed");
     }
@@ -1140,7 +1145,8 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
     typedef typename Cx<R>::T C;
     const Lanes ln = call_lanes<R>(P, coils);
     const bool phases = kind != Grid::abi;
-    if (ln.LS < 8) vals = nullptr;   // narrow lanes read the samples in place
+    // narrow lanes read the samples in place
+    if (ln.LS < (!P->dbl && P->geom.ndim == 3 ? 4 : 8)) vals = nullptr;
     const C* ph = phases && P->has_phase ? reinterpret_cast<const C*>(P->phnat.p) : nullptr;
     const int64_t* foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
     VisitParams<R> p;
@@ -1210,7 +1216,7 @@ template <typename R>
 int run_spread(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, cudaStream_t s) {
     int rc = ensure_scratch(P, coils);
     if (rc) return rc;
-    return launch_visits<R>(P, y, grid, coils, kind, coils >= VALUES_MIN_COILS ? P->vals.p : nullptr,
+    return launch_visits<R>(P, y, grid, coils, kind, use_values(P, coils) ? P->vals.p : nullptr,
                             (int64_t)(P->vals.bytes / sizeof(typename Cx<R>::T)), P->scratch.p, P->scratch_cap, s);
 }
 
@@ -1241,7 +1247,7 @@ int run_spread_noalloc(gbn_plan* P, const void* y, void* grid, int coils, cudaSt
     // else the samples are read in place
     const int64_t used = (need + 255) & ~(int64_t)255;
     const int64_t velems = P->M_total * value_row(coils, sizeof(C));
-    void* vals = coils >= VALUES_MIN_COILS && used + velems * (int64_t)sizeof(C) <= (int64_t)cap
+    void* vals = use_values(P, coils) && used + velems * (int64_t)sizeof(C) <= (int64_t)cap
                      ? static_cast<char*>(scratch) + used : nullptr;
     return launch_visits<R>(P, y, grid, coils, Grid::abi, vals, velems, scratch, need / (int64_t)sizeof(C), s);
 }

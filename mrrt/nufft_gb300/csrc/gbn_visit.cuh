@@ -522,8 +522,8 @@ struct BlockSink {
 
 // ---- values read in place: one (item, block) per warp ---------------------------
 //
-// Up to four coil lanes, and wider batches of calls that may not allocate
-// the coil-minor values.  U visits per slot are in flight at a time.
+// Up to four coil lanes (two of a single-precision volume), and wider batches of calls
+// that may not allocate the coil-minor values.  U visits per slot are in flight at a time.
 constexpr int VISIT_THREADS = 128;   // four (item, block) units per CTA
 
 template <typename R, int NDIM, bool CX, int LS, bool TAB>
@@ -638,7 +638,7 @@ struct StreamLayout {
     static constexpr int VROW = LS * (int)sizeof(C);            // bytes of one visit's values
     // values of a stage: at 32 coils two copies of eight visits each, 9 us of
     // 168 faster than one (256 x 256, 32 coils)
-    static constexpr int VBYTES = LS == 32 && sizeof(C) == 8 ? 4096 : 2048;
+    static constexpr int VBYTES = LS == 32 && sizeof(C) == 8 ? 4096 : VROW < 64 ? 32 * VROW : 2048;
     static constexpr int RV = VBYTES / VROW;                    // visits per stage
     static constexpr int CBYTES = RV * NC * (int)sizeof(R);     // coefficients of a stage
     static constexpr int STAGE = VBYTES + CBYTES;
@@ -650,14 +650,16 @@ struct StreamLayout {
     static_assert(RV % 4 == 0 && RV <= 32 && VROW <= 512 && STAGE % 16 == 0, "stage layout");
 };
 
+// CTAs per SM: what the registers of a block's sums leave (two in double
+// precision: 1048 us at 192 x 192, 16 coils, against 1074 with one).
 template <typename R, int NDIM, bool CX, int LS, bool TAB>
-__global__ void __launch_bounds__(32 * STREAM_WARPS, sizeof(R) == 4 && !CX ? (LS == 32 ? 2 : 3) : 1)
+__global__ void __launch_bounds__(32 * STREAM_WARPS, CX ? 1 : sizeof(R) == 8 || LS == 32 ? 2 : 3)
 spread_stream_kernel(const VisitParams<R> p) {
     typedef typename Cx<R>::T C;
     typedef VisitBlock<NDIM> VB;
     typedef StreamLayout<R, NDIM, CX, LS> SL;
     constexpr int NB = VB::NB, NC = SL::NC, B1 = NDIM > 1 ? VB::B1 : 1, SW = 32 / LS, RV = SL::RV;
-    constexpr int KEEP = NB / SW;
+    constexpr int KEEP = NB / SW, GROUP = SW > 4 ? SW : 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geom<R>& g = p.g;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -818,7 +820,7 @@ spread_stream_kernel(const VisitParams<R> p) {
             left -= n;
             // groups of four visits (blocks begin and end on whole groups)
 #pragma unroll 1
-            for (int q = n; q > 0; q -= 4) {
+            for (int q = n; q > 0; q -= GROUP) {
                 unsigned rows = 0xffffu;
                 if (NDIM > 1 && !CX && SW == 1) {
                     // one visit at a time: bit 4 u + k1 is set where visit u's
@@ -827,7 +829,8 @@ spread_stream_kernel(const VisitParams<R> p) {
                                          lane < 16 && !is_neg_zero(cp[(lane >> 2) * NC + NC - B1 + (lane & 3)]));
                 }
 #pragma unroll
-                for (int u = 0; u < 4 / SW; ++u) {
+                for (int u = 0; u < GROUP / SW; ++u) {
+                    if (GROUP > 4 && slot >= q) break;   // four visits left for eight slots
                     const C v = vp[u * 32];
                     R co[NC];
                     load_run(cp + u * SW * NC, co);
@@ -836,8 +839,9 @@ spread_stream_kernel(const VisitParams<R> p) {
                         if (!(NDIM > 1 && !CX && SW == 1) || (rows >> (4 * u + k1) & 1))
                             add_row<R, NDIM, CX>(acc, v, co, k1);
                 }
-                vp += 4 * LS;
-                cp += 4 * NC;
+                const int step = GROUP > 4 ? min(q, GROUP) : GROUP;
+                vp += step * LS;
+                cp += step * NC;
             }
         }
         // loaded ahead of the exchange between slots, which hides part of it
@@ -948,7 +952,10 @@ cudaError_t visit_lanes(const VisitParams<R>& p, cudaStream_t s) {
     switch (p.LS) {
         case 1: return unit_launch<R, NDIM, CX, 1, TAB>(p, s);
         case 2: return unit_launch<R, NDIM, CX, 2, TAB>(p, s);
-        case 4: return unit_launch<R, NDIM, CX, 4, TAB>(p, s);
+        case 4:
+            if constexpr (sizeof(R) == 4 && NDIM == 3)
+                if (p.vals) return stream_launch<R, NDIM, CX, 4, TAB>(p, s);
+            return unit_launch<R, NDIM, CX, 4, TAB>(p, s);
         case 8: return p.vals ? stream_launch<R, NDIM, CX, 8, TAB>(p, s) : unit_launch<R, NDIM, CX, 8, TAB>(p, s);
         case 16: return p.vals ? stream_launch<R, NDIM, CX, 16, TAB>(p, s) : unit_launch<R, NDIM, CX, 16, TAB>(p, s);
         case 32: return p.vals ? stream_launch<R, NDIM, CX, 32, TAB>(p, s) : unit_launch<R, NDIM, CX, 32, TAB>(p, s);

@@ -50,6 +50,8 @@ def _plan(K, J, tm, rdt, phasing, coils, table_only=False):
     ((6, 7), (6, 6), 32, "single", "real"), ((150,), (6,), 48, "single", "real"), ((9,), (8,), 3, "single", "real"),
     ((18, 13, 10), (6, 6, 6), 8, "single", "real"), ((18, 13, 10), (5, 6, 4), 3, "single", "real"),
     ((40, 38), (6, 6), 6, "double", "real"), ((37, 22), (6, 5), 32, "double", "real"),
+    ((40, 38), (6, 6), 4, "single", "complex"), ((37, 22), (6, 6), 3, "single", "complex"),
+    ((150,), (6,), 4, "single", "real"), ((18, 13, 10), (6, 6, 6), 4, "single", "real"),
     ((40, 38), (6, 6), 12, "single", "complex"), ((18, 13, 10), (6, 6, 6), 2, "double", "complex"),
 ])
 def test_spread_matches_oracle(gpu_lib, K, J, coils, precision, phasing):
