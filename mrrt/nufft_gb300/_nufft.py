@@ -232,11 +232,10 @@ class NufftBase(object):
             pb_order=list(range(self.ndim)), phasing=phasing, max_coils=max_coils,
             tile=tile, stile=stile)
         # per direction: input axes, their Fortran-order strides, values per
-        # repetition, the same of the output, the library's entry point
+        # repetition, the same of the output
         strides = [math.prod(self.__Nd[:d]) for d in range(self.ndim)]
         image, samples = (self.__Nd, tuple(strides), self.nargin1), ((self.M,), (1,), self.M)
-        self._direct = {True: image + samples + (self._plan.lib.gbn_forward,),
-                        False: samples + image + (self._plan.lib.gbn_adjoint,)}
+        self._direct = {True: image + samples, False: samples + image}
         self._p = None
         if mode == "sparse":
             self._weights = sparse_weights(self.__omega, self.__Nd, self.__Jd, self.__Kd, self.kernel,
@@ -484,7 +483,7 @@ class NufftBase(object):
         if type(a) is not torch.Tensor or a.dtype is not plan.ctype or a.device != plan.device or \
                 not self.__on_gpu or self.order != "F" or a.is_conj():
             return None
-        lead, strides, n, out_lead, out_strides, m, call = self._direct[forward]
+        lead, strides, n, out_lead, out_strides, m = self._direct[forward]
         nd = len(lead)
         shape = a.shape
         if n == 0 or shape[:nd] != lead:
@@ -502,6 +501,7 @@ class NufftBase(object):
         if reps > 1:
             out_lead, out_strides = out_lead + (reps,), out_strides + (m,)
         out = torch.empty_strided(out_lead, out_strides, dtype=plan.ctype, device=plan.device)
+        call = plan.lib.gbn_forward if forward else plan.lib.gbn_adjoint
         rc = call(plan.handle, a.data_ptr(), out.data_ptr(), reps, raw_stream(plan.device.index))
         if rc:
             _lib.check_with(plan.lib, rc)
