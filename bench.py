@@ -362,8 +362,8 @@ def our_launches_per_step(Kd, split_tiles, coils=1):
     single-precision plan: with every axis length supported, a pass per axis
     (pad or crop folded in) and the interpolation kernel each way; else pad /
     crop and the interpolation kernel, plus the last-axis pass when its length
-    is supported; the coil-minor sample values from five coils on; the reduce
-    of split tiles."""
+    is supported; the coil-minor sample values from five coils on (three in
+    3-D); the reduce of split tiles."""
     nd = len(Kd)
     if nd >= 2 and all(k in OWN_FFT_LENGTHS for k in Kd):
         per_dir = nd + 1
@@ -371,7 +371,7 @@ def our_launches_per_step(Kd, split_tiles, coils=1):
         per_dir = 3
     else:
         per_dir = 2
-    return 2 * per_dir + (1 if split_tiles > 0 else 0) + (1 if coils >= 5 else 0)
+    return 2 * per_dir + (1 if split_tiles > 0 else 0) + (1 if coils >= (3 if nd == 3 else 5) else 0)
 
 
 def _clock_path(rank):

@@ -71,9 +71,19 @@ __device__ __forceinline__ int wrapk(int k, int K) {
 
 // First tap of the window: 1 + floor(t - J/2), evaluated in double exactly as
 // the reference C does (nufft_table.template.c:577-578).
-template <typename R>
-__device__ __forceinline__ int first_tap(R t, int J) {
-    return 1 + (int)floor((double)t - 0.5 * (double)J);
+__device__ __forceinline__ int first_tap(double t, int J) {
+    return 1 + (int)floor(t - 0.5 * (double)J);
+}
+// The same number for a float without double arithmetic, of which an SM does
+// two operations a cycle: the integer part of J/2 comes off exactly, and of t
+// only the place of its fraction against 1/2 is asked.  Below 2^-26 a negative
+// t may vanish in the double difference, so it takes that way.  (Computing a
+// plan's gather records was bound by this: 128^3 kooshball 1.62 -> 0.81 ms,
+// its visits 11.4 -> 9.9; a re-binning of 65536 samples 281 -> 264 us.)
+__device__ __forceinline__ int first_tap(float t, int J) {
+    if (t < 0.0f && t > -0x1p-26f) return first_tap((double)t, J);
+    const float h = floorf(t);
+    return 1 + (int)h - (J >> 1) - ((J & 1) && t - h < 0.5f ? 1 : 0);
 }
 
 // phase_before(k) = exp(i * sum_d c_d k_d) with every product and partial sum

@@ -22,16 +22,16 @@
 // barriers each, and every warp balloted which of them touched its block:
 // 515 warp instructions a sample at the 2-D 32-coil workload, 101 of them
 // the multiply-adds.)  Measured, spread alone, before -> now, plus the pass
-// that lays the values out: 128^3 kooshball, 8 coils 4892 -> 2014 + 115 us;
-// 64-frame series, 8 coils 949 -> 452 + 64; 2-D 256^2, 32 coils 143 -> 109 +
-// 24; 128^2, one coil 29 -> 18; 192^2 double, 4 coils 345 -> 227.  Bound by
+// that lays the values out: 128^3 kooshball, 8 coils 4892 -> 1860 + 109 us;
+// 64-frame series, 8 coils 949 -> 398 + 64; 2-D 256^2, 32 coils 143 -> 92 +
+// 24; 128^2, one coil 29 -> 18; 192^2 double, 4 coils 345 -> 216.  Bound by
 // instruction issue (3-D: 80% of the issue slots, 45% of them multiply-adds).
 //
 // The sample values come coil-minor, [sample][coil], with conj(sample phase)
 // applied (values_kernel: one transposition per call), so that one visit's
 // coils are one segment: read straight from [coil][sample], a 32-coil visit
-// touches 32 sectors.  Up to four coils, where the segment is no longer than
-// a sector, the values are read in place and the phase applied on reading.
+// touches 32 sectors.  Small batches (use_values in gbn_plan.cu) read the
+// values in place and apply the phase on reading.
 //
 // Order of summation: entry order per slot, slots combined in a fixed
 // pattern, warps sharing a block in warp order, parts of split tiles by

@@ -29,3 +29,24 @@ def test_lists_equal_host_lists(gpu_lib, Nd, Kd, Jd, M):
     yd, xd = _transforms(dev, 2, 3)
     assert torch.equal(yh, yd)
     assert torch.equal(xh, xd)
+
+
+@pytest.mark.parametrize("J", [4, 5, 6, 7])
+def test_first_taps_at_edges(gpu_lib, J):
+    """Coordinates a step of the format around integers, half integers and
+    zero, and small enough to vanish beside J/2 in double: the single-precision
+    first taps of the device are the host's, computed in double."""
+    f = np.float32
+    t = np.concatenate([np.arange(-90, 90) / 2.0, 2.0 ** np.arange(-60, 0), -(2.0 ** np.arange(-140, 0))]).astype(f)
+    up, down = [t], [t]
+    for _ in range(2):
+        up.append(np.nextafter(up[-1], f(np.inf)))
+        down.append(np.nextafter(down[-1], f(-np.inf)))
+    t = np.concatenate(up + down[1:]).astype(np.float64)[:, None]
+    host, dev = _plans((45,), (90,), (J,), [t[::-1].copy(), t], 1)
+    sh, sd = host.stats(), dev.stats()
+    assert {k: sh[k] for k in STAT_KEYS} == {k: sd[k] for k in STAT_KEYS}
+    yh, xh = _transforms(host, 1, 3)
+    yd, xd = _transforms(dev, 1, 3)
+    assert torch.equal(yh, yd)
+    assert torch.equal(xh, xd)
