@@ -50,8 +50,8 @@ extern "C" {
 #define GBN_PHASING_COMPLEX 1
 
 /* Geometry flags.  By default a plan precomputes every sample's table
- * coefficients once (list order, jsum = sum(Jd) values per sample and per
- * spread-list entry) and the kernels read them; TABLE_ONLY keeps no such
+ * coefficients once (per sample for the gather, per visit of a register
+ * block for the spread) and the kernels read them; TABLE_ONLY keeps no such
  * buffers and interpolates the tables inside the kernels instead (same
  * results bit for bit, less device memory).                               */
 #define GBN_FLAG_TABLE_ONLY 1
