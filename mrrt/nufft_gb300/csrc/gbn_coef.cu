@@ -39,14 +39,18 @@ __global__ void __launch_bounds__(256) coef_kernel(const CoefParams<R> p) {
         ++d;
     }
     R cr, ci = (R)0;
-    if (p.wr[0]) {
+    int f = 0;
+    if (p.wr[0] || k == 0) {
         // the gather list is sorted by frame first, one entry per sample
-        int f = 0, hi = p.F;
+        int hi = p.F;
         while (hi - f > 1) {
             const int mid = (f + hi) >> 1;
             if (p.foff[mid] <= e) f = mid;
             else hi = mid;
         }
+    }
+    if (k == 0) p.place[p.foff[f] + p.s.idx[e]] = (int)e;
+    if (p.wr[0]) {
         const int64_t w = (p.foff[f] + p.s.idx[e]) * g.J[d] + j;
         cr = p.wr[d][w];
         if (CX) ci = p.wi[d][w];

@@ -78,8 +78,8 @@ __device__ __forceinline__ int first_tap(double t, int J) {
 // two operations a cycle: the integer part of J/2 comes off exactly, and of t
 // only the place of its fraction against 1/2 is asked.  Below 2^-26 a negative
 // t may vanish in the double difference, so it takes that way.  (Computing a
-// plan's gather records was bound by this: 128^3 kooshball 1.62 -> 0.81 ms,
-// its visits 11.4 -> 9.9; a re-binning of 65536 samples 281 -> 264 us.)
+// plan's gather records was bound by this: 128^3 kooshball 1.62 -> 0.81 ms;
+// a re-binning of 65536 samples 281 -> 264 us.)
 __device__ __forceinline__ int first_tap(float t, int J) {
     if (t < 0.0f && t > -0x1p-26f) return first_tap((double)t, J);
     const float h = floorf(t);

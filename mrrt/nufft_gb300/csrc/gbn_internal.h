@@ -99,6 +99,7 @@ struct CoefParams {
     int off, stride;                // an entry's coefficients lie from out + e * stride + off on
     int jsum;
     int cx;
+    int* place;                     // [samples] list position of each sample
 };
 
 template <typename R>
@@ -129,8 +130,9 @@ struct VisitBuildParams {
     const int4* items;              // {frame, tile, start, count}
     int nitems, nblk;               // register blocks per tile
     const int64_t* foff;
-    const R* wr[3];                 // sparse-matrix weights, or nullptr: the tables
-    const R* wi[3];
+    const R* rec;                   // the gather's coefficients, at rec + place[sample] * stride
+    const int* place;
+    int stride, jsum;
     int cx;
     int* count;                     // [nitems * nblk], multiples of four
     const long long* start;         // exclusive scan of the counts, [nitems * nblk + 1]

@@ -224,7 +224,7 @@ struct gbn_plan {
     // visit lists of the spread (gbn_visit.cuh): offsets per (item, block), sample
     // indices, clipped coefficients; the sample phase in sample order; the values of a
     // call, coil-minor (grown on demand)
-    DevBuf vstart, vidx, vco, vwork, phnat, vals;
+    DevBuf vstart, vidx, vco, vwork, place, phnat, vals;
     int64_t nvisits = 0;  // extent of vidx and vco in visits
     int n_heavy[SPREAD_HEAVY_LEVELS] = {0};   // leading spread items of more entries than 32 << level
     bool coefs = false;   // gcoef and vco hold the current points' coefficients
@@ -1577,7 +1577,11 @@ int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
     b.nitems = P->n_sitems;
     b.nblk = spread_threads(P->geom.ndim, P->Ts) / 32;
     b.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
-    weight_pointers<R>(P, b.wr, b.wi);
+    const GatherRecord rec(P);
+    b.rec = reinterpret_cast<const R*>(P->gcoef.p) + rec.off;
+    b.place = static_cast<const int*>(P->place.p);
+    b.stride = rec.stride;
+    b.jsum = rec.jsum;
     b.cx = P->cx ? 1 : 0;
     const int64_t units = (int64_t)b.nitems * b.nblk;
     auto ensure = [](DevBuf& d, size_t bytes) {
@@ -1626,8 +1630,11 @@ int fill_coefs(gbn_plan* P, cudaStream_t stream = 0, bool sync = true, int64_t t
         const GatherRecord rec(P);
         const size_t bytes = std::max<size_t>((size_t)P->glen * rec.stride * sizeof(R), 16);
         if (P->gcoef.bytes < bytes) GBN_CUDA(P->gcoef.alloc(bytes), "gather coefficient allocation");
+        const size_t pbytes = std::max<size_t>((size_t)P->M_total * sizeof(int), 16);
+        if (P->place.bytes < pbytes) GBN_CUDA(P->place.alloc(pbytes), "sample place allocation");
         CoefParams<R> c;
         std::memset(&c, 0, sizeof(c));
+        c.place = static_cast<int*>(P->place.p);
         c.g = make_geom<R>(P, false);
         c.s = make_list<R>(P, P->glist, P->glen, false);
         c.foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
@@ -2270,7 +2277,7 @@ int gbn_plan_stats(const gbn_plan* P, int64_t* o) {
     o[5] = (int64_t)P->ntiles_s * P->F;
     o[6] = (int64_t)(P->tables.bytes + P->weights.bytes + P->gcoef.bytes +
                      P->vstart.bytes + P->vidx.bytes + P->vco.bytes + P->vwork.bytes + P->phnat.bytes +
-                     P->vals.bytes + P->ptab.bytes + P->half.bytes + P->coil_images.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
+                     P->vals.bytes + P->place.bytes + P->ptab.bytes + P->half.bytes + P->coil_images.bytes + P->mid.bytes + P->sn.bytes + P->glist.bytes + P->slist.bytes + P->pad.bytes +
                      P->grid.bytes + P->scratch.bytes);
     o[7] = P->M_total;
     return GBN_OK;

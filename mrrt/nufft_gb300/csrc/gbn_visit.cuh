@@ -110,26 +110,13 @@ __device__ __forceinline__ void cp_async_wait_pending() {
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-// Coefficient k of the visit of list entry e (sample idx of the frame at
-// offset fo) to the block at (b0, b1, b2): from the per-sample weights when
-// set, else from the tables; conjugated for a complex kernel.
-template <typename R, int NDIM, bool CX>
-__device__ __forceinline__ typename Cx<R>::T visit_coef(const Geom<R>& g, const SampleList<R>& s, int64_t e, short4 ls,
-                                                        int64_t m, const R* const* wr, const R* const* wi, int b0,
-                                                        int b1, int b2, int k) {
+// Coefficient k of a visit to the block at (b0, b1, b2) of a window starting
+// at ls; coef(d, j) gives tap j of axis d.
+template <typename R, int NDIM, bool CX, typename F>
+__device__ __forceinline__ typename Cx<R>::T clipped_coef(const Geom<R>& g, short4 ls, int b0, int b1, int b2, int k,
+                                                          F coef) {
     typedef VisitBlock<NDIM> VB;
     typedef typename Cx<R>::T C;
-    auto coef = [&](int d, int j) -> C {
-        R cr, ci = (R)0;
-        if (wr && wr[0]) {
-            cr = wr[d][m * g.J[d] + j];
-            if (CX) ci = wi[d][m * g.J[d] + j];
-        } else {
-            const R t = s.t[d][e];
-            table_coef<R, CX>(g, d, t, first_tap(t, g.J[d]) + j, cr, ci);
-        }
-        return cmake<R>(cr, CX ? -ci : (R)0);
-    };
     // one path for both axes: lanes of a warp hold coefficients of either
     const int d = NDIM > 1 && k >= VB::B0 ? 1 : 0;
     const int j = d ? b1 + (k - VB::B0) - ls.y : b0 + k - ls.x;
@@ -140,6 +127,18 @@ __device__ __forceinline__ typename Cx<R>::T visit_coef(const Geom<R>& g, const 
         w = CX ? cmul_fixed(w, c2) : cmake<R>(mul_rn(w.x, c2.x), (R)0);
     }
     return w;
+}
+
+// The same of list entry e from the tables, conjugated for a complex kernel.
+template <typename R, int NDIM, bool CX>
+__device__ __forceinline__ typename Cx<R>::T visit_coef(const Geom<R>& g, const SampleList<R>& s, int64_t e, short4 ls,
+                                                        int b0, int b1, int b2, int k) {
+    return clipped_coef<R, NDIM, CX>(g, ls, b0, b1, b2, k, [&](int d, int j) {
+        const R t = s.t[d][e];
+        R cr, ci = (R)0;
+        table_coef<R, CX>(g, d, t, first_tap(t, g.J[d]) + j, cr, ci);
+        return cmake<R>(cr, CX ? -ci : (R)0);
+    });
 }
 
 // ---- plan time ---------------------------------------------------------------
@@ -222,14 +221,16 @@ __global__ void __launch_bounds__(256) visit_fill_kernel(const VisitBuildParams<
     if (at + lane < end) p.vidx[at + lane] = -1;
 }
 
-// Their coefficients, a thread to each, and the sample indices in place of
-// the positions.  A visit waits for four loads in a chain (position, sample,
-// coordinate, table), so an item's visits, up to some thousands, go to the
-// threads of up to VISIT_SLICES CTAs, VISIT_UNROLL at a time; most items need
-// one.  Bound by the instructions of a coefficient: 34 us for 330,000 visits
-// (512 x 512 grid, J = 6).  With the warp of each block computing them where
-// it found the visits, a lane to a visit, one launch took 90 us; with both
-// axes in separate branches this one took 51.
+// Their coefficients, a thread to each, copied from the gather's record of
+// the sample (the same numbers: a sample's coefficients do not depend on the
+// block), and the sample indices in place of the positions.  A visit waits
+// for a chain of loads (position, sample, record's place, record), so an
+// item's visits, up to some thousands, go to the threads of up to
+// VISIT_SLICES CTAs, VISIT_UNROLL at a time; most items need one.  128^3
+// kooshball, 10^8 visits: 3.4 ms for 7.5 GB; computed from the tables, two
+// scattered reads a coefficient, 9.9.  (With the warp of each block making
+// them where it found the visits, a lane to a visit, the 330,000 visits of a
+// 512 x 512 grid took 90 us in place of 34.)
 constexpr int VISIT_SLICES = 4;
 
 template <typename R, int NDIM, bool CX>
@@ -276,7 +277,11 @@ __global__ void __launch_bounds__(256) visit_coef_kernel(const VisitBuildParams<
             c[u] = cmake<R>(!CX && k >= VB::B0 ? (R)-0.0 : (R)0, (R)0);
             if (e[u] >= 0) {
                 const int4 o = block[blk[u]];
-                c[u] = visit_coef<R, NDIM, CX>(g, p.s, e[u], p.s.ls[e[u]], fo + idx[u], p.wr, p.wi, o.x, o.y, o.z, k);
+                const R* r = p.rec + (int64_t)p.place[fo + idx[u]] * p.stride;
+                c[u] = clipped_coef<R, NDIM, CX>(g, p.s.ls[e[u]], o.x, o.y, o.z, k, [&](int d, int j) {
+                    j += (d > 0 ? g.J[0] : 0) + (d > 1 ? g.J[1] : 0);
+                    return cmake<R>(r[j], CX ? -r[p.jsum + j] : (R)0);
+                });
             }
         }
         __syncwarp();   // a visit's lanes, one warp, have read its position
@@ -582,7 +587,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
                 const short4 ls = p.s.ls[e];
 #pragma unroll
                 for (int k = 0; k < VB::NC; ++k) {
-                    const C c = visit_coef<R, NDIM, CX>(g, p.s, e, ls, 0, nullptr, nullptr, b0, b1, b2, k);
+                    const C c = visit_coef<R, NDIM, CX>(g, p.s, e, ls, b0, b1, b2, k);
                     if (CX) {
                         co[u][2 * k] = c.x;
                         co[u][2 * k + (CX ? 1 : 0)] = c.y;
@@ -751,7 +756,7 @@ spread_stream_kernel(const VisitParams<R> p) {
                         for (int b = 1; b < nblk; ++b) blk += (int)(st[b] - base) <= lo + issued + vi;
                         int b0, b1, b2;
                         block_origin_of(p, blk, b0, b1, b2);
-                        const C c = visit_coef<R, NDIM, CX>(g, p.s, e, p.s.ls[e], 0, nullptr, nullptr, b0, b1, b2, k1);
+                        const C c = visit_coef<R, NDIM, CX>(g, p.s, e, p.s.ls[e], b0, b1, b2, k1);
                         if (CX) {
                             cb[2 * q] = c.x;
                             cb[2 * q + 1] = c.y;
