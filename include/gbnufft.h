@@ -107,7 +107,12 @@ int gbn_plan_create(gbn_plan** plan, const gbn_geometry* geom,
                     const void* tm, const void* sample_phase, int device);
 
 /* Replace the sample coordinates (and sample phase) of an existing plan with
- * the same frame offsets; rebuilds the tile lists.                          */
+ * the same frame offsets; rebuilds the tile lists.  Invalid coordinates
+ * (non-finite, |tm| > 2^22) return GBN_ERR_INVALID and keep the previous
+ * points.  A call that fails once it has begun to replace them
+ * (GBN_ERR_NOMEM) may leave the plan without points: every transform then
+ * returns GBN_ERR_INVALID, with nothing launched, until a set_points call
+ * succeeds.                                                                 */
 int gbn_plan_set_points(gbn_plan* plan, const void* tm,
                         const void* sample_phase);
 
@@ -118,9 +123,8 @@ int gbn_plan_set_points(gbn_plan* plan, const void* tm,
  * run); the coordinates never pass through host memory.  The call waits
  * for work already queued on the device, and for two 4-to-16-byte counts it
  * reads back on `stream` (to size the lists and launches), then returns with
- * the rest queued on `stream`.  Invalid coordinates (non-finite, |tm| >
- * 2^22) return GBN_ERR_INVALID and keep the previous lists.  Replaces the
- * host-side tm = omega / gamma recomputation of the reference
+ * the rest queued on `stream`.  Failures as for gbn_plan_set_points.  Replaces
+ * the host-side tm = omega / gamma recomputation of the reference
  * (mrrt/nufft/_nufft.py:338-342) when a trajectory is optimised on the GPU. */
 int gbn_plan_set_points_device(gbn_plan* plan, const void* tm,
                                const void* sample_phase, void* stream);

@@ -66,6 +66,7 @@ class NufftOperator(object):
         self.plan.set_dtables(b.kernel_deriv_tables())
         self._omega = om.copy()
         self._omega_t = torch.as_tensor(om, device=self.device)   # the plan's current trajectory
+        self._moved = True   # the plan holds it (not after a re-planning that failed)
         self._gamma_t = torch.tensor(self.gamma, dtype=torch.float64, device=self.device)
         self._shift_t = torch.as_tensor(self.shift_vec, device=self.device)
         self._inv_gamma_t = torch.tensor(1.0 / self.gamma, dtype=self.rtdtype, device=self.device)
@@ -78,27 +79,31 @@ class NufftOperator(object):
         planner."""
         if isinstance(omega, torch.Tensor) and omega.is_cuda:
             om = omega.detach().to(device=self.device, dtype=self.rtdtype).reshape(self.M, self.ndim)
-            if om.data_ptr() == self._omega_t.data_ptr() or torch.equal(om, self._omega_t):
+            if self._moved and (om.data_ptr() == self._omega_t.data_ptr() or torch.equal(om, self._omega_t)):
                 return
             # tm = omega / gamma (in double, rounded to the operator's dtype) and
             # exp(i omega . (n_shift - n_mid)), as the host path computes them
             tm = (om.to(torch.float64) / self._gamma_t).to(self.rtdtype).contiguous()
             phase = torch.exp(1j * (om @ self._shift_t)).to(self.tdtype)
+            self._moved = False
             self.plan.set_points_device(tm, phase)
             self._omega_t = om.clone()
             self._omega = None
+            self._moved = True
             return
         om = omega.detach().cpu().numpy() if isinstance(omega, torch.Tensor) else np.asarray(omega)
         om = np.ascontiguousarray(om, dtype=self.rdt).reshape(self.M, self.ndim)
-        if self._omega is not None and np.array_equal(om, self._omega):
+        if self._moved and self._omega is not None and np.array_equal(om, self._omega):
             return
         tm = np.zeros_like(om)
         for d in range(self.ndim):
             tm[:, d] = om[:, d] / self.gamma[d]
         phase = np.exp(1j * np.dot(om, self.shift_vec)).astype(self.cdt, copy=False)
+        self._moved = False
         self.plan.set_points(tm, phase)
         self._omega = om.copy()
         self._omega_t = torch.as_tensor(om, device=self.device)
+        self._moved = True
 
     # ---------------------------------------------------------- layout glue
     def _image_to_plan(self, x):

@@ -228,6 +228,11 @@ struct gbn_plan {
     int64_t nvisits = 0;  // extent of vidx and vco in visits
     int n_heavy[SPREAD_HEAVY_LEVELS] = {0};   // leading spread items of more entries than 32 << level
     bool coefs = false;   // gcoef and vco hold the current points' coefficients
+    // A re-planning that fails part way (an allocation) leaves lists that no kernel
+    // may read: `listed` says that the sample lists and work items are those of one
+    // set of points, `ready` that the visits and coefficients are theirs too.
+    // Transforms refuse a plan that is not ready.
+    bool listed = false, ready = false;
     DevBuf glist, gitems;
     DevBuf bin_ws, bin_ws2;   // device binning workspaces (grown on demand)
     DevBuf slist, sitems, sparts, rtiles;
@@ -654,6 +659,8 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
         if (e != cudaSuccess) return cuda_fail(e, "list upload");
         return GBN_OK;
     };
+    P->listed = P->ready = false;
+    P->has_phase = phase != nullptr;
     int rc = pack(gorder, nullptr, P->glist, Mt);
     if (rc) return rc;
     rc = pack(sorder, sls.data(), P->slist, slen);
@@ -728,6 +735,7 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
     P->n_sitems = (int)sa.size();
     P->n_rtiles = (int)rt.size();
     P->n_slots = slots;
+    P->listed = true;
     return GBN_OK;
 }
 
@@ -756,6 +764,7 @@ int ensure_scratch(gbn_plan* P, int coils) {
     // never increases chunks * LS)
     const int64_t need = (int64_t)P->n_slots * chunks * ln.LS * tile_cells;
     if (need > P->scratch_cap) {
+        P->scratch_cap = 0;
         cudaError_t e = P->scratch.alloc((size_t)need * csz);
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "scratch allocation failed");
         P->scratch_cap = need;
@@ -1604,6 +1613,7 @@ int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
         total += 3 * units;   // padding, at most
     }
     const int NC = P->geom.ndim == 1 ? 16 : 8;
+    P->nvisits = 0;
     GBN_CUDA(ensure(P->vidx, (size_t)total * sizeof(int)), "visit allocation");
     if (coefs)
         GBN_CUDA(ensure(P->vco, (size_t)total * NC * (P->cx ? 2 : 1) * sizeof(R)), "visit allocation");
@@ -1623,7 +1633,7 @@ int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
 // kernels (GBN_FLAG_TABLE_ONLY).  `total`: as for build_visits.
 template <typename R>
 int fill_coefs(gbn_plan* P, cudaStream_t stream = 0, bool sync = true, int64_t total = -1) {
-    P->coefs = false;
+    P->coefs = P->ready = false;
     const gbn_geometry& G = P->geom;
     const bool keep = P->weights.p || !(G.flags & GBN_FLAG_TABLE_ONLY);
     if (keep) {
@@ -1653,13 +1663,13 @@ int fill_coefs(gbn_plan* P, cudaStream_t stream = 0, bool sync = true, int64_t t
     if (rc) return rc;
     if (sync) GBN_CUDA(cudaDeviceSynchronize(), "coefficient precompute");
     P->coefs = keep;
+    P->ready = true;
     return GBN_OK;
 }
 
 template <typename R>
 int plan_points(gbn_plan* P, const void* tm, const void* phase) {
     if (!tm && P->M_total > 0) return fail(GBN_ERR_INVALID, "null coordinate array");
-    P->has_phase = phase != nullptr;
     int rc = build_lists<R>(P, reinterpret_cast<const R*>(tm), reinterpret_cast<const R*>(phase));
     if (rc) return rc;
     return fill_coefs<R>(P);
@@ -1861,6 +1871,7 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
         return GBN_OK;
     };
     int rc;
+    P->listed = P->ready = false;
     if ((rc = ensure(P->gitems, (size_t)n_gi * sizeof(int4), "item allocation"))) return rc;
     if ((rc = ensure(P->sitems, (size_t)n_si * sizeof(int4), "item allocation"))) return rc;
     if ((rc = ensure(P->sparts, (size_t)n_si * sizeof(int2), "item allocation"))) return rc;
@@ -1927,6 +1938,7 @@ int device_build_lists(gbn_plan* P, const R* tm, const typename Cx<R>::T* ph, cu
         if ((rc = ensure(P->phnat, (size_t)M * sizeof(C), "phase allocation"))) return rc;
         GBN_CUDA(cudaMemcpyAsync(P->phnat.p, ph, (size_t)M * sizeof(C), cudaMemcpyDeviceToDevice, s), "phase copy");
     }
+    P->listed = true;
     return fill_coefs<R>(P, s, false, (int64_t)nvisits);
 }
 
@@ -2069,6 +2081,13 @@ int gbn_plan_destroy(gbn_plan* P) {
     return GBN_OK;
 }
 
+// Under the plan's lock: its lists are complete.
+static int check_ready(const gbn_plan* P) {
+    if (P->ready) return GBN_OK;
+    return fail(GBN_ERR_INVALID, "the plan has no sample points: its last re-planning failed "
+                                 "(gbn_plan_set_points or gbn_plan_set_points_device gives it new ones)");
+}
+
 static int check_call(gbn_plan* P, const void* a, const void* b, int coils) {
     if (!P) return fail(GBN_ERR_INVALID, "null plan");
     if (coils < 1) return fail(GBN_ERR_INVALID, "coils must be >= 1");
@@ -2083,6 +2102,7 @@ int gbn_forward(gbn_plan* P, const void* x, void* y, int coils, void* stream) {
     if (rc) return rc;
     if (!x) return fail(GBN_ERR_INVALID, "null image");   // read even without samples
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_forward<double>(P, x, y, coils, s) : run_forward<float>(P, x, y, coils, s);
@@ -2093,6 +2113,7 @@ int gbn_adjoint(gbn_plan* P, const void* y, void* x, int coils, void* stream) {
     if (rc) return rc;
     if (!x) return fail(GBN_ERR_INVALID, "null image");   // written even without samples
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_adjoint<double>(P, y, x, coils, s) : run_adjoint<float>(P, y, x, coils, s);
@@ -2103,6 +2124,7 @@ int gbn_forward_host(gbn_plan* P, const void* x, void* y, int coils, void* strea
     if (rc) return rc;
     if (!x) return fail(GBN_ERR_INVALID, "null image");
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_host<double>(P, true, x, y, coils, s) : run_host<float>(P, true, x, y, coils, s);
@@ -2113,6 +2135,7 @@ int gbn_adjoint_host(gbn_plan* P, const void* y, void* x, int coils, void* strea
     if (rc) return rc;
     if (!x) return fail(GBN_ERR_INVALID, "null image");
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_host<double>(P, false, y, x, coils, s) : run_host<float>(P, false, y, x, coils, s);
@@ -2123,6 +2146,7 @@ int gbn_forward_sense(gbn_plan* P, const void* image, const void* maps, void* y,
     if (rc) return rc;
     if (!maps || !image) return fail(GBN_ERR_INVALID, "null image or coil maps");
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_forward<double>(P, image, y, coils, s, maps) : run_forward<float>(P, image, y, coils, s, maps);
@@ -2133,6 +2157,7 @@ int gbn_adjoint_sense(gbn_plan* P, const void* y, const void* maps, void* image,
     if (rc) return rc;
     if (!maps || !image) return fail(GBN_ERR_INVALID, "null image or coil maps");
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_adjoint<double>(P, y, image, coils, s, maps) : run_adjoint<float>(P, y, image, coils, s, maps);
@@ -2142,6 +2167,7 @@ int gbn_interp_forward(gbn_plan* P, const void* grid, void* y, int coils, void* 
     int rc = check_call(P, grid, y, coils);
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_gather<double>(P, grid, y, coils, Grid::abi, s)
@@ -2153,6 +2179,7 @@ int gbn_interp_adjoint(gbn_plan* P, const void* y, void* grid, int coils, void* 
     if (rc) return rc;
     if (!grid) return fail(GBN_ERR_INVALID, "null grid");   // written even without samples
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_spread<double>(P, y, grid, coils, Grid::abi, s)
@@ -2164,6 +2191,7 @@ int gbn_interp_adjoint_noalloc(gbn_plan* P, const void* y, void* grid, int coils
     if (rc) return rc;
     if (!grid) return fail(GBN_ERR_INVALID, "null grid");
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_spread_noalloc<double>(P, y, grid, coils, s)
@@ -2202,6 +2230,7 @@ int gbn_plan_set_weights(gbn_plan* P, const void* const* w_re, const void* const
     if (!P) return fail(GBN_ERR_INVALID, "null plan");
     std::lock_guard<std::mutex> lk(P->mu);
     DeviceGuard guard(P->device);
+    if (!P->listed) return check_ready(P);
     GBN_CUDA(cudaDeviceSynchronize(), "synchronise before replacing weights");
     if (!w_re) {
         GBN_CUDA(P->weights.alloc(0), "weight release");
@@ -2239,6 +2268,7 @@ int gbn_grad_tm(gbn_plan* P, const void* grid, const void* gy, const double* pha
     if (!P->dtables.p) return fail(GBN_ERR_INVALID, "derivative tables not set (gbn_plan_set_dtables)");
     if (P->weights.p) return fail(GBN_ERR_UNSUPPORTED, "coordinate gradient needs table interpolation");
     std::lock_guard<std::mutex> lk(P->mu);
+    if ((rc = check_ready(P))) return rc;
     DeviceGuard guard(P->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return P->dbl ? run_grad<double>(P, grid, gy, phase_shift, gtm, coils, s)
