@@ -13,7 +13,8 @@
 //   dL/dt_d = sum_c Re(conj(gy[m,c]) dy[m,c]/dt_d).
 // One thread per sample (samples in gather-list order, so neighbouring
 // threads read neighbouring grid taps); coils are summed inside the thread.
-// phase_before is separable, so it is folded into the per-axis coefficients
+// The grid of a plan on its own FFT passes holds phase_before already;
+// elsewhere it is separable, so it is folded into the per-axis coefficients
 // (J sincos per axis per sample instead of one per tap per coil).  The
 // kernel has no counterpart in the reference, which has no autograd.
 #include <cuda_runtime.h>

@@ -246,7 +246,7 @@ struct GradParams {
     int coils;
     int apply_pb;
     R grid_scale;
-    const typename Cx<R>::T* grid;  // [coils][Kprod], before phase_before
+    const typename Cx<R>::T* grid;  // as the forward left it: before phase_before (apply_pb) or after
     const typename Cx<R>::T* gy;    // [coils][M] incoming gradient
     R* gtm;                         // [M][ndim] out
 };

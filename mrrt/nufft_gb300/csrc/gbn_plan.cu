@@ -985,10 +985,11 @@ int colfft_2d(gbn_plan* P, int planes, int sign, cudaStream_t s) {
     return run_pass(P, a, sign, s);
 }
 
-// Whether a forward call leaves phase_before (and the orthonormal scale)
-// applied to its grid: plans with derivative tables keep the grid that
-// gbn_grad_tm takes, from before it.
-bool grid_phased(const gbn_plan* P) { return P->geom.phasing == GBN_PHASING_REAL && !P->dtables.p; }
+// Whether a forward call on the plan's own passes leaves phase_before and the
+// orthonormal scale applied to its grid.  The same for every call of a plan:
+// gbn_grad_tm takes that grid whenever its tables were set, also from a graph
+// captured before.
+bool grid_phased(const gbn_plan* P) { return P->geom.phasing == GBN_PHASING_REAL; }
 
 // Transform on the plan's own passes, on coil-minor arrays, widening the axes
 // from the slowest to the contiguous one (sign -1) or narrowing them back:
@@ -1966,8 +1967,9 @@ int run_grad(gbn_plan* P, const void* grid, const void* gy, const double* shift,
     p.ph = L.ph;
     p.M = P->glen;
     p.coils = coils;
-    p.apply_pb = P->geom.phasing == GBN_PHASING_REAL;
-    p.grid_scale = P->geom.ortho ? (R)std::sqrt((double)P->Kprod) : (R)1;
+    const bool done = P->own && grid_phased(P);
+    p.apply_pb = !done && P->geom.phasing == GBN_PHASING_REAL;
+    p.grid_scale = !done && P->geom.ortho ? (R)std::sqrt((double)P->Kprod) : (R)1;
     p.grid = reinterpret_cast<const C*>(grid);
     p.gy = reinterpret_cast<const C*>(gy);
     p.gtm = reinterpret_cast<R*>(gtm);
