@@ -48,7 +48,7 @@ def _run(adjoint, data, omega, shape, n_shift):
     is_torch = isinstance(data, torch.Tensor)
     dev = data.device if is_torch and data.is_cuda else torch.device("cuda")
     if is_torch:
-        arr = data.detach().to(dev, torch.complex128)
+        arr = data.detach().to(dev, torch.complex128).resolve_conj().resolve_neg()
         # Fortran convention: leading axes are the image (or sample) axes
         lead = (M,) if adjoint else shape
         nlead = len(lead)

@@ -372,7 +372,7 @@ class NufftBase(object):
             t = a.detach()
             if not t.is_complex():
                 t = t.to(torch.float64 if self._real_dtype == np.float64 else torch.float32)
-            t = t.to(device=dev, dtype=ct)
+            t = t.to(device=dev, dtype=ct).resolve_conj().resolve_neg()
         else:
             arr = np.asarray(a)
             if arr.dtype != self._cplx_dtype:
@@ -481,7 +481,7 @@ class NufftBase(object):
         else."""
         plan = self._plan
         if type(a) is not torch.Tensor or a.dtype is not plan.ctype or a.device != plan.device or \
-                not self.__on_gpu or self.order != "F" or a.is_conj():
+                not self.__on_gpu or self.order != "F" or a.is_conj() or a.is_neg():
             return None
         lead, strides, n, out_lead, out_strides, m = self._direct[forward]
         nd = len(lead)

@@ -110,22 +110,35 @@ class GpuPlan:
             self.handle = None
 
     # -- transforms on device tensors in the plan's memory layout -------------
+    # The memory of a lazily conjugated or negated view is not what the view means:
+    # an input (_input) is resolved first, an output refused.
     def _check(self, t, numel, name):
         if type(t) is torch.Tensor and t.is_cuda and t.dtype is self.ctype and t.numel() == numel \
-                and t.is_contiguous():
+                and t.is_contiguous() and not (t.is_conj() or t.is_neg()):
             return
         if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
             raise ValueError("%s must be a CUDA tensor" % name)
+        self._check_form(t, numel, name)
+
+    def _check_form(self, t, numel, name):
         if t.dtype != self.ctype:
             raise ValueError("%s must be %s, got %s" % (name, self.ctype, t.dtype))
         if not t.is_contiguous():
             raise ValueError("%s must be contiguous" % name)
         if t.numel() != numel:
             raise ValueError("%s has %d elements, expected %d" % (name, t.numel(), numel))
+        if t.is_conj() or t.is_neg():
+            raise ValueError("%s must not be a lazily conjugated or negated view" % name)
+
+    def _input(self, t, numel, name, host=False):
+        if isinstance(t, torch.Tensor) and (t.is_conj() or t.is_neg()):
+            t = t.resolve_conj().resolve_neg()
+        (self._check_host if host else self._check)(t, numel, name)
+        return t
 
     def forward(self, x, y, coils):
         F = len(self.frame_offsets) - 1
-        self._check(x, F * coils * self.Nprod, "x")
+        x = self._input(x, F * coils * self.Nprod, "x")
         self._check(y, coils * self.M_total, "y")
         # the library switches to the plan's device itself
         rc = self.lib.gbn_forward(self.handle, x.data_ptr(), y.data_ptr(), int(coils), raw_stream(self.device.index))
@@ -135,7 +148,7 @@ class GpuPlan:
 
     def adjoint(self, y, x, coils):
         F = len(self.frame_offsets) - 1
-        self._check(y, coils * self.M_total, "y")
+        y = self._input(y, coils * self.M_total, "y")
         self._check(x, F * coils * self.Nprod, "x")
         # the library switches to the plan's device itself
         rc = self.lib.gbn_adjoint(self.handle, y.data_ptr(), x.data_ptr(), int(coils), raw_stream(self.device.index))
@@ -146,19 +159,14 @@ class GpuPlan:
     def _check_host(self, t, numel, name):
         if not isinstance(t, torch.Tensor) or t.device.type != "cpu":
             raise ValueError("%s must be a CPU tensor" % name)
-        if t.dtype != self.ctype:
-            raise ValueError("%s must be %s, got %s" % (name, self.ctype, t.dtype))
-        if not t.is_contiguous():
-            raise ValueError("%s must be contiguous" % name)
-        if t.numel() != numel:
-            raise ValueError("%s has %d elements, expected %d" % (name, t.numel(), numel))
+        self._check_form(t, numel, name)
 
     def forward_host(self, x, y, coils):
         """Forward transform of host memory into host memory (CPU tensors in
         the device layouts, pageable or pinned); returns when y holds the
         result."""
         F = len(self.frame_offsets) - 1
-        self._check_host(x, F * coils * self.Nprod, "x")
+        x = self._input(x, F * coils * self.Nprod, "x", host=True)
         self._check_host(y, coils * self.M_total, "y")
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_forward_host(self.handle, ctypes.c_void_p(x.data_ptr()),
@@ -168,7 +176,7 @@ class GpuPlan:
     def adjoint_host(self, y, x, coils):
         """Adjoint transform of host memory into host memory."""
         F = len(self.frame_offsets) - 1
-        self._check_host(y, coils * self.M_total, "y")
+        y = self._input(y, coils * self.M_total, "y", host=True)
         self._check_host(x, F * coils * self.Nprod, "x")
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_adjoint_host(self.handle, ctypes.c_void_p(y.data_ptr()),
@@ -179,8 +187,8 @@ class GpuPlan:
         """Coil-sensitivity forward: image [F, N...] and maps [coils, N...]
         (plan layout) -> samples, the map multiply fused into the pad."""
         F = len(self.frame_offsets) - 1
-        self._check(image, F * self.Nprod, "image")
-        self._check(maps, coils * self.Nprod, "maps")
+        image = self._input(image, F * self.Nprod, "image")
+        maps = self._input(maps, coils * self.Nprod, "maps")
         self._check(y, coils * self.M_total, "y")
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_forward_sense(self.handle, ctypes.c_void_p(image.data_ptr()),
@@ -192,8 +200,8 @@ class GpuPlan:
         """Coil-combining adjoint: samples -> image [F, N...] = sum over coils
         of conj(maps) times each coil's adjoint, fused into the crop."""
         F = len(self.frame_offsets) - 1
-        self._check(y, coils * self.M_total, "y")
-        self._check(maps, coils * self.Nprod, "maps")
+        y = self._input(y, coils * self.M_total, "y")
+        maps = self._input(maps, coils * self.Nprod, "maps")
         self._check(image, F * self.Nprod, "image")
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_adjoint_sense(self.handle, ctypes.c_void_p(y.data_ptr()),
@@ -203,7 +211,7 @@ class GpuPlan:
 
     def interp_forward(self, grid, y, coils):
         F = len(self.frame_offsets) - 1
-        self._check(grid, F * coils * self.Kprod, "grid")
+        grid = self._input(grid, F * coils * self.Kprod, "grid")
         self._check(y, coils * self.M_total, "y")
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_interp_forward(self.handle, ctypes.c_void_p(grid.data_ptr()),
@@ -213,7 +221,7 @@ class GpuPlan:
 
     def interp_adjoint(self, y, grid, coils):
         F = len(self.frame_offsets) - 1
-        self._check(y, coils * self.M_total, "y")
+        y = self._input(y, coils * self.M_total, "y")
         self._check(grid, F * coils * self.Kprod, "grid")
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_interp_adjoint(self.handle, ctypes.c_void_p(y.data_ptr()),
@@ -235,7 +243,7 @@ class GpuPlan:
             _lib.check_with(self.lib, self.lib.gbn_plan_set_dtables(self.handle, D))
 
     def grad_tm(self, grid_ptr, gy, phase_shift, gtm, coils):
-        self._check(gy, coils * self.M_total, "gy")
+        gy = self._input(gy, coils * self.M_total, "gy")
         sh = (ctypes.c_double * 3)(*[float(s) for s in phase_shift] + [0.0] * (3 - len(phase_shift)))
         with torch.cuda.device(self.device):
             _lib.check_with(self.lib, self.lib.gbn_grad_tm(self.handle, ctypes.c_void_p(grid_ptr),
@@ -274,13 +282,13 @@ class GpuPlan:
         the tile lists are rebuilt by kernels on the plan's device, on the
         current stream."""
         rt = torch.float32 if self.rdt == np.float32 else torch.float64
-        tm = tm.to(device=self.device, dtype=rt).contiguous()
+        tm = tm.to(device=self.device, dtype=rt).contiguous().resolve_neg()
         if tm.numel() != self.M_total * self.ndim:
             raise ValueError("set_points keeps the sample count; got %d coordinates, expected %d"
                              % (tm.numel(), self.M_total * self.ndim))
         ph = None
         if sample_phase is not None:
-            ph = sample_phase.to(device=self.device, dtype=self.ctype).contiguous()
+            ph = sample_phase.to(device=self.device, dtype=self.ctype).contiguous().resolve_conj().resolve_neg()
             if ph.numel() != self.M_total:
                 raise ValueError("sample_phase needs %d values" % self.M_total)
         with torch.cuda.device(self.device):

@@ -78,7 +78,7 @@ class NufftOperator(object):
         the device (device binning); a host array goes through the host
         planner."""
         if isinstance(omega, torch.Tensor) and omega.is_cuda:
-            om = omega.detach().to(device=self.device, dtype=self.rtdtype).reshape(self.M, self.ndim)
+            om = omega.detach().to(device=self.device, dtype=self.rtdtype).resolve_neg().reshape(self.M, self.ndim)
             if self._moved and (om.data_ptr() == self._omega_t.data_ptr() or torch.equal(om, self._omega_t)):
                 return
             # tm = omega / gamma (in double, rounded to the operator's dtype) and
