@@ -171,7 +171,8 @@ struct VisitParams {
     short4 borg[8];
     int64_t boff[8], bcell[8];
     int bscr[8];
-    int nshared;                    // set by the launcher: leading items shared by a CTA's warps
+    int nshared, nwhole;            // set by the launcher: leading items shared by a CTA's warps, in equal
+                                    // runs, and further on a block to each
     int coils, LS, chunks, row;
     const int64_t* foff;
     const typename Cx<R>::T* vals;  // [frame][m][row] (launch_values), or nullptr: read y in place
