@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(256) coef_kernel(const CoefParams<R> p) {
     }
     R cr, ci = (R)0;
     int f = 0;
-    if (p.wr[0] || k == 0) {
+    if (p.wr[0] || k == 0 || !p.place) {
         // the gather list is sorted by frame first, one entry per sample
         int hi = p.F;
         while (hi - f > 1) {
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(256) coef_kernel(const CoefParams<R> p) {
             else hi = mid;
         }
     }
-    if (k == 0) p.place[p.foff[f] + p.s.idx[e]] = (int)e;
+    if (k == 0 && p.place) p.place[p.foff[f] + p.s.idx[e]] = (int)e;
     if (p.wr[0]) {
         const int64_t w = (p.foff[f] + p.s.idx[e]) * g.J[d] + j;
         cr = p.wr[d][w];
@@ -58,10 +58,10 @@ __global__ void __launch_bounds__(256) coef_kernel(const CoefParams<R> p) {
         const R t = p.s.t[d][e];
         table_coef<R, CX>(g, d, t, first_tap(t, g.J[d]) + j, cr, ci);
     }
-    R* rec = p.out + e * p.stride;
+    R* rec = p.out + (p.place ? e : p.foff[f] + p.s.idx[e]) * p.stride;
     rec[p.off + k] = cr;
     if (CX) rec[p.off + p.jsum + k] = ci;
-    if (sizeof(R) == 4 && !CX && k == 0) {
+    if (sizeof(R) == 4 && !CX && k == 0 && p.place) {
         // the record's head: {cell of the window's start in the staged tile, index, phase}
         int cell = 0, mul = 1;
         for (int a = 0; a < g.ndim; ++a) {

@@ -99,7 +99,8 @@ struct CoefParams {
     int off, stride;                // an entry's coefficients lie from out + e * stride + off on
     int jsum;
     int cx;
-    int* place;                     // [samples] list position of each sample
+    int* place;                     // [samples] list position of each sample; nullptr: the coefficients
+                                    // alone, of sample m (all frames) at out + m * stride + off
 };
 
 template <typename R>
@@ -176,6 +177,8 @@ struct VisitParams {
     int coils, LS, chunks, row;
     const int64_t* foff;
     const typename Cx<R>::T* vals;  // [frame][m][row] (launch_values), or nullptr: read y in place
+    int rec;                        // without vco: place in a row of vals, in reals, of the sample's
+                                    // coefficients (launch_coef), or 0: from the tables
     const typename Cx<R>::T* y;
     const typename Cx<R>::T* ph;    // with y: sample phase, sample order, or nullptr
     typename Cx<R>::T* grid;

@@ -748,10 +748,22 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
 // sectors either way (192 x 192, 4 coils: 521 against 506).
 bool use_values(const gbn_plan* P, int coils) { return coils >= (!P->dbl && P->geom.ndim == 3 ? 3 : 5); }
 
-// Values per sample of the coil-minor buffer: the coils, rounded up to 16 bytes.
-int value_row(int coils, size_t csz) {
-    const int unit = (int)(16 / csz);
-    return (coils + unit - 1) / unit * unit;
+// A double precision plan that stores no coefficients computes each sample's
+// once a call, beside its values, and the spread copies them per visit: 12
+// interpolations a sample in place of 40 at 256 x 256, of which an SM does few
+// (8 coils: 736 us, against 1079 computed per visit).  In single precision the
+// copies' loads cost more than the interpolation (112 against 96).
+bool call_records(const gbn_plan* P) { return P->dbl && !P->coefs; }
+
+// A sample's row of the coil-minor buffer, in complex values rounded up to 16
+// bytes: its values, then its coefficients (call_records).
+int values_extent(const gbn_plan* P, int n) {
+    const int unit = P->dbl ? 1 : 2;
+    return (n + unit - 1) / unit * unit;
+}
+int value_row(const gbn_plan* P, int coils) {
+    const int reals = call_records(P) ? GatherRecord(P).jsum * (P->cx ? 2 : 1) : 0;
+    return values_extent(P, coils) + values_extent(P, (reals + 1) / 2);
 }
 
 // Scratch for the partial tiles of split spread work items.
@@ -770,7 +782,7 @@ int ensure_scratch(gbn_plan* P, int coils) {
         P->scratch_cap = need;
     }
     // the coil-minor values of the visit-list spread
-    const size_t vbytes = (size_t)P->M_total * value_row(coils, csz) * csz;
+    const size_t vbytes = (size_t)P->M_total * value_row(P, coils) * csz;
     if (use_values(P, coils) && vbytes > P->vals.bytes) {
         cudaError_t e = P->vals.alloc(vbytes);
         if (e != cudaSuccess) return fail(GBN_ERR_NOMEM, "sample value allocation failed");
@@ -1178,7 +1190,7 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
     p.coils = coils;
     p.LS = ln.LS;
     p.chunks = (coils + ln.LS - 1) / ln.LS;
-    p.row = value_row(coils, sizeof(C));
+    p.row = value_row(P, coils);
     p.foff = foff;
     p.vals = static_cast<const C*>(vals);
     p.y = static_cast<const C*>(y);
@@ -1202,6 +1214,20 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
         v.check = p.g.check;
         v.out_elems = vals_elems;
         GBN_CUDA(launch_values<R>(v, s), "sample values launch");
+        if (call_records(P)) {
+            CoefParams<R> c;
+            std::memset(&c, 0, sizeof(c));
+            c.g = make_geom<R>(P, false);
+            c.s = make_list<R>(P, P->glist, P->glen, false);
+            c.foff = foff;
+            c.F = P->F;
+            c.out = static_cast<R*>(vals);
+            c.off = p.rec = 2 * values_extent(P, coils);
+            c.stride = 2 * p.row;
+            c.jsum = GatherRecord(P).jsum;
+            c.cx = P->cx ? 1 : 0;
+            GBN_CUDA(launch_coef<R>(c, s), "sample coefficients launch");
+        }
     }
     GBN_CUDA(launch_spread_visits<R>(p, s), "spread launch");
     if (P->n_rtiles) {
@@ -1256,7 +1282,7 @@ int run_spread_noalloc(gbn_plan* P, const void* y, void* grid, int coils, cudaSt
     // the values take what the partial sums leave of the array, if they fit;
     // else the samples are read in place
     const int64_t used = (need + 255) & ~(int64_t)255;
-    const int64_t velems = P->M_total * value_row(coils, sizeof(C));
+    const int64_t velems = P->M_total * value_row(P, coils);
     void* vals = use_values(P, coils) && used + velems * (int64_t)sizeof(C) <= (int64_t)cap
                      ? static_cast<char*>(scratch) + used : nullptr;
     return launch_visits<R>(P, y, grid, coils, Grid::abi, vals, velems, scratch, need / (int64_t)sizeof(C), s);

@@ -99,6 +99,28 @@ __device__ __forceinline__ void load_run(const double* src, double (&o)[N]) {
     }
 }
 
+template <int N>
+__device__ __forceinline__ void store_run(float* dst, const float (&v)[N]) {
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4)
+            *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) dst[i] = v[i];
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_run(double* dst, const double (&v)[N]) {
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) *reinterpret_cast<double2*>(dst + i) = make_double2(v[i], v[i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) dst[i] = v[i];
+    }
+}
+
 // 16-byte asynchronous copy of `bytes` (16 or 0) source bytes, zero-filled.
 __device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, bool valid) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -129,16 +151,93 @@ __device__ __forceinline__ typename Cx<R>::T clipped_coef(const Geom<R>& g, shor
     return w;
 }
 
-// The same of list entry e from the tables, conjugated for a complex kernel.
-template <typename R, int NDIM, bool CX>
-__device__ __forceinline__ typename Cx<R>::T visit_coef(const Geom<R>& g, const SampleList<R>& s, int64_t e, short4 ls,
-                                                        int b0, int b1, int b2, int k) {
-    return clipped_coef<R, NDIM, CX>(g, ls, b0, b1, b2, k, [&](int d, int j) {
-        const R t = s.t[d][e];
+// What the coefficients of a visit to list entry e (-1: padding) are computed
+// from.
+template <typename R, int NDIM>
+struct VisitEntry {
+    short4 ls;
+    R t[3];
+    int idx;   // sample index, -1: padding
+    __device__ __forceinline__ void load(const SampleList<R>& s, int e) {
+        idx = -1;
+        ls = make_short4(0, 0, 0, 0);
+#pragma unroll
+        for (int d = 0; d < NDIM; ++d) t[d] = (R)0;
+        if (e < 0) return;
+        idx = s.idx[e];
+        ls = s.ls[e];
+#pragma unroll
+        for (int d = 0; d < NDIM; ++d) t[d] = s.t[d][e];
+    }
+};
+
+// The part-th of P equal runs of the coefficients of a visit to the block at (b0, b1, b2),
+// from the tables, into out: the numbers a plan that keeps them has stored.
+// P lanes share a visit, and a lane reads the entry once for all of its
+// coefficients.  Spread alone: 256 x 256, 4 and 8 coils 47 and 76 us, 60 x 72 x
+// 45, 3 and 8 coils 380 and 462.  (A lane to each coefficient, which read the
+// entry and, of w = c1 c2, the table for c2 anew, and where the samples are read
+// in place each coil lane for itself: 222 and 226, 1331 and 1467.)
+template <typename R, int NDIM, bool CX, int P>
+__device__ __forceinline__ void table_visit(const Geom<R>& g, const VisitEntry<R, NDIM>& v, int b0, int b1, int b2,
+                                            int part, R* out) {
+    typedef VisitBlock<NDIM> VB;
+    typedef typename Cx<R>::T C;
+    int first[3] = {0, 0, 0};
+#pragma unroll
+    for (int d = 0; d < NDIM; ++d) first[d] = first_tap(v.t[d], g.J[d]);
+    auto tap = [&](int d, R td, int k) {
         R cr, ci = (R)0;
-        table_coef<R, CX>(g, d, t, first_tap(t, g.J[d]) + j, cr, ci);
+        table_coef<R, CX>(g, d, td, k, cr, ci);
         return cmake<R>(cr, CX ? -ci : (R)0);
-    });
+    };
+    C c2 = cmake<R>((R)0, (R)0);
+    if (NDIM > 2) c2 = tap(2, v.t[2], first[2] + b2 - v.ls.z);
+    constexpr int NK = VB::NC / P, W = CX ? 2 : 1;
+    R co[NK * W];
+#pragma unroll
+    for (int i = 0; i < NK; ++i) {
+        const int k = part * NK + i, d = NDIM > 1 && k >= VB::B0 ? 1 : 0;
+        const int j = d ? b1 + (k - VB::B0) - v.ls.y : b0 + k - v.ls.x;
+        const bool in = v.idx >= 0 && j >= 0 && j < g.J[d];
+        C c = cmake<R>(d ? (R)-0.0 : (R)0, (R)0);
+        // a tap past the window is computed too (its table index is clamped) and
+        // dropped: behind a branch each, the taps' loads waited for one another
+        if (NDIM > 1 || in) {
+            C w = tap(d, d ? v.t[1] : v.t[0], (d ? first[1] : first[0]) + j);
+            if (NDIM > 2 && d) w = CX ? cmul_fixed(w, c2) : cmake<R>(mul_rn(w.x, c2.x), (R)0);
+            if (in) c = w;
+        }
+        co[i * W] = c.x;
+        if (CX) co[i * W + W - 1] = c.y;
+    }
+    store_run(out + part * NK * W, co);
+}
+
+// The same from the sample's coefficients, J_0 + J_1 + J_2 at rec (imaginary
+// parts behind them).
+template <typename R, int NDIM, bool CX, int P>
+__device__ __forceinline__ void record_visit(const Geom<R>& g, bool on, short4 ls, const R* rec, int b0, int b1, int b2,
+                                             int part, R* out) {
+    typedef VisitBlock<NDIM> VB;
+    typedef typename Cx<R>::T C;
+    const int at1 = g.J[0], at2 = g.J[0] + (NDIM > 1 ? g.J[1] : 0), jsum = at2 + (NDIM > 2 ? g.J[2] : 0);
+    auto tap = [&](int j) { return cmake<R>(rec[j], CX ? -rec[jsum + j] : (R)0); };
+    C c2 = cmake<R>((R)0, (R)0);
+    if (NDIM > 2 && on) c2 = tap(at2 + b2 - ls.z);
+    constexpr int NK = VB::NC / P, W = CX ? 2 : 1;
+    R co[NK * W];
+#pragma unroll
+    for (int i = 0; i < NK; ++i) {
+        const int k = part * NK + i;
+        C c = cmake<R>(NDIM > 1 && k >= VB::B0 ? (R)-0.0 : (R)0, (R)0);
+        if (on)
+            c = clipped_coef<R, NDIM, CX>(g, ls, b0, b1, b2, k,
+                                          [&](int d, int j) { return d == 2 ? c2 : tap((d ? at1 : 0) + j); });
+        co[i * W] = c.x;
+        if (CX) co[i * W + W - 1] = c.y;
+    }
+    store_run(out + part * NK * W, co);
 }
 
 // ---- plan time ---------------------------------------------------------------
@@ -539,7 +638,12 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
     constexpr int SW = 32 / LS;
     // visits in flight per slot, fewer the more registers one takes
     constexpr int WORDS = (int)sizeof(R) / 4 * (CX ? 2 : 1) * (NDIM == 1 ? 2 : 1);
-    constexpr int U = WORDS > 2 || SW > 8 || TAB ? 1 : (WORDS > 1 || SW > 4 ? 2 : 4);
+    constexpr int U = WORDS > 2 || SW > 8 ? 1 : (WORDS > 1 || SW > 4 ? 2 : 4);
+    // coefficients and sample indices of 32 visits, a lane to each, where they
+    // are computed on the way
+    __shared__ __align__(16) R tab_co[TAB ? VISIT_THREADS : 1][NC];
+    __shared__ int tab_id[TAB ? VISIT_THREADS : 1];
+    const int own = TAB ? threadIdx.x & ~31 : 0;
     const Geom<R>& g = p.g;
     const int lane = threadIdx.x & 31;
     const unsigned unit = blockIdx.x * (VISIT_THREADS / 32) + (threadIdx.x >> 5);
@@ -568,36 +672,35 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
 #pragma unroll
     for (int q = 0; q < NB; ++q) acc[q] = cmake<R>((R)0, (R)0);
     const int* vidx = p.vidx + st;
+    VisitEntry<R, NDIM> entry;   // of the 32 visits to come, and the entries after them
+    int next = -1;
+    if (TAB) {
+        entry.load(p.s, lane < n ? vidx[lane] : -1);
+        next = 32 + lane < n ? vidx[32 + lane] : -1;
+    }
     for (int i0 = 0; i0 < n; i0 += U * SW) {
+        if (TAB && (i0 & 31) == 0) {
+            __syncwarp();   // the visits before these have been read
+            tab_id[threadIdx.x] = entry.idx;
+            table_visit<R, NDIM, CX, 1>(g, entry, b0, b1, b2, 0, tab_co[threadIdx.x]);
+            entry.load(p.s, next);
+            next = i0 + 64 + lane < n ? vidx[i0 + 64 + lane] : -1;
+            __syncwarp();
+        }
         // past the last visit, and for padding, the value is zero by selection:
         // an infinity or NaN must not meet a zero coefficient
         int id[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int i = i0 + u * SW + slot;
-            id[u] = i < n ? vidx[i] : -1;
+            id[u] = TAB ? tab_id[own + (i & 31)] : i < n ? vidx[i] : -1;
         }
         C v[U], w[U];
         R co[U][NC];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (TAB) {
-                const int64_t e = max(id[u], 0);
-                id[u] = id[u] < 0 ? -1 : p.s.idx[e];
-                const short4 ls = p.s.ls[e];
-#pragma unroll
-                for (int k = 0; k < VB::NC; ++k) {
-                    const C c = visit_coef<R, NDIM, CX>(g, p.s, e, ls, b0, b1, b2, k);
-                    if (CX) {
-                        co[u][2 * k] = c.x;
-                        co[u][2 * k + (CX ? 1 : 0)] = c.y;
-                    } else {
-                        co[u][k] = c.x;
-                    }
-                }
-            } else {
-                load_run(p.vco + (st + min(i0 + u * SW + slot, n - 1)) * NC, co[u]);
-            }
+            if (TAB) load_run(tab_co[own + ((i0 + u * SW + slot) & 31)], co[u]);
+            else load_run(p.vco + (st + min(i0 + u * SW + slot, n - 1)) * NC, co[u]);
             const int m = max(id[u], 0);
             v[u] = cmake<R>((R)0, (R)0);
             if (GBN_INB(g.check, m < Mf, CHK_SAMPLE_READ)) v[u] = yb[m];
@@ -636,11 +739,14 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
 // leaves the last warps alone with the heavy tiles of the k-space centre.
 constexpr int STREAM_WARPS = 8;
 
-// Where a visit costs a warp more (double precision), the lighter items end a
-// launch on their one warp each; they go to a CTA too, a block to each warp.  No
-// block is cut, so no sum changes.  256 x 256, 8 coils: 658 us in place of 804.
-template <typename R, int LS>
-constexpr bool share_whole() { return sizeof(R) == 8 && LS >= 8; }
+// Where a visit costs a warp more (double precision, coefficients computed on
+// the way), the lighter items end a launch on their one warp each; they go to a
+// CTA too, a block to each warp.  No block is cut, so no sum changes.  (With
+// eight slots a stage's end decides which slot a visit goes to: not there.)
+// 256 x 256, 8 coils: double 658 us in place of 804; computed coefficients 80
+// in place of 96, complex 115 and 147, double 738 and 878.
+template <typename R, int LS, bool TAB>
+constexpr bool share_whole() { return (TAB || sizeof(R) == 8) && LS >= 8; }
 
 template <typename R, int NDIM, bool CX, int LS>
 struct StreamLayout {
@@ -662,16 +768,19 @@ struct StreamLayout {
 };
 
 // CTAs per SM: what the registers of a block's sums leave (two in double
-// precision: 1048 us at 192 x 192, 16 coils, against 1074 with one).
+// precision: 1048 us at 192 x 192, 16 coils, against 1074 with one), and those
+// of coefficients computed on the way (two: 60 x 72 x 45, complex, 3 coils 607
+// us against 849 where 163 registers left one).
 template <typename R, int NDIM, bool CX, int LS, bool TAB>
-__global__ void __launch_bounds__(32 * STREAM_WARPS, CX ? 1 : sizeof(R) == 8 || LS == 32 ? 2 : 3)
+__global__ void __launch_bounds__(32 * STREAM_WARPS,
+                                  TAB && sizeof(R) == 4 ? 2 : CX ? 1 : sizeof(R) == 8 || LS == 32 ? 2 : 3)
 spread_stream_kernel(const VisitParams<R> p) {
     typedef typename Cx<R>::T C;
     typedef VisitBlock<NDIM> VB;
     typedef StreamLayout<R, NDIM, CX, LS> SL;
     constexpr int NB = VB::NB, NC = SL::NC, B1 = NDIM > 1 ? VB::B1 : 1, SW = 32 / LS, RV = SL::RV;
     constexpr int KEEP = NB / SW, GROUP = SW > 4 ? SW : 4;
-    constexpr bool WHOLE = share_whole<R, LS>();
+    constexpr bool WHOLE = share_whole<R, LS, TAB>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geom<R>& g = p.g;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -729,22 +838,29 @@ spread_stream_kernel(const VisitParams<R> p) {
     const int off = lane * 16 % SL::VROW;
     const bool lane_ok = c0 * (int)sizeof(C) + off < row_bytes;
     const char* vsrc = reinterpret_cast<const char*>(p.vals + fo * p.row + c0) + (lane_ok ? off : 0);
-    const int* isrc = p.vidx + base + lo + lane;
+    const int visit = TAB ? lane % RV : lane;
+    const int* isrc = p.vidx + base + lo + visit;
     const char* csrc = reinterpret_cast<const char*>(p.vco + (base + lo) * NC) + lane * 16;
-    int to_load = hi - lo - lane;                        // this lane's visits not yet read
+    int to_load = hi - lo - visit;                       // this lane's visits not yet read
     int to_copy = (hi - lo) * NC * (int)sizeof(R) - lane * 16;   // coefficient bytes not yet copied
     int issued = 0;                                      // visits whose copies were issued
-    // index of the visit this lane reads for the stage to come (-1: none)
+    // index of the visit this lane reads for the stage to come (-1: none); with
+    // TAB its list entry, visit lane % RV of the stage, and what it holds
+    VisitEntry<R, NDIM> entry;
+    int origin = 0;   // lane b: block b's, for the visits' blocks
+    if (TAB) {
+        const short4 o = p.borg[min(lane, 7)];
+        origin = o.x | o.y << 8 | o.z << 16;
+    }
     auto load_id = [&]() {
-        const int id = lane < RV && to_load > 0 ? *isrc : -1;
+        const int id = (TAB || lane < RV) && to_load > 0 ? *isrc : -1;
         isrc += RV;
         to_load -= RV;
         return id;
     };
     auto issue = [&](unsigned char* sb, int id) {
         if (issued < hi - lo) {
-            const int e_mine = id;
-            if (TAB) id = id < 0 ? -1 : p.s.idx[id];
+            if (TAB) id = entry.idx;
             // no copy of a sample out of range, nor past the last coil: zeros
             if (!GBN_INB(g.check, id < Mf, CHK_SAMPLE_READ)) id = -1;
 #pragma unroll
@@ -754,26 +870,19 @@ spread_stream_kernel(const VisitParams<R> p) {
                 cp_async16_zfill(sb + lane * 16 + j * 512, vsrc + (ok ? (int64_t)m * row_bytes : 0), ok);
             }
             if (TAB) {
-                R* cb = reinterpret_cast<R*>(sb + SL::VBYTES);
-                for (int q = lane; q - lane < RV * VB::NC; q += 32) {
-                    const int vi = q / VB::NC, k1 = q - vi * VB::NC;
-                    const int e = __shfl_sync(0xffffffffu, e_mine, min(vi, RV - 1));
-                    if (vi < RV && e >= 0) {
-                        int blk = 0;   // the block this visit belongs to
-                        for (int b = 1; b < nblk; ++b) blk += (int)(st[b] - base) <= lo + issued + vi;
-                        int b0, b1, b2;
-                        block_origin_of(p, blk, b0, b1, b2);
-                        const C c = visit_coef<R, NDIM, CX>(g, p.s, e, p.s.ls[e], b0, b1, b2, k1);
-                        if (CX) {
-                            cb[2 * q] = c.x;
-                            cb[2 * q + 1] = c.y;
-                        } else {
-                            cb[q] = c.x;
-                        }
-                    } else if (vi < RV) {
-                        cb[(CX ? 2 : 1) * q] = (R)0;
-                        if (CX) cb[2 * q + 1] = (R)0;
-                    }
+                const int vi = lane % RV;
+                int blk = 0;   // the block the visit belongs to: the last that begins at or before it
+#pragma unroll
+                for (int h = 4; h > 0; h /= 2)
+                    if (__shfl_sync(0xffffffffu, rel, blk + h) <= lo + issued + vi) blk += h;
+                const int o = __shfl_sync(0xffffffffu, origin, blk);
+                const int b0 = o & 0xff, b1 = o >> 8 & 0xff, b2 = o >> 16;
+                R* co = reinterpret_cast<R*>(sb + SL::VBYTES) + vi * NC;
+                if (sizeof(R) == 8 && p.rec) {
+                    const R* rec = reinterpret_cast<const R*>(p.vals + (fo + max(entry.idx, 0)) * p.row) + p.rec;
+                    record_visit<R, NDIM, CX, 32 / RV>(g, entry.idx >= 0, entry.ls, rec, b0, b1, b2, lane / RV, co);
+                } else {
+                    table_visit<R, NDIM, CX, 32 / RV>(g, entry, b0, b1, b2, lane / RV, co);
                 }
             } else {
 #pragma unroll
@@ -793,8 +902,13 @@ spread_stream_kernel(const VisitParams<R> p) {
     int id = load_id();
     {
         const int nx = load_id();
+        if (TAB) entry.load(p.s, id);
         issue(ring, id);
         id = nx;
+        if (TAB) {
+            entry.load(p.s, id);
+            id = load_id();
+        }
     }
 
     C acc[NB], phase = cmake<R>((R)1, (R)0);
@@ -822,6 +936,7 @@ spread_stream_kernel(const VisitParams<R> p) {
                 unsigned char* done = const_cast<unsigned char*>(sb);
                 sb = sb == ring ? ring + SL::STAGE : ring;
                 issue(done, id);
+                if (TAB) entry.load(p.s, id);
                 id = nx;
                 left = RV;
                 vp = reinterpret_cast<const C*>(sb) + slot * LS + coil;
@@ -941,7 +1056,7 @@ cudaError_t stream_launch(const VisitParams<R>& p0, cudaStream_t s) {
     while (q < SPREAD_HEAVY_LEVELS - 1 && (SPREAD_SHARE_ENTRIES << q) < load) ++q;
     p.nshared = p.nheavy[q];
     p.nwhole = max(p.nshared, p.nheavy[0]);
-    const int shared = share_whole<R, LS>() ? p.nwhole : p.nshared;
+    const int shared = share_whole<R, LS, TAB>() ? p.nwhole : p.nshared;
     const int64_t ctas = shared + ((int64_t)p.nitems - shared + STREAM_WARPS - 1) / STREAM_WARPS;
     if (ctas > INT32_MAX || p.chunks > 65535) return cudaErrorInvalidValue;
     constexpr size_t smem = StreamLayout<R, NDIM, CX, LS>::SMEM;

@@ -56,3 +56,27 @@ def test_tiles_of_every_weight(gpu_lib, K, J, coils, rdt):
     P.interp_adjoint(torch.from_numpy(y).cuda(), g, coils)
     ref = O.interp_adjoint(y.T, h, (J,) * len(K), L, tm, K)
     assert rel_l2(g.cpu().numpy().T, ref) < (1e-5 if rdt == np.float32 else 1e-12)
+
+
+@pytest.mark.parametrize("coils", [1, 3, 4, 5, 8, 19, 32])
+@pytest.mark.parametrize("K,J,phasing", [((150, 141), 6, "real"), ((150, 141), 5, "complex"), ((1500,), 6, "real"),
+                                         ((1500,), 8, "complex"), ((37, 30, 26), 6, "real"), ((37, 30, 26), 4, "complex")])
+@pytest.mark.parametrize("rdt", [np.float32, np.float64])
+def test_computed_coefficients(gpu_lib, K, J, phasing, coils, rdt):
+    """Plans that keep no coefficients: the sums of those that do, bit for bit,
+    in several frames (one empty), and with the samples read in place."""
+    tm = _weights(np.asarray(K), coils)
+    M = len(tm)
+    fo = [0, M // 3, M // 3, M]
+    P, _ = plan_of(K, J, tm, rdt, phasing, coils, frame_offsets=fo)
+    T, _ = plan_of(K, J, tm, rdt, phasing, coils, table_only=True, frame_offsets=fo)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    y = torch.randn(coils * M, dtype=P.ctype, device="cuda", generator=g)
+    out = [torch.full((3 * coils, int(np.prod(K))), 7.0, dtype=P.ctype, device="cuda") for _ in range(2)]
+    P.interp_adjoint(y, out[0], coils)
+    T.interp_adjoint(y, out[1], coils)
+    assert torch.equal(out[0], out[1])
+    ys = [torch.empty_like(y) for _ in range(2)]
+    P.interp_forward(out[0], ys[0], coils)
+    T.interp_forward(out[0], ys[1], coils)
+    assert torch.equal(ys[0], ys[1])
