@@ -243,10 +243,15 @@ gather_kernel(const GatherParams<R> p) {
 
     // an equal share of the samples per warp (whole rounds of SW): items hold
     // some 70 to 100 samples at the workloads here, which in turns of 32 per
-    // warp occupied three of the eight warps
-    const int share = ((count + nwarps - 1) / nwarps + SW - 1) / SW * SW;
-    const int last = min(count, (warp + 1) * share);
-    for (int base = warp * share; base < last; base += 32) {
+    // warp occupied three of the eight warps.  Double precision coefficients
+    // computed on the way cost a warp as much for 10 samples as for 32: turns of
+    // 32 where that outweighs the sums (256 x 256: 4 coils 229 in place of 242 us,
+    // 8 coils 376 and 385; not with 32, 1822 and 1296, nor in a volume,
+    // 60 x 72 x 45 with 3: 2147 and 1635)
+    const bool turns = sizeof(R) == 8 && NDIM < 3 && !p.s.cr && SW > 2;
+    const int share = turns ? 32 : ((count + nwarps - 1) / nwarps + SW - 1) / SW * SW;
+    const int last = turns ? count : min(count, (warp + 1) * share);
+    for (int base = warp * share; base < last; base += turns ? nwarps * 32 : 32) {
         const int nb = min(32, last - base);
         R mcr[NDIM][JL], mci[NDIM][JL];
         int mbase = 0;  // shared-memory index of the window's first cell
