@@ -194,17 +194,20 @@ int gbn_interp_adjoint(gbn_plan* plan, const void* y, void* grid, int coils,
  * libgbnufft reserves it on each device it initialises.                     */
 #define GBN_NOALLOC_SCRATCH_BYTES (64u * 1024u * 1024u)
 
-/* Same result as gbn_interp_adjoint, for callers that must not allocate
+/* Same result as gbn_interp_adjoint (to rounding), for callers that must not allocate
  * device memory during a call: a process whose device memory is committed
  * up front to a fixed budget, or a pipeline that cannot let a cudaMalloc or
  * cudaFree (which may synchronise the whole device) happen between its
- * launches.  gbn_interp_adjoint grows a per-plan buffer for the partial sums
- * of tiles split across CTAs; this variant keeps them in one statically
- * sized array per device instead and never calls an allocator.
+ * launches.  gbn_interp_adjoint grows per-plan buffers for the partial sums
+ * of tiles split across CTAs and for the samples laid out coil-minor; this
+ * variant keeps both in one statically sized array per device instead and
+ * never calls an allocator.
  * No counterpart in the reference.
  *   - Limit: the partial sums of one call must fit GBN_NOALLOC_SCRATCH_BYTES
  *     (64 MiB); a larger request returns GBN_ERR_TOOLARGE before anything
  *     is launched.  Fewer coils per call, or gbn_interp_adjoint, fit it.
+ *     The coil-minor samples take the rest, a group of coils at a time if
+ *     need be, and are left out if not even one group fits.
  *   - Every call looks up the array's address on the current device (no
  *     allocation; it stays right after a device reset).  The first call on
  *     a device can also load the module holding the array: make that first

@@ -2,8 +2,9 @@
 //
 // The adjoint spread splits a crowded tile over several CTAs; each writes its
 // partial sums to scratch memory and reduce_kernel adds them up in part order.
-// gbn_interp_adjoint keeps that scratch in a per-plan buffer that it grows
-// with cudaMalloc.  Callers that cannot allocate during a call (a fixed
+// With several coils the samples are laid out coil-minor first.
+// gbn_interp_adjoint keeps both in per-plan buffers that it grows with
+// cudaMalloc.  Callers that cannot allocate during a call (a fixed
 // device-memory budget, or no room for the device-wide synchronisation a
 // cudaMalloc / cudaFree may cause) use this array instead: it is part of the
 // module image, so the CUDA driver reserves it when the module loads and no
@@ -21,7 +22,8 @@
 #include "gbn_internal.h"
 
 // Nothing in it has to start at zero: every part of a split tile writes all
-// cells that reduce_kernel later reads, before it reads them.
+// cells that reduce_kernel later reads, before it reads them, and the samples
+// are laid out before the spread reads them.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[GBN_NOALLOC_SCRATCH_BYTES];
 
 namespace gbn {

@@ -1159,16 +1159,28 @@ int run_gather(gbn_plan* P, const void* grid, void* y, int coils, Grid kind, cud
 }
 
 // The spread over visit lists into `grid`, then the reduction of split tiles.
-// vals: room for the coil-minor values (or nullptr: the samples are read in
-// place), scratch: the partial sums.
+// vals: room for the coil-minor values.  If it does not hold them all they are
+// laid out a group of coil chunks at a time; if not even one chunk (of as few
+// lanes as that path takes, inplace_lanes), the spread copies the samples as
+// they lie, as narrow lanes always do.  scratch: the partial sums.
 template <typename R>
 int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, void* vals, int64_t vals_elems,
                   void* scratch, int64_t scratch_elems, cudaStream_t s) {
     typedef typename Cx<R>::T C;
-    const Lanes ln = call_lanes<R>(P, coils);
+    Lanes ln = call_lanes<R>(P, coils);
     const bool phases = kind != Grid::abi;
-    // narrow lanes read the samples in place
-    if (ln.LS < (!P->dbl && P->geom.ndim == 3 ? 4 : 8)) vals = nullptr;
+    auto coils_held = [&]() {
+        int n = vals ? coils : 0;   // no samples: no values
+        while (n > 0 && P->M_total * value_row(P, n) > vals_elems) n = (n - 1) / ln.LS * ln.LS;
+        return n;
+    };
+    int group = coils_held();
+    if (group == 0 && ln.LS > inplace_lanes<R>()) {
+        ln = make_lanes(P->geom.ndim, inplace_lanes<R>());
+        group = coils_held();
+    }
+    if (group == 0 || ln.LS < (!P->dbl && P->geom.ndim == 3 ? 4 : 8)) vals = nullptr;
+    if (!vals) group = coils;
     const C* ph = phases && P->has_phase ? reinterpret_cast<const C*>(P->phnat.p) : nullptr;
     const int64_t* foff = reinterpret_cast<const int64_t*>(P->dfoff.p);
     VisitParams<R> p;
@@ -1190,7 +1202,7 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
     p.coils = coils;
     p.LS = ln.LS;
     p.chunks = (coils + ln.LS - 1) / ln.LS;
-    p.row = value_row(P, coils);
+    p.row = value_row(P, group);
     p.foff = foff;
     p.vals = static_cast<const C*>(vals);
     p.y = static_cast<const C*>(y);
@@ -1200,36 +1212,43 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
     p.tile_cells = (int64_t)P->Ts[0] * P->Ts[1] * P->Ts[2];
     p.scratch_elems = scratch_elems;
     p.apply_pb = phases && P->geom.phasing == GBN_PHASING_REAL;
-    if (vals) {
-        ValuesParams<R> v;
-        std::memset(&v, 0, sizeof(v));
-        v.y = p.y;
-        v.ph = ph;
-        v.out = static_cast<C*>(vals);
-        v.foff = foff;
-        v.F = P->F;
-        v.coils = coils;
-        v.row = p.row;
-        v.M = P->M_total;
-        v.check = p.g.check;
-        v.out_elems = vals_elems;
-        GBN_CUDA(launch_values<R>(v, s), "sample values launch");
-        if (call_records(P)) {
-            CoefParams<R> c;
-            std::memset(&c, 0, sizeof(c));
-            c.g = make_geom<R>(P, false);
-            c.s = make_list<R>(P, P->glist, P->glen, false);
-            c.foff = foff;
-            c.F = P->F;
-            c.out = static_cast<R*>(vals);
-            c.off = p.rec = 2 * values_extent(P, coils);
-            c.stride = 2 * p.row;
-            c.jsum = GatherRecord(P).jsum;
-            c.cx = P->cx ? 1 : 0;
-            GBN_CUDA(launch_coef<R>(c, s), "sample coefficients launch");
-        }
+    if (vals && call_records(P)) {
+        CoefParams<R> c;
+        std::memset(&c, 0, sizeof(c));
+        c.g = make_geom<R>(P, false);
+        c.s = make_list<R>(P, P->glist, P->glen, false);
+        c.foff = foff;
+        c.F = P->F;
+        c.out = static_cast<R*>(vals);
+        c.off = p.rec = 2 * values_extent(P, group);
+        c.stride = 2 * p.row;
+        c.jsum = GatherRecord(P).jsum;
+        c.cx = P->cx ? 1 : 0;
+        GBN_CUDA(launch_coef<R>(c, s), "sample coefficients launch");
     }
-    GBN_CUDA(launch_spread_visits<R>(p, s), "spread launch");
+    for (int first = 0; first < coils; first += group) {
+        const int n = std::min(group, coils - first);
+        p.chunk0 = first / ln.LS;
+        p.nchunk = (n + ln.LS - 1) / ln.LS;
+        if (vals) {
+            ValuesParams<R> v;
+            std::memset(&v, 0, sizeof(v));
+            v.y = p.y;
+            v.ph = ph;
+            v.out = static_cast<C*>(vals);
+            v.foff = foff;
+            v.F = P->F;
+            v.coils = coils;
+            v.first = first;
+            v.n = n;
+            v.row = p.row;
+            v.M = P->M_total;
+            v.check = p.g.check;
+            v.out_elems = vals_elems;
+            GBN_CUDA(launch_values<R>(v, s), "sample values launch");
+        }
+        GBN_CUDA(launch_spread_visits<R>(p, s), "spread launch");
+    }
     if (P->n_rtiles) {
         ReduceParams<R> q;
         std::memset(&q, 0, sizeof(q));
@@ -1256,8 +1275,9 @@ int run_spread(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, cud
                             (int64_t)(P->vals.bytes / sizeof(typename Cx<R>::T)), P->scratch.p, P->scratch_cap, s);
 }
 
-// The spread of run_spread with the split-tile partial sums kept in the
-// fixed no-alloc array instead of the plan's scratch buffer.  Nothing here
+// The spread of run_spread with the split-tile partial sums and the
+// coil-minor values kept in the fixed no-alloc array instead of the plan's
+// buffers.  Nothing here
 // allocates: the size check happens before any launch, and the array's
 // address comes from a lookup on the current device at every call.
 template <typename R>
@@ -1279,13 +1299,11 @@ int run_spread_noalloc(gbn_plan* P, const void* y, void* grid, int coils, cudaSt
                       (long long)need, coils, cap);
         return fail(GBN_ERR_TOOLARGE, msg);
     }
-    // the values take what the partial sums leave of the array, if they fit;
-    // else the samples are read in place
-    const int64_t used = (need + 255) & ~(int64_t)255;
-    const int64_t velems = P->M_total * value_row(P, coils);
-    void* vals = use_values(P, coils) && used + velems * (int64_t)sizeof(C) <= (int64_t)cap
-                     ? static_cast<char*>(scratch) + used : nullptr;
-    return launch_visits<R>(P, y, grid, coils, Grid::abi, vals, velems, scratch, need / (int64_t)sizeof(C), s);
+    // the values take what the partial sums leave of the array
+    const int64_t used = std::min((need + 255) & ~(int64_t)255, (int64_t)cap);
+    void* vals = use_values(P, coils) ? static_cast<char*>(scratch) + used : nullptr;
+    return launch_visits<R>(P, y, grid, coils, Grid::abi, vals, ((int64_t)cap - used) / (int64_t)sizeof(C), scratch,
+                            need / (int64_t)sizeof(C), s);
 }
 
 template <typename R>

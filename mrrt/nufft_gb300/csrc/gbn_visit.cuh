@@ -121,15 +121,13 @@ __device__ __forceinline__ void store_run(double* dst, const double (&v)[N]) {
     }
 }
 
-// 16-byte asynchronous copy of `bytes` (16 or 0) source bytes, zero-filled.
-__device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, bool valid) {
+// Asynchronous copy of BYTES (8 or 16) source bytes, of none and zeros if not
+// valid.
+template <int BYTES>
+__device__ __forceinline__ void cp_async_zfill(void* smem, const void* gmem, bool valid) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    const int n = valid ? 16 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(n) : "memory");
-}
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait_pending() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+    const int n = valid ? BYTES : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(BYTES), "r"(n) : "memory");
 }
 
 // Coefficient k of a visit to the block at (b0, b1, b2) of a window starting
@@ -409,7 +407,7 @@ __global__ void __launch_bounds__(256) values_kernel(const ValuesParams<R> p) {
     const int64_t m0 = (int64_t)blockIdx.x * VAL_SAMPLES;
     const int ns = (int)min((int64_t)VAL_SAMPLES, p.M - m0);
     const int c0 = blockIdx.y * VAL_COILS;
-    const int nc = min(VAL_COILS, p.coils - c0);
+    const int nc = min(VAL_COILS, p.n - c0);
     const int sl = threadIdx.x % VAL_SAMPLES, cg = threadIdx.x / VAL_SAMPLES;
     constexpr int NG = 256 / VAL_SAMPLES;
     if (sl < ns) {
@@ -421,7 +419,7 @@ __global__ void __launch_bounds__(256) values_kernel(const ValuesParams<R> p) {
             else hi = mid;
         }
         const int64_t fo = p.foff[f], Mf = p.foff[f + 1] - fo;
-        const C* src = p.y + fo * p.coils + (m - fo) + (int64_t)c0 * Mf;
+        const C* src = p.y + fo * p.coils + (m - fo) + (int64_t)(p.first + c0) * Mf;
         const C ph = p.ph ? p.ph[m] : cmake<R>((R)1, (R)0);
         for (int c = cg; c < nc; c += 4 * NG) {
             C v[4];
@@ -429,7 +427,7 @@ __global__ void __launch_bounds__(256) values_kernel(const ValuesParams<R> p) {
             for (int u = 0; u < 4; ++u) {
                 v[u] = cmake<R>((R)0, (R)0);
                 if (c + u * NG < nc &&
-                    GBN_INB(p.check, fo * p.coils + (m - fo) + (int64_t)(c0 + c + u * NG) * Mf < p.M * p.coils,
+                    GBN_INB(p.check, fo * p.coils + (m - fo) + (int64_t)(p.first + c0 + c + u * NG) * Mf < p.M * p.coils,
                             CHK_SAMPLE_READ))
                     v[u] = src[(int64_t)(c + u * NG) * Mf];
             }
@@ -626,8 +624,8 @@ struct BlockSink {
 
 // ---- values read in place: one (item, block) per warp ---------------------------
 //
-// Up to four coil lanes (two of a single-precision volume), and wider batches of calls
-// that may not allocate the coil-minor values.  U visits per slot are in flight at a time.
+// Up to four coil lanes (two of a single-precision volume).  U visits per slot
+// are in flight at a time.
 constexpr int VISIT_THREADS = 128;   // four (item, block) units per CTA
 
 template <typename R, int NDIM, bool CX, int LS, bool TAB>
@@ -649,7 +647,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
     const unsigned unit = blockIdx.x * (VISIT_THREADS / 32) + (threadIdx.x >> 5);
     if (unit >= (unsigned)(p.nitems * p.nblk)) return;   // whole warps only; no barrier below
     const int item = (int)(unit / (unsigned)p.nblk), blk = (int)(unit - (unsigned)item * p.nblk);
-    const int chunk = blockIdx.y;
+    const int chunk = p.chunk0 + blockIdx.y;
     const int4 it = p.items[item];
     const int2 part = p.parts[item];
     const int f = it.x;
@@ -728,7 +726,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
 // The visits of an item's blocks lie one after another, so a warp runs over
 // a whole range of them, blocks in turn, with the copies (values and
 // coefficients, cp.async into the warp's own ring, no barrier) running
-// STAGES - 1 stages ahead across block boundaries: with loads into registers
+// one stage ahead across block boundaries: with loads into registers
 // the same sums waited 58% of the time on the four visits a lane could hold.
 //
 // An item of many entries is shared by the eight warps of a CTA, each taking
@@ -737,6 +735,12 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
 // memory, in warp order); lighter items go one to a warp, eight to a CTA.
 // Sharing costs a barrier and, where blocks are cut, an exchange; not sharing
 // leaves the last warps alone with the heavy tiles of the k-space centre.
+//
+// Calls that may not allocate and whose values do not fit the fixed array have
+// them copied from [coil][sample] value by value (INPLACE): the same sums in the
+// same order.  Adjacent lanes copy a coil's values for adjacent visits, whose
+// samples tend to be adjacent, into rows of one value more, which keeps the lanes
+// on different banks.
 constexpr int STREAM_WARPS = 8;
 
 // Where a visit costs a warp more (double precision, coefficients computed on
@@ -748,7 +752,7 @@ constexpr int STREAM_WARPS = 8;
 template <typename R, int LS, bool TAB>
 constexpr bool share_whole() { return (TAB || sizeof(R) == 8) && LS >= 8; }
 
-template <typename R, int NDIM, bool CX, int LS>
+template <typename R, int NDIM, bool CX, int LS, bool INPLACE>
 struct StreamLayout {
     typedef typename Cx<R>::T C;
     static constexpr int NC = VisitBlock<NDIM>::NC * (CX ? 2 : 1);
@@ -758,26 +762,28 @@ struct StreamLayout {
     static constexpr int VBYTES = LS == 32 && sizeof(C) == 8 ? 4096 : VROW < 64 ? 32 * VROW : 2048;
     static constexpr int RV = VBYTES / VROW;                    // visits per stage
     static constexpr int CBYTES = RV * NC * (int)sizeof(R);     // coefficients of a stage
-    static constexpr int STAGE = VBYTES + CBYTES;
+    static constexpr int COFF = VBYTES + (INPLACE ? RV * (int)sizeof(C) : 0);   // where they begin
+    static constexpr int STAGE = COFF + CBYTES;
+    static constexpr int LSP = LS + (INPLACE ? 1 : 0);          // values from a visit's to the next's
     static constexpr int HEAD = 16 * LS * (int)sizeof(C);       // one combined block
     static constexpr int SINK = 32;                             // the item's BlockSink
     static constexpr int WARP = 2 * STAGE + HEAD + SINK;
     static constexpr int SMEM = STREAM_WARPS * WARP;
     static_assert(sizeof(BlockSink<R, 2, LS>) <= SINK, "sink");
-    static_assert(RV % 4 == 0 && RV <= 32 && VROW <= 512 && STAGE % 16 == 0, "stage layout");
+    static_assert(RV % 4 == 0 && RV <= 32 && VROW <= 512 && COFF % 16 == 0 && STAGE % 16 == 0, "stage layout");
 };
 
 // CTAs per SM: what the registers of a block's sums leave (two in double
 // precision: 1048 us at 192 x 192, 16 coils, against 1074 with one), and those
 // of coefficients computed on the way (two: 60 x 72 x 45, complex, 3 coils 607
 // us against 849 where 163 registers left one).
-template <typename R, int NDIM, bool CX, int LS, bool TAB>
+template <typename R, int NDIM, bool CX, int LS, bool TAB, bool INPLACE>
 __global__ void __launch_bounds__(32 * STREAM_WARPS,
                                   TAB && sizeof(R) == 4 ? 2 : CX ? 1 : sizeof(R) == 8 || LS == 32 ? 2 : 3)
 spread_stream_kernel(const VisitParams<R> p) {
     typedef typename Cx<R>::T C;
     typedef VisitBlock<NDIM> VB;
-    typedef StreamLayout<R, NDIM, CX, LS> SL;
+    typedef StreamLayout<R, NDIM, CX, LS, INPLACE> SL;
     constexpr int NB = VB::NB, NC = SL::NC, B1 = NDIM > 1 ? VB::B1 : 1, SW = 32 / LS, RV = SL::RV;
     constexpr int KEEP = NB / SW, GROUP = SW > 4 ? SW : 4;
     constexpr bool WHOLE = share_whole<R, LS, TAB>();
@@ -788,7 +794,7 @@ spread_stream_kernel(const VisitParams<R> p) {
     const bool shared_item = (int)blockIdx.x < nshared;
     const int item = shared_item ? (int)blockIdx.x : nshared + ((int)blockIdx.x - nshared) * STREAM_WARPS + warp;
     if (item >= p.nitems) return;   // only in a CTA of unshared items: no barrier there
-    const int chunk = blockIdx.y;
+    const int chunk = p.chunk0 + blockIdx.y;
     const int4 it = p.items[item];
     const int part = p.parts[item].x;
     const int f = it.x;
@@ -836,8 +842,10 @@ spread_stream_kernel(const VisitParams<R> p) {
     // A lane copies 16 bytes at a fixed place of every (512 / VROW)-th visit.
     const int row_bytes = p.row * (int)sizeof(C);
     const int off = lane * 16 % SL::VROW;
-    const bool lane_ok = c0 * (int)sizeof(C) + off < row_bytes;
-    const char* vsrc = reinterpret_cast<const char*>(p.vals + fo * p.row + c0) + (lane_ok ? off : 0);
+    const int v0 = blockIdx.y * LS;   // the chunk's place in a row of values
+    const bool lane_ok = v0 * (int)sizeof(C) + off < row_bytes;
+    const char* vsrc = reinterpret_cast<const char*>(p.vals + fo * p.row + v0) + (lane_ok ? off : 0);
+    const C* ysrc = p.y + fo * p.coils + (int64_t)c0 * Mf;
     const int visit = TAB ? lane % RV : lane;
     const int* isrc = p.vidx + base + lo + visit;
     const char* csrc = reinterpret_cast<const char*>(p.vco + (base + lo) * NC) + lane * 16;
@@ -863,11 +871,21 @@ spread_stream_kernel(const VisitParams<R> p) {
             if (TAB) id = entry.idx;
             // no copy of a sample out of range, nor past the last coil: zeros
             if (!GBN_INB(g.check, id < Mf, CHK_SAMPLE_READ)) id = -1;
+            if (INPLACE) {
 #pragma unroll
-            for (int j = 0; j < SL::VBYTES / 512; ++j) {
-                const int m = __shfl_sync(0xffffffffu, id, lane * 16 / SL::VROW + j * (512 / SL::VROW));
-                const bool ok = m >= 0 && lane_ok;
-                cp_async16_zfill(sb + lane * 16 + j * 512, vsrc + (ok ? (int64_t)m * row_bytes : 0), ok);
+                for (int j = 0; j < LS * RV / 32; ++j) {
+                    const int c = j * (32 / RV) + lane / RV, m = __shfl_sync(0xffffffffu, id, lane % RV);
+                    const bool ok = m >= 0 && c0 + c < p.coils;
+                    cp_async_zfill<sizeof(C)>(sb + (lane % RV * SL::LSP + c) * sizeof(C),
+                                              ysrc + (ok ? (int64_t)c * Mf + m : 0), ok);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < SL::VBYTES / 512; ++j) {
+                    const int m = __shfl_sync(0xffffffffu, id, lane * 16 / SL::VROW + j * (512 / SL::VROW));
+                    const bool ok = m >= 0 && lane_ok;
+                    cp_async_zfill<16>(sb + lane * 16 + j * 512, vsrc + (ok ? (int64_t)m * row_bytes : 0), ok);
+                }
             }
             if (TAB) {
                 const int vi = lane % RV;
@@ -877,8 +895,8 @@ spread_stream_kernel(const VisitParams<R> p) {
                     if (__shfl_sync(0xffffffffu, rel, blk + h) <= lo + issued + vi) blk += h;
                 const int o = __shfl_sync(0xffffffffu, origin, blk);
                 const int b0 = o & 0xff, b1 = o >> 8 & 0xff, b2 = o >> 16;
-                R* co = reinterpret_cast<R*>(sb + SL::VBYTES) + vi * NC;
-                if (sizeof(R) == 8 && p.rec) {
+                R* co = reinterpret_cast<R*>(sb + SL::COFF) + vi * NC;
+                if (sizeof(R) == 8 && !INPLACE && p.rec) {
                     const R* rec = reinterpret_cast<const R*>(p.vals + (fo + max(entry.idx, 0)) * p.row) + p.rec;
                     record_visit<R, NDIM, CX, 32 / RV>(g, entry.idx >= 0, entry.ls, rec, b0, b1, b2, lane / RV, co);
                 } else {
@@ -889,8 +907,8 @@ spread_stream_kernel(const VisitParams<R> p) {
                 for (int q = 0; q < SL::CBYTES; q += 512) {
                     if (SL::CBYTES - q < 512 && lane * 16 >= SL::CBYTES - q) break;
                     const bool ok = q < to_copy;
-                    cp_async16_zfill(sb + SL::VBYTES + lane * 16 + q,
-                                     ok ? csrc + q : reinterpret_cast<const char*>(p.vco), ok);
+                    cp_async_zfill<16>(sb + SL::COFF + lane * 16 + q,
+                                       ok ? csrc + q : reinterpret_cast<const char*>(p.vco), ok);
                 }
                 csrc += SL::CBYTES;
                 to_copy -= SL::CBYTES;
@@ -939,8 +957,8 @@ spread_stream_kernel(const VisitParams<R> p) {
                 if (TAB) entry.load(p.s, id);
                 id = nx;
                 left = RV;
-                vp = reinterpret_cast<const C*>(sb) + slot * LS + coil;
-                cp = reinterpret_cast<const R*>(sb + SL::VBYTES) + slot * NC;
+                vp = reinterpret_cast<const C*>(sb) + slot * SL::LSP + coil;
+                cp = reinterpret_cast<const R*>(sb + SL::COFF) + slot * NC;
             }
             const int n = min(end - pos, left);
             pos += n;
@@ -958,7 +976,7 @@ spread_stream_kernel(const VisitParams<R> p) {
 #pragma unroll
                 for (int u = 0; u < GROUP / SW; ++u) {
                     if (GROUP > 4 && slot >= q) break;   // four visits left for eight slots
-                    const C v = vp[u * 32];
+                    const C v = vp[u * SW * SL::LSP];
                     R co[NC];
                     load_run(cp + u * SW * NC, co);
 #pragma unroll
@@ -967,7 +985,7 @@ spread_stream_kernel(const VisitParams<R> p) {
                             add_row<R, NDIM, CX>(acc, v, co, k1);
                 }
                 const int step = GROUP > 4 ? min(q, GROUP) : GROUP;
-                vp += step * LS;
+                vp += step * SL::LSP;
                 cp += step * NC;
             }
         }
@@ -1037,17 +1055,18 @@ cudaError_t launch_visit_fill(const VisitBuildParams<R>& p, cudaStream_t s) {
 
 template <typename R>
 cudaError_t launch_values(const ValuesParams<R>& p, cudaStream_t s) {
-    if (p.M == 0 || p.coils == 0) return cudaSuccess;
+    if (p.M == 0 || p.n == 0) return cudaSuccess;
     const int64_t bx = (p.M + VAL_SAMPLES - 1) / VAL_SAMPLES;
-    const int64_t by = (p.coils + VAL_COILS - 1) / VAL_COILS;
+    const int64_t by = (p.n + VAL_COILS - 1) / VAL_COILS;
     if (bx > INT32_MAX || by > 65535) return cudaErrorInvalidValue;
     values_kernel<R><<<dim3((unsigned)bx, (unsigned)by), 256, 0, s>>>(p);
     return cudaGetLastError();
 }
 
-template <typename R, int NDIM, bool CX, int LS, bool TAB>
+template <typename R, int NDIM, bool CX, int LS, bool TAB, bool INPLACE>
 cudaError_t stream_launch(const VisitParams<R>& p0, cudaStream_t s) {
     VisitParams<R> p = p0;
+    if (INPLACE && p.ph && p.s.len > 0) return cudaErrorInvalidValue;   // the values hold the phase
     // An item goes to one warp up to 32 entries per slot (a longer one would
     // outlast the rest of a small launch), more where each of the device's
     // warps has many times that to do anyway.
@@ -1058,12 +1077,12 @@ cudaError_t stream_launch(const VisitParams<R>& p0, cudaStream_t s) {
     p.nwhole = max(p.nshared, p.nheavy[0]);
     const int shared = share_whole<R, LS, TAB>() ? p.nwhole : p.nshared;
     const int64_t ctas = shared + ((int64_t)p.nitems - shared + STREAM_WARPS - 1) / STREAM_WARPS;
-    if (ctas > INT32_MAX || p.chunks > 65535) return cudaErrorInvalidValue;
-    constexpr size_t smem = StreamLayout<R, NDIM, CX, LS>::SMEM;
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(spread_stream_kernel<R, NDIM, CX, LS, TAB>), smem);
+    if (ctas > INT32_MAX || p.nchunk > 65535) return cudaErrorInvalidValue;
+    constexpr size_t smem = StreamLayout<R, NDIM, CX, LS, INPLACE>::SMEM;
+    const auto kernel = spread_stream_kernel<R, NDIM, CX, LS, TAB, INPLACE>;
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
-    spread_stream_kernel<R, NDIM, CX, LS, TAB>
-        <<<dim3((unsigned)ctas, (unsigned)p.chunks), 32 * STREAM_WARPS, smem, s>>>(p);
+    kernel<<<dim3((unsigned)ctas, (unsigned)p.nchunk), 32 * STREAM_WARPS, smem, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -1071,9 +1090,16 @@ template <typename R, int NDIM, bool CX, int LS, bool TAB>
 cudaError_t unit_launch(const VisitParams<R>& p, cudaStream_t s) {
     const int64_t units = (int64_t)p.nitems * p.nblk;
     const int64_t ctas = (units + VISIT_THREADS / 32 - 1) / (VISIT_THREADS / 32);
-    if (units > INT32_MAX || p.chunks > 65535) return cudaErrorInvalidValue;
-    spread_unit_kernel<R, NDIM, CX, LS, TAB><<<dim3((unsigned)ctas, (unsigned)p.chunks), VISIT_THREADS, 0, s>>>(p);
+    if (units > INT32_MAX || p.nchunk > 65535) return cudaErrorInvalidValue;
+    spread_unit_kernel<R, NDIM, CX, LS, TAB><<<dim3((unsigned)ctas, (unsigned)p.nchunk), VISIT_THREADS, 0, s>>>(p);
     return cudaGetLastError();
+}
+
+template <typename R, int NDIM, bool CX, int LS, bool TAB>
+cudaError_t stream_values(const VisitParams<R>& p, cudaStream_t s) {
+    if (p.vals) return stream_launch<R, NDIM, CX, LS, TAB, false>(p, s);
+    if constexpr (LS <= inplace_lanes<R>()) return stream_launch<R, NDIM, CX, LS, TAB, true>(p, s);
+    return cudaErrorInvalidValue;
 }
 
 template <typename R, int NDIM, bool CX, bool TAB>
@@ -1082,12 +1108,12 @@ cudaError_t visit_lanes(const VisitParams<R>& p, cudaStream_t s) {
         case 1: return unit_launch<R, NDIM, CX, 1, TAB>(p, s);
         case 2: return unit_launch<R, NDIM, CX, 2, TAB>(p, s);
         case 4:
-            if constexpr (sizeof(R) == 4 && NDIM == 3)
-                if (p.vals) return stream_launch<R, NDIM, CX, 4, TAB>(p, s);
-            return unit_launch<R, NDIM, CX, 4, TAB>(p, s);
-        case 8: return p.vals ? stream_launch<R, NDIM, CX, 8, TAB>(p, s) : unit_launch<R, NDIM, CX, 8, TAB>(p, s);
-        case 16: return p.vals ? stream_launch<R, NDIM, CX, 16, TAB>(p, s) : unit_launch<R, NDIM, CX, 16, TAB>(p, s);
-        case 32: return p.vals ? stream_launch<R, NDIM, CX, 32, TAB>(p, s) : unit_launch<R, NDIM, CX, 32, TAB>(p, s);
+            if constexpr (sizeof(R) == 4 && NDIM == 3) return stream_values<R, NDIM, CX, 4, TAB>(p, s);
+            else return unit_launch<R, NDIM, CX, 4, TAB>(p, s);
+        case 8: return stream_values<R, NDIM, CX, 8, TAB>(p, s);
+        // volumes have eight lanes at most
+        case 16: if constexpr (NDIM < 3) return stream_values<R, NDIM, CX, 16, TAB>(p, s); break;
+        case 32: if constexpr (NDIM < 3) return stream_values<R, NDIM, CX, 32, TAB>(p, s); break;
     }
     return cudaErrorInvalidValue;
 }
