@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(256) coef_kernel(const CoefParams<R> p) {
             else hi = mid;
         }
     }
+    if ((k == 0 || !p.place) && !GBN_INB(g.check, p.foff[f] + p.s.idx[e] < p.s.len, CHK_LIST)) return;
     if (k == 0 && p.place) p.place[p.foff[f] + p.s.idx[e]] = (int)e;
     if (p.wr[0]) {
         const int64_t w = (p.foff[f] + p.s.idx[e]) * g.J[d] + j;

@@ -133,6 +133,7 @@ struct VisitBuildParams {
     const int64_t* foff;
     const R* rec;                   // the gather's coefficients, at rec + place[sample] * stride
     const int* place;
+    int64_t samples, nvisits;       // extents: of place and the records, of vidx and vco
     int stride, jsum;
     int cx;
     int* count;                     // [nitems * nblk], multiples of four

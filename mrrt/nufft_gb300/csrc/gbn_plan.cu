@@ -1665,6 +1665,8 @@ int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
     else
         GBN_CUDA(P->vco.alloc(0), "coefficient release");
     b.start = start;
+    b.nvisits = total;
+    b.samples = P->glen;
     b.vidx = static_cast<int*>(P->vidx.p);
     b.vco = static_cast<R*>(P->vco.p);
     GBN_CUDA(launch_visit_fill<R>(b, stream), "visit launch");

@@ -156,12 +156,12 @@ struct VisitEntry {
     short4 ls;
     R t[3];
     int idx;   // sample index, -1: padding
-    __device__ __forceinline__ void load(const SampleList<R>& s, int e) {
+    __device__ __forceinline__ void load(const SampleList<R>& s, int e, unsigned* check) {
         idx = -1;
         ls = make_short4(0, 0, 0, 0);
 #pragma unroll
         for (int d = 0; d < NDIM; ++d) t[d] = (R)0;
-        if (e < 0) return;
+        if (e < 0 || !GBN_INB(check, e < s.len, CHK_LIST)) return;
         idx = s.idx[e];
         ls = s.ls[e];
 #pragma unroll
@@ -282,10 +282,11 @@ template <typename R, int NDIM>
 __global__ void __launch_bounds__(256) visit_count_kernel(const VisitBuildParams<R> p) {
     const int item = blockIdx.x, blk = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int4 it = p.items[item];
+    const bool ok = GBN_INB(p.g.check, it.z >= 0 && it.w >= 0 && it.z + (int64_t)it.w <= p.s.len, CHK_LIST);
     int b0, b1, b2;
     block_origin<NDIM>(p.g, blk, b0, b1, b2);
     int n = 0;
-    const int count = block_in_grid<NDIM>(p.g, it.y, b0, b1, b2) ? it.w : 0;
+    const int count = ok && block_in_grid<NDIM>(p.g, it.y, b0, b1, b2) ? it.w : 0;
     for (int base = 0; base < count; base += 32 * VISIT_UNROLL) {
         unsigned mask[VISIT_UNROLL];
         block_hits<R, NDIM>(p, it.z, count, base, lane, b0, b1, b2, mask);
@@ -300,10 +301,13 @@ template <typename R, int NDIM>
 __global__ void __launch_bounds__(256) visit_fill_kernel(const VisitBuildParams<R> p) {
     const int item = blockIdx.x, blk = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int4 it = p.items[item];
+    if (!GBN_INB(p.g.check, it.z >= 0 && it.w >= 0 && it.z + (int64_t)it.w <= p.s.len, CHK_LIST)) return;
     int b0, b1, b2;
     block_origin<NDIM>(p.g, blk, b0, b1, b2);
     int64_t at = p.start[(int64_t)item * p.nblk + blk];
-    const int64_t end = p.start[(int64_t)item * p.nblk + blk + 1];
+    // device binning sizes the lists by a bound on the sum of the counts
+    const int64_t stop = p.start[(int64_t)item * p.nblk + blk + 1], end = min(stop, (int64_t)p.nvisits);
+    if (!GBN_INB(p.g.check, stop <= p.nvisits, CHK_LIST)) return;
     const int count = block_in_grid<NDIM>(p.g, it.y, b0, b1, b2) ? it.w : 0;
     for (int base = 0; base < count; base += 32 * VISIT_UNROLL) {
         unsigned mask[VISIT_UNROLL];
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(256) visit_coef_kernel(const VisitBuildParams<
     const int item = blockIdx.x;
     const long long* st = p.start + (int64_t)item * p.nblk;
     const int64_t first = st[0];
-    const int n = (int)(st[p.nblk] - first);
+    const int n = (int)(min(st[p.nblk], (long long)p.nvisits) - first);
     if ((int)blockIdx.y * PER * VISIT_UNROLL >= n) return;   // the whole CTA
     // origins and first visits of the item's blocks
     __shared__ int4 block[8];
@@ -370,11 +374,15 @@ __global__ void __launch_bounds__(256) visit_coef_kernel(const VisitBuildParams<
         }
 #pragma unroll
         for (int u = 0; u < VISIT_UNROLL; ++u) {
+            if (!GBN_INB(g.check, e[u] < p.s.len, CHK_LIST)) e[u] = -1;
             idx[u] = e[u] < 0 ? -1 : p.s.idx[e[u]];
+            if (!GBN_INB(g.check, fo + idx[u] < p.samples, CHK_LIST)) e[u] = idx[u] = -1;
             c[u] = cmake<R>(!CX && k >= VB::B0 ? (R)-0.0 : (R)0, (R)0);
             if (e[u] >= 0) {
                 const int4 o = block[blk[u]];
-                const R* r = p.rec + (int64_t)p.place[fo + idx[u]] * p.stride;
+                int at = p.place[fo + idx[u]];
+                if (!GBN_INB(g.check, at >= 0 && at < p.samples, CHK_LIST)) at = 0;
+                const R* r = p.rec + (int64_t)at * p.stride;
                 c[u] = clipped_coef<R, NDIM, CX>(g, p.s.ls[e[u]], o.x, o.y, o.z, k, [&](int d, int j) {
                     j += (d > 0 ? g.J[0] : 0) + (d > 1 ? g.J[1] : 0);
                     return cmake<R>(r[j], CX ? -r[p.jsum + j] : (R)0);
@@ -673,7 +681,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
     VisitEntry<R, NDIM> entry;   // of the 32 visits to come, and the entries after them
     int next = -1;
     if (TAB) {
-        entry.load(p.s, lane < n ? vidx[lane] : -1);
+        entry.load(p.s, lane < n ? vidx[lane] : -1, g.check);
         next = 32 + lane < n ? vidx[32 + lane] : -1;
     }
     for (int i0 = 0; i0 < n; i0 += U * SW) {
@@ -681,7 +689,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
             __syncwarp();   // the visits before these have been read
             tab_id[threadIdx.x] = entry.idx;
             table_visit<R, NDIM, CX, 1>(g, entry, b0, b1, b2, 0, tab_co[threadIdx.x]);
-            entry.load(p.s, next);
+            entry.load(p.s, next, g.check);
             next = i0 + 64 + lane < n ? vidx[i0 + 64 + lane] : -1;
             __syncwarp();
         }
@@ -896,6 +904,7 @@ spread_stream_kernel(const VisitParams<R> p) {
                 const int o = __shfl_sync(0xffffffffu, origin, blk);
                 const int b0 = o & 0xff, b1 = o >> 8 & 0xff, b2 = o >> 16;
                 R* co = reinterpret_cast<R*>(sb + SL::COFF) + vi * NC;
+                if (!GBN_INB(g.check, entry.idx < Mf, CHK_SAMPLE_READ)) entry.idx = -1;
                 if (sizeof(R) == 8 && !INPLACE && p.rec) {
                     const R* rec = reinterpret_cast<const R*>(p.vals + (fo + max(entry.idx, 0)) * p.row) + p.rec;
                     record_visit<R, NDIM, CX, 32 / RV>(g, entry.idx >= 0, entry.ls, rec, b0, b1, b2, lane / RV, co);
@@ -920,11 +929,11 @@ spread_stream_kernel(const VisitParams<R> p) {
     int id = load_id();
     {
         const int nx = load_id();
-        if (TAB) entry.load(p.s, id);
+        if (TAB) entry.load(p.s, id, g.check);
         issue(ring, id);
         id = nx;
         if (TAB) {
-            entry.load(p.s, id);
+            entry.load(p.s, id, g.check);
             id = load_id();
         }
     }
@@ -954,7 +963,7 @@ spread_stream_kernel(const VisitParams<R> p) {
                 unsigned char* done = const_cast<unsigned char*>(sb);
                 sb = sb == ring ? ring + SL::STAGE : ring;
                 issue(done, id);
-                if (TAB) entry.load(p.s, id);
+                if (TAB) entry.load(p.s, id, g.check);
                 id = nx;
                 left = RV;
                 vp = reinterpret_cast<const C*>(sb) + slot * SL::LSP + coil;
