@@ -53,7 +53,9 @@ extern "C" {
  * coefficients once (per sample for the gather, per visit of a register
  * block for the spread) and the kernels read them; TABLE_ONLY keeps no such
  * buffers and interpolates the tables inside the kernels instead (same
- * results bit for bit, less device memory).                               */
+ * results bit for bit, less device memory, a slower adjoint).  The spread of
+ * a plan whose visit coefficients do not fit the free device memory beside
+ * the buffers of a max_coils transform does so by itself.                 */
 #define GBN_FLAG_TABLE_ONLY 1
 /* By default single-precision 2-D and 3-D plans run the FFT on the library's
  * own pruned passes (which read only the rows that hold data and write only
@@ -296,7 +298,8 @@ int gbn_debug_check_status(gbn_plan* plan, unsigned* out);
  * for the allocation-failure paths.  After this call, `after` more device
  * allocations made by the library succeed and the next one fails as if
  * cudaMalloc had reported cudaErrorMemoryAllocation (nothing is requested
- * from the device for it); the call that needed it returns GBN_ERR_NOMEM.
+ * from the device for it); the call that needed it returns GBN_ERR_NOMEM, or
+ * does without where it can (visit coefficients).
  * A negative value turns the injection off.  Process-wide.                 */
 int gbn_debug_fail_alloc(long long after);
 

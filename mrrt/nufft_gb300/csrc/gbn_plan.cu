@@ -161,6 +161,7 @@ struct DevBuf {
         if (injected_alloc_failure()) return cudaErrorMemoryAllocation;
         cudaError_t e = cudaMalloc(&p, b);
         if (e == cudaSuccess) bytes = b;
+        else cudaGetLastError();   // reported here: not to a later launch
         return e;
     }
 };
@@ -227,7 +228,7 @@ struct gbn_plan {
     DevBuf vstart, vidx, vco, vwork, place, phnat, vals;
     int64_t nvisits = 0;  // extent of vidx and vco in visits
     int n_heavy[SPREAD_HEAVY_LEVELS] = {0};   // leading spread items of more entries than 32 << level
-    bool coefs = false;   // gcoef and vco hold the current points' coefficients
+    bool coefs = false;   // gcoef holds the current points' coefficients, and so does vco if allocated
     // A re-planning that fails part way (an allocation) leaves lists that no kernel
     // may read: `listed` says that the sample lists and work items are those of one
     // set of points, `ready` that the visits and coefficients are theirs too.
@@ -748,12 +749,12 @@ int build_lists(gbn_plan* P, const R* tm, const R* phase) {
 // sectors either way (192 x 192, 4 coils: 521 against 506).
 bool use_values(const gbn_plan* P, int coils) { return coils >= (!P->dbl && P->geom.ndim == 3 ? 3 : 5); }
 
-// A double precision plan that stores no coefficients computes each sample's
+// A double precision plan that stores no visit coefficients computes each sample's
 // once a call, beside its values, and the spread copies them per visit: 12
 // interpolations a sample in place of 40 at 256 x 256, of which an SM does few
 // (8 coils: 736 us, against 1079 computed per visit).  In single precision the
 // copies' loads cost more than the interpolation (112 against 96).
-bool call_records(const gbn_plan* P) { return P->dbl && !P->coefs; }
+bool call_records(const gbn_plan* P) { return P->dbl && !P->vco.p; }
 
 // A sample's row of the coil-minor buffer, in complex values rounded up to 16
 // bytes: its values, then its coefficients (call_records).
@@ -1192,7 +1193,7 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
     p.s = make_list<R>(P, P->slist, P->slen, true);
     p.start = static_cast<const long long*>(P->vstart.p);
     p.vidx = static_cast<const int*>(P->vidx.p);
-    p.vco = P->coefs ? static_cast<const R*>(P->vco.p) : nullptr;
+    p.vco = static_cast<const R*>(P->vco.p);
     for (int q = 0; q < SPREAD_HEAVY_LEVELS; ++q) p.nheavy[q] = P->n_heavy[q];
     p.nvisits = P->nvisits;
     p.items = reinterpret_cast<const int4*>(P->sitems.p);
@@ -1617,10 +1618,24 @@ void weight_pointers(const gbn_plan* P, const R* (&wr)[3], const R* (&wi)[3]) {
         }
 }
 
+// Bytes of the buffers that a transform of max_coils coils still has to allocate.
+size_t transform_bytes(const gbn_plan* P) {
+    const size_t csz = (size_t)2 * P->rsize;
+    const int coils = P->geom.max_coils;
+    const size_t grid = (size_t)P->F * coils * P->Kprod * csz;
+    const size_t need = grid + (P->own ? grid / P->geom.Kd[0] * P->geom.Nd[0] : 2 * grid) +
+                        (use_values(P, coils) ? (size_t)P->M_total * value_row(P, coils) * csz : 0);
+    const size_t held = P->grid.bytes + P->half.bytes + P->pad.bytes + P->mid.bytes + P->vals.bytes;
+    return need > held ? need - held : 0;
+}
+
 // Visit lists of the spread (gbn_visit.cuh), with their coefficients unless
-// the geometry asks for table interpolation inside the kernels.  `total`: the
-// visits before padding where the caller knows them (device binning), else -1
-// and the padded sum is read back.
+// the geometry asks for table interpolation inside the kernels.  The
+// coefficients are the most of a plan (32 bytes a visit, some 33 visits a sample
+// in single-precision volumes): where they do not fit beside the buffers of a
+// transform, and there are no weights that they alone hold, the spread
+// interpolates too.  `total`: the visits before padding where the caller knows
+// them (device binning), else -1 and the padded sum is read back.
 template <typename R>
 int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
     VisitBuildParams<R> b;
@@ -1660,10 +1675,17 @@ int build_visits(gbn_plan* P, bool coefs, cudaStream_t stream, int64_t total) {
     const int NC = P->geom.ndim == 1 ? 16 : 8;
     P->nvisits = 0;
     GBN_CUDA(ensure(P->vidx, (size_t)total * sizeof(int)), "visit allocation");
-    if (coefs)
-        GBN_CUDA(ensure(P->vco, (size_t)total * NC * (P->cx ? 2 : 1) * sizeof(R)), "visit allocation");
-    else
+    const size_t bytes = std::max<size_t>((size_t)total * NC * (P->cx ? 2 : 1) * sizeof(R), 256);
+    if (!coefs) {
         GBN_CUDA(P->vco.alloc(0), "coefficient release");
+    } else if (P->vco.bytes < bytes) {
+        GBN_CUDA(P->vco.alloc(0), "coefficient release");
+        size_t room = 0, all = 0;
+        GBN_CUDA(cudaMemGetInfo(&room, &all), "free memory");
+        const bool fits = room >= bytes && room - bytes >= transform_bytes(P);
+        const cudaError_t e = fits || P->weights.p ? P->vco.alloc(bytes) : cudaErrorMemoryAllocation;
+        if (e != cudaSuccess && (e != cudaErrorMemoryAllocation || P->weights.p)) return cuda_fail(e, "visit allocation");
+    }
     b.start = start;
     b.nvisits = total;
     b.samples = P->glen;

@@ -179,3 +179,43 @@ def test_operator_after_a_failed_move(gpu_lib, on_device):
     finally:
         gpu_lib.gbn_debug_fail_alloc(-1)
     assert seen > 0
+
+
+@pytest.mark.parametrize("rdt", [np.float32, np.float64])
+def test_visit_coefficients_that_do_not_fit(gpu_lib, rdt):
+    """A plan whose visit coefficients cannot be allocated works without them,
+    to the same bits, and takes them up with weights, or when moved, with room."""
+    from mrrt.nufft_gb300._kernels import kernel_table
+    from mrrt.nufft_gb300._plan import GpuPlan
+
+    h = [kernel_table(N[d], J[d], K[d], 512, "real", rdt) for d in range(2)]
+    _, many, ph = _points()
+
+    def plan():
+        return GpuPlan(N, K, J, 512, rdt, h, None, np.ones(N[0] * N[1], rdt), many, ph, max_coils=COILS)
+
+    x, y = (t.to(torch.complex64 if rdt == np.float32 else torch.complex128) for t in _data())
+    P = plan()
+    want, held = _results(P, x, y), P.stats()["device_bytes"]
+    lean = None
+    try:
+        for k in range(64):   # the last allocation of a construction is that of the visit coefficients
+            gpu_lib.gbn_debug_fail_alloc(k)
+            try:
+                lean = plan()
+                break
+            except GbnError as e:
+                assert e.code == GBN_ERR_NOMEM
+    finally:
+        gpu_lib.gbn_debug_fail_alloc(-1)
+    got = _results(lean, x, y)
+    assert lean.stats()["device_bytes"] < held
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    rng = np.random.default_rng(4)
+    w = [rng.standard_normal((M, 6)) for _ in range(2)]
+    P.set_weights(w)
+    lean.set_weights(w)
+    assert all(torch.equal(a, b) for a, b in zip(_results(lean, x, y), _results(P, x, y)))
+    lean.set_points(many, ph)
+    assert all(torch.equal(a, b) for a, b in zip(_results(lean, x, y), want))
+    assert lean.stats()["device_bytes"] >= held
