@@ -67,13 +67,12 @@ __host__ __device__ constexpr size_t exchange_bytes() {
 // CTAs per SM asked of the compiler: as many as the register transforms leave
 // room for, left to itself it may take 148 registers for loads in flight.  (At
 // 128 in place of 96 registers the 256-point passes of a 128^3, 8-coil pair
-// took 70 us more.)  The 512-point passes gain by more loads in flight instead:
-// 256^2, 32 coils 154 -> 142 us forward and 196 -> 182 us adjoint at 2 in place
-// of 3 CTAs.
+// took 70 us more.)  96 for the longest transforms give a 256-thread CTA two,
+// with room for loads in flight; with three the 512-point passes took 154 in
+// place of 142 us (256^2, 32 coils, forward) and 196 in place of 182 (adjoint).
 template <int L1, int L2, int TC>
 __host__ __device__ constexpr int pass_ctas(PassMode mode) {
     const int big = L1 > L2 ? L1 : L2, threads = TC * L1;
-    if (L1 * L2 == 512 && TC == 16) return 2;
     const int regs = (big <= 12 ? 48 : big <= 16 ? 64 : big <= 24 ? 80 : 96) +
                      // the phases held beside a column
                      (mode == PHASE && (L1 == 32 || L2 == 12) ? 16 : 0);
