@@ -74,8 +74,8 @@ template <int L1, int L2, int TC>
 __host__ __device__ constexpr int pass_ctas(PassMode mode) {
     const int big = L1 > L2 ? L1 : L2, threads = TC * L1;
     const int regs = (big <= 12 ? 48 : big <= 16 ? 64 : big <= 24 ? 80 : 96) +
-                     // the phases held beside a column
-                     (mode == PHASE && (L1 == 32 || L2 == 12) ? 16 : 0);
+                     // the phases held beside a column (16 x 12 spilled at 64)
+                     (mode == PHASE && L2 == 12 ? 16 : 0);
     const int ctas = 65536 / (threads * regs);
     return ctas < 1 ? 1 : ctas > 16 ? 16 : ctas;
 }
