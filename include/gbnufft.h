@@ -240,8 +240,10 @@ int gbn_plan_set_dtables(gbn_plan* plan, const void* const* dtab);
 /* Gradient of a real loss with respect to the sample coordinates tm
  * (single-frame plans, real phasing).
  *   grid : the oversampled grid as a gbn_forward call with the same coil count
- *          leaves it in the buffer that gbn_forward_grid returns (callers copy
- *          it if they need it later), before or after the tables were set.
+ *          leaves it in the buffer that gbn_forward_grid returns, before or
+ *          after the tables were set.  Callers copy it if they need it later;
+ *          a copy is taken to be in the form (before phase_before or after)
+ *          in which the plan's last forward call left its own.
  *   gy   : [coils][M] dL/dy in torch's convention (dL/dRe + i dL/dIm).
  *   phase_shift : host [ndim], d(sample phase)/d(tm_d) divided by i, i.e.
  *          (n_shift_d - n_mid_d) * 2 pi / Kd[d] for phase_after.
@@ -255,10 +257,10 @@ int gbn_grad_tm(gbn_plan* plan, const void* grid, const void* gy,
  * [K_{ndim-1}]...[K_0][coils] per frame, for single-precision 2-D and 3-D
  * plans whose every axis length the library's FFT passes implement (see
  * GBN_FLAG_CUFFT_ONLY), else [K1][coils][K0] for 2-D plans and [coils][K...]
- * for 1-D and 3-D ones.  For real phasing the coil-minor grid holds
- * phase_before and the orthonormal scale already; the other two are the FFT's
- * output, from before them.  The interpolation-only entry points keep the
- * [planes][K...] layout.                                                    */
+ * for 1-D and 3-D ones.  It is the FFT's output, from before phase_before and
+ * the orthonormal scale, but for the coil-minor grid of real phasing in a plan
+ * without derivative tables, which holds both already.  The interpolation-only
+ * entry points keep the [planes][K...] layout.                              */
 int gbn_forward_grid(gbn_plan* plan, void** grid);
 
 /* Exact direct NUDFT in double precision on the GPU (the reference's

@@ -84,6 +84,7 @@ template <int L1, int L2, int TC, int SIGN, PassMode MODE, bool RM>
 __global__ void __launch_bounds__(TC * L1, (pass_ctas<L1, L2, TC>(MODE))) fftpass_kernel(const FftPassParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sm = reinterpret_cast<float2*>(smem_raw);
+    if (MODE != IMAGE && SIGN < 0 && p.state && blockIdx.x == 0 && threadIdx.x == 0) *p.state = MODE == PHASE;
     auto at = [](int col, int k2, int n1) {
         return RM ? col * row_block<L1, L2>() + k2 * (L1 | 1) + n1 : (k2 * L1 + n1) * TC + col;
     };

@@ -13,9 +13,9 @@
 //   dL/dt_d = sum_c Re(conj(gy[m,c]) dy[m,c]/dt_d).
 // One thread per sample (samples in gather-list order, so neighbouring
 // threads read neighbouring grid taps); coils are summed inside the thread.
-// The grid of a plan on its own FFT passes holds phase_before already;
-// elsewhere it is separable, so it is folded into the per-axis coefficients
-// (J sincos per axis per sample instead of one per tap per coil).  The
+// phase_before is separable, so it is folded into the per-axis coefficients
+// (J sincos per axis per sample instead of one per tap per coil); a grid left
+// by a forward call before the derivative tables were set holds it already.  The
 // kernel has no counterpart in the reference, which has no autograd.
 #include <cuda_runtime.h>
 
@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(128) grad_kernel(const GradParams<R> p) {
     const Geom<R>& g = p.g;
     const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= p.M) return;
+    const bool held = p.phased && *p.phased, apply_pb = p.apply_pb && !held;
     // Per axis and tap: the table coefficient and its derivative, each
     // times that axis's factor of phase_before.  phase_before(k) =
     // exp(i sum_d c_d k_d) is a product over axes, so the phases cost
@@ -52,14 +53,14 @@ __global__ void __launch_bounds__(128) grad_kernel(const GradParams<R> p) {
                 const int n = min(max((int)nf + g.ncenter[d], -2), g.J[d] * g.L + 1);
                 const R dc = lerp_rn(pp - nf, __ldg(p.dh[d] + n), __ldg(p.dh[d] + n + 1));
                 R sn = (R)0, cs = (R)1;
-                if (p.apply_pb) sincos_r(mul_rn(g.pbc[d], (R)wrapk(kf[d] + j, g.K[d])), &sn, &cs);
+                if (apply_pb) sincos_r(mul_rn(g.pbc[d], (R)wrapk(kf[d] + j, g.K[d])), &sn, &cs);
                 cc[d][j] = cmake<R>(c * cs, c * sn);
                 dd[d][j] = cmake<R>(dc * cs, dc * sn);
             }
         }
     }
     const C ph = p.ph ? p.ph[m] : cmake<R>((R)1, (R)0);
-    const R inv_scale = (R)1 / p.grid_scale;
+    const R inv_scale = held ? (R)1 : (R)1 / p.grid_scale;
     R out[3] = {0, 0, 0};
     constexpr int D1 = NDIM > 1 ? 1 : 0, D2 = NDIM > 2 ? 2 : 0;
     for (int co = 0; co < p.coils; ++co) {
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(256) grad2d_group_kernel(const GradParams<R> p
     const int base = lane & ~7;
     const bool ok = m < p.M;
     const int64_t mm = ok ? m : 0;
+    const bool held = p.phased && *p.phased, apply_pb = p.apply_pb && !held;
     // tap j of each axis: coefficient and derivative times the axis's phase_before factor
     C cc[2], dd[2];
     int kf[2];
@@ -149,7 +151,7 @@ __global__ void __launch_bounds__(256) grad2d_group_kernel(const GradParams<R> p
             const int n = min(max((int)nf + g.ncenter[d], -2), g.J[d] * g.L + 1);
             const R dc = lerp_rn(pp - nf, __ldg(p.dh[d] + n), __ldg(p.dh[d] + n + 1));
             R sn = (R)0, cs = (R)1;
-            if (p.apply_pb) sincos_r(mul_rn(g.pbc[d], (R)wrapk(kf[d] + j, g.K[d])), &sn, &cs);
+            if (apply_pb) sincos_r(mul_rn(g.pbc[d], (R)wrapk(kf[d] + j, g.K[d])), &sn, &cs);
             cc[d] = cmake<R>(c * cs, c * sn);
             dd[d] = cmake<R>(dc * cs, dc * sn);
         }
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(256) grad2d_group_kernel(const GradParams<R> p
     const bool row = ok && j < g.J[1];
     const int64_t o1 = (int64_t)wrapk(kf[1] + j, g.K[1]) * g.gs1;
     const C ph = (ok && p.ph) ? p.ph[mm] : cmake<R>((R)1, (R)0);
-    const R inv_scale = (R)1 / p.grid_scale;
+    const R inv_scale = held ? (R)1 : (R)1 / p.grid_scale;
     R out[2] = {0, 0};
     for (int co = 0; co < p.coils; ++co) {
         const C* gb = p.grid + (int64_t)co * g.gsp;

@@ -259,7 +259,8 @@ struct GradParams {
     int coils;
     int apply_pb;
     R grid_scale;
-    const typename Cx<R>::T* grid;  // as the forward left it: before phase_before (apply_pb) or after
+    const int* phased;              // the grid holds phase_before and the scale already (or nullptr: it does not)
+    const typename Cx<R>::T* grid;  // as the forward left it
     const typename Cx<R>::T* gy;    // [coils][M] incoming gradient
     R* gtm;                         // [M][ndim] out
 };
@@ -370,6 +371,7 @@ struct FftPassParams {
     const float2* phase;
     int prows;
     float div;
+    int* state;                     // receives whether they were (or nullptr)
     unsigned* check;                // checked builds: status word and extents
     int64_t in_elems, out_elems;
 };

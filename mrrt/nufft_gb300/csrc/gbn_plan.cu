@@ -219,7 +219,7 @@ struct gbn_plan {
 
     DevBuf tables, dtables, sn, dfoff;
     DevBuf check;         // status word of the checked build's bounds tests
-    DevBuf tickets;       // work counters of the persistent gather launch
+    DevBuf tickets;       // work counters of the persistent gather launch (two), grid_state
     DevBuf weights;       // sparse-matrix mode: per-axis [M_total][J] weights (re, then im)
     DevBuf gcoef;         // precomputed coefficients in gather list order
     // visit lists of the spread (gbn_visit.cuh): offsets per (item, block), sample
@@ -877,6 +877,7 @@ struct AxisPass {
     int64_t S, arrays, psi, pso;
     int nin, nout;
     bool phase = false;   // coil-minor grid rows: times phase_before
+    int* state = nullptr; // where to note that
 };
 int run_pass(gbn_plan* P, const AxisPass& a, int sign, cudaStream_t s) {
     const gbn_geometry& G = P->geom;
@@ -896,6 +897,7 @@ int run_pass(gbn_plan* P, const AxisPass& a, int sign, cudaStream_t s) {
         p.phase = static_cast<const float2*>(P->ptab.p);
         p.prows = (int)(P->Kprod / G.Kd[0]);
     }
+    p.state = a.state;
     p.div = G.ortho ? (float)std::sqrt((double)P->Kprod) : 1.f;
     p.check = static_cast<unsigned*>(P->check.p);
     p.in_elems = a.in_elems;
@@ -999,10 +1001,13 @@ int colfft_2d(gbn_plan* P, int planes, int sign, cudaStream_t s) {
 }
 
 // Whether a forward call on the plan's own passes leaves phase_before and the
-// orthonormal scale applied to its grid.  The same for every call of a plan:
-// gbn_grad_tm takes that grid whenever its tables were set, also from a graph
-// captured before.
-bool grid_phased(const gbn_plan* P) { return P->geom.phasing == GBN_PHASING_REAL; }
+// orthonormal scale applied to its grid: plans with derivative tables keep the
+// grid that gbn_grad_tm takes, from before it.  The tables may come after a
+// forward call, or after the capture of one, so the pass that writes the grid
+// also notes on the device which of the two it holds (grid_state), and
+// gbn_grad_tm's kernels read that.
+bool grid_phased(const gbn_plan* P) { return P->geom.phasing == GBN_PHASING_REAL && !P->dtables.p; }
+int* grid_state(const gbn_plan* P) { return reinterpret_cast<int*>(P->tickets.p) + 2; }
 
 // Transform on the plan's own passes, on coil-minor arrays, widening the axes
 // from the slowest to the contiguous one (sign -1) or narrowing them back:
@@ -1021,7 +1026,8 @@ int own_transform(gbn_plan* P, const void* x, void* xa, const void* maps, int co
         if (d3 && (rc = run_pass(P, AxisPass{grid, ge, half, he, 1, rn, (int64_t)P->F * G.Kd[2], rn * G.Nd[1],
                                              rn * G.Kd[1], G.Nd[1], G.Kd[1]}, -1, s)))
             return rc;
-        return run_pass(P, AxisPass{half, he, grid, ge, 0, coils, rows, rn, rk, G.Nd[0], G.Kd[0], grid_phased(P)}, -1, s);
+        return run_pass(P, AxisPass{half, he, grid, ge, 0, coils, rows, rn, rk, G.Nd[0], G.Kd[0], grid_phased(P),
+                                   grid_state(P)}, -1, s);
     }
     if ((rc = run_pass(P, AxisPass{grid, ge, half, he, 0, coils, rows, rk, rn, G.Kd[0], G.Nd[0]}, 1, s))) return rc;
     if (d3 && (rc = run_pass(P, AxisPass{half, he, grid, ge, 1, rn, (int64_t)P->F * G.Kd[2], rn * G.Kd[1],
@@ -2035,9 +2041,9 @@ int run_grad(gbn_plan* P, const void* grid, const void* gy, const double* shift,
     p.ph = L.ph;
     p.M = P->glen;
     p.coils = coils;
-    const bool done = P->own && grid_phased(P);
-    p.apply_pb = !done && P->geom.phasing == GBN_PHASING_REAL;
-    p.grid_scale = !done && P->geom.ortho ? (R)std::sqrt((double)P->Kprod) : (R)1;
+    p.apply_pb = P->geom.phasing == GBN_PHASING_REAL;
+    p.grid_scale = P->geom.ortho ? (R)std::sqrt((double)P->Kprod) : (R)1;
+    p.phased = P->own ? grid_state(P) : nullptr;
     p.grid = reinterpret_cast<const C*>(grid);
     p.gy = reinterpret_cast<const C*>(gy);
     p.gtm = reinterpret_cast<R*>(gtm);
