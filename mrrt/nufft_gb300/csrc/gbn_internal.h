@@ -183,7 +183,7 @@ struct VisitParams {
     int nshared, nwhole;            // set by the launcher: leading items shared by a CTA's warps, in equal
                                     // runs, and further on a block to each
     int coils, LS, chunks, row;
-    int chunk0, nchunk;             // coil chunks of the launch; vals holds those alone
+    int nchunk;                     // coil chunks of the launch (chunks: of the scratch's layout)
     const int64_t* foff;
     const typename Cx<R>::T* vals;  // [frame][m][row] (launch_values), or nullptr: read y in place
     int rec;                        // without vco: place in a row of vals, in reals, of the sample's

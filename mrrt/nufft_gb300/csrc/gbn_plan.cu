@@ -1234,9 +1234,17 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
         GBN_CUDA(launch_coef<R>(c, s), "sample coefficients launch");
     }
     for (int first = 0; first < coils; first += group) {
+        // the coils of the group as a call of their own, but for the scratch,
+        // which is laid out for all
         const int n = std::min(group, coils - first);
-        p.chunk0 = first / ln.LS;
-        p.nchunk = (n + ln.LS - 1) / ln.LS;
+        const int64_t part = (int64_t)first / ln.LS * p.tile_cells * ln.LS;
+        VisitParams<R> q = p;
+        q.coils = n;
+        q.nchunk = (n + ln.LS - 1) / ln.LS;
+        q.grid += first * p.g.gsp;
+        q.g.grid_elems -= first * p.g.gsp;
+        q.scratch += part;
+        q.scratch_elems -= part;
         if (vals) {
             ValuesParams<R> v;
             std::memset(&v, 0, sizeof(v));
@@ -1254,7 +1262,7 @@ int launch_visits(gbn_plan* P, const void* y, void* grid, int coils, Grid kind, 
             v.out_elems = vals_elems;
             GBN_CUDA(launch_values<R>(v, s), "sample values launch");
         }
-        GBN_CUDA(launch_spread_visits<R>(p, s), "spread launch");
+        GBN_CUDA(launch_spread_visits<R>(q, s), "spread launch");
     }
     if (P->n_rtiles) {
         ReduceParams<R> q;

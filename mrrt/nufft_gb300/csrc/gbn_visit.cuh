@@ -603,7 +603,7 @@ struct BlockSink {
         int n0, n1;
         extent(p, blk, n0, n1);
         const Geom<R>& g = p.g;
-        // within a block offsets fit 32 bits
+        // strides fit 32 bits (the launcher has looked), three of them need not
         const int s0 = direct ? (int)g.gs0 : LS, s1 = direct ? (int)g.gs1 : g.T[0] * LS;
         const bool vec = sizeof(R) == 4 && direct && g.gs0 == 1 && ((g.K[0] | g.gsf | g.gsp | g.gs1 | g.gs2) & 1) == 0;
         C* d = dst + (direct ? p.boff[blk] : p.bscr[blk] * LS);
@@ -612,7 +612,7 @@ struct BlockSink {
         for (int i = 0; i < KEEP; i += STEP) {
             const int q = q0 + i, k0 = q % B0, k1 = q / B0;
             const bool in0 = k0 < n0 && k1 < n1, in1 = STEP == 2 && k0 + 1 < n0 && k1 < n1;
-            C* o = d + k0 * s0 + k1 * s1;
+            C* o = d + (int64_t)k0 * s0 + (int64_t)k1 * s1;
 #ifdef GBN_CHECKED
             C* last = o + (in1 ? s0 : 0);
             if ((in0 || in1) && !(direct ? GBN_INB(p.g.check, o >= p.grid && last < p.grid + p.g.grid_elems, CHK_GRID_WRITE)
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, 5) spread_unit_kernel(const Vis
     const unsigned unit = blockIdx.x * (VISIT_THREADS / 32) + (threadIdx.x >> 5);
     if (unit >= (unsigned)(p.nitems * p.nblk)) return;   // whole warps only; no barrier below
     const int item = (int)(unit / (unsigned)p.nblk), blk = (int)(unit - (unsigned)item * p.nblk);
-    const int chunk = p.chunk0 + blockIdx.y;
+    const int chunk = blockIdx.y;
     const int4 it = p.items[item];
     const int2 part = p.parts[item];
     const int f = it.x;
@@ -802,7 +802,7 @@ spread_stream_kernel(const VisitParams<R> p) {
     const bool shared_item = (int)blockIdx.x < nshared;
     const int item = shared_item ? (int)blockIdx.x : nshared + ((int)blockIdx.x - nshared) * STREAM_WARPS + warp;
     if (item >= p.nitems) return;   // only in a CTA of unshared items: no barrier there
-    const int chunk = p.chunk0 + blockIdx.y;
+    const int chunk = blockIdx.y;
     const int4 it = p.items[item];
     const int part = p.parts[item].x;
     const int f = it.x;
@@ -850,9 +850,8 @@ spread_stream_kernel(const VisitParams<R> p) {
     // A lane copies 16 bytes at a fixed place of every (512 / VROW)-th visit.
     const int row_bytes = p.row * (int)sizeof(C);
     const int off = lane * 16 % SL::VROW;
-    const int v0 = blockIdx.y * LS;   // the chunk's place in a row of values
-    const bool lane_ok = v0 * (int)sizeof(C) + off < row_bytes;
-    const char* vsrc = reinterpret_cast<const char*>(p.vals + fo * p.row + v0) + (lane_ok ? off : 0);
+    const bool lane_ok = c0 * (int)sizeof(C) + off < row_bytes;
+    const char* vsrc = reinterpret_cast<const char*>(p.vals + fo * p.row + c0) + (lane_ok ? off : 0);
     const C* ysrc = p.y + fo * p.coils + (int64_t)c0 * Mf;
     const int visit = TAB ? lane % RV : lane;
     const int* isrc = p.vidx + base + lo + visit;
@@ -1136,7 +1135,7 @@ template <typename R>
 cudaError_t launch_spread_visits(const VisitParams<R>& p0, cudaStream_t s) {
     if (p0.nitems == 0 || p0.coils == 0) return cudaSuccess;
     VisitParams<R> p = p0;
-    if (p.nblk < 1 || p.nblk > 8) return cudaErrorInvalidValue;
+    if (p.nblk < 1 || p.nblk > 8 || p.g.gs0 > INT32_MAX || p.g.gs1 > INT32_MAX) return cudaErrorInvalidValue;
     for (int b = 0; b < p.nblk; ++b) {
         int b0, b1, b2;
         if (p.g.ndim == 1) block_origin<1>(p.g, b, b0, b1, b2);
