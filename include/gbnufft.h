@@ -123,9 +123,9 @@ int gbn_plan_set_points(gbn_plan* plan, const void* tm,
  * tile lists are built on the device by a sort of the samples (stable, so
  * the spread's summation order, hence its result, is the same in every
  * run); the coordinates never pass through host memory.  The call waits
- * for work already queued on the device, and for two 4-to-16-byte counts it
- * reads back on `stream` (to size the lists and launches), then returns with
- * the rest queued on `stream`.  Failures as for gbn_plan_set_points.  Replaces
+ * for work already queued on the device, and for two blocks of counts, 128 and
+ * 40 bytes, that it reads back on `stream` (to size the lists and launches),
+ * then returns with the rest queued on `stream`.  Failures as for gbn_plan_set_points.  Replaces
  * the host-side tm = omega / gamma recomputation of the reference
  * (mrrt/nufft/_nufft.py:338-342) when a trajectory is optimised on the GPU. */
 int gbn_plan_set_points_device(gbn_plan* plan, const void* tm,
@@ -175,7 +175,8 @@ int gbn_forward_sense(gbn_plan* plan, const void* image, const void* maps,
                       void* y, int coils, void* stream);
 
 /* Coil-combining adjoint: image[f] = sum_c conj(maps[c]) * adjoint_c, the
- * sum (in coil order) fused into the crop pass.                             */
+ * sum in coil order: fused into the crop pass around cuFFT, else one more
+ * pass over the coil images that the last FFT pass wrote.                    */
 int gbn_adjoint_sense(gbn_plan* plan, const void* y, const void* maps,
                       void* image, int coils, void* stream);
 

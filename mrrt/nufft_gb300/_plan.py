@@ -185,7 +185,8 @@ class GpuPlan:
 
     def forward_sense(self, image, maps, y, coils):
         """Coil-sensitivity forward: image [F, N...] and maps [coils, N...]
-        (plan layout) -> samples, the map multiply fused into the pad."""
+        (plan layout) -> samples, the map multiply fused into the pass that
+        reads the image."""
         F = len(self.frame_offsets) - 1
         image = self._input(image, F * self.Nprod, "image")
         maps = self._input(maps, coils * self.Nprod, "maps")
@@ -198,7 +199,7 @@ class GpuPlan:
 
     def adjoint_sense(self, y, maps, image, coils):
         """Coil-combining adjoint: samples -> image [F, N...] = sum over coils
-        of conj(maps) times each coil's adjoint, fused into the crop."""
+        of conj(maps) times each coil's adjoint."""
         F = len(self.frame_offsets) - 1
         y = self._input(y, coils * self.M_total, "y")
         maps = self._input(maps, coils * self.Nprod, "maps")

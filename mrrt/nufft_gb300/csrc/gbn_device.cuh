@@ -54,7 +54,7 @@ __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fm
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 // Complex product with its roundings fixed (which of a product's two terms
 // is contracted is otherwise the compiler's choice at each call site): the
-// spread kernels of the entry and the visit lists agree bit for bit.
+// spread gives the same bits with stored coefficients and with computed ones.
 template <typename C>
 __device__ __forceinline__ C cmul_fixed(C a, C b) {
     C r;
@@ -169,15 +169,6 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
     return d;
 }
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-    unsigned long long ra, rb, rd;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-    float2 d;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-    return d;
-}
 // Asynchronous global -> shared copies (cp.async, cached in L1 and L2).
 // BYTES is 4, 8 or 16; both addresses must be aligned to BYTES.
 template <int BYTES>
@@ -191,9 +182,7 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 
-// Element-wise pair operations: a * b and a * b + c on (re, im) pairs.
-__device__ __forceinline__ float2 pmul(float2 a, float2 b) { return fmul2(a, b); }
-__device__ __forceinline__ double2 pmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+// Element-wise a * b + c on (re, im) pairs.
 __device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) { return ffma2(a, b, c); }
 __device__ __forceinline__ double2 pfma(double2 a, double2 b, double2 c) {
     return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));

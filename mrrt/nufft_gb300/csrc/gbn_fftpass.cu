@@ -7,7 +7,8 @@ namespace gbn {
 cudaError_t launch_fftpass_short(const FftPassParams& p, int sign, cudaStream_t s);
 cudaError_t launch_fftpass_long(const FftPassParams& p, int sign, cudaStream_t s);
 
-// Lengths with a compile-time split L1 x L2, both dividing 480 and at most 32.
+// The lengths with kernels: a selection of the products of two factors up to 32
+// that divide 480, each a compile-time split.
 bool fftpass_supported(int L) {
     switch (L) {
         case 64: case 96: case 128: case 192: case 256: case 384: case 512: case 768:

@@ -33,7 +33,7 @@
 // four coils: RM), consecutive elements of one.
 // The register transforms are Stockham autosort FFTs (Govindaraju et al.,
 // "High performance discrete Fourier transforms on graphics processors",
-// SC 2008), radix 4, 2 and 3 stages fully unrolled; their roots are compile-
+// SC 2008), radix 4, 2, 3 and 5 stages fully unrolled; their roots are compile-
 // time constants in constant memory, the W_L^(n1 k2) twiddles a per-plan
 // table computed on the host in double precision.  Single precision only;
 // other lengths and double precision run through cuFFT.

@@ -1076,8 +1076,9 @@ cudaError_t stream_launch(const VisitParams<R>& p0, cudaStream_t s) {
     VisitParams<R> p = p0;
     if (INPLACE && p.ph && p.s.len > 0) return cudaErrorInvalidValue;   // the values hold the phase
     // An item goes to one warp up to 32 entries per slot (a longer one would
-    // outlast the rest of a small launch), more where each of the device's
-    // warps has many times that to do anyway.
+    // outlast the rest of a small launch), more where each warp of three CTAs on
+    // each of 152 SMs would have many times that to do anyway.  (Where fewer CTAs
+    // fit, complex kernels above all, this shares items sooner than that asks.)
     const int64_t load = p.s.len * p.chunks / (3 * STREAM_WARPS * 152) / 8;
     int q = LS >= 32 ? 0 : LS >= 16 ? 1 : 2;
     while (q < SPREAD_HEAVY_LEVELS - 1 && (SPREAD_SHARE_ENTRIES << q) < load) ++q;

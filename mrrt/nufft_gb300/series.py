@@ -146,7 +146,8 @@ class NufftSeries(object):
 
     def adjoint_sense(self, y, maps, image=None):
         """Frame-major samples -> ``[F, *reversed(Nd)]``, the coil sum of
-        conj(maps) times each coil's adjoint fused into the crop pass."""
+        conj(maps) times each coil's adjoint (fused into the crop around cuFFT,
+        a pass over the coil images otherwise)."""
         c = maps.shape[0]
         if image is None:
             image = torch.empty((self.n_frames,) + tuple(reversed(self.Nd)), dtype=self.ctype,
