@@ -603,7 +603,8 @@ struct BlockSink {
         int n0, n1;
         extent(p, blk, n0, n1);
         const Geom<R>& g = p.g;
-        // strides fit 32 bits (the launcher has looked), three of them need not
+        // strides fit 32 bits (the launcher has looked), three rows need not (unsigned:
+        // signed products of 64 bits cost the series' adjoint 2 us of 680)
         const int s0 = direct ? (int)g.gs0 : LS, s1 = direct ? (int)g.gs1 : g.T[0] * LS;
         const bool vec = sizeof(R) == 4 && direct && g.gs0 == 1 && ((g.K[0] | g.gsf | g.gsp | g.gs1 | g.gs2) & 1) == 0;
         C* d = dst + (direct ? p.boff[blk] : p.bscr[blk] * LS);
@@ -612,7 +613,7 @@ struct BlockSink {
         for (int i = 0; i < KEEP; i += STEP) {
             const int q = q0 + i, k0 = q % B0, k1 = q / B0;
             const bool in0 = k0 < n0 && k1 < n1, in1 = STEP == 2 && k0 + 1 < n0 && k1 < n1;
-            C* o = d + (int64_t)k0 * s0 + (int64_t)k1 * s1;
+            C* o = d + ((unsigned long long)(unsigned)k1 * (unsigned)s1 + (unsigned)(k0 * s0));
 #ifdef GBN_CHECKED
             C* last = o + (in1 ? s0 : 0);
             if ((in0 || in1) && !(direct ? GBN_INB(p.g.check, o >= p.grid && last < p.grid + p.g.grid_elems, CHK_GRID_WRITE)
@@ -1136,7 +1137,7 @@ template <typename R>
 cudaError_t launch_spread_visits(const VisitParams<R>& p0, cudaStream_t s) {
     if (p0.nitems == 0 || p0.coils == 0) return cudaSuccess;
     VisitParams<R> p = p0;
-    if (p.nblk < 1 || p.nblk > 8 || p.g.gs0 > INT32_MAX || p.g.gs1 > INT32_MAX) return cudaErrorInvalidValue;
+    if (p.nblk < 1 || p.nblk > 8 || p.g.gs0 > INT32_MAX / 4 || p.g.gs1 > INT32_MAX) return cudaErrorInvalidValue;
     for (int b = 0; b < p.nblk; ++b) {
         int b0, b1, b2;
         if (p.g.ndim == 1) block_origin<1>(p.g, b, b0, b1, b2);
