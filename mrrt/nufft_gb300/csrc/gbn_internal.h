@@ -158,9 +158,9 @@ struct ValuesParams {
 };
 
 // Coil lanes of a spread that copies the samples as they lie.  1024 x 1024 with
-// 1.2 million radial (0.7 million uniform) samples, 32 coils, single precision:
-// 1132 (864) us in four chunks of 8 lanes, 1926 (3416) with 32 lanes; double, whose
-// values fill half a sector each, 15.7 ms and 9.5 ms.
+// 1.2 million radial samples, 32 coils, single precision: 1035 us in four chunks of
+// 8 lanes, 1926 with 32 lanes.  Double, whose values fill half a sector each: 3.9 ms
+// for one chunk of 8, 9.5 with 32 lanes for all.
 template <typename R> constexpr int inplace_lanes() { return sizeof(R) == 4 ? 8 : 32; }
 
 template <typename R>
